@@ -82,12 +82,34 @@ int make_accum_map(CUtensorMap* map, float* base, int Z, int N, int H, int D) {
 long long* g_timeline = nullptr;
 int g_timeline_block = 0;
 
-int sm_count() {
-  int dev = 0, n = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0)
-    return 148;
+constexpr int kMaxDevices = 64;
+
+int current_device() {
+  int dev = -1;
+  return cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kMaxDevices ? dev : -1;
+}
+
+// SMs of a device, asked once per device (the query costs as much host time as a tensor map)
+int sm_count(int dev) {
+  static std::atomic<int> cached[kMaxDevices];
+  if (dev < 0) return 148;
+  int n = cached[dev].load(std::memory_order_relaxed);
+  if (n == 0) {
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) return 148;
+    cached[dev].store(n, std::memory_order_relaxed);
+  }
   return n;
+}
+
+// Raises a kernel's dynamic shared-memory limit, once per kernel and device.
+template <auto kKernel>
+bool allow_smem(int dev, int bytes) {
+  static std::atomic<bool> done[kMaxDevices];
+  if (dev >= 0 && done[dev].load(std::memory_order_acquire)) return true;
+  if (cudaFuncSetAttribute(kKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess)
+    return false;
+  if (dev >= 0) done[dev].store(true, std::memory_order_release);
+  return true;
 }
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
@@ -206,12 +228,11 @@ int launch_fwd(const FmhaFwdParams* p, cudaStream_t stream) {
   kp.timeline = g_timeline;
   kp.timeline_block = g_timeline_block;
   auto kernel = fmha::fmha_fwd_kernel<D, kBf16>;
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, T::kSmemBytes) !=
-      cudaSuccess)
-    return FMHA_ERR_LAUNCH;
+  const int dev = current_device();
+  if (!allow_smem<fmha::fmha_fwd_kernel<D, kBf16>>(dev, T::kSmemBytes)) return FMHA_ERR_LAUNCH;
   // persistent grid: one CTA per SM (or per super-item = pair of query blocks, if fewer)
   const long long n_super = (long long)((kp.num_q_blocks + 1) / 2) * kp.num_heads_total;
-  const int sms = std::max(1, sm_count() - std::max(0, (int)p->sm_margin));
+  const int sms = std::max(1, sm_count(dev) - std::max(0, (int)p->sm_margin));
   const unsigned grid = (unsigned)std::min<long long>(n_super, sms);
   kernel<<<grid, T::kThreads, T::kSmemBytes, stream>>>(tq, tk, tv, to, kp);
   return cudaGetLastError() == cudaSuccess ? FMHA_OK : FMHA_ERR_LAUNCH;
@@ -285,8 +306,7 @@ int launch_bwd(const FmhaBwdParams* p, const BwdWorkspace& w, cudaStream_t strea
     kp.timeline = g_timeline;
     kp.timeline_block = g_timeline_block;
     auto kernel = fmha::fmha_bwd_kernel<D, kBf16, DR>;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, T::kSmemBytes) !=
-        cudaSuccess)
+    if (!allow_smem<fmha::fmha_bwd_kernel<D, kBf16, DR>>(current_device(), T::kSmemBytes))
       return FMHA_ERR_LAUNCH;
     const unsigned grid = (unsigned)((long long)kp.num_kv_blocks * H * Z);
     kernel<<<grid, T::kThreads, T::kSmemBytes, stream>>>(tq, tk, tv, tdo, tdk, tdv, tacc, kp);
@@ -320,13 +340,12 @@ FmhaStrides dense_strides(int n, int head, int k) {
 // ---------------------------------------------------------------------------------------
 static __device__ __align__(256) unsigned char g_fmha_static_scratch[FMHA_STATIC_SCRATCH_BYTES];
 
-constexpr int kMaxDevices = 64;
 std::atomic<void*> g_static_scratch_addr[kMaxDevices];  // per device, filled on first use
 
 // Device address of the scratch area on the CURRENT device, or nullptr (rc set) on failure.
 void* static_scratch_for_current_device(int* rc) {
-  int dev = -1;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) {
+  const int dev = current_device();
+  if (dev < 0) {
     *rc = FMHA_ERR_NO_DEVICE;
     return nullptr;
   }

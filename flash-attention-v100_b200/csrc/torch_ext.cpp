@@ -17,10 +17,14 @@
 //   - `bwd` ignores the fp16 `D` argument (flash_attn_interface.py:43-44) and computes
 //     D = rowsum(dO o O) itself in fp32.
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
+#include <torch/csrc/autograd/autograd_not_implemented_fallback.h>
 #include <torch/extension.h>
 
+#include <cmath>
 #include <optional>
+#include <tuple>
 #include <vector>
 
 #include "../../include/fmha_b200.h"
@@ -41,6 +45,15 @@ void check_input(const at::Tensor& t, const char* name) {
               "This repo only supports fp16 and bf16 data types (", name, ")");
   TORCH_CHECK(t.dim() == 4, name, " must have shape (batch, seqlen, heads, head_size)");
   TORCH_CHECK(t.stride(-1) == 1, name, " must have contiguous last dimension");
+}
+
+// uninitialised memory, straight from the caching allocator (the dispatcher's at::empty costs
+// about a microsecond more per tensor, and a backward makes four)
+at::Tensor empty_on(const at::Tensor& like, at::IntArrayRef sizes, at::ScalarType type) {
+  return at::detail::empty_cuda(sizes, type, like.device(), std::nullopt);
+}
+at::Tensor fresh_like(const at::Tensor& t) {
+  return t.is_contiguous() ? empty_on(t, t.sizes(), t.scalar_type()) : at::empty_like(t);
 }
 
 void check_status(int rc, const char* what) {
@@ -88,11 +101,10 @@ std::vector<at::Tensor> fwd_impl(const at::Tensor& q, const at::Tensor& k, const
     TORCH_CHECK(out.sizes() == q.sizes() && out.scalar_type() == q.scalar_type(),
                 "out must have the shape and type of q");
   } else {
-    out = at::empty_like(q);
+    out = fresh_like(q);
   }
   c10::cuda::CUDAGuard guard(q.device());
-  auto fopts = q.options().dtype(at::kFloat);
-  at::Tensor lse = at::empty({B, H, Nq}, fopts);
+  at::Tensor lse = empty_on(q, {B, H, Nq}, at::kFloat);
 
   FmhaFwdParams p = {};
   p.q = q.data_ptr();
@@ -117,7 +129,7 @@ std::vector<at::Tensor> fwd_impl(const at::Tensor& q, const at::Tensor& k, const
   p.seqused_k = seqused_ptr(seqused_k, q, "seqused_k");
   check_status(fmha_fwd(&p, at::cuda::getCurrentCUDAStream().stream()), "fmha_fwd");
   if (!want_sum) return {out, lse};
-  return {out, lse, at::ones({B, H, Nq}, fopts)};
+  return {out, lse, at::ones({B, H, Nq}, q.options().dtype(at::kFloat))};
 }
 
 // the reference's entry point: {out, softmax_max := lse, softmax_sum := 1}
@@ -172,7 +184,7 @@ std::vector<at::Tensor> bwd_impl(const at::Tensor& dout, const at::Tensor& q, co
                   " must have the shape and type of its input");
       return t.value();
     }
-    return at::empty_like(like);
+    return fresh_like(like);
   };
   at::Tensor dq = take(dq_, q, "dq");
   at::Tensor dk = take(dk_, k, "dk");
@@ -208,7 +220,7 @@ std::vector<at::Tensor> bwd_impl(const at::Tensor& dout, const at::Tensor& q, co
   p.seqused_k = seqused_ptr(seqused_k, q, "seqused_k");
   p.flags = deterministic ? FMHA_BWD_DETERMINISTIC : 0;
   const size_t ws_bytes = fmha_bwd_workspace_bytes(&p);
-  at::Tensor ws = at::empty({static_cast<int64_t>(ws_bytes)}, q.options().dtype(at::kByte));
+  at::Tensor ws = empty_on(q, {static_cast<int64_t>(ws_bytes)}, at::kByte);
   check_status(fmha_bwd(&p, ws.data_ptr(), ws_bytes, at::cuda::getCurrentCUDAStream().stream()),
                "fmha_bwd");
   return {dq, dk, dv};
@@ -237,7 +249,130 @@ std::vector<at::Tensor> mha_bwd_lse(const at::Tensor& dout, const at::Tensor& q,
                   softmax_scale, is_causal, seqused_q, seqused_k, deterministic);
 }
 
+// ---------------------------------------------------------------------------------------------
+// Dispatcher ops and autograd.  Registered here rather than as Python custom ops: on the smallest
+// calls the host is what takes the time (a training step of Z2 H4 N128 D64 spent 137 us in the
+// Python op wrappers and the Python autograd function around 19 us of GPU work).
+// ---------------------------------------------------------------------------------------------
+using OptTensor = std::optional<at::Tensor>;
+
+std::tuple<at::Tensor, at::Tensor> op_fwd(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v,
+                                          double softmax_scale, bool causal, const OptTensor& seqused_q,
+                                          const OptTensor& seqused_k) {
+  auto r = fwd_impl(q, k, v, std::nullopt, softmax_scale, causal, false, seqused_q, seqused_k);
+  return {std::move(r[0]), std::move(r[1])};
+}
+
+std::tuple<at::Tensor, at::Tensor, at::Tensor> op_bwd(const at::Tensor& dout, const at::Tensor& q,
+                                                      const at::Tensor& k, const at::Tensor& v,
+                                                      const at::Tensor& out, const at::Tensor& softmax_lse,
+                                                      double softmax_scale, bool causal,
+                                                      const OptTensor& seqused_q, const OptTensor& seqused_k,
+                                                      bool deterministic) {
+  auto r = mha_bwd_lse(dout, q, k, v, out, softmax_lse, softmax_scale, causal, seqused_q, seqused_k,
+                       deterministic);
+  return {std::move(r[0]), std::move(r[1]), std::move(r[2])};
+}
+
+// Both calls go through the dispatcher, so that every mode that intercepts ops (fake tensors,
+// tensor subclasses, tracing) still sees them.
+std::tuple<at::Tensor, at::Tensor> call_fwd(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v,
+                                            double softmax_scale, bool causal, const OptTensor& seqused_q,
+                                            const OptTensor& seqused_k) {
+  static const auto op = c10::Dispatcher::singleton()
+                             .findSchemaOrThrow("flash_attn_v100::fwd", "")
+                             .typed<decltype(op_fwd)>();
+  return op.call(q, k, v, softmax_scale, causal, seqused_q, seqused_k);
+}
+
+std::tuple<at::Tensor, at::Tensor, at::Tensor> call_bwd(const at::Tensor& dout, const at::Tensor& q,
+                                                        const at::Tensor& k, const at::Tensor& v,
+                                                        const at::Tensor& out, const at::Tensor& lse,
+                                                        double softmax_scale, bool causal,
+                                                        const OptTensor& seqused_q,
+                                                        const OptTensor& seqused_k, bool deterministic) {
+  static const auto op = c10::Dispatcher::singleton()
+                             .findSchemaOrThrow("flash_attn_v100::bwd", "")
+                             .typed<decltype(op_bwd)>();
+  return op.call(dout, q, k, v, out, lse, softmax_scale, causal, seqused_q, seqused_k, deterministic);
+}
+
+at::Tensor last_dim_contiguous(const at::Tensor& t) {
+  return t.dim() > 0 && t.stride(-1) != 1 ? t.contiguous() : t;
+}
+
+// The autograd node of flash_attn_func / flash_attn_padded_func (the Python class FlashAttnFunc
+// is the same computation for code that torch.compile traces).
+struct AttentionFunction : public torch::autograd::Function<AttentionFunction> {
+  static at::Tensor forward(torch::autograd::AutogradContext* ctx, const at::Tensor& q_, const at::Tensor& k_,
+                            const at::Tensor& v_, const OptTensor& seqused_q, const OptTensor& seqused_k,
+                            double softmax_scale, bool causal, bool deterministic) {
+    at::AutoDispatchBelowADInplaceOrView guard;
+    const at::Tensor q = last_dim_contiguous(q_), k = last_dim_contiguous(k_), v = last_dim_contiguous(v_);
+    auto [out, lse] = call_fwd(q, k, v, softmax_scale, causal, seqused_q, seqused_k);
+    ctx->save_for_backward({q, k, v, out, lse, seqused_q.value_or(at::Tensor()), seqused_k.value_or(at::Tensor())});
+    ctx->saved_data["scale"] = softmax_scale;
+    ctx->saved_data["causal"] = causal;
+    ctx->saved_data["deterministic"] = deterministic;
+    return out;
+  }
+
+  static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx,
+                                                 torch::autograd::variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    auto opt = [](const at::Tensor& t) { return t.defined() ? OptTensor(t) : OptTensor(); };
+    const double scale = ctx->saved_data["scale"].toDouble();
+    const bool causal = ctx->saved_data["causal"].toBool();
+    const bool deterministic = ctx->saved_data["deterministic"].toBool();
+    const at::Tensor dout = last_dim_contiguous(grads[0]);
+    auto call = [&]() {
+      return call_bwd(dout, saved[0], saved[1], saved[2], saved[3], saved[4], scale, causal, opt(saved[5]),
+                      opt(saved[6]), deterministic);
+    };
+    at::Tensor dq, dk, dv;
+    if (at::GradMode::is_enabled()) {
+      // create_graph: the op's own autograd entry records that it has no derivative
+      std::tie(dq, dk, dv) = call();
+    } else {
+      at::AutoDispatchBelowADInplaceOrView guard;
+      std::tie(dq, dk, dv) = call();
+    }
+    return {dq, dk, dv, at::Tensor(), at::Tensor(), at::Tensor(), at::Tensor(), at::Tensor()};
+  }
+};
+
+// flash_attn_func / flash_attn_padded_func outside of tracing
+at::Tensor attention(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v,
+                     std::optional<double> softmax_scale, bool causal, const OptTensor& seqused_q,
+                     const OptTensor& seqused_k, bool deterministic) {
+  TORCH_CHECK(q.dim() > 0 && k.dim() > 0 && v.dim() > 0, "q, k and v must have shape (batch, seqlen, heads, head_size)");
+  const double scale = softmax_scale.has_value() ? *softmax_scale : std::pow((double)q.size(-1), -0.5);
+  if (at::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad()))
+    return AttentionFunction::apply(q, k, v, seqused_q, seqused_k, scale, causal, deterministic);
+  at::AutoDispatchBelowADInplaceOrView guard;
+  return std::get<0>(call_fwd(last_dim_contiguous(q), last_dim_contiguous(k), last_dim_contiguous(v), scale,
+                              causal, seqused_q, seqused_k));
+}
+
 }  // namespace
+
+TORCH_LIBRARY(flash_attn_v100, m) {
+  m.def("fwd(Tensor q, Tensor k, Tensor v, float softmax_scale, bool causal, Tensor? seqused_q=None, "
+        "Tensor? seqused_k=None) -> (Tensor, Tensor)", {at::Tag::pt2_compliant_tag});
+  m.def("bwd(Tensor dout, Tensor q, Tensor k, Tensor v, Tensor out, Tensor softmax_lse, float softmax_scale, "
+        "bool causal, Tensor? seqused_q=None, Tensor? seqused_k=None, bool deterministic=False) -> (Tensor, "
+        "Tensor, Tensor)", {at::Tag::pt2_compliant_tag});
+}
+TORCH_LIBRARY_IMPL(flash_attn_v100, CUDA, m) {
+  m.impl("fwd", TORCH_FN(op_fwd));
+  m.impl("bwd", TORCH_FN(op_bwd));
+}
+// the ops themselves have no derivative (the functions above do): differentiating through a direct
+// call is an error, not a silent zero
+TORCH_LIBRARY_IMPL(flash_attn_v100, Autograd, m) {
+  m.impl("fwd", torch::autograd::autogradNotImplementedFallback());
+  m.impl("bwd", torch::autograd::autogradNotImplementedFallback());
+}
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.doc() = "B200 (sm_100a) fused multi-head attention";
@@ -252,5 +387,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("bwd", &mha_bwd,
         "Backward pass: bwd(dout, q, k, v, out, D|None, softmax_sum|None, softmax_max, dq|None, "
         "dk|None, dv|None, softmax_scale, is_causal)");
+  m.def("attention", &attention,
+        "Attention with autograd: attention(q, k, v, softmax_scale|None, causal, seqused_q|None, "
+        "seqused_k|None, deterministic)");
   m.def("version", []() { return std::string(fmha_version()); });
 }

@@ -15,12 +15,14 @@ What changed underneath:
   * the contract "N_CTX is a multiple of 32, right-padded by the caller" (README.md:3) is
     checked, and tail tiles are masked inside the kernels.
 
-  * the two extension calls are registered as ``torch.library`` custom ops
-    (``flash_attn_v100::fwd`` / ``flash_attn_v100::bwd``, each with a fake implementation that
-    only describes output shapes), so that ``flash_attn_func`` can sit inside a
+  * the two extension calls are dispatcher ops (``flash_attn_v100::fwd`` / ``flash_attn_v100::bwd``,
+    each with a fake implementation that only describes output shapes), so that ``flash_attn_func`` can sit inside a
     ``torch.compile(fullgraph=True)`` region: the compiler sees two opaque ops instead of a
     pybind call it cannot trace.  The reference's glue (:62-99) calls the extension directly
     and breaks the graph.
+
+  * outside of tracing the autograd node is the extension's own (C++): the Python classes below are
+    the form ``torch.compile`` traces.
 
 There is no CPU path: importing this module needs the compiled extension, and calling it needs
 a CUDA device.
@@ -37,32 +39,18 @@ def _maybe_contiguous(x):
     return x.contiguous() if x.stride(-1) != 1 else x
 
 
-@torch.library.custom_op("flash_attn_v100::fwd", mutates_args=(), device_types="cuda")
-def _fwd_op(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, softmax_scale: float, causal: bool,
-            seqused_q: Optional[torch.Tensor] = None, seqused_k: Optional[torch.Tensor] = None
-            ) -> Tuple[torch.Tensor, torch.Tensor]:
-    out, softmax_lse = flash_attn_cuda.fwd_lse(q, k, v, None, softmax_scale, causal, seqused_q, seqused_k)
-    return out, softmax_lse
+# the two ops are registered by the extension; these describe their outputs to fake-tensor tracing
+_fwd_op = torch.ops.flash_attn_v100.fwd.default
+_bwd_op = torch.ops.flash_attn_v100.bwd.default
 
 
-@_fwd_op.register_fake
+@torch.library.register_fake("flash_attn_v100::fwd")
 def _fwd_fake(q, k, v, softmax_scale, causal, seqused_q=None, seqused_k=None):
     Z, N, H, _ = q.shape
     return torch.empty_like(q), q.new_empty((Z, H, N), dtype=torch.float32)
 
 
-@torch.library.custom_op("flash_attn_v100::bwd", mutates_args=(), device_types="cuda")
-def _bwd_op(dout: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: torch.Tensor,
-            softmax_lse: torch.Tensor, softmax_scale: float, causal: bool,
-            seqused_q: Optional[torch.Tensor] = None, seqused_k: Optional[torch.Tensor] = None,
-            deterministic: bool = False) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
-    # D = rowsum(dO * O) is computed by the extension in fp32; softmax_lse already is max + ln(sum)
-    dq, dk, dv = flash_attn_cuda.bwd_lse(dout, q, k, v, out, softmax_lse, softmax_scale, causal,
-                                         seqused_q, seqused_k, deterministic)
-    return dq, dk, dv
-
-
-@_bwd_op.register_fake
+@torch.library.register_fake("flash_attn_v100::bwd")
 def _bwd_fake(dout, q, k, v, out, softmax_lse, softmax_scale, causal, seqused_q=None, seqused_k=None,
               deterministic=False):
     return torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
@@ -141,7 +129,9 @@ def flash_attn_padded_func(q, k, v, seqused_q=None, seqused_k=None, softmax_scal
     batch entry.  Padding keys are masked, padding tiles are skipped instead of computed, the
     padding rows of the output and of every gradient are zero.  ``deterministic=True`` adds the
     partial sums of dQ in a fixed order (bit-for-bit reproducible, slower)."""
-    return FlashAttnPaddedFunc.apply(q, k, v, seqused_q, seqused_k, softmax_scale, causal, deterministic)
+    if torch.compiler.is_compiling():
+        return FlashAttnPaddedFunc.apply(q, k, v, seqused_q, seqused_k, softmax_scale, causal, deterministic)
+    return flash_attn_cuda.attention(q, k, v, softmax_scale, causal, seqused_q, seqused_k, deterministic)
 
 
 def flash_attn_func(q, k, v, softmax_scale: Optional[float] = None, causal: bool = False):
@@ -151,4 +141,6 @@ def flash_attn_func(q, k, v, softmax_scale: Optional[float] = None, causal: bool
     seqlen a multiple of 32.  softmax_scale defaults to head_dim ** -0.5.  Returns (batch,
     seqlen, heads, head_dim) in the inputs' type.
     """
-    return FlashAttnFunc.apply(q, k, v, softmax_scale, causal)
+    if torch.compiler.is_compiling():
+        return FlashAttnFunc.apply(q, k, v, softmax_scale, causal)
+    return flash_attn_cuda.attention(q, k, v, softmax_scale, causal, None, None, False)
