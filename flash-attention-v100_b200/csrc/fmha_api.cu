@@ -192,26 +192,107 @@ BwdWorkspace carve_workspace(void* ws, int Z, int H, int Nq, int D) {
   return w;
 }
 
+// ---------------------------------------------------------------------------------------
+// How the forward's work is cut.  A query block (256 rows) is one item unless that leaves SMs
+// idle: then its KV range is cut into chunks of chunk_tiles tiles, each an item of its own that
+// leaves an fp32 partial result, and a second kernel joins them.
+// ---------------------------------------------------------------------------------------
+struct FwdPlan {
+  int chunk_tiles = 1 << 30;
+  int max_chunks = 1;      // of any query block
+  int items_per_head = 0;
+  int first_cut_row = 0;   // rows from here on belong to cut query blocks
+  size_t workspace = 0;    // bytes of the partial results
+};
+
+FwdPlan plan_fwd(const FmhaFwdParams* p, int sms) {
+  FwdPlan plan;
+  const bool causal = p->causal != 0;
+  const int nqb = (p->seqlen_q + 255) / 256, nk = (p->seqlen_k + 127) / 128;
+  const double heads = (double)p->batch * p->heads;
+  plan.items_per_head = nqb;
+  // In units of one round (256 query rows x 128 keys, about 1.2 us): an item costs its rounds and
+  // half a round of its own.
+  auto visible = [&](int qb) {
+    return fmha::fwd_visible_tiles(causal, p->causal_shift, std::min(qb * 256 + 255, p->seqlen_q - 1), nk);
+  };
+  const int n_max = visible(nqb - 1);
+  if (n_max < 4 || heads * nqb > 8.0 * sms) return plan;  // nothing to cut, or enough items to balance
+  auto cost = [&](int chunk, int& items) {  // makespan with chunks of `chunk` tiles
+    double total = 0;
+    items = 0;
+    for (int qb = causal ? 0 : nqb - 1; qb < nqb; ++qb) {
+      const int n = visible(qb), c = n <= chunk ? 1 : (n + chunk - 1) / chunk;
+      items += c;
+      total += n + 0.5 * c;
+    }
+    const int rep = causal ? 1 : nqb;
+    items *= rep;
+    total *= rep;
+    const int longest = std::min(chunk, n_max);
+    // equal items run in whole waves; unequal ones, longest first, fill the gaps
+    const double waves = causal ? std::max(longest + 0.5, total * heads / sms + 0.5 * (longest < n_max ? longest : 2))
+                                : std::ceil(items * heads / sms) * (longest + 0.5);
+    return waves;
+  };
+  int items = 0;
+  double best = 0.85 * cost(n_max, items);  // a cut has to be worth it: the estimate is rough
+  // without a mask the work per SM is what it is unless SMs idle; under one, unless one block dominates
+  for (int k = 2; k <= 64 && n_max / k >= 2; ++k) {
+    const int chunk = (n_max + k - 1) / k;
+    const double t0 = cost(chunk, items);
+    // the joining kernel: its launch, and the partial rows written and read (at about 4 TB/s)
+    const double t = t0 + 2.5 + heads * items * 256.0 * p->head_dim * 8.0 / 4e12 / 1.2e-6;
+    if (t < best) {
+      best = t;
+      plan.chunk_tiles = chunk;
+      plan.items_per_head = items;
+      plan.max_chunks = (n_max + chunk - 1) / chunk;
+    }
+    if (heads * items > 8.0 * sms) break;
+  }
+  if (plan.max_chunks > 1) {
+    int qb = 0;
+    while (visible(qb) <= plan.chunk_tiles) ++qb;
+    plan.first_cut_row = qb * 256;
+    plan.workspace = (size_t)plan.max_chunks * p->batch * p->heads * p->seqlen_q * (p->head_dim + 1) * sizeof(float);
+  }
+  return plan;
+}
+
+// Heads whose items are interleaved in the forward's order, so that the last items are the short
+// ones of a causal mask: as many as have their K and V in 48 of the 126 MB of L2.
+int fwd_head_group(const FmhaFwdParams* p) {
+  const double kv_bytes = 4.0 * p->seqlen_k * p->head_dim;
+  return (int)std::max(1.0, std::min((double)p->batch * p->heads, 48e6 / kv_bytes));
+}
+
 // D is the head dimension the kernel runs at; the tensors have p->head_dim <= D elements per row
 // (96 runs at D = 128: the tensor maps describe 96 columns, the loads fill the rest of a
 // 128-wide tile with zeros and the stores clip it)
 template <int D, bool kBf16>
 int launch_fwd(const FmhaFwdParams* p, cudaStream_t stream) {
   using T = fmha::FwdTraits<D, kBf16>;
+  using E = typename std::conditional<kBf16, __nv_bfloat16, __half>::type;
   CUtensorMap tq, tk, tv, to;
   int rc;
   const int Dr = p->head_dim;
   if ((rc = make_tensor_map(&tq, p->q, p->batch, p->seqlen_q, p->heads, Dr, p->q_strides, kBf16)))
     return rc;
-  // K and V are loaded in half tiles of kStepN rows
-  if ((rc = make_tensor_map(&tk, p->k, p->batch, p->seqlen_k, p->heads, Dr, p->k_strides, kBf16,
-                            T::kStepN)))
+  if ((rc = make_tensor_map(&tk, p->k, p->batch, p->seqlen_k, p->heads, Dr, p->k_strides, kBf16)))
     return rc;
-  if ((rc = make_tensor_map(&tv, p->v, p->batch, p->seqlen_k, p->heads, Dr, p->v_strides, kBf16,
-                            T::kStepN)))
+  if ((rc = make_tensor_map(&tv, p->v, p->batch, p->seqlen_k, p->heads, Dr, p->v_strides, kBf16)))
     return rc;
   if ((rc = make_tensor_map(&to, p->o, p->batch, p->seqlen_q, p->heads, Dr, p->o_strides, kBf16)))
     return rc;
+  const int dev = current_device();
+  const int sms = std::max(1, sm_count(dev) - std::max(0, (int)p->sm_margin));
+  FwdPlan plan;
+  if (p->workspace != nullptr) plan = plan_fwd(p, sms);
+  if (plan.workspace > p->workspace_bytes || plan.max_chunks <= 1) {
+    plan = FwdPlan();
+    plan.items_per_head = (p->seqlen_q + 255) / 256;
+  }
   fmha::FwdKernelParams kp;
   kp.lse = p->lse;
   kp.heads = p->heads;
@@ -219,23 +300,39 @@ int launch_fwd(const FmhaFwdParams* p, cudaStream_t stream) {
   kp.seqlen_k = p->seqlen_k;
   kp.num_q_blocks = (p->seqlen_q + 255) / 256;
   kp.num_heads_total = p->batch * p->heads;
-  kp.scale_log2 = p->scale * 1.4426950408889634f;
+  kp.head_group = fwd_head_group(p);
+  kp.items_per_head = plan.items_per_head;
+  kp.num_items = plan.items_per_head * kp.num_heads_total;
+  kp.chunk_tiles = plan.chunk_tiles;
+  kp.scale_log2 = std::fabs(p->scale) * 1.4426950408889634f;
+  kp.negate = p->scale < 0.f;
   kp.causal = p->causal ? 1 : 0;
   kp.causal_shift = p->causal_shift;
   kp.status = p->status;
   kp.seqused_q = p->seqused_q;
   kp.seqused_k = p->seqused_k;
-  kp.timeline = g_timeline;
-  kp.timeline_block = g_timeline_block;
+  kp.row_elems = Dr;
+  kp.o_part = nullptr;
+  kp.lse_part = nullptr;
+  if (plan.max_chunks > 1) {
+    kp.o_part = static_cast<float*>(p->workspace);
+    kp.lse_part = kp.o_part + (size_t)plan.max_chunks * kp.num_heads_total * p->seqlen_q * Dr;
+  }
   auto kernel = fmha::fmha_fwd_kernel<D, kBf16>;
-  const int dev = current_device();
   if (!allow_smem<fmha::fmha_fwd_kernel<D, kBf16>>(dev, T::kSmemBytes)) return FMHA_ERR_LAUNCH;
-  // persistent grid: one CTA per SM (or per super-item = pair of query blocks, if fewer)
-  const long long n_super = (long long)((kp.num_q_blocks + 1) / 2) * kp.num_heads_total;
-  const int sms = std::max(1, sm_count(dev) - std::max(0, (int)p->sm_margin));
-  const unsigned grid = (unsigned)std::min<long long>(n_super, sms);
+  // One block per item, taken over by running blocks; dealt out instead where every item has an SM
+  // of its own (nothing to take over) or the caller wants SMs left free.
+  kp.deal = kp.num_items <= sms || p->sm_margin > 0;
+  const unsigned grid = kp.deal ? (unsigned)std::min(kp.num_items, sms) : (unsigned)kp.num_items;
   kernel<<<grid, T::kThreads, T::kSmemBytes, stream>>>(tq, tk, tv, to, kp);
-  return cudaGetLastError() == cudaSuccess ? FMHA_OK : FMHA_ERR_LAUNCH;
+  if (cudaGetLastError() != cudaSuccess) return FMHA_ERR_LAUNCH;
+  if (plan.max_chunks > 1) {
+    const long long rows = (long long)kp.num_heads_total * (p->seqlen_q - plan.first_cut_row);
+    fmha::fmha_fwd_combine_kernel<E><<<(unsigned)((rows + 7) / 8), 256, 0, stream>>>(
+        kp, static_cast<E*>(p->o), p->o_strides.batch, p->o_strides.row, p->o_strides.head, plan.first_cut_row, rows);
+    if (cudaGetLastError() != cudaSuccess) return FMHA_ERR_LAUNCH;
+  }
+  return FMHA_OK;
 }
 
 // D: the head dimension the kernels run at; DR <= D: what the tensors have (p->head_dim)
@@ -373,7 +470,7 @@ int fmha_fwd(const FmhaFwdParams* p, void* stream) {
     return FMHA_ERR_NULL_POINTER;
   int rc = check_common(p->batch, p->heads, p->seqlen_q, p->seqlen_k, p->head_dim, p->scale, p->dtype);
   if (rc) return rc;
-  if (!aligned16(p->q) || !aligned16(p->k) || !aligned16(p->v) || !aligned16(p->o))
+  if (!aligned16(p->q) || !aligned16(p->k) || !aligned16(p->v) || !aligned16(p->o) || !aligned16(p->workspace))
     return FMHA_ERR_BAD_ALIGNMENT;
   if ((rc = check_strides(p->q_strides, p->seqlen_q, p->heads, p->batch))) return rc;
   if ((rc = check_strides(p->k_strides, p->seqlen_k, p->heads, p->batch))) return rc;
@@ -383,6 +480,12 @@ int fmha_fwd(const FmhaFwdParams* p, void* stream) {
   if (p->dtype == FMHA_DTYPE_BF16)
     return p->head_dim > 64 ? launch_fwd<128, true>(p, s) : launch_fwd<64, true>(p, s);
   return p->head_dim > 64 ? launch_fwd<128, false>(p, s) : launch_fwd<64, false>(p, s);
+}
+
+size_t fmha_fwd_workspace_bytes(const FmhaFwdParams* p) {
+  if (p == nullptr || check_common(p->batch, p->heads, p->seqlen_q, p->seqlen_k, p->head_dim, p->scale, p->dtype))
+    return 0;
+  return plan_fwd(p, std::max(1, sm_count(current_device()) - std::max(0, (int)p->sm_margin))).workspace;
 }
 
 size_t fmha_bwd_workspace_bytes(const FmhaBwdParams* p) {

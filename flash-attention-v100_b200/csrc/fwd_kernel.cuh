@@ -2,55 +2,64 @@
 //
 // Replaces fused_mha_forward_kernel of the reference (kernel/fused_mha_kernel.cu:20-323):
 // same mathematics (online softmax over KV tiles, running max / sum, O rescale), none of its
-// structure.  The kernel is PERSISTENT: one CTA per SM walks a list of work items; a work item
-// is 256 query rows (two 128-row tiles) of one (batch, head), processed against the KV sequence
-// in 128-row tiles, each consumed in two 64-row halves ("steps"):
+// structure.  A work item is 256 query rows (two 128-row tiles) of one (batch, head), processed
+// against the KV sequence (or a chunk of it) in 128-row tiles, one per ROUND:
 //
-//   warp 8      TMA producer for K and V, in half tiles of 64 rows, through a ring of
-//               shared-memory slots (full / empty mbarriers per slot); a slot holds what one
-//               step consumes, V(h) and K(h+2); runs ahead into the next item as slots free
+//   warp 8      TMA producer for K and V through a ring of shared-memory slots of one tile (full /
+//               empty mbarriers per slot); it is also the one that takes the next item
 //   warp 10     TMA producer for the two Q tiles of an item, as soon as the previous item's
 //               last S = Q K^T has released them
-//   warps 9, 11 MMA issuers, one per query tile t: S_t(h) = Q_t K(h)^T (128 x 64, both operands
-//               in shared memory) and O_t += P_t(h) V(h) (P_t read from tensor memory),
-//               accumulators in tensor memory.  The whole warp runs the loop so that
-//               descriptors stay in uniform registers; one elected lane issues.  Two issuers
-//               because the tensor pipe queues very little: with one, every barrier wait
-//               between two blocks of MMAs let the pipe run dry.
-//   warps 0-3   softmax of query tile 0: one thread per row, S_0(h) read with tcgen05.ld,
-//               online exp2 softmax, P_0(h) written back over S_0(h) as fp16, lazy O_0
-//               rescale, epilogue
+//   warp 9      MMA issuer.  A round is two turns, one per query tile t: O_t += P_t(j) V(j) (P_t
+//               read from tensor memory, in two halves of 64 keys), S_t(j+1) = Q_t K(j+1)^T
+//               (128 x 128).  The whole warp runs the loop so that descriptors stay in uniform
+//               registers; one elected lane issues.
+//   warps 0-3   softmax of query tile 0: one thread per row, a whole 128-column row of S_0(j) in
+//               registers, online exp2 softmax, P_0(j) written back over S_0(j) as fp16 in two
+//               halves (each released to the MMA warp as soon as it is there), lazy O_0 rescale,
+//               epilogue
 //   warps 4-7   the same for query tile 1
 //
-// S_t is double buffered in tensor memory: while the softmax group works on S_t(h), the tensor
-// pipe already holds or computes S_t(h+1), so the group never waits for the latency of an MMA
-// round trip, and the MMA warps only ever wait for P.  The price is N = 64 per S MMA, which the
-// tensor pipe runs at 3/4 of the rate of N = 128.
+// What bounds it at D = 128: shared memory, then power.  Per round the tensor pipe needs 2048 clk, and
+// its operands with the TMA writes are 256 KB, which at 128 bytes/clk is 2048 clk as well; a round takes
+// 2850 clk with the exponentials left out and 3250 with them (1500-1700 clk per group).  At D = 64
+// it is the softmax groups.  What made it faster than S tiles of 64 keys, double buffered, with two
+// issuing warps (Z=8, H=32, N=2048 / Z=1, N=16384 sustained, TFLOP/s; D=128 without a mask 947 / 1055
+// -> 1024 / 1195, causal 847 / 1057 -> 902 / 1136; D=64 614 -> 698):
+//   - S tiles of 128 keys read Q from shared memory half as often;
+//   - the turns come in a fixed order, which keeps the two softmax groups half a round apart: while
+//     one group's exponentials run, the tensor pipe works for the other;
+//   - the code is small: the roles of a CTA share one instruction cache, and at 200 KB of code the MMA
+//     warp waited for instructions (2850 clk of a round became 4000).  Control flow of the issuing
+//     warps is made warp-uniform for the compiler, slow paths are rolled loops;
+//   - no row maximum in the ordinary round (see the softmax groups), and the epilogue of an item waits
+//     for nothing;
+//   - 1/8 (D = 128) or 1/4 (D = 64) of the exponentials are a polynomial on the FMA pipe; more gives
+//     nothing (1/2: 6 % slower).
 //
-// While the groups run an item's epilogue the producer and the MMA warp already start the next
-// item (its Q / K loads and first S = Q K^T), so that the load latency at the head of an item
-// and the store at its tail are hidden.
+// While the groups run an item's epilogue the producers and the MMA warp already work on the next
+// item, so that the load latency at the head of an item and the store at its tail are hidden.
 //
 // Element type: fp16 (the reference's only type, kernel/fused_mha_api.cpp:25-29) or bf16
 // (kBf16): the tensor cores take either by two bits of the instruction descriptor; P and O are
 // then rounded to bf16 instead of fp16, everything in between stays fp32.
 //
-// Tensor memory (512 columns): S_t buffer b at [t * 128 + b * 64, + 64); O_0 [256, 256 + D),
-// O_1 [256 + D, 256 + 2 D); P_t(h) aliases the first 32 columns of the S_t buffer it came from
-// (two fp16 per 32-bit column).
+// Tensor memory (512 columns): S_t [t * 128, + 128); O_0 [256, 256 + D), O_1 [256 + D, 256 + 2 D);
+// P_t aliases the first 64 columns of S_t (two fp16 per 32-bit column).
 //
 // Shared memory: rows of 64 fp16 (128 bytes) in the TMA / UMMA 128-byte swizzle.  A 128 x D
-// tile is D/64 boxes of 128 x 64, box b at byte offset b * 16384 (a 64-row half tile of K or V:
-// boxes of 64 x 64, 8192 bytes apart).  Per softmax group one extra tile stages the output for
-// the TMA store.
+// tile is D/64 boxes of 128 x 64, box b at byte offset b * 16384.  Per softmax group one box
+// stages the output for the TMA store, 64 columns at a time.
 //
-// Work items are paired (heaviest with lightest query block of a head) into super-items of
-// equal cost, and super-items are dealt round-robin to the CTAs: balanced without a global
-// work counter, and CTAs that run at the same time work on neighbouring heads (K/V stay in L2).
+// Work distribution: the grid has one block per item, heaviest first; a running CTA takes over
+// further blocks through cluster launch control, i.e. the hardware balances the load.  A caller
+// that wants SMs left free (sm_margin) gets a smaller grid with the items dealt round robin.
 #pragma once
 #include <cuda.h>
 #include <math_constants.h>
 
+#include <type_traits>
+
+#include "aux_kernels.cuh"
 #include "ptx.cuh"
 
 namespace fmha {
@@ -60,54 +69,45 @@ struct FwdKernelParams {
   int heads, seqlen_q, seqlen_k;
   int num_q_blocks;     // ceil(seqlen_q / 256)
   int num_heads_total;  // batch * heads
-  float scale_log2;     // scale * log2(e)
+  int head_group;       // heads whose items are interleaved (>= 1)
+  int items_per_head;   // query blocks, or chunks of them
+  int num_items;
+  int deal;             // 1: items are dealt round robin to the blocks; 0: cluster launch control
+  int chunk_tiles;      // KV tiles of 128 an item covers at most
+  float scale_log2;     // |scale| * log2(e)
+  int negate;           // scale < 0: the tensor cores form -Q K^T, so that a row's maximum is a maximum
   int causal, causal_shift;
   int* status;
   // optional per-batch lengths (right-padded batches): rows >= seqused_q[z] and keys >=
   // seqused_k[z] are padding, skipped tile-wise and masked inside partial tiles
   const int* seqused_q;
   const int* seqused_k;
-  // debug builds (-DFMHA_TIMELINE) only: clock64 stamps of one CTA, see FMHA_TL
-  long long* timeline;
-  int timeline_block;
+  // query blocks cut in several chunks: fp32 partial outputs (chunk, Z*H, seqlen_q, row_elems),
+  // each normalised by its own row sum, and their log-sum-exp (chunk, Z*H, seqlen_q)
+  float* o_part;
+  float* lse_part;
+  int row_elems;        // elements per row of the tensors (head_dim)
 };
 
-#ifndef FMHA_ABLATE
-#define FMHA_ABLATE 0  // debug builds: bit 0 no exp2, bit 1 no row max, bit 2 no P store
-#endif
-
-// pairs out of every 4 whose exponential is a polynomial on the FMA pipe (the rest use MUFU),
-// for head_dim 128 and for head_dim 64
-#ifndef FMHA_FWD_POLY_PAIRS
-#define FMHA_FWD_POLY_PAIRS 0
-#endif
-#ifndef FMHA_FWD_POLY_PAIRS_D64
-#define FMHA_FWD_POLY_PAIRS_D64 0
-#endif
+// pairs out of every 8 whose exponential is a polynomial on the FMA pipe (the rest use MUFU)
+constexpr int kFwdPolyPairsD128 = 1, kFwdPolyPairsD64 = 2;
 
 template <int D, bool kBf16 = false>
 struct FwdTraits {
   static constexpr int kBlockM = 128;  // rows per query tile
   static constexpr int kTilesM = 2;    // query tiles per work item
-  static constexpr int kBlockN = 128;  // rows per KV tile (one TMA load)
-  static constexpr int kStepN = 64;    // KV rows per S = Q K^T / softmax / O += P V step
+  static constexpr int kBlockN = 128;  // rows per KV tile
   static constexpr int kBoxes = D / 64;
   static constexpr int kBoxBytes = 128 * 128;  // 128 rows x 128 bytes
   static constexpr int kTileBytes = kBoxes * kBoxBytes;
-  // K and V travel in half tiles of kStepN rows: the same shared memory holds twice as many
-  // ring slots, each released as soon as its step is done, so loads run several steps ahead
-  static constexpr int kHalfBoxBytes = kStepN * 128;  // 64 rows x 128 bytes
-  static constexpr int kHalfTileBytes = kBoxes * kHalfBoxBytes;
-  // a ring slot holds the two half tiles one step consumes: V(h) and K(h+2) (one barrier pair
-  // and one release per step); the slot of an item's head holds K(0) and K(1)
-  static constexpr int kSlotBytes = 2 * kHalfTileBytes;
-  static constexpr int kStages = (D == 128) ? 3 : 6;
-  static constexpr int kThreads = 384;  // softmax 0, softmax 1, {TMA, MMA, 2 idle} warpgroups
-  // Q tiles, K/V ring, one output staging tile per softmax group
-  static constexpr int kSmemBytes = 1024 + (kTilesM + 2) * kTileBytes + kStages * kSlotBytes;
+  static constexpr int kStages = (D == 128) ? 4 : 8;  // ring slots of one K or V tile
+  static constexpr int kItemStages = 4;  // item ids published ahead
+  static constexpr int kThreads = 384;   // softmax 0, softmax 1, {K/V, MMA, Q, idle} warps
+  // Q tiles, K/V ring, one 64-column output box per softmax group
+  static constexpr int kSmemBytes = 1024 + kTilesM * (kTileBytes + kBoxBytes) + kStages * kTileBytes;
   static constexpr int kTmemCols = 512;
-  static constexpr int kPolyPairs = (D == 64) ? FMHA_FWD_POLY_PAIRS_D64 : FMHA_FWD_POLY_PAIRS;
-  static constexpr uint32_t kIdescQK = umma_idesc_f16(128, kStepN, 0, 0, kBf16);
+  static constexpr int kPolyPairs = (D == 128) ? kFwdPolyPairsD128 : kFwdPolyPairsD64;
+  static constexpr uint32_t kIdescQK = umma_idesc_f16(128, kBlockN, 0, 0, kBf16);
   static constexpr uint32_t kIdescPV = umma_idesc_f16(128, D, 0, 1, kBf16);
 };
 
@@ -116,37 +116,22 @@ constexpr int kFwdRegsSoftmax = 168 + (168 - kFwdRegsIssue) / 2;  // warps 0-7: 
 static_assert(kFwdRegsIssue <= 168 && kFwdRegsSoftmax >= 168 && kFwdRegsSoftmax % 8 == 0,
               "setmaxnreg.dec must not raise and .inc must not lower the 168 registers of the launch");
 
-// lazy rescale threshold in the log2 domain: P may grow to 2^8 before O is rescaled
-constexpr float kRescaleThreshold = 8.0f;
+// lazy rescale: the exponentials of 64 keys of a row may add up to 2^10 before O is rescaled to a
+// new reference (P has to stay far from the 65504 of fp16; O and the row sum are fp32)
+constexpr float kRescaleSum = 1024.0f;
 
-// The work list of one CTA.  Super-item s = (head zh, pair k): query blocks nqb-1-k (heavy,
-// first) and k (light), one item only when they coincide.  Every role of the CTA walks the
-// same list with its own copy of this iterator.
-struct FwdWorkIter {
-  int s, sub, n_super, pairs_per_head, nqb, stride;
-  __device__ FwdWorkIter(int first, int stride_, int nqb_, int heads_total)
-      : s(first), sub(0), pairs_per_head((nqb_ + 1) / 2), nqb(nqb_), stride(stride_) {
-    n_super = pairs_per_head * heads_total;
-  }
-  __device__ bool next(int& zh, int& qb) {
-    while (s < n_super) {
-      const int k = s % pairs_per_head;
-      const int hi = nqb - 1 - k;
-      zh = s / pairs_per_head;
-      if (sub == 0) {
-        sub = 1;
-        qb = hi;
-        return true;
-      }
-      sub = 0;
-      s += stride;
-      if (k != hi) {
-        qb = k;
-        return true;
-      }
-    }
-    return false;
-  }
+// A work item: 256 query rows from q0 of head zh = z * heads + h, KV tiles [kv_first, kv_first + n_t)
+// for its query tile t (n_t = 0: the tile sees nothing of this chunk).  The producer warp works it
+// out and publishes it in shared memory.
+struct __align__(16) FwdItem {
+  int id;      // -1: no more items
+  int n0, n1;  // KV tiles of the two query tiles
+  int q0;
+  int z, h, zh;
+  int kv_first;
+  int sq, sk;  // lengths of the batch entry
+  int chunk;   // index of the chunk among those of its query block, -1: the block is not cut
+  int pad;
 };
 
 // the lengths that count for batch entry z: the tensors' own, or the caller's per-batch ones
@@ -155,27 +140,67 @@ __device__ __forceinline__ void fwd_lengths(const FwdKernelParams& p, int z, int
   sk = p.seqused_k == nullptr ? p.seqlen_k : max(0, min(p.seqlen_k, __ldg(p.seqused_k + z)));
 }
 
-// KV tiles each of the two query tiles of an item has to visit (0 = none)
-template <int D>
-__device__ __forceinline__ void fwd_item_extent(const FwdKernelParams& p, int z, int q0,
-                                                int (&n_kv)[2]) {
-  using T = FwdTraits<D>;
-  int sq, sk;
-  fwd_lengths(p, z, sq, sk);
-  const int nk_total = (sk + T::kBlockN - 1) / T::kBlockN;
-#pragma unroll
-  for (int t = 0; t < 2; ++t) {
-    const int r0 = q0 + t * T::kBlockM;
-    if (r0 >= sq) {
-      n_kv[t] = 0;
-    } else if (!p.causal) {
-      n_kv[t] = nk_total;
-    } else {
-      const int r_last = min(r0 + T::kBlockM - 1, sq - 1);
-      const long long lim = (long long)r_last + p.causal_shift;
-      n_kv[t] = lim < 0 ? 0 : (int)min((long long)nk_total, lim / T::kBlockN + 1);
+// KV tiles the query rows up to r_last see, of nk_total
+__host__ __device__ __forceinline__ int fwd_visible_tiles(bool causal, int shift, int r_last, int nk_total) {
+  if (!causal) return nk_total;
+  const long long lim = (long long)r_last + shift;
+  if (lim < 0) return 0;
+  return lim / 128 + 1 < nk_total ? (int)(lim / 128 + 1) : nk_total;
+}
+// chunks of a query block, by the tensors' own lengths (also on the host, where the per-batch
+// lengths are not known)
+__host__ __device__ __forceinline__ int fwd_chunks(bool causal, int shift, int qb, int seqlen_q, int nk_total,
+                                                   int chunk_tiles) {
+  const int r_last = (qb * 256 + 255 < seqlen_q - 1) ? qb * 256 + 255 : seqlen_q - 1;
+  const int n = fwd_visible_tiles(causal, shift, r_last, nk_total);
+  return n <= chunk_tiles ? 1 : (n + chunk_tiles - 1) / chunk_tiles;
+}
+
+// Items in groups of head_group heads (their K and V share the L2); in a group the last query
+// blocks first (under a causal mask the heaviest), heads innermost.
+__device__ __forceinline__ FwdItem fwd_item(const FwdKernelParams& p, int id) {
+  FwdItem it;
+  it.id = id;
+  it.pad = 0;
+  const int per_group = p.head_group * p.items_per_head;
+  const int group = id / per_group, within = id % per_group;
+  const int heads_here = min(p.head_group, p.num_heads_total - group * p.head_group);
+  int u = within / heads_here;
+  it.zh = group * p.head_group + within % heads_here;
+  it.z = it.zh / p.heads;
+  it.h = it.zh % p.heads;
+  int qb = p.num_q_blocks - 1;
+  it.chunk = -1;
+  it.kv_first = 0;
+  int most = 0x7fffffff;
+  if (p.o_part == nullptr) {
+    qb -= u;
+  } else {
+    for (;; --qb) {
+      const int chunks =
+          fwd_chunks(p.causal != 0, p.causal_shift, qb, p.seqlen_q, (p.seqlen_k + 127) / 128, p.chunk_tiles);
+      if (u < chunks || qb == 0) {
+        if (chunks > 1) {
+          it.chunk = u;
+          it.kv_first = u * p.chunk_tiles;
+          most = p.chunk_tiles;
+        }
+        break;
+      }
+      u -= chunks;
     }
   }
+  it.q0 = qb * 256;
+  fwd_lengths(p, it.z, it.sq, it.sk);
+  const int nk_total = (it.sk + 127) / 128;
+  auto tiles = [&](int r0) {
+    if (r0 >= it.sq) return 0;
+    const int n = fwd_visible_tiles(p.causal != 0, p.causal_shift, min(r0 + 127, it.sq - 1), nk_total);
+    return max(0, min(most, n - it.kv_first));
+  };
+  it.n0 = tiles(it.q0);
+  it.n1 = tiles(it.q0 + 128);
+  return it;
 }
 
 template <int D, bool kBf16 = false>
@@ -185,23 +210,24 @@ __global__ void __launch_bounds__(384, 1)
                     const FwdKernelParams p) {
   using T = FwdTraits<D, kBf16>;
   extern __shared__ uint8_t smem_raw[];
+  __shared__ __align__(16) uint8_t clc_word[16];
+  __shared__ uint64_t bar_clc;                        // the answer to the last request is in clc_word
+  __shared__ FwdItem items[T::kItemStages];           // items of this CTA
+  __shared__ uint64_t bar_item_full[T::kItemStages], bar_item_empty[T::kItemStages];
   __shared__ uint64_t bar_q_full[2];   // Q_t of the current item has landed
   __shared__ uint64_t bar_q_free[2];   // the last S_t = Q_t K^T of the item is done: Q_t reusable
   __shared__ uint64_t bar_kv_full[T::kStages];
   __shared__ uint64_t bar_kv_empty[T::kStages];
-  __shared__ uint64_t bar_s_full[2][2];  // [tile][buffer]
-  __shared__ uint64_t bar_pv_done[2];    // one of the last two O_t += of an item has completed
-  // One barrier per S/P buffer: a softmax warp may be a step ahead of its neighbours, and its
-  // arrival for step h+1 must not be counted towards step h.  Per buffer that cannot happen:
-  // the buffer's next S only exists after everybody's P of this step has been consumed.
-  __shared__ uint64_t bar_p_full[2][2];  // [tile][buffer]
+  __shared__ uint64_t bar_s_full[2];     // S_t(j) is there, and so is the result of O_t += of round j - 1
+  __shared__ uint64_t bar_p_full[2][2];  // [tile][half]: P_t for 64 keys is there
+  __shared__ uint64_t bar_pv_half[2];    // O_t += of the first 64 keys of the round has completed
   __shared__ uint64_t bar_o_full[2];
   __shared__ uint64_t bar_o_read[2];   // the softmax group has O_t in registers: O_t reusable
   __shared__ uint32_t tmem_base_slot;
   __shared__ int abort_word;
   __shared__ int skip_cta;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);  // warp-uniform for the compiler, too
   const int lane = threadIdx.x & 31;
 
   // a status word already set by an earlier launch / CTA means: drain the grid quickly
@@ -215,23 +241,29 @@ __global__ void __launch_bounds__(384, 1)
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t q_smem = smem_base;                                    // 2 query tiles
   const uint32_t ring_smem = smem_base + T::kTilesM * T::kTileBytes;    // K/V ring
-  const uint32_t ostage_smem = ring_smem + T::kStages * T::kSlotBytes;  // 2 output tiles
+  const uint32_t ostage_smem = ring_smem + T::kStages * T::kTileBytes;  // 2 output boxes
 
   // ---- set-up: barriers (thread 0), tensor memory (warp 9)
   if (threadIdx.x == 0) {
+    mbar_init(smem_u32(&bar_clc), 1);
+    for (int s = 0; s < T::kItemStages; ++s) {
+      mbar_init(smem_u32(&bar_item_full[s]), 1);
+      mbar_init(smem_u32(&bar_item_empty[s]), 10);  // MMA warp, Q warp, eight softmax warps
+    }
     for (int s = 0; s < T::kStages; ++s) {
       mbar_init(smem_u32(&bar_kv_full[s]), 1);
-      mbar_init(smem_u32(&bar_kv_empty[s]), 2);  // one release by each MMA warp
+      mbar_init(smem_u32(&bar_kv_empty[s]), 1);
     }
     for (int t = 0; t < 2; ++t) {
       mbar_init(smem_u32(&bar_q_full[t]), 1);
       mbar_init(smem_u32(&bar_q_free[t]), 1);
-      mbar_init(smem_u32(&bar_s_full[t][0]), 1);
-      mbar_init(smem_u32(&bar_s_full[t][1]), 1);
-      mbar_init(smem_u32(&bar_pv_done[t]), 1);
-      // one arrival per softmax warp: 128 arrivals on one word are 128 serialised atomics
+      mbar_init(smem_u32(&bar_s_full[t]), 1);
+      // one arrival per softmax warp: 128 arrivals on one word are 128 serialised atomics.  A warp
+      // cannot arrive twice in one phase: it needs the next S_t in between, which is only issued
+      // once all four warps' P_t has been consumed.
       mbar_init(smem_u32(&bar_p_full[t][0]), 4);
       mbar_init(smem_u32(&bar_p_full[t][1]), 4);
+      mbar_init(smem_u32(&bar_pv_half[t]), 1);
       mbar_init(smem_u32(&bar_o_full[t]), 1);
       mbar_init(smem_u32(&bar_o_read[t]), 4);
     }
@@ -244,10 +276,30 @@ __global__ void __launch_bounds__(384, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = tmem_base_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, tmem_base_slot, 0);
 
-  FwdWorkIter work(blockIdx.x, gridDim.x, p.num_q_blocks, p.num_heads_total);
-  int zh, qb;
+  // The next item published by the producer warp (every consuming warp keeps its own count); id = -1
+  // when there is none, and when a wait ran out.
+  uint32_t item_cnt = 0;
+  auto take_item = [&]() -> FwdItem {
+    const uint32_t s = item_cnt % T::kItemStages;
+    FwdItem it;
+    if (mbar_wait_warp(smem_u32(&bar_item_full[s]), (item_cnt / T::kItemStages) & 1, &abort_word, 12)) {
+      it = items[s];
+      // what decides over branches is made warp-uniform for the compiler: only in control flow that
+      // it knows to be uniform can it keep addresses and MMA descriptors in uniform registers
+      it.id = __shfl_sync(0xffffffffu, it.id, 0);
+      it.n0 = __shfl_sync(0xffffffffu, it.n0, 0);
+      it.n1 = __shfl_sync(0xffffffffu, it.n1, 0);
+    } else {
+      it.id = -1;
+      it.n0 = it.n1 = 0;
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(smem_u32(&bar_item_empty[s]));
+    ++item_cnt;
+    return it;
+  };
 
   // Register budget: 384 threads leave 168 per thread.  The producer / MMA warpgroup hands part
   // of its share to the softmax warpgroups, whose threads hold a 128-column row of S.  Each
@@ -255,230 +307,229 @@ __global__ void __launch_bounds__(384, 1)
   if (warp >= 8) {
     reg_dealloc<kFwdRegsIssue>();
     if (warp == 8) {
-      // =========================== TMA producer (converged warp, elected issue) ==========
+      // =========================== K/V producer, item source (converged warp) ==========
       if (elect_one()) {
         tma_prefetch_desc(&tm_q);
         tma_prefetch_desc(&tm_k);
         tma_prefetch_desc(&tm_v);
       }
       __syncwarp();
-      uint32_t kv_it = 0;  // ring slots loaded so far (slot index and phase)
       bool ok = true;
-      while (ok && work.next(zh, qb)) {
-        const int z = zh / p.heads, h = zh % p.heads;
-        const int q0 = qb * (T::kBlockM * T::kTilesM);
-        int n_kv[2];
-        fwd_item_extent<D>(p, z, q0, n_kv);
-        // slot loads in the order the MMA warps consume them:
-        //   [K(0) K(1)]  [V(0) K(2)]  [V(1) K(3)]  ...  [V(nh-3) K(nh-1)]  [V(nh-2)]  [V(nh-1)]
-        const int nh = 2 * max(n_kv[0], n_kv[1]);
-        const int n_loads = nh > 0 ? nh + 1 : 0;
-        for (int it = 0; it < n_loads; ++it, ++kv_it) {
-          const uint32_t slot = kv_it % T::kStages;
-          const uint32_t round = kv_it / T::kStages;
-          if (round > 0 &&
-              !mbar_wait_warp(smem_u32(&bar_kv_empty[slot]), (round - 1) & 1, &abort_word, 2)) {
-            ok = false;
-            break;
-          }
-          // first and second half tile of the slot (-1 = none)
-          const int k_first = (it == 0) ? 0 : -1;               // K half in the first place
-          const int v_first = (it == 0) ? -1 : it - 1;          // V(h), h = it - 1
-          const int k_second = (it == 0) ? 1 : (it + 1 < nh ? it + 1 : -1);  // K(h+2)
-          if (elect_one()) {
-            const uint32_t fbar = smem_u32(&bar_kv_full[slot]);
-            const uint32_t base = ring_smem + slot * T::kSlotBytes;
-            mbar_arrive_expect_tx(fbar, (k_second >= 0 ? 2 : 1) * T::kHalfTileBytes);
+      uint32_t published = 0, asked = 0;
+      // Asking for a block is separate from taking it: the answer takes a microsecond, and asking as
+      // late as possible is what lets the CTA that is done first have the block.
+      bool pending = false;
+      auto ask = [&]() {
+        if (p.deal || pending) return;
+        if (elect_one()) {
+          fence_proxy_async_smem();  // the last answer has been read
+          mbar_arrive_expect_tx(smem_u32(&bar_clc), 16);
+          clc_request(smem_u32(clc_word), smem_u32(&bar_clc));
+        }
+        __syncwarp();
+        pending = true;
+      };
+      // finds the next item and publishes it
+      int id = -1;
+      auto next_item = [&]() -> FwdItem {
+        if (published == 0) {
+          id = blockIdx.x;
+        } else if (p.deal) {
+          id = p.num_items - id > (int)gridDim.x ? id + (int)gridDim.x : -1;
+        } else {
+          ask();
+          ok = mbar_wait_warp(smem_u32(&bar_clc), asked & 1, &abort_word, 14);
+          ++asked;
+          pending = false;
+          id = ok ? clc_answer(smem_u32(clc_word)) : -1;
+        }
+        id = __shfl_sync(0xffffffffu, id, 0);
+        FwdItem it;
+        it.id = -1;
+        it.n0 = it.n1 = 0;
+        if (id >= 0) it = fwd_item(p, id);
+        it.n0 = __shfl_sync(0xffffffffu, it.n0, 0);
+        it.n1 = __shfl_sync(0xffffffffu, it.n1, 0);
+        const uint32_t s = published % T::kItemStages, round = published / T::kItemStages;
+        if (round > 0 && !mbar_wait_warp(smem_u32(&bar_item_empty[s]), (round - 1) & 1, &abort_word, 13)) ok = false;
+        if (ok && lane == 0) {
+          items[s] = it;
+          mbar_arrive(smem_u32(&bar_item_full[s]));
+        }
+        __syncwarp();
+        ++published;
+        if (!ok) it.id = -1;
+        return it;
+      };
+      uint32_t slot = 0, phase = 1;  // the next ring slot, parity of its last release (none yet: passes)
+      auto load = [&](const CUtensorMap* tm, const FwdItem& it, int tile) {
+        if (!(ok = mbar_wait_warp(smem_u32(&bar_kv_empty[slot]), phase, &abort_word, 2))) return;
+        if (elect_one()) {
+          const uint32_t fbar = smem_u32(&bar_kv_full[slot]);
+          mbar_arrive_expect_tx(fbar, T::kTileBytes);
 #pragma unroll
-            for (int b = 0; b < T::kBoxes; ++b) {
-              if (k_first >= 0)
-                tma_load_4d(base + b * T::kHalfBoxBytes, &tm_k, fbar, b * 64, k_first * T::kStepN, h, z);
-              else
-                tma_load_4d(base + b * T::kHalfBoxBytes, &tm_v, fbar, b * 64, v_first * T::kStepN, h, z);
-              if (k_second >= 0)
-                tma_load_4d(base + T::kHalfTileBytes + b * T::kHalfBoxBytes, &tm_k, fbar, b * 64,
-                            k_second * T::kStepN, h, z);
-            }
-          }
-          __syncwarp();
+          for (int b = 0; b < T::kBoxes; ++b)
+            tma_load_4d(ring_smem + slot * T::kTileBytes + b * T::kBoxBytes, tm, fbar, b * 64,
+                        (it.kv_first + tile) * T::kBlockN, it.h, it.z);
+        }
+        __syncwarp();
+        if (++slot == T::kStages) {
+          slot = 0;
+          phase ^= 1u;
+        }
+      };
+      // K(0) V(0) K(1) V(1) ... of one item after the other
+      while (ok) {
+        const FwdItem it = next_item();
+        if (it.id < 0) break;
+        const int n = max(it.n0, it.n1);
+#pragma unroll 1
+        for (int i = 0; ok && i < 2 * n; ++i) {
+          if (i >= 2 * n - 5) ask();
+          load((i & 1) ? &tm_v : &tm_k, it, i >> 1);
         }
       }
     } else if (warp == 10) {
       // =========================== Q producer ===========================
       // its own warp, so that waiting for the Q buffers of the running item never holds back
       // the K/V prefetch of the next one
-      uint32_t items = 0;  // items with work seen so far (phase of the Q barriers)
+      uint32_t phase = 0;  // bit t: Q_t tiles loaded so far, modulo 2 (phase of the Q barriers)
+      uint32_t used = 0;   // bit t: Q_t has been loaded before
       bool ok = true;
-      while (ok && work.next(zh, qb)) {
-        const int z = zh / p.heads, h = zh % p.heads;
-        const int q0 = qb * (T::kBlockM * T::kTilesM);
-        int n_kv[2];
-        fwd_item_extent<D>(p, z, q0, n_kv);
-        if (max(n_kv[0], n_kv[1]) == 0) continue;
-#pragma unroll
+      while (ok) {
+        const FwdItem it = take_item();
+        if (it.id < 0) break;
+#pragma unroll 1
         for (int t = 0; t < T::kTilesM; ++t) {
-          if (items > 0 &&
-              !mbar_wait_warp(smem_u32(&bar_q_free[t]), (items - 1) & 1, &abort_word, 1)) {
-            ok = false;
-            break;
+          if ((t == 0 ? it.n0 : it.n1) == 0) continue;
+          const int row = it.q0 + t * T::kBlockM;
+          if ((used >> t) & 1) {
+            // cold from HBM this takes microseconds: start towards L2 before waiting for the buffer
+            if (elect_one())
+#pragma unroll
+              for (int b = 0; b < T::kBoxes; ++b) tma_prefetch_l2_4d(&tm_q, b * 64, row, it.h, it.z);
+            __syncwarp();
+            if (!mbar_wait_warp(smem_u32(&bar_q_free[t]), ((phase >> t) & 1) ^ 1, &abort_word, 1)) {
+              ok = false;
+              break;
+            }
           }
           if (elect_one()) {
             const uint32_t qbar = smem_u32(&bar_q_full[t]);
             mbar_arrive_expect_tx(qbar, T::kTileBytes);
 #pragma unroll
             for (int b = 0; b < T::kBoxes; ++b)
-              tma_load_4d(q_smem + t * T::kTileBytes + b * T::kBoxBytes, &tm_q, qbar, b * 64,
-                          q0 + t * T::kBlockM, h, z);
+              tma_load_4d(q_smem + t * T::kTileBytes + b * T::kBoxBytes, &tm_q, qbar, b * 64, row, it.h, it.z);
           }
           __syncwarp();
-        }
-        ++items;
-        // the next item's Q tiles come cold from HBM (microseconds): start them towards L2 now,
-        // a whole item ahead of the load that needs them
-        {
-          FwdWorkIter peek = work;
-          int zh2, qb2;
-          if (peek.next(zh2, qb2) && elect_one()) {
-#pragma unroll
-            for (int t = 0; t < T::kTilesM; ++t)
-#pragma unroll
-              for (int b = 0; b < T::kBoxes; ++b)
-                tma_prefetch_l2_4d(&tm_q, b * 64, qb2 * (T::kBlockM * T::kTilesM) + t * T::kBlockM,
-                                   zh2 % p.heads, zh2 / p.heads);
-          }
-          __syncwarp();
+          phase ^= 1u << t;
+          used |= 1u << t;
         }
       }
-    } else if (warp == 9 || warp == 11) {
-      // =========================== MMA issuers, one warp per query tile ===================
-      // Two issuers, because the tensor pipe queues very little: whenever a single issuer sat in
-      // a barrier wait between two blocks of MMAs the pipe ran dry.  With one warp per tile the
-      // other warp's MMAs fill those gaps.
-      // (converged warp, elected issue)
+    } else if (warp == 9) {
+      // =========================== MMA issuer (converged warp, elected issue) ===================
       // All 32 lanes run the loop so that addresses and descriptors live in uniform registers;
       // a loop run by one lane only makes every operand a per-thread value that has to be moved
       // to a uniform register before each tcgen05.mma, and the issue rate falls below the
       // tensor pipe's 64 cycles per 128x128x16 MMA.
       const uint32_t q_lo0 = umma_desc_lo(q_smem, kLboKMajor);
-      // S_t buffer `buf` = Q_t K(h)^T, K(h) = the half tile at k_addr
-      auto issue_qk = [&](int t, int buf, uint32_t k_addr) {
-        const uint32_t d = tmem_base + t * 128 + buf * T::kStepN;
-        const uint32_t a_lo = q_lo0 + ((t * T::kTileBytes) >> 4);
-        const uint32_t b_lo = umma_desc_lo(k_addr, kLboKMajor);
-#pragma unroll
-        for (int ks = 0; ks < D / 16; ++ks) {
-          const uint32_t a_off = ((ks >> 2) * T::kBoxBytes + (ks & 3) * 32) >> 4;
-          const uint32_t b_off = ((ks >> 2) * T::kHalfBoxBytes + (ks & 3) * 32) >> 4;
-          umma_ss_elect(d, a_lo + a_off, b_lo + b_off, T::kIdescQK, ks > 0 ? 1u : 0u);
+      const uint32_t idesc_qk = T::kIdescQK | (p.negate ? kIdescNegateA : 0u);
+      uint32_t slot = 0, slot_phase = 0;
+      uint32_t phase_q = 0;  // bit t: parity of the next q_full[t]
+      uint32_t phase_p = 0;  // bit t: parity of the next p_full[t]
+      uint32_t phase_o = 0;  // bit t: parity of the next o_read[t], of the first one already waited for
+      uint32_t used_o = 0;   // bit t: O_t has been written before
+      auto slot_wait = [&]() {
+        return mbar_wait_warp(smem_u32(&bar_kv_full[slot]), slot_phase, &abort_word, 4);
+      };
+      auto slot_next = [&]() {
+        umma_commit_elect(smem_u32(&bar_kv_empty[slot]));
+        if (++slot == T::kStages) {
+          slot = 0;
+          slot_phase ^= 1u;
         }
       };
-      // O_t (+)= P_t (in S_t buffer `buf`) V(h), V(h) = the half tile at v_addr; its 64-column
-      // boxes are kHalfBoxBytes apart
-      auto issue_pv = [&](int t, int buf, uint32_t v_addr, bool accumulate) {
-        const uint32_t d = tmem_base + 256 + t * D;
-        const uint32_t a = tmem_base + t * 128 + buf * T::kStepN;
-        const uint32_t b_lo = umma_desc_lo(v_addr, T::kHalfBoxBytes);
-#pragma unroll
-        for (int ks = 0; ks < T::kStepN / 16; ++ks)
-          umma_ts_elect(d, a + ks * 8, b_lo + ((ks * 2048) >> 4), T::kIdescPV,
-                        (accumulate || ks > 0) ? 1u : 0u);
-      };
-      auto kv_addr = [&](uint32_t it) { return ring_smem + (it % T::kStages) * T::kSlotBytes; };
-      auto kv_wait = [&](uint32_t it, int who) {
-        return mbar_wait_warp(smem_u32(&bar_kv_full[it % T::kStages]), (it / T::kStages) & 1,
-                              &abort_word, who);
-      };
-      auto kv_release = [&](uint32_t it) {
-        umma_commit_elect(smem_u32(&bar_kv_empty[it % T::kStages]));
-      };
-      const int t = (warp == 9) ? 0 : 1;  // the query tile this warp issues for
-      uint32_t items = 0, kv_it = 0;  // kv_it: ring slots consumed before this item
-      int tl_base = 0;     // timeline slot offset of the current item (debug builds)
-      uint32_t p_cnt = 0;  // P_t steps consumed so far (even at item boundaries)
-      uint32_t o_cnt = 0;  // items in which tile t produced an O_t (phase of o_read[t])
+      FwdItem cur = take_item();
+      int j = -1;
       bool ok = true;
-      while (ok && work.next(zh, qb)) {
-        const int q0 = qb * (T::kBlockM * T::kTilesM);
-        int n_kv[2];
-        fwd_item_extent<D>(p, zh / p.heads, q0, n_kv);
-        const int n_max = max(n_kv[0], n_kv[1]);
-        if (n_max == 0) continue;
-        const int nh = 2 * n_kv[t];  // steps of this tile
-        const int nhm = 2 * n_max;   // steps of the item (the K/V ring serves both tiles)
-        {
-          // the first two S_t of the item, one per buffer, from K(0) and K(1) in the head slot
-          ok = ok && mbar_wait_warp(smem_u32(&bar_q_full[t]), items & 1, &abort_word, 3) &&
-               kv_wait(kv_it, 4);
-          if (!ok) break;
-          tc_fence_after();
-          if (nh > 0) {
-#pragma unroll
-            for (int b = 0; b < 2; ++b) {
-              issue_qk(t, b, kv_addr(kv_it) + b * T::kHalfTileBytes);
-              umma_commit_elect(smem_u32(&bar_s_full[t][b]));
-            }
-          }
-          // with at most one KV tile these were the item's last uses of Q_t
-          if (nh <= 2) umma_commit_elect(smem_u32(&bar_q_free[t]));
-          kv_release(kv_it);
+      // One pass per round: V(j) of cur (j = -1: none) and K(j+1), which after the last round is K(0) of
+      // the item behind it (nxt).
+      while (ok && cur.id >= 0) {
+        const int n = max(cur.n0, cur.n1);
+        if (n == 0) {
+          cur = take_item();
+          continue;
         }
-        for (int h = 0; ok && h < nhm; ++h) {
-          const int buf = h & 1;
-          const uint32_t it_s = kv_it + 1 + h;  // the slot with V(h) and K(h+2)
-          // The step's two waits (its slot, P_t(h)) with both probes in flight together; when
-          // both are ready, as they normally are, the bounded waits below are skipped.  A slot
-          // is only released after it was seen full, used or not: otherwise this warp could
-          // release the same slot twice within one round of the ring.
-          const uint32_t bs = smem_u32(&bar_kv_full[it_s % T::kStages]);
-          const uint32_t ps = (it_s / T::kStages) & 1;
-          const bool use_p = h < nh;
-          const uint32_t bp = use_p ? smem_u32(&bar_p_full[t][buf]) : bs;
-          const uint32_t pp = use_p ? ((p_cnt >> 1) & 1) : ps;
-          const bool all_ready = __all_sync(0xffffffffu, mbar_try_wait3(bs, ps, bp, pp, bs, ps));
-          if (!all_ready && !kv_wait(it_s, 5)) {
-            ok = false;
-            break;
-          }
-          if (h < nh) {
-            FMHA_TL(2, tl_base + h, t * 4 + 0);
-            if (!all_ready &&
-                !mbar_wait_warp(smem_u32(&bar_p_full[t][buf]), (p_cnt >> 1) & 1, &abort_word, 6)) {
-              ok = false;
-              break;
+        const bool last = j == n - 1;
+        FwdItem nxt = cur;
+        if (last) nxt = take_item();
+        const bool has_k = !last || max(nxt.n0, nxt.n1) > 0;
+        const int jk = last ? 0 : j + 1;
+        // V(j) sits in the current slot, K(jk) in the one behind it
+        const uint32_t v_addr = ring_smem + slot * T::kTileBytes;
+        const uint32_t k_slot = j < 0 ? slot : (slot + 1 == T::kStages ? 0 : slot + 1);
+        const uint32_t k_addr = ring_smem + k_slot * T::kTileBytes;
+        const uint32_t k_phase = k_slot < slot ? slot_phase ^ 1u : slot_phase;
+        if (j >= 0 && !(ok = slot_wait())) break;
+#pragma unroll 1
+        for (int t = 0; t < 2; ++t) {
+          const int nt = t == 0 ? cur.n0 : cur.n1;
+          if (j >= 0 && j < nt) {
+            // ---- O_t (+)= P_t V(j), as the two halves of P_t come in
+            // the first O_t += of an item overwrites O_t: the previous item's epilogue must have
+            // read it out of tensor memory
+            if (j == 0) {
+              if ((used_o >> t) & 1) {
+                ok = mbar_wait_warp(smem_u32(&bar_o_read[t]), (phase_o >> t) & 1, &abort_word, 7);
+                phase_o ^= 1u << t;
+              }
+              used_o |= 1u << t;
             }
-            ++p_cnt;
-            // the first O_t += of an item overwrites O_t: the previous item's epilogue must
-            // have read it out of tensor memory
-            if (h == 0 && o_cnt > 0 &&
-                !mbar_wait_warp(smem_u32(&bar_o_read[t]), (o_cnt - 1) & 1, &abort_word, 7)) {
-              ok = false;
-              break;
+            const uint32_t v_lo = umma_desc_lo(v_addr, kLboMnMajor);
+            const uint32_t d = tmem_base + 256 + t * D, a = tmem_base + t * 128;
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+              ok = ok && mbar_wait_warp(smem_u32(&bar_p_full[t][half]), (phase_p >> t) & 1, &abort_word, 6);
+              tc_fence_after();
+#pragma unroll
+              for (int ks = half * 4; ks < half * 4 + 4; ++ks)
+                umma_ts_elect(d, a + ks * 8, v_lo + ((ks * 2048) >> 4), T::kIdescPV, (j > 0 || ks > 0) ? 1u : 0u);
+              // told to the softmax group, for the rare case that it has to rescale in mid-round
+              if (half == 0) umma_commit_elect(smem_u32(&bar_pv_half[t]));
+            }
+            phase_p ^= 1u << t;
+            if (j == nt - 1) umma_commit_elect(smem_u32(&bar_o_full[t]));
+            if (!ok) break;
+          }
+          if (t == 1 && j >= 0) slot_next();
+          // ---- S_t = Q_t K^T of the round after, which may be the first of the next item
+          if (t == 0 && has_k && !(ok = mbar_wait_warp(smem_u32(&bar_kv_full[k_slot]), k_phase, &abort_word, 5))) break;
+          const int nk = t == 0 ? nxt.n0 : nxt.n1;
+          if (jk < nk) {
+            if (jk == 0) {
+              ok = mbar_wait_warp(smem_u32(&bar_q_full[t]), (phase_q >> t) & 1, &abort_word, 3);
+              phase_q ^= 1u << t;
+              if (!ok) break;
             }
             tc_fence_after();
-            FMHA_TL(2, tl_base + h, t * 4 + 1);
-            issue_pv(t, buf, kv_addr(it_s), h > 0);
-            FMHA_TL(2, tl_base + h, t * 4 + 2);
-            if (h + 2 < nh) {
-              // S_t(h+2) goes where P_t(h) was; the tensor pipe runs one warp's MMAs in order.
-              // Its commit also tells the softmax group that O_t += P_t(h) V(h) is complete.
-              issue_qk(t, buf, kv_addr(it_s) + T::kHalfTileBytes);
-              umma_commit_elect(smem_u32(&bar_s_full[t][buf]));
-              if (h + 3 == nh) umma_commit_elect(smem_u32(&bar_q_free[t]));
-            } else {
-              // no S follows: the completion of this O_t += gets a barrier of its own
-              umma_commit_elect(smem_u32(&bar_pv_done[t]));
-              if (h + 1 == nh) {
-                umma_commit_elect(smem_u32(&bar_o_full[t]));
-                ++o_cnt;
-              }
+            const uint32_t a_lo = q_lo0 + ((t * T::kTileBytes) >> 4);
+            const uint32_t b_lo = umma_desc_lo(k_addr, kLboKMajor);
+#pragma unroll
+            for (int ks = 0; ks < D / 16; ++ks) {
+              const uint32_t off = ((ks >> 2) * T::kBoxBytes + (ks & 3) * 32) >> 4;
+              umma_ss_elect(tmem_base + t * 128, a_lo + off, b_lo + off, idesc_qk, ks > 0 ? 1u : 0u);
             }
-            FMHA_TL(2, tl_base + h, t * 4 + 3);
+            umma_commit_elect(smem_u32(&bar_s_full[t]));
+            if (jk == nk - 1) umma_commit_elect(smem_u32(&bar_q_free[t]));
           }
-          kv_release(it_s);
         }
-        kv_it += nhm + 1;
-        ++items;
-        tl_base += 64;
+        if (!ok) break;
+        if (has_k) slot_next();
+        ++j;
+        if (last) {
+          cur = nxt;
+          j = has_k ? 0 : -1;
+        }
       }
     }
   } else {
@@ -490,215 +541,245 @@ __global__ void __launch_bounds__(384, 1)
     const uint32_t lane_addr = uint32_t(quad * 32) << 16;
     const uint32_t tS = tmem_base + lane_addr + t * 128;
     const uint32_t tO = tmem_base + lane_addr + 256 + t * D;
-    const uint32_t o_stage = ostage_smem + t * T::kTileBytes;
-    bool stored = false;  // a TMA store of this group may still be reading the staging box
+    const uint32_t o_stage = ostage_smem + t * T::kBoxBytes;
     const float c = p.scale_log2;
-    // a masked score must give exp2(s * c - m * c) = 0 whatever the sign of c
-    const float mask_val = (c >= 0.f) ? -CUDART_INF_F : CUDART_INF_F;
-    const bool tl = (lane == 0 && quad == 0);
-    uint32_t step = 0;    // steps of this tile so far, over all items (even at item boundaries)
-    uint32_t o_cnt = 0;   // O_t tiles read so far (phase of o_full[t])
-    int tl_base = 0;      // timeline slot offset of the current item (debug builds)
+    uint32_t phase_s = 0, phase_o = 0;  // parities of the next s_full[t], o_full[t]
+    bool stored = false;  // a TMA store of this group may still be reading the staging box
 
-    while (work.next(zh, qb)) {
-      const int z = zh / p.heads, h = zh % p.heads;
-      const int q0 = qb * (T::kBlockM * T::kTilesM);
-      int n_kv[2];
-      fwd_item_extent<D>(p, z, q0, n_kv);
-      int sq, sk;
-      fwd_lengths(p, z, sq, sk);
-      const int n = n_kv[t];
-      const bool tile_valid = (q0 + t * T::kBlockM) < p.seqlen_q;
-      const int row = q0 + t * T::kBlockM + row_in_tile;
-      long long lim_ll = p.causal ? (long long)row + p.causal_shift : (long long)sk - 1;
-      lim_ll = min(lim_ll, (long long)sk - 1);
-      if (row >= sq) lim_ll = -1;  // a padding row sees nothing: O = 0, LSE = -inf
-      lim_ll = max(lim_ll, -1ll);
-      const int row_limit = (int)lim_ll;  // last visible key of this row (-1 = none)
+    // The epilogue of an item is done after the first round of the next one: its O_t is complete by
+    // then (nothing to wait for), and what follows the read of O_t (normalising, staging, storing)
+    // runs while the tensor pipe works on the second round.
+    bool pending = false;
+    FwdItem done;           // the item whose epilogue is pending
+    float done_m = 0.f, done_l = 0.f;
 
-      float m_ref = mask_val;  // reference score of the running softmax (raw, unscaled)
-      float l = 0.f;           // running sum of exp2((s - m_ref) * c)
-
-      for (int hs = 0; hs < 2 * n; ++hs, ++step) {
-        const uint32_t buf = step & 1;  // == hs & 1
-        const uint32_t tSb = tS + buf * T::kStepN;
-        if (tl) FMHA_TL(t, tl_base + hs, 0);
-        // on a time-out keep going: every later wait returns at once, and all 128 threads of
-        // the group still meet at the named barriers of the epilogue
-        mbar_wait(smem_u32(&bar_s_full[t][buf]), (step >> 1) & 1, &abort_word, 9);
-        tc_fence_after();
-        if (tl) FMHA_TL(t, tl_base + hs, 1);
-        uint32_t s[2][32];
-        tmem_ld32(tSb + 0, s[0]);
-        tmem_ld32(tSb + 32, s[1]);
-        tmem_wait_ld();
-        if (tl) FMHA_TL(t, tl_base + hs, 2);
-
-        const int lim = row_limit - hs * T::kStepN;  // columns > lim of this step are masked
-        if (lim < T::kStepN - 1) {
-#pragma unroll
-          for (int cc = 0; cc < 2; ++cc)
-#pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (cc * 32 + i > lim) s[cc][i] = __float_as_uint(mask_val);
-        }
-
-        // row extreme: max of s when c >= 0, min when c < 0, so that m * c = max(s * c)
-        float mx0 = __uint_as_float(s[0][0]), mx1 = __uint_as_float(s[1][0]);
-        if (c >= 0.f) {
-          mx0 = fmaxf(mx0, __uint_as_float(s[0][1]));
-          mx1 = fmaxf(mx1, __uint_as_float(s[1][1]));
-#pragma unroll
-          for (int i = 2; i < 32; i += 2) {
-            mx0 = max3(mx0, __uint_as_float(s[0][i]), __uint_as_float(s[0][i + 1]));
-            mx1 = max3(mx1, __uint_as_float(s[1][i]), __uint_as_float(s[1][i + 1]));
-          }
-        } else {
-          mx0 = fminf(mx0, __uint_as_float(s[0][1]));
-          mx1 = fminf(mx1, __uint_as_float(s[1][1]));
-#pragma unroll
-          for (int i = 2; i < 32; i += 2) {
-            mx0 = min3(mx0, __uint_as_float(s[0][i]), __uint_as_float(s[0][i + 1]));
-            mx1 = min3(mx1, __uint_as_float(s[1][i]), __uint_as_float(s[1][i + 1]));
-          }
-        }
-        float mx = (c >= 0.f) ? fmaxf(mx0, mx1) : fminf(mx0, mx1);
-        if (FMHA_ABLATE & 2) mx = __uint_as_float(s[0][0]);
-
-        if (hs == 0) {
-          m_ref = mx;
-        } else {
-          const float m_new = (c >= 0.f) ? fmaxf(m_ref, mx) : fminf(m_ref, mx);
-          // growth of the scaled maximum; NaN (inf - inf) compares false
-          const bool need = (m_new - m_ref) * c > kRescaleThreshold;
-          const bool any_need = __any_sync(0xffffffffu, need);
-#ifdef FMHA_COUNT_RESCALE
-          // debug builds: how often a warp takes the rescale path (word 0), per warp-step (word 1)
-          if (lane == 0 && p.timeline != nullptr) {
-            atomicAdd(reinterpret_cast<unsigned long long*>(p.timeline) + 1, 1ull);
-            if (any_need) atomicAdd(reinterpret_cast<unsigned long long*>(p.timeline), 1ull);
-          }
-#endif
-          if (any_need) {
-            // O_t may still be accumulating the previous step: wait for that MMA.  The next
-            // one is not issued before this thread has arrived on p_full.
-            // That is known from the commit of S_t(hs+1), issued right behind it, or, for
-            // the last step of an item (no S follows the last two O_t +=, which complete
-            // bar_pv_done twice per item), from the first of those two completions.
-            if (hs + 1 < 2 * n)
-              mbar_wait(smem_u32(&bar_s_full[t][buf ^ 1]), ((step + 1) >> 1) & 1, &abort_word, 11);
-            else
-              mbar_wait(smem_u32(&bar_pv_done[t]), 0, &abort_word, 11);
-            tc_fence_after();
-            const float alpha = isinf(m_new) ? 1.f : fast_exp2((m_ref - m_new) * c);
-            l *= alpha;
-            m_ref = m_new;
-#pragma unroll
-            for (int cc = 0; cc < D / 32; ++cc) {
-              uint32_t o[32];
-              tmem_ld32(tO + cc * 32, o);
-              tmem_wait_ld();
-#pragma unroll
-              for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-              tmem_st32(tO + cc * 32, o);
-            }
-          }
-        }
-
-        if (tl) FMHA_TL(t, tl_base + hs, 3);
-        const float neg_mc = isinf(m_ref) ? 0.f : -m_ref * c;
-        const uint64_t c2 = pack2f(c, c), nm2 = pack2f(neg_mc, neg_mc);
-        uint64_t la = pack2f(0.f, 0.f), lb = pack2f(0.f, 0.f);
-        uint32_t pk[32];  // 64 scores -> 32 packed columns of P
-#pragma unroll
-        for (int cc = 0; cc < 2; ++cc) {
-#pragma unroll
-          for (int i = 0; i < 32; i += 2) {
-            const uint64_t x2 = fma2(pack2(s[cc][i], s[cc][i + 1]), c2, nm2);
-            uint64_t p2;
-            // kPolyPairs of every 4 pairs go through the FMA pipe instead of the MUFU unit
-            if (((i >> 1) & 3) < T::kPolyPairs) {
-              p2 = poly_exp2_pair(x2);
-            } else {
-              uint32_t x0, x1;
-              unpack2(x2, x0, x1);
-              p2 = pack2f(fast_exp2(__uint_as_float(x0)), fast_exp2(__uint_as_float(x1)));
-            }
-            if (i & 2) lb = add2(lb, p2); else la = add2(la, p2);
-            uint32_t p0, p1;
-            unpack2(p2, p0, p1);
-            pk[cc * 16 + (i >> 1)] = pack16x2<kBf16>(__uint_as_float(p0), __uint_as_float(p1));
-          }
-        }
-        if (!(FMHA_ABLATE & 4)) tmem_st32(tSb, pk);
-        {
-          uint32_t a0, a1;
-          unpack2(add2(la, lb), a0, a1);
-          l += __uint_as_float(a0) + __uint_as_float(a1);
-        }
-        if (tl) FMHA_TL(t, tl_base + hs, 4);
-        tmem_wait_st();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&bar_p_full[t][buf]));
-        if (tl) FMHA_TL(t, tl_base + hs, 5);
+    for (;;) {
+      const FwdItem it = take_item();
+      const int n = t == 0 ? it.n0 : it.n1;
+      float m_ref = -CUDART_INF_F;  // reference score of the running softmax (raw, unscaled)
+      float neg_mc = 0.f;           // -m_ref * c, 0 while there is no reference
+      float l = 0.f;                // running sum of exp2((s - m_ref) * c)
+      int lim;                      // last visible column of this row in the round
+      {
+        const int row = it.q0 + t * T::kBlockM + row_in_tile;
+        long long last_key = p.causal ? (long long)row + p.causal_shift : (long long)it.sk - 1;
+        last_key = min(last_key, (long long)it.sk - 1);
+        if (row >= it.sq) last_key = -1;  // a padding row sees nothing: O = 0, LSE = -inf
+        lim = (int)max(last_key, -1ll) - it.kv_first * T::kBlockN;
       }
-      if (tl) FMHA_TL(t, tl_base + 31, 6);
 
-      // ---- epilogue: O_t / l -> fp16 registers (tensor memory released) -> staging box -> TMA
-      //      store; LSE
-      if (tile_valid) {
-        uint32_t oh[D / 2];  // the output row, fp16 pairs
-        if (n > 0) {
-          mbar_wait(smem_u32(&bar_o_full[t]), o_cnt & 1, &abort_word, 10);
-          ++o_cnt;
+      for (int j = 0; j < n || j == 0; ++j, lim -= T::kBlockN) {
+        if (j < n) {
+          // on a time-out keep going: every later wait returns at once, and all 128 threads of
+          // the group still meet at the named barriers of the epilogue
+          mbar_wait(smem_u32(&bar_s_full[t]), phase_s, &abort_word, 9);
+          phase_s ^= 1u;
           tc_fence_after();
-          if (tl) FMHA_TL(t, tl_base + 31, 8);
-          const float inv_l = (l > 0.f) ? 1.f / l : 0.f;
-          uint32_t o[D / 32][32];
+          uint32_t s[4][32];
+#pragma unroll
+          for (int cc = 0; cc < 4; ++cc) tmem_ld32(tS + cc * 32, s[cc]);
+          tmem_wait_ld();
+          if (lim < T::kBlockN - 1) {
+#pragma unroll
+            for (int cc = 0; cc < 4; ++cc)
+#pragma unroll
+              for (int i = 0; i < 32; ++i)
+                if (cc * 32 + i > lim) s[cc][i] = __float_as_uint(-CUDART_INF_F);
+          }
+          // P of 64 keys -> tensor memory.  The reference m_ref stays what it was unless an exponential
+          // comes out too large; what tells is their sum, which the row sum needs anyway, so that
+          // in the ordinary case no maximum is looked for at all.  (The first round has to look: it
+          // has no reference yet.)
+          auto half_round = [&](auto half_tag) {
+            constexpr int half = decltype(half_tag)::value;
+            const uint64_t c2 = pack2f(c, c), nm2 = pack2f(neg_mc, neg_mc);
+            uint64_t la = pack2f(0.f, 0.f), lb = pack2f(0.f, 0.f);
+            uint32_t pk[32];
+#pragma unroll
+            for (int ch = 0; ch < 2; ++ch) {
+              const int cc = half * 2 + ch;
+#pragma unroll
+              for (int i = 0; i < 32; i += 2) {
+                const uint64_t x2 = fma2(pack2(s[cc][i], s[cc][i + 1]), c2, nm2);
+                uint64_t p2;
+                // kPolyPairs of every 8 pairs go through the FMA pipe instead of the MUFU unit
+                if (((i >> 1) & 7) < T::kPolyPairs) {
+                  p2 = poly_exp2_pair(x2);
+                } else {
+                  uint32_t x0, x1;
+                  unpack2(x2, x0, x1);
+                  p2 = pack2f(fast_exp2(__uint_as_float(x0)), fast_exp2(__uint_as_float(x1)));
+                }
+                if (i & 2) lb = add2(lb, p2); else la = add2(la, p2);
+                uint32_t p0, p1;
+                unpack2(p2, p0, p1);
+                pk[ch * 16 + (i >> 1)] = pack16x2<kBf16>(__uint_as_float(p0), __uint_as_float(p1));
+              }
+            }
+            uint32_t a0, a1;
+            unpack2(add2(la, lb), a0, a1);
+            float sum = __uint_as_float(a0) + __uint_as_float(a1);
+            // (a row that has not seen anything yet has no reference to compare with)
+            const bool need = !(sum <= kRescaleSum) || (m_ref == -CUDART_INF_F && lim >= half * 64);
+            if (!__any_sync(0xffffffffu, need)) {
+              tmem_st32(tS + half * 32, pk);
+            } else {
+              // Rare: a new reference.  The scores of this half are still in tensor memory (P of the
+              // half goes where columns before the ones read next were).
+              // O_t += of the keys before is complete: that of the previous round because its MMAs
+              // precede S_t(j), that of keys 0-63 of this round by a commit of its own.  The next
+              // one is not issued before this warp has arrived on p_full.
+              float m_new = m_ref;
+#pragma unroll 1
+              for (int ch = 0; ch < 2; ++ch) {
+                uint32_t x[32];
+                tmem_ld32(tS + half * 64 + ch * 32, x);
+                tmem_wait_ld();
+#pragma unroll
+                for (int i = 0; i < 32; ++i)
+                  if (half * 64 + ch * 32 + i <= lim) m_new = fmaxf(m_new, __uint_as_float(x[i]));
+              }
+              if (half == 1) mbar_wait(smem_u32(&bar_pv_half[t]), phase_s ^ 1u, &abort_word, 11);
+              if (half == 1 || j > 0) {
+                tc_fence_after();
+                const float alpha = isinf(m_new) ? 1.f : fast_exp2((m_ref - m_new) * c);
+                l *= alpha;
+#pragma unroll 1
+                for (int cc = 0; cc < D / 16; ++cc) {
+                  uint32_t o[16];
+                  tmem_ld16(tO + cc * 16, o);
+                  tmem_wait_ld();
+#pragma unroll
+                  for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+                  tmem_st16(tO + cc * 16, o);
+                }
+              }
+              m_ref = m_new;
+              neg_mc = isinf(m_ref) ? 0.f : -m_ref * c;
+              sum = 0.f;
+#pragma unroll 1
+              for (int ch = 0; ch < 2; ++ch) {
+                uint32_t x[32], h[16];
+                tmem_ld32(tS + half * 64 + ch * 32, x);
+                tmem_wait_ld();
+#pragma unroll
+                for (int i = 0; i < 32; i += 2) {
+                  const int col = half * 64 + ch * 32 + i;
+                  const float e0 = col <= lim ? fast_exp2(fmaf(__uint_as_float(x[i]), c, neg_mc)) : 0.f;
+                  const float e1 = col + 1 <= lim ? fast_exp2(fmaf(__uint_as_float(x[i + 1]), c, neg_mc)) : 0.f;
+                  sum += e0 + e1;
+                  h[i >> 1] = pack16x2<kBf16>(e0, e1);
+                }
+                tmem_st16(tS + half * 32 + ch * 16, h);
+              }
+            }
+            l += sum;
+            tmem_wait_st();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&bar_p_full[t][half]));
+          };
+          if (j == 0) {
+            float mx[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              mx[k] = fmaxf(__uint_as_float(s[k >> 1][(k & 1) * 16]), __uint_as_float(s[k >> 1][(k & 1) * 16 + 1]));
+#pragma unroll
+              for (int i = 2; i < 16; i += 2)
+                mx[k] = max3(mx[k], __uint_as_float(s[k >> 1][(k & 1) * 16 + i]),
+                             __uint_as_float(s[k >> 1][(k & 1) * 16 + i + 1]));
+            }
+            m_ref = fmaxf(max3(mx[0], mx[1], mx[2]), mx[3]);
+            neg_mc = isinf(m_ref) ? 0.f : -m_ref * c;
+          }
+          half_round(std::integral_constant<int, 0>{});
+          half_round(std::integral_constant<int, 1>{});
+        }
+
+        if (j > 0 || !pending) continue;
+        // ---- epilogue of the item before: O_t / l -> registers (tensor memory released) -> 16 bit ->
+        //      staging box -> TMA store; LSE.  A chunk of a query block leaves fp32 rows instead.
+        pending = false;
+        const int row = done.q0 + t * T::kBlockM + row_in_tile;
+        const int nd = t == 0 ? done.n0 : done.n1;
+        const bool split = done.chunk >= 0;
+        const float inv_l = (done_l > 0.f) ? 1.f / done_l : 0.f;
+        if (row < p.seqlen_q) {
+          const float lse =
+              (done_l > 0.f) ? (done_m * c + log2f(done_l)) * 0.6931471805599453f : -CUDART_INF_F;
+          const size_t stat = (size_t)done.zh * p.seqlen_q + row;
+          if (split) p.lse_part[(size_t)done.chunk * p.num_heads_total * p.seqlen_q + stat] = lse;
+          else p.lse[stat] = lse;
+        }
+        if (nd > 0) {
+          mbar_wait(smem_u32(&bar_o_full[t]), phase_o, &abort_word, 10);
+          phase_o ^= 1u;
+          tc_fence_after();
+        }
+        if (split) {
+          if (nd == 0) continue;  // LSE = -inf: the combine kernel reads no row
+          float* dst = p.o_part + (((size_t)done.chunk * p.num_heads_total + done.zh) * p.seqlen_q + row) * p.row_elems;
+#pragma unroll 1
+          for (int cc = 0; cc < D / 16; ++cc) {
+            uint32_t o[16];
+            tmem_ld16(tO + cc * 16, o);
+            tmem_wait_ld();
+            if (row < p.seqlen_q && cc * 16 < p.row_elems) {
+#pragma unroll
+              for (int i = 0; i < 16; i += 4)
+                *reinterpret_cast<float4*>(dst + cc * 16 + i) =
+                    make_float4(__uint_as_float(o[i]) * inv_l, __uint_as_float(o[i + 1]) * inv_l,
+                                __uint_as_float(o[i + 2]) * inv_l, __uint_as_float(o[i + 3]) * inv_l);
+            }
+          }
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(smem_u32(&bar_o_read[t]));
+          continue;
+        }
+        uint32_t o[D / 32][32];
+        if (nd > 0) {
 #pragma unroll
           for (int cc = 0; cc < D / 32; ++cc) tmem_ld32(tO + cc * 32, o[cc]);
           tmem_wait_ld();
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(smem_u32(&bar_o_read[t]));
-          if (tl) FMHA_TL(t, tl_base + 31, 9);
+        } else {
 #pragma unroll
           for (int cc = 0; cc < D / 32; ++cc)
 #pragma unroll
-            for (int i = 0; i < 32; i += 2)
-              oh[cc * 16 + (i >> 1)] = pack16x2<kBf16>(__uint_as_float(o[cc][i]) * inv_l,
-                                                       __uint_as_float(o[cc][i + 1]) * inv_l);
-        } else {
-#pragma unroll
-          for (int i = 0; i < D / 2; ++i) oh[i] = 0u;
+            for (int i = 0; i < 32; ++i) o[cc][i] = 0u;
         }
-        if (row < p.seqlen_q) {
-          const float lse =
-              (l > 0.f) ? (m_ref * c + log2f(l)) * 0.6931471805599453f : -CUDART_INF_F;
-          p.lse[((size_t)z * p.heads + h) * p.seqlen_q + row] = lse;
-        }
-        // through this group's staging tile and TMA stores (per-thread stores of whole rows are
-        // uncoalesced and clog the load/store pipe for everybody)
-        if (row_in_tile == 0 && stored) tma_wait_group_read<0>();  // previous item's store
-        named_bar_sync(1 + t, 128);
+        // through this group's staging box and TMA stores, 64 columns at a time (per-thread stores of
+        // whole rows are uncoalesced and clog the load/store pipe for everybody)
 #pragma unroll
-        for (int ch = 0; ch < D / 8; ++ch)  // 16-byte chunk (8 fp16) of this row
-          sts128(o_stage + (ch >> 3) * T::kBoxBytes + row_in_tile * 128 +
-                     (((ch & 7) ^ (row_in_tile & 7)) << 4),
-                 oh[ch * 4 + 0], oh[ch * 4 + 1], oh[ch * 4 + 2], oh[ch * 4 + 3]);
-        fence_proxy_async_smem();
-        named_bar_sync(1 + t, 128);
-        if (row_in_tile == 0) {
+        for (int b = 0; b < T::kBoxes; ++b) {
+          if (row_in_tile == 0 && stored) tma_wait_group_read<0>();  // the box's last store has been read
+          named_bar_sync(1 + t, 128);
 #pragma unroll
-          for (int b = 0; b < T::kBoxes; ++b)
-            tma_store_4d(&tm_o, o_stage + b * T::kBoxBytes, b * 64, q0 + t * T::kBlockM, h, z);
-          tma_commit_group();
+          for (int ch = 0; ch < 8; ++ch) {  // 16-byte chunk (8 fp16) of this row
+            const uint32_t* w = &o[b * 2 + (ch >> 2)][(ch & 3) * 8];
+            uint32_t h4[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+              h4[i] = pack16x2<kBf16>(__uint_as_float(w[2 * i]) * inv_l, __uint_as_float(w[2 * i + 1]) * inv_l);
+            sts128(o_stage + row_in_tile * 128 + ((ch ^ (row_in_tile & 7)) << 4), h4[0], h4[1], h4[2], h4[3]);
+          }
+          fence_proxy_async_smem();
+          named_bar_sync(1 + t, 128);
+          if (row_in_tile == 0) {
+            tma_store_4d(&tm_o, o_stage, b * 64, done.q0 + t * T::kBlockM, done.h, done.z);
+            tma_commit_group();
+          }
+          stored = true;
         }
-        stored = true;
       }
-      if (tl) FMHA_TL(t, tl_base + 31, 7);
-      tl_base += 64;
+      if (it.id < 0) break;
+      pending = it.q0 + t * T::kBlockM < p.seqlen_q;
+      done = it;
+      done_m = m_ref;
+      done_l = l;
     }
     if (row_in_tile == 0) tma_wait_group<0>();
   }
@@ -714,6 +795,50 @@ __global__ void __launch_bounds__(384, 1)
   if (warp == 9) {
     tc_fence_after();
     tmem_dealloc(tmem_base, T::kTmemCols);
+  }
+}
+
+// Joins the chunks of the query blocks that were cut: one warp per row, rows from row_begin on.
+// Every partial row is normalised; its weight is exp(lse_part - lse).
+template <typename E>
+__global__ void __launch_bounds__(256)
+    fmha_fwd_combine_kernel(const FwdKernelParams p, E* __restrict__ o, long long so_batch, long long so_row,
+                            long long so_head, int row_begin, long long total_rows) {
+  const long long idx = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (idx >= total_rows) return;
+  const int lane = threadIdx.x & 31;
+  const int rows = p.seqlen_q - row_begin;
+  const int zh = (int)(idx / rows), row = row_begin + (int)(idx % rows);
+  const int chunks = fwd_chunks(p.causal != 0, p.causal_shift, row / 256, p.seqlen_q, (p.seqlen_k + 127) / 128,
+                                p.chunk_tiles);
+  if (chunks <= 1) return;
+  const size_t stat = (size_t)zh * p.seqlen_q + row, plane = (size_t)p.num_heads_total * p.seqlen_q;
+  float mx = -CUDART_INF_F;
+  for (int c = lane; c < chunks; c += 32) mx = fmaxf(mx, p.lse_part[c * plane + stat]);
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+  const float base = mx > -CUDART_INF_F ? mx : 0.f;
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  float sum = 0.f;
+  const int col = lane * 4;
+  for (int c = 0; c < chunks; ++c) {
+    const float lp = p.lse_part[c * plane + stat];
+    if (lp == -CUDART_INF_F) continue;  // nothing visible in this chunk: its row was not written
+    const float w = expf(lp - base);
+    sum += w;
+    if (col < p.row_elems) {
+      const float4 v = *reinterpret_cast<const float4*>(p.o_part + (c * plane + stat) * p.row_elems + col);
+      acc.x += w * v.x, acc.y += w * v.y, acc.z += w * v.z, acc.w += w * v.w;
+    }
+  }
+  const float inv = sum > 0.f ? 1.f / sum : 0.f;
+  if (lane == 0) p.lse[stat] = sum > 0.f ? base + logf(sum) : -CUDART_INF_F;
+  if (col < p.row_elems) {
+    constexpr bool kBf16 = std::is_same<E, __nv_bfloat16>::value;
+    uint2 v;
+    v.x = pack16x2<kBf16>(acc.x * inv, acc.y * inv);
+    v.y = pack16x2<kBf16>(acc.z * inv, acc.w * inv);
+    *reinterpret_cast<uint2*>(o + (zh / p.heads) * so_batch + row * so_row + (zh % p.heads) * so_head + col) = v;
   }
 }
 

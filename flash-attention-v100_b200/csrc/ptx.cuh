@@ -88,14 +88,16 @@ constexpr uint32_t kWaitPollLimit = 1u << 22;
 
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_word,
                                           int who) {
-  if (mbar_try_wait(bar, parity)) return true;
-  if (*abort_word != 0) return false;  // some wait already gave up: drain without polling
-  for (uint32_t i = 0; i < kWaitPollLimit; ++i) {
-    if (mbar_try_wait(bar, parity)) return true;
-    if ((i & 255u) == 255u && *abort_word != 0) return false;
+  // kept to a handful of instructions: there are dozens of waits in a kernel, and the instruction
+  // cache is what the roles of a CTA share
+  for (uint32_t i = 0; !mbar_try_wait(bar, parity); ++i) {
+    if (*abort_word != 0) return false;  // some wait already gave up: drain without polling
+    if (i == kWaitPollLimit) {
+      *abort_word = kErrWaitTimeout | (who & 0xff);
+      return false;
+    }
   }
-  atomicCAS(const_cast<int*>(abort_word), 0, kErrWaitTimeout | (who & 0xff));
-  return false;
+  return true;
 }
 
 // Bounded wait for a word in global memory to reach `want`; another CTA of the same grid with a
@@ -244,7 +246,27 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32
         "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
       : "memory");
 }
-
+// 16 columns
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+        "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+      :
+      : "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]),
+        "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]),
+        "r"(r[14]), "r"(r[15])
+      : "memory");
+}
 
 // ---------------------------------------------------------------------------------
 // UMMA descriptors (16-bit operands, fp32 accumulate, dense, cta_group::1, M = 128)
@@ -256,6 +278,8 @@ __host__ __device__ constexpr uint32_t umma_idesc_f16(int m, int n, int a_mn_maj
   return (1u << 4) | (uint32_t(bf16) << 7) | (uint32_t(bf16) << 10) | (uint32_t(a_mn_major) << 15) |
          (uint32_t(b_mn_major) << 16) | (uint32_t(n >> 3) << 17) | (uint32_t(m >> 4) << 24);
 }
+
+constexpr uint32_t kIdescNegateA = 1u << 13;  // the product is formed with -A
 
 // Shared-memory matrix descriptor, 128-byte swizzle.  Bits: [0,14) address >> 4;
 // [16,30) leading byte offset >> 4; [32,46) stride byte offset >> 4; [46,48) version = 1;
@@ -301,9 +325,9 @@ __device__ __forceinline__ void umma_ss(uint32_t d_tmem, uint32_t a_lo, uint32_t
       "mov.b64 da, {%1, %3};\n\t"
       "mov.b64 db, {%2, %3};\n\t"
       "setp.ne.b32 p, %5, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, {%6, %6, %6, %6}, p;\n\t}"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, p;\n\t}"
       :
-      : "r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(kDescHi), "r"(idesc), "r"(accumulate), "r"(0u)
+      : "r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(kDescHi), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 // D[tmem] (+)= A[tmem] * B[smem]   (A: 128 lanes x K fp16, two per 32-bit column)
@@ -313,9 +337,9 @@ __device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint32
       "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\t"
       "mov.b64 db, {%2, %3};\n\t"
       "setp.ne.b32 p, %5, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, {%6, %6, %6, %6}, p;\n\t}"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}"
       :
-      : "r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(kDescHi), "r"(idesc), "r"(accumulate), "r"(0u)
+      : "r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(kDescHi), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 
@@ -342,30 +366,51 @@ __device__ __forceinline__ void umma_ts_elect(uint32_t d_tmem, uint32_t a_tmem, 
 __device__ __forceinline__ void umma_commit_elect(uint32_t bar) {
   if (elect_one()) umma_commit(bar);
 }
-// Three barriers tested with the three probes in flight together: a probe that finds its phase
-// complete still costs a round trip through the shared-memory pipe, and three in a row cost
-// three.  Returns true when all three phases are complete.
-__device__ __forceinline__ bool mbar_try_wait3(uint32_t bar0, uint32_t par0, uint32_t bar1,
-                                               uint32_t par1, uint32_t bar2, uint32_t par2) {
-  uint32_t r0, r1, r2;
+// has the phase completed?  A single test by a whole converged warp, without waiting.
+__device__ __forceinline__ bool mbar_probe_warp(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
   asm volatile(
-      "{\n\t.reg .pred p0, p1, p2;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p0, [%3], %4;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p1, [%5], %6;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p2, [%7], %8;\n\t"
-      "selp.u32 %0, 1, 0, p0;\n\t"
-      "selp.u32 %1, 1, 0, p1;\n\t"
-      "selp.u32 %2, 1, 0, p2;\n\t}"
-      : "=r"(r0), "=r"(r1), "=r"(r2)
-      : "r"(bar0), "r"(par0), "r"(bar1), "r"(par1), "r"(bar2), "r"(par2)
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
       : "memory");
-  return (r0 & r1 & r2) != 0;
+  return __all_sync(0xffffffffu, ok != 0);
 }
 // bounded wait by a whole converged warp, with a warp-uniform result
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity,
                                                volatile int* abort_word, int who) {
   const bool ok = mbar_wait(bar, parity, abort_word, who);
   return __all_sync(0xffffffffu, ok);
+}
+
+// ---------------------------------------------------------------------------------
+// cluster launch control: a running CTA takes over the block index of one that has not started.
+// The answer (16 bytes) lands in shared memory and completes 16 bytes on the mbarrier.  No
+// request may follow one that was answered "nothing left".
+// ---------------------------------------------------------------------------------
+__device__ __forceinline__ void clc_request(uint32_t answer_smem, uint32_t bar) {
+  asm volatile(
+      "clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(
+          answer_smem),
+      "r"(bar)
+      : "memory");
+}
+// block index (x) taken over, or -1 when no block was left
+__device__ __forceinline__ int clc_answer(uint32_t answer_smem) {
+  uint32_t got, x;
+  asm volatile(
+      "{\n\t.reg .b128 h;\n\t.reg .pred p;\n\t.reg .b32 y, z, w;\n\t"
+      "ld.shared.b128 h, [%2];\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, h;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t"
+      "mov.u32 %1, 0;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid.v4.b32.b128 {%1, y, z, w}, h;\n\t}"
+      : "=r"(got), "=r"(x)
+      : "r"(answer_smem)
+      : "memory");
+  return got ? (int)x : -1;
 }
 
 // warpgroup-wide register re-budgeting: every warp of an aligned group of 4 warps executes it
@@ -434,21 +479,22 @@ __device__ __forceinline__ float min3(float a, float b, float c) {
   return d;
 }
 // exp2 on the FMA / ALU pipes (no MUFU): x = n + f with n = floor(x) from a round-down add of
-// 1.5 * 2^23, 2^f by a cubic (relative error 7.5e-5, far below the fp16 rounding P gets anyway),
-// 2^n by adding n into the exponent field.  An option of the forward kernel (FMHA_FWD_POLY_PAIRS) for a
-// fraction of the softmax exponentials, off by default.  x is clamped to >= -126
-// (masked -inf scores give 2^-126, which rounds to 0 in fp16).
+// 1.5 * 2^23, 2^f on [0, 1) by the degree-4 polynomial with constant term 1 of least maximal
+// relative error (2.9e-6, found by iterated weighted least squares; an order of magnitude below
+// the fp16 rounding that P gets anyway), 2^n by adding n into the exponent field.  x is clamped to
+// >= -127, where the result is exactly 0 (a masked -inf score).
 // Works on a packed pair; the result is the packed pair of 2^x.
 __device__ __forceinline__ uint64_t poly_exp2_pair(uint64_t x2) {
   uint32_t x0, x1;
   unpack2(x2, x0, x1);
-  x2 = pack2f(fmaxf(__uint_as_float(x0), -126.f), fmaxf(__uint_as_float(x1), -126.f));
+  x2 = pack2f(fmaxf(__uint_as_float(x0), -127.f), fmaxf(__uint_as_float(x1), -127.f));
   const uint64_t magic = pack2f(12582912.f, 12582912.f);
   const uint64_t t2 = add2_rm(x2, magic);
   const uint64_t f2 = sub2(x2, sub2(t2, magic));
-  uint64_t p2 = fma2(f2, pack2f(0.0780244917f, 0.0780244917f), pack2f(0.2260672003f, 0.2260672003f));
-  p2 = fma2(p2, f2, pack2f(0.6958335042f, 0.6958335042f));
-  p2 = fma2(p2, f2, pack2f(0.9999251962f, 0.9999251962f));
+  uint64_t p2 = fma2(f2, pack2f(0.0134266876f, 0.0134266876f), pack2f(0.0522424690f, 0.0522424690f));
+  p2 = fma2(p2, f2, pack2f(0.241280213f, 0.241280213f));
+  p2 = fma2(p2, f2, pack2f(0.693044841f, 0.693044841f));
+  p2 = fma2(p2, f2, pack2f(1.f, 1.f));
   uint32_t p0, p1, t0, t1;
   unpack2(p2, p0, p1);
   unpack2(t2, t0, t1);

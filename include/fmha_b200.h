@@ -104,6 +104,11 @@ typedef struct {
    * the contract "the caller pads" (README.md:3) and computes the padding like real rows. */
   const int32_t* seqused_q;
   const int32_t* seqused_k;
+  /* Optional device scratch of fmha_fwd_workspace_bytes bytes, 16-byte aligned.  With it, a call whose
+   * query blocks alone would leave SMs idle (few queries over a long context) cuts their KV
+   * ranges into chunks and joins the partial results; without it such a call runs uncut. */
+  void* workspace;
+  size_t workspace_bytes;
 } FmhaFwdParams;
 
 typedef struct {
@@ -175,6 +180,7 @@ typedef struct {
 
 /* Forward: O = softmax(scale * Q K^T [+ causal mask]) V and LSE.
  * Replaces fused_mha_forward (include/fused_mha.h:1-2, kernel/fused_mha_kernel.cu:891-902). */
+size_t fmha_fwd_workspace_bytes(const FmhaFwdParams* p); /* 0 where a workspace would not be used */
 int fmha_fwd(const FmhaFwdParams* p, void* stream);
 
 /* Bytes of device workspace the backward needs for these sizes: an fp32 dQ accumulator
