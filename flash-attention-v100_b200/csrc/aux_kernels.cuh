@@ -66,23 +66,27 @@ __global__ void __launch_bounds__(256)
     fmha_bwd_preprocess_kernel(const E* __restrict__ o, Strides3 so,
                                const E* __restrict__ dout, Strides3 sdo,
                                const float* __restrict__ lse, float* __restrict__ dq_accum,
-                               float* __restrict__ lse2, float* __restrict__ delta, int heads,
+                               float* __restrict__ neg_lse2, void* __restrict__ neg_delta, int heads,
                                int seqlen_q, int seqlen_q_pad, long long total_rows,
                                const int* __restrict__ seqused_q) {
   constexpr int kGroup = D / 8;  // threads per row
   constexpr int kRowsPerBlock = 256 / kGroup;
   const int part = threadIdx.x % kGroup;
   const long long row_id = (long long)blockIdx.x * kRowsPerBlock + threadIdx.x / kGroup;
+  // the statistics in the form the backward kernel's inner loop adds them: negated, and delta in the
+  // precision it is used in (fp16 pairs with fp16 tensors)
+  auto put = [&](float l2, float dl) {
+    neg_lse2[row_id] = -l2;
+    if constexpr (std::is_same<E, __nv_bfloat16>::value) static_cast<float*>(neg_delta)[row_id] = -dl;
+    else static_cast<__half*>(neg_delta)[row_id] = __float2half_rn(-dl);
+  };
   if (row_id >= total_rows) return;  // whole groups leave together (256 % kGroup == 0)
   const long long zh = row_id / seqlen_q_pad;
   const int q = (int)(row_id % seqlen_q_pad);
   const int z = (int)(zh / heads);
   const int h = (int)(zh % heads);
   if (q >= seqlen_q) {
-    if (part == 0) {
-      lse2[row_id] = CUDART_INF_F;
-      delta[row_id] = 0.f;
-    }
+    if (part == 0) put(CUDART_INF_F, 0.f);
     return;
   }
   // a padding row of a right-padded batch: P = exp2(s - inf) = 0 for it, it adds nothing to any
@@ -104,8 +108,7 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
   for (int off = kGroup / 2; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
   if (part == 0) {
-    delta[row_id] = padding ? 0.f : acc;
-    lse2[row_id] = padding ? CUDART_INF_F : lse[zh * seqlen_q + q] * 1.4426950408889634f;
+    put(padding ? CUDART_INF_F : lse[zh * seqlen_q + q] * 1.4426950408889634f, padding ? 0.f : acc);
   }
   if (dq_accum != nullptr && mine) {
     float4* dst = reinterpret_cast<float4*>(

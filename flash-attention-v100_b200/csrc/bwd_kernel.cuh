@@ -5,8 +5,10 @@
 // dS = P o (dP - D) * scale,  dQ = dS K,  dK = dS^T Q  (kernel/fused_mha_kernel.cu:453-458,
 // 503-506), with dQ accumulated in fp32 instead of the reference's fp16 atomics (:543,693).
 //
-// One CTA owns one 128-row KV tile of one (batch, head) and walks the query tiles (128 rows)
-// that can see it.  Everything is computed TRANSPOSED so that the KV rows sit on the 128
+// A work item is one 128-row KV tile of one (batch, head) and the query tiles (128 rows) that can
+// see it.  A CTA stays on its SM and takes item after item (cluster launch control); the first S^T
+// and P^T of an item run beside the last dS^T, dQ and dK of the one before.  Everything is computed
+// TRANSPOSED so that the KV rows sit on the 128
 // tensor-memory lanes, which lets P^T feed the dV MMA straight from tensor memory:
 //
 //   S^T  = K  Q_i^T    (A = K  smem K-major,  B = Q_i  smem K-major)      -> TMEM [0,128)
@@ -23,24 +25,37 @@
 //   warps 8-11      dQ group: one thread per query row; tensor memory -> registers ->
 //                   shared-memory staging -> TMA reduce-add into the fp32 dQ accumulator
 //                   (bulk async adds: no per-thread atomics in the load/store pipeline)
-//   warp 12         TMA producer (K, V once; Q_i through a 2-stage ring, dO_i single stage)
+//   warp 12         TMA producer (K, V once; Q_i through a 2-stage ring, dO_i single stage) and
+//                   source of the items
 //   warp 13         MMA issuer: the whole warp runs the loop, one elected lane issues
 //
-// The per-row statistics come from the workspace the preprocess kernel fills:
-// lse2 = lse * log2(e) (+inf on padding rows) and delta = rowsum(dO o O) (0 on padding rows),
-// both padded to a multiple of 128 rows per (batch, head); a tile's 2 x 128 values are staged
-// through shared memory once instead of being re-read by every thread.
+// The per-row statistics come from the workspace the preprocess kernel fills, negated (they are
+// added): lse2 = lse * log2(e) (+inf on padding rows) and delta = rowsum(dO o O) (0 on padding rows),
+// both padded to a multiple of 128 rows per (batch, head); a tile's 2 x 128 values come in with Q_i.
+//
+// What bounds it: per query tile 2560 clk of MMA at D = 128, in a period of about 4000, beside which
+// the roles compete for shared memory (MMA operands, dQ staging, statistics) and for the
+// instruction cache.  The latter decides more than it seems: the same kernel with its MMA loops and
+// write-outs unrolled fetched 1.7 times the instructions from behind the first-level cache
+// and ran 10-18 % SLOWER than one CTA per item did, rolled up it is faster.  Hence the loops below.
+// One CTA per item spent about 7 us of its life on its head and tail (a causal item at N = 2048 has
+// 8.5 tiles of 2.2 us).  Whole backward, one CTA per item -> this, steady state: Z8 H32 N2048 D128
+// causal 1025 -> 955 us, without a mask 1665 -> 1570, Z64 H16 N512 D64 422 -> 385, Z1 H16 N16384
+// causal 2870 -> 2740.
 #pragma once
 #include <cuda.h>
 #include <math_constants.h>
 
+#include <type_traits>
+
+#include "aux_kernels.cuh"
 #include "ptx.cuh"
 
 namespace fmha {
 
 struct BwdKernelParams {
-  const float* lse2;    // fp32 (Z*H, seqlen_q_pad)
-  const float* delta;   // fp32 (Z*H, seqlen_q_pad)
+  const float* neg_lse2;  // fp32 (Z*H, seqlen_q_pad)
+  const void* neg_delta;  // (Z*H, seqlen_q_pad): fp32 with bf16 tensors, else fp16
   float* dk_accum;      // optional fp32 (Z, seqlen_k, H, D) contiguous
   float* dv_accum;      // optional
   long long accum_batch_stride;  // elements between batch entries of dk_accum / dv_accum
@@ -50,6 +65,9 @@ struct BwdKernelParams {
   int num_heads_total;  // batch * heads
   int head_group;       // heads whose CTAs are interleaved in the grid (>= 1)
   int q_tile_begin;     // query tiles before this one take no part (FmhaBwdParams.q_row_begin / 128)
+  int deal;             // 1: every block has the one item of its index; 0: cluster launch control
+  uint16_t *dk, *dv;    // 16-bit outputs (element strides), for KV tiles that no query sees
+  Strides3 dk_strides, dv_strides;
   float scale, scale_log2;
   int causal, causal_shift;
   int* status;
@@ -67,7 +85,7 @@ struct BwdKernelParams {
 };
 
 constexpr int kBwdRegsIssue = 80;     // warps 12-15
-constexpr int kBwdRegsCompute = 120;  // warps 0-7
+constexpr int kBwdRegsCompute = 128;  // warps 0-7
 constexpr int kBwdRegsDq = 128 + (128 - kBwdRegsIssue) + 2 * (128 - kBwdRegsCompute);  // warps 8-11
 static_assert(kBwdRegsIssue <= 128 && kBwdRegsCompute <= 128 && kBwdRegsDq >= 128,
               "setmaxnreg.dec must not raise and .inc must not lower the 128 registers of the launch");
@@ -79,19 +97,88 @@ struct BwdTraits {
   static constexpr int kBoxBytes = 128 * 128;
   static constexpr int kTileBytes = kBoxes * kBoxBytes;  // a 128 x D fp16 tile
   static constexpr int kDsBytes = 2 * kBoxBytes;         // dS^T: 128 x 128 fp16
-  static constexpr int kQStages = 2;
+  // Tile slots.  K, V and dO are in slots 0-2 and change places from item to item (see the kernel);
+  // slots 3 and 4 take the query tiles in turn.
+  static constexpr int kSlots = 5;
   static constexpr int kStageBytes = 2 * 16384;          // dQ staging: 2 x (128 rows x 32 fp32)
-  static constexpr int kStatBytes = 256 * 4;             // lse2[128] + delta[128] of one tile
+  // statistics of one query tile: -lse2[128] (fp32), -delta[128] (fp32 with bf16 tensors, else fp16)
+  static constexpr int kDeltaBytes = kBf16 ? 512 : 256;
+  static constexpr int kStatBytes = 512 + kDeltaBytes;
+  static constexpr int kItemStages = 4;                  // item ids published ahead
   static constexpr int kThreads = 512;  // 4 warpgroups; warps 14, 15 only take part in barriers
-  // K, V, Q x2, dO, dS^T, dQ staging, statistics
-  static constexpr int kSmemBytes =
-      1024 + (3 + kQStages) * kTileBytes + kDsBytes + kStageBytes + kStatBytes;
   static constexpr int kTmemCols = 512;
   static constexpr int kColS = 0, kColDP = 128, kColDQ = 128, kColDK = 256, kColDV = 256 + D;
+  // warps that read dK (and as many dV) out of tensor memory at the end of an item
+  static constexpr int kDrainWarps = (D == 128) ? 8 : 4;
   static constexpr uint32_t kIdescST = umma_idesc_f16(128, 128, 0, 0, kBf16);  // S^T, dP^T
   static constexpr uint32_t kIdescDV = umma_idesc_f16(128, D, 0, 1, kBf16);    // dV, dK
   static constexpr uint32_t kIdescDQ = umma_idesc_f16(128, D, 1, 1, kBf16);    // dQ
 };
+
+// A work item: one KV tile of one (batch, head) and the query tiles that see it.  The producer warp
+// works it out and publishes it in shared memory.
+struct __align__(16) BwdItem {
+  int id;       // -1: no more items
+  int cnt;      // query tiles to walk (0: dK and dV of this KV tile are zeros)
+  int i_begin;  // the first of them
+  int kb;       // KV tile
+  int z, h, zh;
+  int sk;       // keys of the batch entry
+};
+
+// what the roles share beside the tiles, at the end of the dynamic shared memory
+template <int D, bool kBf16>
+struct __align__(16) BwdControl {
+  using T = BwdTraits<D, kBf16>;
+  uint8_t clc_word[16];  // the answer to the last request for an item
+  BwdItem items[T::kItemStages];
+  uint64_t bar_clc, bar_item_full[T::kItemStages], bar_item_empty[T::kItemStages];
+  uint64_t bar_full[T::kSlots], bar_empty[T::kSlots];  // per tile slot
+  uint64_t bar_s_full, bar_dp_full, bar_p_ready, bar_ds_ready, bar_dq_full, bar_dq_empty;
+  uint64_t bar_acc_full;               // dK and dV of an item are complete
+  uint64_t bar_dv_read, bar_dk_read;   // ... and have been read out of tensor memory
+  uint32_t tmem_base;
+  int abort_word;
+  int skip_cta;
+};
+
+template <int D, bool kBf16>
+constexpr int bwd_smem_bytes() {
+  using T = BwdTraits<D, kBf16>;
+  return T::kSlots * T::kTileBytes + T::kDsBytes + T::kStageBytes + 2 * T::kStatBytes +
+         (int)sizeof(BwdControl<D, kBf16>);
+}
+
+// Heads are taken in groups of head_group; within a group the items are ordered by KV tile first
+// (early KV tiles see the most query tiles under a causal mask and take longest), head second: the
+// items in work at any time still belong to a handful of heads (their Q / dO tiles and dQ
+// accumulators stay in L2), and what comes last, at the end of a group and of the grid, are the
+// short ones.  head_group = 1: all items of a head in a row.
+__device__ __forceinline__ BwdItem bwd_item(const BwdKernelParams& p, int id) {
+  BwdItem it;
+  it.id = id;
+  const int per_group = p.head_group * p.num_kv_blocks;
+  const int group = id / per_group, within = id % per_group;
+  const int heads_here = min(p.head_group, p.num_heads_total - group * p.head_group);
+  it.zh = group * p.head_group + within % heads_here;
+  it.kb = within / heads_here;
+  it.z = it.zh / p.heads;
+  it.h = it.zh % p.heads;
+  // the lengths that count for this batch entry: query tiles and keys beyond them are padding
+  const int sq = p.seqused_q == nullptr ? p.seqlen_q : max(0, min(p.seqlen_q, __ldg(p.seqused_q + it.z)));
+  it.sk = p.seqused_k == nullptr ? p.seqlen_k : max(0, min(p.seqlen_k, __ldg(p.seqused_k + it.z)));
+  const int nq_tiles = (sq + 127) / 128;
+  int i_begin = 0;
+  if (p.causal) {
+    // query row r sees key kv0 iff r + shift >= kv0
+    const long long first_row = (long long)it.kb * 128 - p.causal_shift;
+    i_begin = first_row <= 0 ? 0 : (int)min((long long)nq_tiles, first_row / 128);
+  }
+  it.i_begin = max(i_begin, p.q_tile_begin);
+  // a KV tile that is all padding walks no query tile
+  it.cnt = it.kb * 128 < it.sk ? max(0, nq_tiles - it.i_begin) : 0;
+  return it;
+}
 
 // DR <= D: elements per row of the tensors.  96 runs at D = 128: the tile loads fill columns
 // 96-127 with zeros, so those columns of dQ, dK and dV are zeros that are never written out, and
@@ -103,123 +190,106 @@ __global__ void __launch_bounds__(512, 1)
                     const __grid_constant__ CUtensorMap tm_dk, const __grid_constant__ CUtensorMap tm_dv,
                     const __grid_constant__ CUtensorMap tm_dqacc, const BwdKernelParams p) {
   using T = BwdTraits<D, kBf16>;
-  extern __shared__ uint8_t smem_raw[];
-  __shared__ uint64_t bar_kv_full;
-  __shared__ uint64_t bar_q_full[T::kQStages], bar_q_empty[T::kQStages];
-  __shared__ uint64_t bar_do_full, bar_do_empty;
-  __shared__ uint64_t bar_s_full, bar_dp_full, bar_p_ready, bar_ds_ready, bar_dq_full,
-      bar_dq_empty, bar_ds_free, bar_done;
-  __shared__ uint32_t tmem_base_slot;
-  __shared__ int abort_word;
-  __shared__ int skip_cta;
+  // (no static shared memory: the tiles need every byte, and 1024-byte alignment)
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  const uint32_t smem_base = smem_u32(smem_raw);
+  const uint32_t ds_smem = smem_base + T::kSlots * T::kTileBytes;   // dS^T, later dK / dV on their way out
+  const uint32_t stg_smem = ds_smem + T::kDsBytes;                  // dQ staging, 2 x 16 KB
+  const uint32_t stat_smem = stg_smem + T::kStageBytes;             // statistics, one block per query slot
+  auto& sh = *reinterpret_cast<BwdControl<D, kBf16>*>(smem_raw + T::kSlots * T::kTileBytes + T::kDsBytes +
+                                                      T::kStageBytes + 2 * T::kStatBytes);
+  volatile int* const abort_word = &sh.abort_word;
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);  // warp-uniform for the compiler, too
   const int lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
-    skip_cta = (p.status != nullptr && *reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
-    abort_word = 0;
+    sh.skip_cta = (p.status != nullptr && *reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
+    sh.abort_word = 0;
   }
   __syncthreads();
-  if (skip_cta) return;
+  if (sh.skip_cta) return;
 
-  const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  const uint32_t k_smem = smem_base;
-  const uint32_t v_smem = k_smem + T::kTileBytes;
-  const uint32_t q_smem = v_smem + T::kTileBytes;                   // kQStages tiles
-  const uint32_t do_smem = q_smem + T::kQStages * T::kTileBytes;    // one tile
-  const uint32_t ds_smem = do_smem + T::kTileBytes;                 // dS^T
-  const uint32_t stg_smem = ds_smem + T::kDsBytes;                  // dQ staging, 2 x 16 KB
-  const uint32_t stat_smem = stg_smem + T::kStageBytes;             // statistics
+  // one tile into its slot; a query tile brings its lse2 and delta along
+  auto send = [&](int slot, const CUtensorMap* tm, const BwdItem& it, int row, bool is_q) {
+    if (elect_one()) {
+      const uint32_t bar = smem_u32(&sh.bar_full[slot]);
+      mbar_arrive_expect_tx(bar, T::kTileBytes + (is_q ? T::kStatBytes : 0));
+#pragma unroll
+      for (int b = 0; b < T::kBoxes; ++b)
+        tma_load_4d(smem_base + slot * T::kTileBytes + b * T::kBoxBytes, tm, bar, b * 64, row, it.h, it.z);
+      if (is_q) {
+        const uint32_t st = stat_smem + (slot - 3) * T::kStatBytes;
+        const size_t at = (size_t)it.zh * p.seqlen_q_pad + row;
+        bulk_load(st, p.neg_lse2 + at, 512, bar);
+        bulk_load(st + 512, static_cast<const char*>(p.neg_delta) + at * (T::kDeltaBytes / 128), T::kDeltaBytes, bar);
+      }
+    }
+    __syncwarp();
+  };
 
-  // ---- coordinates.  Heads are taken in groups of head_group; within a group the CTAs are
-  // ordered by KV tile first (early KV tiles see the most query tiles under a causal mask and
-  // live longest), head second: the CTAs running at any time still belong to a handful of heads
-  // (their Q / dO tiles and dQ accumulators stay in L2), and what is dispatched last, at the end
-  // of a group and of the grid, are the short CTAs.  head_group = 1: all CTAs of a head in a row.
-  const int nkb = p.num_kv_blocks;
-  const int per_group = p.head_group * nkb;
-  const int group = blockIdx.x / per_group;
-  const int within = blockIdx.x % per_group;
-  const int heads_here = min(p.head_group, p.num_heads_total - group * p.head_group);
-  const int zh = group * p.head_group + within % heads_here;
-  const int kb = within / heads_here;
-  const int z = zh / p.heads;
-  const int h = zh % p.heads;
-  const int kv0 = kb * T::kBlock;
-
-  // the lengths that count for this batch entry: query tiles and keys beyond them are padding
-  const int sq = p.seqused_q == nullptr ? p.seqlen_q : max(0, min(p.seqlen_q, __ldg(p.seqused_q + z)));
-  const int sk = p.seqused_k == nullptr ? p.seqlen_k : max(0, min(p.seqlen_k, __ldg(p.seqused_k + z)));
-  const int nq_tiles = (sq + T::kBlock - 1) / T::kBlock;
-  int i_begin = 0;
-  if (p.causal) {
-    // query row r sees key kv0 iff r + shift >= kv0
-    const long long first_row = (long long)kv0 - p.causal_shift;
-    i_begin = first_row <= 0 ? 0 : (int)min((long long)nq_tiles, first_row / T::kBlock);
-  }
-  i_begin = max(i_begin, p.q_tile_begin);
-  // query tiles this CTA walks (may be 0; a KV tile that is all padding walks none)
-  const int cnt = kv0 < sk ? max(0, nq_tiles - i_begin) : 0;
-  // the n-th query tile this CTA visits
-  auto tile_of = [&](int n) { return i_begin + n; };
-
-  // The producer warp sets the barriers up itself and sends the loads of K, V and of the first
-  // Q / dO tile off at once, before the CTA-wide barrier below that waits for the tensor-memory
-  // allocation: the load latency at the head of a CTA runs beside the rest of the set-up.
+  // The producer warp sets the barriers up itself and sends the first tiles of its first item off at
+  // once, before the CTA-wide barrier below that waits for the tensor-memory allocation.
   if (warp == 12) {
     if (lane == 0) {
-      mbar_init(smem_u32(&bar_kv_full), 1);
-      for (int s = 0; s < T::kQStages; ++s) {
-        mbar_init(smem_u32(&bar_q_full[s]), 1);
-        mbar_init(smem_u32(&bar_q_empty[s]), 1);
+      mbar_init(smem_u32(&sh.bar_clc), 1);
+      for (int s = 0; s < T::kItemStages; ++s) {
+        mbar_init(smem_u32(&sh.bar_item_full[s]), 1);
+        mbar_init(smem_u32(&sh.bar_item_empty[s]), 13);  // MMA warp, four dQ warps, eight compute warps
       }
-      mbar_init(smem_u32(&bar_do_full), 1);
-      mbar_init(smem_u32(&bar_do_empty), 1);
-      mbar_init(smem_u32(&bar_s_full), 1);
-      mbar_init(smem_u32(&bar_dp_full), 1);
-      mbar_init(smem_u32(&bar_p_ready), 256);
-      mbar_init(smem_u32(&bar_ds_ready), 256);
-      mbar_init(smem_u32(&bar_dq_full), 1);
-      mbar_init(smem_u32(&bar_dq_empty), 128);
-      mbar_init(smem_u32(&bar_ds_free), 1);
-      mbar_init(smem_u32(&bar_done), 1);
+      for (int s = 0; s < T::kSlots; ++s) {
+        mbar_init(smem_u32(&sh.bar_full[s]), 1);
+        mbar_init(smem_u32(&sh.bar_empty[s]), 1);
+      }
+      mbar_init(smem_u32(&sh.bar_s_full), 1);
+      mbar_init(smem_u32(&sh.bar_dp_full), 1);
+      mbar_init(smem_u32(&sh.bar_p_ready), 8);  // one arrival per warp
+      mbar_init(smem_u32(&sh.bar_ds_ready), 8);
+      mbar_init(smem_u32(&sh.bar_dq_full), 1);
+      mbar_init(smem_u32(&sh.bar_dq_empty), 4);
+      mbar_init(smem_u32(&sh.bar_acc_full), 1);
+      mbar_init(smem_u32(&sh.bar_dv_read), T::kDrainWarps);
+      mbar_init(smem_u32(&sh.bar_dk_read), T::kDrainWarps);
       fence_barrier_init();
     }
     __syncwarp();
-    if (cnt > 0 && elect_one()) {
-      tma_prefetch_desc(&tm_q);
-      tma_prefetch_desc(&tm_k);
-      tma_prefetch_desc(&tm_v);
-      tma_prefetch_desc(&tm_do);
-      const uint32_t kvbar = smem_u32(&bar_kv_full);
-      mbar_arrive_expect_tx(kvbar, 2 * T::kTileBytes);
-      const uint32_t qbar = smem_u32(&bar_q_full[0]);
-      mbar_arrive_expect_tx(qbar, T::kTileBytes);
-      const uint32_t dbar = smem_u32(&bar_do_full);
-      mbar_arrive_expect_tx(dbar, T::kTileBytes);
-      const int row0 = tile_of(0) * T::kBlock;
-#pragma unroll
-      for (int b = 0; b < T::kBoxes; ++b) {
-        tma_load_4d(k_smem + b * T::kBoxBytes, &tm_k, kvbar, b * 64, kv0, h, z);
-        tma_load_4d(q_smem + b * T::kBoxBytes, &tm_q, qbar, b * 64, row0, h, z);
-      }
-#pragma unroll
-      for (int b = 0; b < T::kBoxes; ++b) {
-        tma_load_4d(v_smem + b * T::kBoxBytes, &tm_v, kvbar, b * 64, kv0, h, z);
-        tma_load_4d(do_smem + b * T::kBoxBytes, &tm_do, dbar, b * 64, row0, h, z);
-      }
+    const BwdItem it = bwd_item(p, blockIdx.x);
+    if (it.cnt > 0) {
+      const int row0 = it.i_begin * T::kBlock;
+      send(3, &tm_q, it, row0, true);
+      send(0, &tm_k, it, it.kb * T::kBlock, false);
+      send(1, &tm_v, it, it.kb * T::kBlock, false);
+      send(2, &tm_do, it, row0, false);
     }
-    __syncwarp();
   }
   if (warp == 13) {
-    tmem_alloc(smem_u32(&tmem_base_slot), T::kTmemCols);
+    tmem_alloc(smem_u32(&sh.tmem_base), T::kTmemCols);
     tmem_relinquish();
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = tmem_base_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, sh.tmem_base, 0);
+
+  // The next item published by the producer warp (every consuming warp keeps its own count); id = -1
+  // when there is none, and when a wait ran out.
+  uint32_t item_cnt = 0;
+  auto take_item = [&]() -> BwdItem {
+    const uint32_t s = item_cnt % T::kItemStages;
+    BwdItem it;
+    if (mbar_wait_warp(smem_u32(&sh.bar_item_full[s]), (item_cnt / T::kItemStages) & 1, abort_word, 16)) {
+      it = sh.items[s];
+      it.id = __shfl_sync(0xffffffffu, it.id, 0);  // warp-uniform for the compiler
+      it.cnt = __shfl_sync(0xffffffffu, it.cnt, 0);
+    } else {
+      it.id = -1;
+      it.cnt = 0;
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(smem_u32(&sh.bar_item_empty[s]));
+    ++item_cnt;
+    return it;
+  };
 
   // Register budget: 512 threads leave 128 per thread.  The producer / MMA warpgroup and the
   // compute warpgroups hand part of their share to the dQ warpgroup, which must hold a whole
@@ -228,268 +298,491 @@ __global__ void __launch_bounds__(512, 1)
   // compiler budgets registers per region only when the instruction dominates the region.
   if (warp >= 12) {
     reg_dealloc<kBwdRegsIssue>();
-  if (warp == 12) {
-    // =========================== TMA producer ===========================
-    if (cnt > 0) {
-      // K, V and the first Q / dO tile were sent off during the set-up
-      for (int n = 1; n < cnt; ++n) {
-        const int st = n % T::kQStages;
-        const int round = n / T::kQStages;
-        const int row = tile_of(n) * T::kBlock;
-        if (round > 0 &&
-            !mbar_wait_warp(smem_u32(&bar_q_empty[st]), (round - 1) & 1, &abort_word, 1))
-          break;
+    // Slots of the running item's K, V and dO.  At the end of an item they fall free in the order
+    // V (after the last dP^T), dO (after the last dV), K (after the last dQ), and the next item
+    // needs K first, V and dO a while later: it takes them over in that order, so that its first
+    // S^T is issued like any other query tile's.
+    int slot_k = 0, slot_v = 1, slot_do = 2;
+    auto next_slots = [&]() {
+      const int k = slot_k;
+      slot_k = slot_v;
+      slot_v = slot_do;
+      slot_do = k;
+    };
+    if (warp == 12) {
+      // =========================== TMA producer, item source ===========================
+      bool ok = true;
+      uint32_t published = 0, asked = 0;
+      bool pending = false;  // a request is out
+      auto ask = [&]() {
+        if (p.deal || pending) return;
         if (elect_one()) {
-          const uint32_t qbar = smem_u32(&bar_q_full[st]);
-          mbar_arrive_expect_tx(qbar, T::kTileBytes);
-#pragma unroll
-          for (int b = 0; b < T::kBoxes; ++b)
-            tma_load_4d(q_smem + st * T::kTileBytes + b * T::kBoxBytes, &tm_q, qbar, b * 64, row, h,
-                        z);
+          fence_proxy_async_smem();  // the last answer has been read
+          mbar_arrive_expect_tx(smem_u32(&sh.bar_clc), 16);
+          clc_request(smem_u32(sh.clc_word), smem_u32(&sh.bar_clc));
         }
         __syncwarp();
-        if (!mbar_wait_warp(smem_u32(&bar_do_empty), (n - 1) & 1, &abort_word, 2)) break;
-        if (elect_one()) {
-          const uint32_t dbar = smem_u32(&bar_do_full);
-          mbar_arrive_expect_tx(dbar, T::kTileBytes);
-#pragma unroll
-          for (int b = 0; b < T::kBoxes; ++b)
-            tma_load_4d(do_smem + b * T::kBoxBytes, &tm_do, dbar, b * 64, row, h, z);
+        pending = true;
+      };
+      // a KV tile without query tiles: zeros.  They are written here, so that only
+      // items with query tiles to walk are published
+      auto write_zeros = [&](const BwdItem& it) {
+        const int rows = min(T::kBlock, p.seqlen_k - it.kb * T::kBlock);
+        for (int which = 0; which < 2; ++which) {
+          float* accum = which ? p.dk_accum : p.dv_accum;
+          const uint4 zero = make_uint4(0, 0, 0, 0);
+          if (accum != nullptr) {
+            if (p.accum_overwrite == 0) continue;
+            float* dst = accum + (size_t)it.z * p.accum_batch_stride +
+                         ((size_t)it.kb * T::kBlock * p.heads + it.h) * DR;
+            for (int i = lane; i < rows * (DR / 4); i += 32)
+              *reinterpret_cast<uint4*>(dst + (size_t)(i / (DR / 4)) * p.heads * DR + (i % (DR / 4)) * 4) = zero;
+          } else {
+            const Strides3& s = which ? p.dk_strides : p.dv_strides;
+            uint16_t* dst = (which ? p.dk : p.dv) + it.z * s.batch + (long long)it.kb * T::kBlock * s.row + it.h * s.head;
+            for (int i = lane; i < rows * (DR / 8); i += 32)
+              *reinterpret_cast<uint4*>(dst + (i / (DR / 8)) * s.row + (i % (DR / 8)) * 8) = zero;
+          }
+        }
+      };
+
+      // finds the next item with query tiles to walk and publishes it
+      int id = -1;
+      bool first = true;  // the item of the block's own index comes first
+      auto next_item = [&]() -> BwdItem {
+        BwdItem it;
+        for (;; first = false) {
+          if (first) {
+            id = blockIdx.x;
+          } else if (p.deal) {
+            id = -1;
+          } else {
+            ask();
+            ok = mbar_wait_warp(smem_u32(&sh.bar_clc), asked & 1, abort_word, 17);
+            ++asked;
+            pending = false;
+            id = ok ? clc_answer(smem_u32(sh.clc_word)) : -1;
+          }
+          id = __shfl_sync(0xffffffffu, id, 0);
+          it.id = -1;
+          it.cnt = 0;
+          if (id < 0) break;
+          it = bwd_item(p, id);
+          it.cnt = __shfl_sync(0xffffffffu, it.cnt, 0);
+          if (it.cnt > 0) break;
+          ask();
+          write_zeros(it);
+        }
+        const uint32_t s = published % T::kItemStages, round = published / T::kItemStages;
+        if (round > 0 && !mbar_wait_warp(smem_u32(&sh.bar_item_empty[s]), (round - 1) & 1, abort_word, 18)) ok = false;
+        if (ok && lane == 0) {
+          sh.items[s] = it;
+          mbar_arrive(smem_u32(&sh.bar_item_full[s]));
         }
         __syncwarp();
+        ++published;
+        if (!ok) it.id = -1;
+        return it;
+      };
+      uint32_t used = 0;  // bit s: loads into slot s so far, modulo 2
+      auto load = [&](int slot, const CUtensorMap* tm, const BwdItem& it, int row, bool is_q) {
+        ok = ok && mbar_wait_warp(smem_u32(&sh.bar_empty[slot]), ((used >> slot) & 1) ^ 1, abort_word, 1);
+        if (ok) send(slot, tm, it, row, is_q);
+        used ^= 1u << slot;
+      };
+      uint32_t g = 0;  // query tiles so far, over all items
+      while (ok) {
+        const BwdItem it = next_item();
+        if (it.id < 0) break;
+        const int row0 = it.i_begin * T::kBlock, kv0 = it.kb * T::kBlock;
+        if (first) {
+          used = 0xf;  // sent off during the set-up
+          first = false;
+        } else {
+          if (published > 1) next_slots();
+          // cold from HBM these take microseconds: start towards L2 before waiting for the slots
+          if (elect_one()) {
+#pragma unroll
+            for (int b = 0; b < T::kBoxes; ++b) {
+              tma_prefetch_l2_4d(&tm_k, b * 64, kv0, it.h, it.z);
+              tma_prefetch_l2_4d(&tm_v, b * 64, kv0, it.h, it.z);
+              tma_prefetch_l2_4d(&tm_do, b * 64, row0, it.h, it.z);
+            }
+          }
+          __syncwarp();
+          // in the order in which the slots fall free
+          load(3 + (g & 1), &tm_q, it, row0, true);
+          load(slot_k, &tm_k, it, kv0, false);
+          load(slot_v, &tm_v, it, kv0, false);
+          load(slot_do, &tm_do, it, row0, false);
+        }
+        ++g;
+        if (it.cnt == 1) ask();
+#pragma unroll 1
+        for (int n = 1; ok && n < it.cnt; ++n, ++g) {
+          const int row = (it.i_begin + n) * T::kBlock;
+          if (n == it.cnt - 1) ask();  // the answer takes a microsecond
+          load(3 + (g & 1), &tm_q, it, row, true);
+          load(slot_do, &tm_do, it, row, false);
+        }
       }
-    }
-  } else if (warp == 13) {
-    // =========================== MMA issuer (converged warp) ===========================
-    if (cnt > 0) {
-      // C[128 x 128] = A[128 x D] B[128 x D]^T, both K-major in shared memory
-      auto issue_kmajor = [&](uint32_t d_col, uint32_t a_addr, uint32_t b_addr) {
-        const uint32_t a_lo = umma_desc_lo(a_addr, kLboKMajor);
-        const uint32_t b_lo = umma_desc_lo(b_addr, kLboKMajor);
+    } else if (warp == 13) {
+      // =========================== MMA issuer (converged warp) ===========================
+      // D (+)= A B with A and B in shared memory, the contraction in blocks of 64.  Loops, not straight
+      // code: what the roles of the CTA execute has to fit the instruction cache together.
+      auto issue_ss = [&](int blocks, uint32_t d_col, uint32_t a_lo, uint32_t a_block, uint32_t a_step, uint32_t b_lo,
+                          uint32_t b_block, uint32_t b_step, uint32_t idesc, uint32_t accumulate) {
+#pragma unroll 1
+        for (int b = 0; b < blocks; ++b) {
 #pragma unroll
-        for (int ks = 0; ks < D / 16; ++ks) {
-          const uint32_t off = ((ks >> 2) * T::kBoxBytes + (ks & 3) * 32) >> 4;
-          umma_ss_elect(tmem_base + d_col, a_lo + off, b_lo + off, T::kIdescST, ks > 0 ? 1u : 0u);
+          for (int i = 0; i < 4; ++i)
+            umma_ss_elect(tmem_base + d_col, a_lo + i * a_step, b_lo + i * b_step, idesc, i > 0 ? 1u : accumulate);
+          a_lo += a_block;
+          b_lo += b_block;
+          accumulate = 1u;
         }
+      };
+      // steps of 16 along the contraction and blocks of 64, in descriptor units
+      constexpr uint32_t kStepK = 32 >> 4, kBlockK = T::kBoxBytes >> 4;  // K-major operand
+      constexpr uint32_t kStepMn = 2048 >> 4, kBlockMn = 4 * kStepMn;    // MN-major operand
+      // C[128 x 128] = A[128 x D] B[128 x D]^T, both K-major
+      auto issue_kmajor = [&](uint32_t d_col, uint32_t a_addr, uint32_t b_addr) {
+        issue_ss(T::kBoxes, d_col, umma_desc_lo(a_addr, kLboKMajor), kBlockK, kStepK, umma_desc_lo(b_addr, kLboKMajor),
+                 kBlockK, kStepK, T::kIdescST, 0u);
+      };
+      auto slot_addr = [&](int slot) { return smem_base + slot * T::kTileBytes; };
+      uint32_t filled = 0;  // bit s: fills of slot s waited for so far, modulo 2
+      auto wait_full = [&](int slot, int who) {
+        const bool got = mbar_wait_warp(smem_u32(&sh.bar_full[slot]), (filled >> slot) & 1, abort_word, who);
+        filled ^= 1u << slot;
+        return got;
       };
       const uint32_t ds_lo_k = umma_desc_lo(ds_smem, kLboKMajor);    // dS^T as K-major A (dK)
       const uint32_t ds_lo_mn = umma_desc_lo(ds_smem, kLboMnMajor);  // dS^T read as MN-major A (dQ)
-      const uint32_t k_lo_mn = umma_desc_lo(k_smem, kLboMnMajor);    // K as MN-major B (dQ)
-      const uint32_t do_lo_mn = umma_desc_lo(do_smem, kLboMnMajor);  // dO as MN-major B (dV)
 
-      bool ok = mbar_wait_warp(smem_u32(&bar_kv_full), 0, &abort_word, 3);
-      ok = ok && mbar_wait_warp(smem_u32(&bar_q_full[0]), 0, &abort_word, 4);
+      BwdItem cur = take_item();
+      bool ok = cur.id >= 0;
+      ok = ok && wait_full(slot_k, 3) && wait_full(3, 4);
       if (ok) {
         tc_fence_after();
-        issue_kmajor(T::kColS, k_smem, q_smem);
-        umma_commit_elect(smem_u32(&bar_s_full));
+        issue_kmajor(T::kColS, slot_addr(slot_k), slot_addr(3));
+        umma_commit_elect(smem_u32(&sh.bar_s_full));
       }
-      ok = ok && mbar_wait_warp(smem_u32(&bar_do_full), 0, &abort_word, 5);
+      ok = ok && wait_full(slot_v, 5) && wait_full(slot_do, 5);
       if (ok) {
         tc_fence_after();
-        issue_kmajor(T::kColDP, v_smem, do_smem);
-        umma_commit_elect(smem_u32(&bar_dp_full));
+        issue_kmajor(T::kColDP, slot_addr(slot_v), slot_addr(slot_do));
+        umma_commit_elect(smem_u32(&sh.bar_dp_full));
+        if (cur.cnt == 1) umma_commit_elect(smem_u32(&sh.bar_empty[slot_v]));
       }
-      for (int n = 0; ok && n < cnt; ++n) {
-        const int st = n % T::kQStages;
-        const uint32_t q_addr = q_smem + st * T::kTileBytes;
-        // ---- dV += P^T dO_i
-        FMHA_TL(2, n, 0);
-        if (!mbar_wait_warp(smem_u32(&bar_p_ready), n & 1, &abort_word, 6)) break;
+      uint32_t item_no = 0;
+      int n = 0;  // query tile of the item
+#pragma unroll 1
+      for (uint32_t g = 0; ok; ++g) {  // one pass per query tile, from one item into the next
+        const bool last = n == cur.cnt - 1;
+        const uint32_t q_addr = slot_addr(3 + (g & 1));
+        // ---- dV += P^T dO_i; the first one overwrites the last item's dV
+        FMHA_TL(2, g, 0);
+        if (n == 0 && item_no > 0 && !mbar_wait_warp(smem_u32(&sh.bar_dv_read), (item_no - 1) & 1, abort_word, 19)) break;
+        if (!mbar_wait_warp(smem_u32(&sh.bar_p_ready), g & 1, abort_word, 6)) break;
         tc_fence_after();
-        FMHA_TL(2, n, 1);
+        FMHA_TL(2, g, 1);
+        const uint32_t do_lo_mn = umma_desc_lo(slot_addr(slot_do), kLboMnMajor);  // dO as MN-major B
+#pragma unroll 1
+        for (int b = 0; b < 2; ++b)
 #pragma unroll
-        for (int ks = 0; ks < T::kBlock / 16; ++ks)
-          umma_ts_elect(tmem_base + T::kColDV,
-                        tmem_base + T::kColS + (ks >> 2) * 64 + (ks & 3) * 8, do_lo_mn + ks * 128,
-                        T::kIdescDV, (n > 0 || ks > 0) ? 1u : 0u);
-        umma_commit_elect(smem_u32(&bar_do_empty));
-        // ---- S^T of the next query tile (the S region is free once dV has read P^T)
-        if (n + 1 < cnt) {
-          const int st1 = (n + 1) % T::kQStages;
-          if (!mbar_wait_warp(smem_u32(&bar_q_full[st1]), ((n + 1) / T::kQStages) & 1, &abort_word,
-                              7))
-            break;
+          for (int i = 0; i < 4; ++i)
+            umma_ts_elect(tmem_base + T::kColDV, tmem_base + T::kColS + b * 64 + i * 8,
+                          do_lo_mn + b * kBlockMn + i * kStepMn, T::kIdescDV, (n > 0 || b > 0 || i > 0) ? 1u : 0u);
+        umma_commit_elect(smem_u32(&sh.bar_empty[slot_do]));
+        // ---- S^T of the next query tile (the S region is free once dV has read P^T), which may be
+        // the first one of the next item
+        BwdItem nxt = cur;
+        if (last) nxt = take_item();
+        if (nxt.id >= 0) {
+          if (last && !wait_full(slot_v, 3)) break;  // the next K is where V was
+          if (!wait_full(3 + ((g + 1) & 1), 7)) break;
           tc_fence_after();
-          issue_kmajor(T::kColS, k_smem, q_smem + st1 * T::kTileBytes);
-          umma_commit_elect(smem_u32(&bar_s_full));
+          issue_kmajor(T::kColS, slot_addr(last ? slot_v : slot_k), slot_addr(3 + ((g + 1) & 1)));
+          umma_commit_elect(smem_u32(&sh.bar_s_full));
         }
         // ---- dQ_i = dS K first (its read-out is on the critical path), then dK += dS^T Q_i
-        FMHA_TL(2, n, 2);
-        if (!mbar_wait_warp(smem_u32(&bar_ds_ready), n & 1, &abort_word, 8)) break;
+        FMHA_TL(2, g, 2);
+        if (!mbar_wait_warp(smem_u32(&sh.bar_ds_ready), g & 1, abort_word, 8)) break;
         tc_fence_after();
-        FMHA_TL(2, n, 3);
-#pragma unroll
-        for (int ks = 0; ks < T::kBlock / 16; ++ks)
-          umma_ss_elect(tmem_base + T::kColDQ, ds_lo_mn + ks * 128, k_lo_mn + ks * 128, T::kIdescDQ,
-                        ks > 0 ? 1u : 0u);
-        umma_commit_elect(smem_u32(&bar_dq_full));
-        const uint32_t q_lo_mn = umma_desc_lo(q_addr, kLboMnMajor);
-#pragma unroll
-        for (int ks = 0; ks < T::kBlock / 16; ++ks) {
-          const uint32_t off = ((ks >> 2) * T::kBoxBytes + (ks & 3) * 32) >> 4;
-          umma_ss_elect(tmem_base + T::kColDK, ds_lo_k + off, q_lo_mn + ks * 128, T::kIdescDV,
-                        (n > 0 || ks > 0) ? 1u : 0u);
-        }
-        umma_commit_elect(smem_u32(&bar_q_empty[st]));
-        umma_commit_elect(smem_u32(&bar_ds_free));
-        FMHA_TL(2, n, 4);
-        // ---- dP^T of the next query tile (its columns hold dQ_i until the dQ group read it)
-        if (n + 1 < cnt) {
-          if (!mbar_wait_warp(smem_u32(&bar_do_full), (n + 1) & 1, &abort_word, 9)) break;
-          if (!mbar_wait_warp(smem_u32(&bar_dq_empty), n & 1, &abort_word, 10)) break;
+        FMHA_TL(2, g, 3);
+        const uint32_t k_lo_mn = umma_desc_lo(slot_addr(slot_k), kLboMnMajor);  // K as MN-major B
+        issue_ss(2, T::kColDQ, ds_lo_mn, kBlockMn, kStepMn, k_lo_mn, kBlockMn, kStepMn, T::kIdescDQ, 0u);
+        umma_commit_elect(smem_u32(&sh.bar_dq_full));
+        if (last) umma_commit_elect(smem_u32(&sh.bar_empty[slot_k]));
+        if (n == 0 && item_no > 0) {
+          if (!mbar_wait_warp(smem_u32(&sh.bar_dk_read), (item_no - 1) & 1, abort_word, 20)) break;
           tc_fence_after();
-          FMHA_TL(2, n, 5);
-          issue_kmajor(T::kColDP, v_smem, do_smem);
-          umma_commit_elect(smem_u32(&bar_dp_full));
-          FMHA_TL(2, n, 6);
         }
+        const uint32_t q_lo_mn = umma_desc_lo(q_addr, kLboMnMajor);
+        issue_ss(2, T::kColDK, ds_lo_k, kBlockK, kStepK, q_lo_mn, kBlockMn, kStepMn, T::kIdescDV, n > 0 ? 1u : 0u);
+        umma_commit_elect(smem_u32(&sh.bar_empty[3 + (g & 1)]));  // Q_i, and dS^T, have been read
+        if (last) umma_commit_elect(smem_u32(&sh.bar_acc_full));
+        FMHA_TL(2, g, 4);
+        if (nxt.id < 0) break;
+        // ---- dP^T of the next query tile (its columns hold dQ_i until the dQ group read it)
+        if (last) {
+          next_slots();
+          cur = nxt;
+          ++item_no;
+          n = 0;
+          if (!wait_full(slot_v, 5)) break;
+        } else {
+          ++n;
+        }
+        if (!wait_full(slot_do, 9)) break;
+        if (!mbar_wait_warp(smem_u32(&sh.bar_dq_empty), g & 1, abort_word, 10)) break;
+        tc_fence_after();
+        FMHA_TL(2, g, 5);
+        issue_kmajor(T::kColDP, slot_addr(slot_v), slot_addr(slot_do));
+        umma_commit_elect(smem_u32(&sh.bar_dp_full));
+        if (n == cur.cnt - 1) umma_commit_elect(smem_u32(&sh.bar_empty[slot_v]));
+        FMHA_TL(2, g, 6);
       }
-      umma_commit_elect(smem_u32(&bar_done));
     }
-  }
   } else {
     const int quad = warp & 3;
     const int r = quad * 32 + lane;  // TMEM lane of this thread
     const uint32_t lane_addr = uint32_t(quad * 32) << 16;
-    const size_t stat_base = (size_t)zh * p.seqlen_q_pad;
 
     if (warp < 8) {
-      // =========================== compute groups: P^T, dS^T ===========================
+      // =========================== compute groups: P^T, dS^T; dK, dV out ===================
       reg_dealloc<kBwdRegsCompute>();
       const int cg = warp >> 2;           // query-column half of this group
-      const int ct = threadIdx.x;         // 0..255 among the compute threads
-      const int kvi = kv0 + r;            // key of this thread
-      const float c = p.scale_log2;
+      const uint64_t c2 = pack2f(p.scale_log2, p.scale_log2);
       const uint32_t tS = tmem_base + lane_addr + T::kColS + cg * 64;
       // P^T (32 packed columns) goes over the start of this group's own S^T half, which only
       // this group reads: no ordering between the two groups is needed
       const uint32_t tP = tS;
       const uint32_t tDP = tmem_base + lane_addr + T::kColDP + cg * 64;
-      // statistics: thread ct < 128 carries lse2[q0 + ct], the others delta[q0 + ct - 128]
-      const float* stat_src = (ct < 128 ? p.lse2 : p.delta) + stat_base + (ct & 127);
-      float stat_next = (cnt > 0) ? __ldg(stat_src + (size_t)tile_of(0) * T::kBlock) : 0.f;
+      // this thread's 128-byte row of dS^T; a warp's 32 rows (4 KB) are also its own staging area for
+      // dK and dV
+      const uint32_t row_addr = ds_smem + cg * T::kBoxBytes + r * 128;
       const bool tl = (threadIdx.x == 0);
+      uint32_t g = 0, drained = 0;
 
-      for (int n = 0; n < cnt; ++n) {
-        const int qbase = tile_of(n) * T::kBlock;
-        const uint32_t sb = stat_smem;  // lse2 at [0, 512), delta at [512, 1024)
-        named_bar_sync(3, 256);  // every thread is done reading the previous tile's values
-        asm volatile("st.shared.f32 [%0], %1;" ::"r"(sb + ct * 4), "f"(stat_next) : "memory");
-        if (n + 1 < cnt) stat_next = __ldg(stat_src + (size_t)tile_of(n + 1) * T::kBlock);
-        named_bar_sync(4, 256);  // this tile's values are visible
-
-        // first visible query column of this thread's half (>= 64: none)
-        int first_visible = 0;
-        if (kvi >= sk) {
-          first_visible = T::kBlock;
-        } else if (p.causal) {
-          const long long fv = (long long)kvi - p.causal_shift - qbase;
-          first_visible = fv <= 0 ? 0 : (int)min(fv, (long long)T::kBlock);
-        }
-        const int fvh = first_visible - cg * 64;
-
-        uint32_t pp[32];  // P^T of this row and half, 16-bit pairs
-        // fp16 only: -(P^T o delta) as fp16 pairs, so that dS^T = P^T o dP^T - P^T o delta is one
-        // half2 FMA per pair; with bf16 (8 mantissa bits) dS^T is formed in fp32 instead
-        uint32_t npd[kBf16 ? 1 : 32];
-        if (tl) FMHA_TL(0, n, 0);
-        mbar_wait(smem_u32(&bar_s_full), n & 1, &abort_word, 11);  // on a time-out: keep going,
-        // every later wait returns at once and all 256 threads still meet at the named barrier
-        tc_fence_after();
-        if (tl) FMHA_TL(0, n, 1);
-        {
-          uint32_t s[2][32];
-          tmem_ld32(tS, s[0]);
-          tmem_ld32(tS + 32, s[1]);
-          tmem_wait_ld();
+      // dK (is_dk) or dV columns [col0, col0 + 64) of an item: tensor memory -> 16-bit, staging, TMA
+      // store; or (ring attention) into an fp32 buffer, added to what is there or, with
+      // accum_overwrite, in its place
+      auto drain_half = [&](bool is_dk, const BwdItem& it, int col0, bool restage) {
+        const uint32_t tAcc = tmem_base + lane_addr + (is_dk ? T::kColDK : T::kColDV) + col0;
+        const float mul = is_dk ? p.scale : 1.f;
+        float* accum = is_dk ? p.dk_accum : p.dv_accum;
+        const uint32_t read_bar = smem_u32(is_dk ? &sh.bar_dk_read : &sh.bar_dv_read);
+        if (accum != nullptr) {
+          const int kvi = it.kb * T::kBlock + r;
+          const bool have = kvi < it.sk;  // this thread's row has a result
+          const bool touch = kvi < p.seqlen_k && (have || p.accum_overwrite != 0);
+          float* dst = accum + (size_t)it.z * p.accum_batch_stride + ((size_t)kvi * p.heads + it.h) * DR + col0;
+#pragma unroll 1
+          for (int cc = 0; cc < 4; ++cc) {
+            uint32_t a[16];
+            tmem_ld16(tAcc + cc * 16, a);
+            tmem_wait_ld();
+            if (touch && col0 + cc * 16 < DR) {
 #pragma unroll
-          for (int cc = 0; cc < 2; ++cc)
-#pragma unroll
-            for (int i = 0; i < 32; i += 4) {
-              const float4 L = lds128(sb + (cg * 64 + cc * 32 + i) * 4);
-              const float x0 = fmaf(__uint_as_float(s[cc][i + 0]), c, -L.x);
-              const float x1 = fmaf(__uint_as_float(s[cc][i + 1]), c, -L.y);
-              const float x2 = fmaf(__uint_as_float(s[cc][i + 2]), c, -L.z);
-              const float x3 = fmaf(__uint_as_float(s[cc][i + 3]), c, -L.w);
-              if constexpr (kBf16) {
-                // a bf16 argument would cost P two to three digits: exponentials in fp32
-                pp[cc * 16 + (i >> 1) + 0] = pack_bf16x2(fast_exp2(x0), fast_exp2(x1));
-                pp[cc * 16 + (i >> 1) + 1] = pack_bf16x2(fast_exp2(x2), fast_exp2(x3));
-              } else {
-                pp[cc * 16 + (i >> 1) + 0] = exp2_half2(pack_half2(x0, x1));
-                pp[cc * 16 + (i >> 1) + 1] = exp2_half2(pack_half2(x2, x3));
+              for (int i = 0; i < 16; i += 4) {
+                float4 cur = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (p.accum_overwrite == 0) cur = *reinterpret_cast<float4*>(dst + cc * 16 + i);
+                if (have) {
+                  cur.x += __uint_as_float(a[i + 0]) * mul;
+                  cur.y += __uint_as_float(a[i + 1]) * mul;
+                  cur.z += __uint_as_float(a[i + 2]) * mul;
+                  cur.w += __uint_as_float(a[i + 3]) * mul;
+                }
+                *reinterpret_cast<float4*>(dst + cc * 16 + i) = cur;
               }
             }
-          if (fvh > 0) {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {  // pair j = columns 2j, 2j+1 of this half
-              if (2 * j + 1 < fvh) pp[j] = 0u;
-              else if (2 * j < fvh) pp[j] &= 0xffff0000u;
-            }
           }
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(read_bar);
+          return;
         }
-        tmem_st32(tP, pp);
-        tmem_wait_st();
+        uint32_t w[32];
+#pragma unroll
+        for (int cc = 0; cc < 2; ++cc) {
+          uint32_t a[32];
+          tmem_ld32(tAcc + cc * 32, a);
+          tmem_wait_ld();
+#pragma unroll
+          for (int i = 0; i < 16; ++i)
+            w[cc * 16 + i] =
+                pack16x2<kBf16>(__uint_as_float(a[2 * i]) * mul, __uint_as_float(a[2 * i + 1]) * mul);
+        }
         tc_fence_before();
-        mbar_arrive(smem_u32(&bar_p_ready));
-        if (tl) FMHA_TL(0, n, 2);
-        // off the critical path (dP^T is not there yet): -(P o delta)
-        if constexpr (!kBf16) {
+        if (restage && lane == 0) tma_wait_group_read<0>();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(read_bar);
 #pragma unroll
-          for (int j = 0; j < 32; j += 2) {
-            const float4 Dl = lds128(sb + 512 + (cg * 64 + 2 * j) * 4);
-            npd[j + 0] = mul_half2(pp[j + 0], pack_half2(-Dl.x, -Dl.y));
-            npd[j + 1] = mul_half2(pp[j + 1], pack_half2(-Dl.z, -Dl.w));
-          }
+        for (int ch = 0; ch < 8; ++ch)
+          sts128(row_addr + ((ch ^ (r & 7)) << 4), w[4 * ch], w[4 * ch + 1], w[4 * ch + 2], w[4 * ch + 3]);
+        fence_proxy_async_smem();
+        __syncwarp();
+        const int row = it.kb * T::kBlock + quad * 32;
+        if (lane == 0 && row < p.seqlen_k) {
+          tma_store_4d(is_dk ? &tm_dk : &tm_dv, row_addr, col0, row, it.h, it.z);
+          tma_commit_group();
         }
-
-        mbar_wait(smem_u32(&bar_dp_full), n & 1, &abort_word, 12);
-        if (tl) FMHA_TL(0, n, 3);
-        // dS^T of the previous tile must have been consumed by its dK / dQ MMAs
-        if (n > 0) mbar_wait(smem_u32(&bar_ds_free), (n - 1) & 1, &abort_word, 13);
+      };
+      // dK and dV of an item whose MMAs have all been issued
+      auto drain = [&](const BwdItem& it) {
+        mbar_wait(smem_u32(&sh.bar_acc_full), drained & 1, abort_word, 15);
+        ++drained;
         tc_fence_after();
-        if (tl) FMHA_TL(0, n, 4);
-        {
-          uint32_t dp[2][32];
-          tmem_ld32(tDP, dp[0]);
-          tmem_ld32(tDP + 32, dp[1]);
-          tmem_wait_ld();
-          const uint32_t row_addr = ds_smem + cg * T::kBoxBytes + r * 128;
+        // dV, then dK (D = 64: one group each)
+#pragma unroll 1
+        for (int i = 0; i < T::kBoxes; ++i)
+          drain_half(D == 128 ? i == 1 : cg == 1, it, D == 128 ? cg * 64 : 0, i > 0);
+      };
+      // An item's dK and dV are written out behind the first P^T of the next item: they are complete
+      // by then, and the group would wait for the next item's first dP^T (whose V and dO tiles come
+      // in last) anyway.
+      bool pending = false;
+      BwdItem done;
+      for (;;) {
+        const BwdItem it = take_item();
+        if (it.id < 0) break;
+        const int kvi = it.kb * T::kBlock + r;  // key of this thread
+#pragma unroll 1
+        for (int n = 0; n < it.cnt; ++n, ++g) {
+          const int qbase = (it.i_begin + n) * T::kBlock;
+          const uint32_t sb = stat_smem + (g & 1) * T::kStatBytes;  // lse2 at [0, 512), delta at [512, 1024)
+
+          // first visible query column of this thread's half (>= 64: none)
+          int first_visible = 0;
+          if (kvi >= it.sk) {
+            first_visible = T::kBlock;
+          } else if (p.causal) {
+            const long long fv = (long long)kvi - p.causal_shift - qbase;
+            first_visible = fv <= 0 ? 0 : (int)min(fv, (long long)T::kBlock);
+          }
+          const int fvh = first_visible - cg * 64;
+
+          uint32_t pp[32];  // P^T of this row and half, 16-bit pairs
+          // fp16 only: -(P^T o delta) as fp16 pairs, so that dS^T = P^T o dP^T - P^T o delta is one
+          // half2 FMA per pair; with bf16 (8 mantissa bits) dS^T is formed in fp32 instead
+          uint32_t npd[kBf16 ? 1 : 32];
+          if (tl) FMHA_TL(0, g, 0);
+          // on a time-out: keep going, every later wait returns at once
+          mbar_wait(smem_u32(&sh.bar_full[3 + (g & 1)]), (g >> 1) & 1, abort_word, 21);  // the statistics
+          mbar_wait(smem_u32(&sh.bar_s_full), g & 1, abort_word, 11);
+          tc_fence_after();
+          if (tl) FMHA_TL(0, g, 1);
+          {
+            uint32_t s[2][32];
+            tmem_ld32(tS, s[0]);
+            tmem_ld32(tS + 32, s[1]);
+            tmem_wait_ld();
 #pragma unroll
-          for (int cc = 0; cc < 2; ++cc)
+            for (int cc = 0; cc < 2; ++cc)
 #pragma unroll
-            for (int k8 = 0; k8 < 4; ++k8) {  // 8 columns = one 16-byte chunk
-              uint32_t w[4];
-              float dl[8];  // bf16 only: delta of this chunk's 8 query columns
-              if constexpr (kBf16) {
-                const float4 Da = lds128(sb + 512 + (cg * 64 + cc * 32 + k8 * 8) * 4);
-                const float4 Db = lds128(sb + 512 + (cg * 64 + cc * 32 + k8 * 8 + 4) * 4);
-                dl[0] = Da.x, dl[1] = Da.y, dl[2] = Da.z, dl[3] = Da.w;
-                dl[4] = Db.x, dl[5] = Db.y, dl[6] = Db.z, dl[7] = Db.w;
-              }
+              for (int i = 0; i < 32; i += 4) {
+                const float4 nl = lds128(sb + (cg * 64 + cc * 32 + i) * 4);
+                uint32_t x[4];
+                unpack2(fma2(pack2(s[cc][i + 0], s[cc][i + 1]), c2, pack2f(nl.x, nl.y)), x[0], x[1]);
+                unpack2(fma2(pack2(s[cc][i + 2], s[cc][i + 3]), c2, pack2f(nl.z, nl.w)), x[2], x[3]);
 #pragma unroll
-              for (int q2 = 0; q2 < 4; ++q2) {
-                const int i = k8 * 8 + q2 * 2;     // column within this 32-column block
-                const int j = cc * 16 + (i >> 1);  // its fp16 pair
-                if constexpr (kBf16) {
-                  w[q2] = pack_bf16x2(bf16_lo(pp[j]) * (__uint_as_float(dp[cc][i]) - dl[q2 * 2]),
-                                      bf16_hi(pp[j]) * (__uint_as_float(dp[cc][i + 1]) - dl[q2 * 2 + 1]));
-                } else {
-                  w[q2] = fma_half2(pp[j],
-                                    pack_half2(__uint_as_float(dp[cc][i]), __uint_as_float(dp[cc][i + 1])),
-                                    npd[j]);
+                for (int k = 0; k < 2; ++k) {
+                  const float xa = __uint_as_float(x[2 * k]), xb = __uint_as_float(x[2 * k + 1]);
+                  // a bf16 argument would cost P two to three digits: exponentials in fp32
+                  if constexpr (kBf16) pp[cc * 16 + (i >> 1) + k] = pack_bf16x2(fast_exp2(xa), fast_exp2(xb));
+                  else pp[cc * 16 + (i >> 1) + k] = exp2_half2(pack_half2(xa, xb));
                 }
               }
-              const int ch = cc * 4 + k8;  // chunk of this thread's 128-byte row
-              sts128(row_addr + ((ch ^ (r & 7)) << 4), w[0], w[1], w[2], w[3]);
+            if (fvh > 0) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) {  // pair j = columns 2j, 2j+1 of this half
+                if (2 * j + 1 < fvh) pp[j] = 0u;
+                else if (2 * j < fvh) pp[j] &= 0xffff0000u;
+              }
             }
+          }
+          tmem_st32(tP, pp);
+          tmem_wait_st();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(smem_u32(&sh.bar_p_ready));
+          if (tl) FMHA_TL(0, g, 2);
+          if (pending) {
+            drain(done);
+            pending = false;
+          }
+          // off the critical path (dP^T is not there yet): -(P o delta)
+          if constexpr (!kBf16) {
+#pragma unroll
+            for (int j = 0; j < 32; j += 4) {
+              const float4 nd = lds128(sb + 512 + (cg * 32 + j) * 4);  // eight fp16 values
+              npd[j + 0] = mul_half2(pp[j + 0], __float_as_uint(nd.x));
+              npd[j + 1] = mul_half2(pp[j + 1], __float_as_uint(nd.y));
+              npd[j + 2] = mul_half2(pp[j + 2], __float_as_uint(nd.z));
+              npd[j + 3] = mul_half2(pp[j + 3], __float_as_uint(nd.w));
+            }
+          }
+
+          mbar_wait(smem_u32(&sh.bar_dp_full), g & 1, abort_word, 12);
+          if (tl) FMHA_TL(0, g, 3);
+          // dS^T of the previous tile must have been consumed by its dK / dQ MMAs (which also
+          // released its query tile), and dK / dV must have left the staging area
+          if (g > 0) mbar_wait(smem_u32(&sh.bar_empty[3 + ((g - 1) & 1)]), ((g - 1) >> 1) & 1, abort_word, 13);
+          if (n == 0) {
+            if (lane == 0) tma_wait_group_read<0>();
+            __syncwarp();
+          }
+          tc_fence_after();
+          if (tl) FMHA_TL(0, g, 4);
+          {
+            uint32_t dp[2][32];
+            tmem_ld32(tDP, dp[0]);
+            tmem_ld32(tDP + 32, dp[1]);
+            tmem_wait_ld();
+#pragma unroll
+            for (int cc = 0; cc < 2; ++cc)
+#pragma unroll
+              for (int k8 = 0; k8 < 4; ++k8) {  // 8 columns = one 16-byte chunk
+                uint32_t w[4];
+                uint64_t nd[4];  // bf16 only: -delta of this chunk's 8 query columns, in pairs
+                if constexpr (kBf16) {
+                  const float4 a = lds128(sb + 512 + (cg * 64 + cc * 32 + k8 * 8) * 4);
+                  const float4 b = lds128(sb + 512 + (cg * 64 + cc * 32 + k8 * 8 + 4) * 4);
+                  nd[0] = pack2f(a.x, a.y), nd[1] = pack2f(a.z, a.w);
+                  nd[2] = pack2f(b.x, b.y), nd[3] = pack2f(b.z, b.w);
+                }
+#pragma unroll
+                for (int q2 = 0; q2 < 4; ++q2) {
+                  const int i = k8 * 8 + q2 * 2;     // column within this 32-column block
+                  const int j = cc * 16 + (i >> 1);  // its fp16 pair
+                  if constexpr (kBf16) {
+                    uint32_t lo, hi;
+                    unpack2(mul2(pack2f(bf16_lo(pp[j]), bf16_hi(pp[j])), add2(pack2(dp[cc][i], dp[cc][i + 1]), nd[q2])),
+                            lo, hi);
+                    w[q2] = pack_bf16x2(__uint_as_float(lo), __uint_as_float(hi));
+                  } else {
+                    w[q2] = fma_half2(pp[j],
+                                      pack_half2(__uint_as_float(dp[cc][i]), __uint_as_float(dp[cc][i + 1])),
+                                      npd[j]);
+                  }
+                }
+                const int ch = cc * 4 + k8;  // chunk of this thread's 128-byte row
+                sts128(row_addr + ((ch ^ (r & 7)) << 4), w[0], w[1], w[2], w[3]);
+              }
+          }
+          fence_proxy_async_smem();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(smem_u32(&sh.bar_ds_ready));
+          if (tl) FMHA_TL(0, g, 5);
         }
-        fence_proxy_async_smem();
-        tc_fence_before();
-        mbar_arrive(smem_u32(&bar_ds_ready));
-        if (tl) FMHA_TL(0, n, 5);
+        pending = true;
+        done = it;
       }
+      if (pending) drain(done);
+      if (lane == 0) tma_wait_group<0>();
     } else {
       // =========================== dQ group ===========================
       reg_alloc<kBwdRegsDq>();
@@ -499,154 +792,81 @@ __global__ void __launch_bounds__(512, 1)
       // an odd number of chunks per tile breaks the alternation of the two staging buffers by
       // chunk index: count the chunks staged so far instead
       [[maybe_unused]] uint32_t chunk_no = 0;
-      for (int n = 0; n < cnt; ++n) {
-        if (tl) FMHA_TL(1, n, 0);
-        // on a time-out keep going (like the compute groups): every later wait returns at once,
-        // and all 128 threads still meet at the named barriers
-        mbar_wait(smem_u32(&bar_dq_full), n & 1, &abort_word, 14);
-        tc_fence_after();
-        if (tl) FMHA_TL(1, n, 1);
-        // The whole dQ row goes to registers first so that the dQ columns are released to the
-        // next dP^T as early as possible; then 32-column chunks go out through shared memory.
-        uint32_t acc[D / 32][32];
+      uint32_t g = 0;
+      for (;;) {
+        const BwdItem it = take_item();
+        if (it.id < 0) break;
+#pragma unroll 1
+        for (int n = 0; n < it.cnt; ++n, ++g) {
+          const int tile = it.i_begin + n;
+          if (tl) FMHA_TL(1, g, 0);
+          // on a time-out keep going (like the compute groups): every later wait returns at once,
+          // and all 128 threads still meet at the named barriers
+          mbar_wait(smem_u32(&sh.bar_dq_full), g & 1, abort_word, 14);
+          tc_fence_after();
+          if (tl) FMHA_TL(1, g, 1);
+          // The whole dQ row goes to registers first so that the dQ columns are released to the
+          // next dP^T as early as possible; then 32-column chunks go out through shared memory.
+          uint32_t acc[D / 32][32];
 #pragma unroll
-        for (int cc = 0; cc < D / 32; ++cc) tmem_ld32(tDQ + cc * 32, acc[cc]);
-        tmem_wait_ld();
-        tc_fence_before();
-        mbar_arrive(smem_u32(&bar_dq_empty));
-        if (tl) FMHA_TL(1, n, 2);
+          for (int cc = 0; cc < D / 32; ++cc) tmem_ld32(tDQ + cc * 32, acc[cc]);
+          tmem_wait_ld();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(smem_u32(&sh.bar_dq_empty));
+          if (tl) FMHA_TL(1, g, 2);
+          int* const order_word =
+              p.dq_order == nullptr ? nullptr : p.dq_order + (size_t)it.zh * (p.seqlen_q_pad / T::kBlock) + tile;
 #pragma unroll
-        for (int cc = 0; cc < kChunks; ++cc) {
-          // One reduce-add per 32-column chunk for the whole 128-row tile (16 KB): few large
-          // bulk operations instead of many small ones.  The buffer was last used two
-          // reduce-adds ago: at most one group may still be reading.
-          uint32_t stg_buf;
-          if constexpr (kChunks % 2 == 0) {
-            stg_buf = stg_smem + (cc & 1) * 16384;
-          } else {
-            stg_buf = stg_smem + (chunk_no & 1u) * 16384;
-            ++chunk_no;
-          }
-          if (r == 0) tma_wait_group_read<1>();
-          named_bar_sync(2, 128);
-          const uint32_t buf_row = stg_buf + r * 128;
-#pragma unroll
-          for (int k4 = 0; k4 < 8; ++k4)
-            sts128(buf_row + ((k4 ^ (r & 7)) << 4), acc[cc][k4 * 4 + 0], acc[cc][k4 * 4 + 1],
-                   acc[cc][k4 * 4 + 2], acc[cc][k4 * 4 + 3]);
-          fence_proxy_async_smem();
-          named_bar_sync(2, 128);
-          if (r == 0) {
-            int* order_word = p.dq_order == nullptr
-                                  ? nullptr
-                                  : p.dq_order + (size_t)zh * (p.seqlen_q_pad / T::kBlock) + tile_of(n);
-            if (order_word != nullptr && cc == 0) {
-              // the KV tiles before this one have added their share of this query tile
-              global_flag_wait(order_word, kb, &abort_word, p.status, 17);
-              fence_proxy_async_all();
+          for (int cc = 0; cc < kChunks; ++cc) {
+            // One reduce-add per 32-column chunk for the whole 128-row tile (16 KB): few large
+            // bulk operations instead of many small ones.  The buffer was last used two
+            // reduce-adds ago: at most one group may still be reading.
+            uint32_t stg_buf;
+            if constexpr (kChunks % 2 == 0) {
+              stg_buf = stg_smem + (cc & 1) * 16384;
+            } else {
+              stg_buf = stg_smem + (chunk_no & 1u) * 16384;
+              ++chunk_no;
             }
-            tma_reduce_add_4d(&tm_dqacc, stg_buf, cc * 32,
-                              tile_of(n) * T::kBlock, h, z);
-            tma_commit_group();
-            if (order_word != nullptr && cc == kChunks - 1) {
-              tma_wait_group<0>();  // the adds have been performed, not just read from shared memory
-              fence_proxy_async_all();
-              __threadfence();
-              global_flag_release(order_word, kb + 1);
+            if (r == 0) tma_wait_group_read<1>();
+            named_bar_sync(2, 128);
+            const uint32_t buf_row = stg_buf + r * 128;
+#pragma unroll
+            for (int k4 = 0; k4 < 8; ++k4)
+              sts128(buf_row + ((k4 ^ (r & 7)) << 4), acc[cc][k4 * 4 + 0], acc[cc][k4 * 4 + 1],
+                     acc[cc][k4 * 4 + 2], acc[cc][k4 * 4 + 3]);
+            fence_proxy_async_smem();
+            named_bar_sync(2, 128);
+            if (r == 0) {
+              if (order_word != nullptr && cc == 0) {
+                // the KV tiles before this one have added their share of this query tile
+                global_flag_wait(order_word, it.kb, &sh.abort_word, p.status, 17);
+                fence_proxy_async_all();
+              }
+              tma_reduce_add_4d(&tm_dqacc, stg_buf, cc * 32, tile * T::kBlock, it.h, it.z);
+              tma_commit_group();
+              if (order_word != nullptr && cc == kChunks - 1) {
+                tma_wait_group<0>();  // the adds have been performed, not just read from shared memory
+                fence_proxy_async_all();
+                __threadfence();
+                global_flag_release(order_word, it.kb + 1);
+              }
             }
           }
+          if (tl) FMHA_TL(1, g, 3);
         }
-        if (tl) FMHA_TL(1, n, 3);
       }
       if (r == 0) tma_wait_group<0>();
-      named_bar_sync(2, 128);  // the group leaves its loop together
-    }
-
-    // ============ epilogue: dK (warps 0-3), dV (warps 4-7) ============
-    // The two compute groups, which are done with the last query tile before the dQ group is:
-    // dK and dV leave while the last dQ tile is still being staged and reduce-added.
-    if (warp < 8) {
-      const bool is_dk = warp < 4;
-      if (cnt > 0) mbar_wait(smem_u32(&bar_done), 0, &abort_word, 15);
-      tc_fence_after();
-      const uint32_t tAcc = tmem_base + lane_addr + (is_dk ? T::kColDK : T::kColDV);
-      const float mul = is_dk ? p.scale : 1.f;
-      float* accum = is_dk ? p.dk_accum : p.dv_accum;
-      const int kvi = kv0 + r;
-      if (accum != nullptr) {
-        // ring attention: this block's contribution goes into an fp32 buffer, added to what is
-        // there or (accum_overwrite) in its place; then also rows nobody contributes to are
-        // written, as zeros, so that the buffer needs no clearing beforehand
-        const bool have = cnt > 0 && kvi < sk;                  // this thread's row has a result
-        const bool touch = kvi < p.seqlen_k && (have || p.accum_overwrite != 0);
-        float* dst =
-            accum + (size_t)z * p.accum_batch_stride + ((size_t)kvi * p.heads + h) * DR;
-#pragma unroll
-        for (int cc = 0; cc < D / 32; ++cc) {
-          uint32_t a[32];
-          if (cnt > 0) {  // uniform over the CTA: the tensor-memory load is a warp-wide instruction
-            tmem_ld32(tAcc + cc * 32, a);
-            tmem_wait_ld();
-          }
-          if (touch && cc * 32 < DR) {
-#pragma unroll
-            for (int i = 0; i < 32; i += 4) {
-              float4 cur = make_float4(0.f, 0.f, 0.f, 0.f);
-              if (p.accum_overwrite == 0) cur = *reinterpret_cast<float4*>(dst + cc * 32 + i);
-              if (have) {
-                cur.x += __uint_as_float(a[i + 0]) * mul;
-                cur.y += __uint_as_float(a[i + 1]) * mul;
-                cur.z += __uint_as_float(a[i + 2]) * mul;
-                cur.w += __uint_as_float(a[i + 3]) * mul;
-              }
-              *reinterpret_cast<float4*>(dst + cc * 32 + i) = cur;
-            }
-          }
-        }
-      } else {
-        // fp16 tile -> shared memory (over Q stage 0 / dO) -> TMA store
-        const uint32_t out_smem = is_dk ? q_smem : do_smem;
-#pragma unroll
-        for (int cc = 0; cc < D / 32; ++cc) {
-          uint32_t a[32];
-          if (cnt > 0) {
-            tmem_ld32(tAcc + cc * 32, a);
-            tmem_wait_ld();
-          } else {
-#pragma unroll
-            for (int i = 0; i < 32; ++i) a[i] = 0u;
-          }
-#pragma unroll
-          for (int k4 = 0; k4 < 4; ++k4) {
-            const int ch = cc * 4 + k4;
-            const uint32_t addr =
-                out_smem + (ch >> 3) * T::kBoxBytes + r * 128 + (((ch & 7) ^ (r & 7)) << 4);
-            sts128(addr,
-                   pack16x2<kBf16>(__uint_as_float(a[k4 * 8 + 0]) * mul, __uint_as_float(a[k4 * 8 + 1]) * mul),
-                   pack16x2<kBf16>(__uint_as_float(a[k4 * 8 + 2]) * mul, __uint_as_float(a[k4 * 8 + 3]) * mul),
-                   pack16x2<kBf16>(__uint_as_float(a[k4 * 8 + 4]) * mul, __uint_as_float(a[k4 * 8 + 5]) * mul),
-                   pack16x2<kBf16>(__uint_as_float(a[k4 * 8 + 6]) * mul, __uint_as_float(a[k4 * 8 + 7]) * mul));
-          }
-        }
-        fence_proxy_async_smem();
-        named_bar_sync(is_dk ? 1 : 5, 128);
-        if (r == 0) {
-          const CUtensorMap* tm = is_dk ? &tm_dk : &tm_dv;
-#pragma unroll
-          for (int b = 0; b < T::kBoxes; ++b)
-            tma_store_4d(tm, out_smem + b * T::kBoxBytes, b * 64, kv0, h, z);
-          tma_commit_group();
-          tma_wait_group<0>();
-        }
-      }
     }
   }
 
   // ---- teardown
   tc_fence_before();
   __syncthreads();
-  if (abort_word != 0) {
-    if (threadIdx.x == 0 && p.status != nullptr) atomicCAS(p.status, 0, abort_word);
+  if (sh.abort_word != 0) {
+    if (threadIdx.x == 0 && p.status != nullptr) atomicCAS(p.status, 0, sh.abort_word);
+    // let copies that may still be in flight land before the shared memory is released
     for (int i = 0; i < 64; ++i) __nanosleep(1000);
   }
   if (warp == 13) {

@@ -366,14 +366,14 @@ int launch_bwd(const FmhaBwdParams* p, const BwdWorkspace& w, cudaStream_t strea
     // with fp32 accumulation the fp16 outputs are not touched: any valid map will do
     const bool acc_k = p->dk_accum != nullptr, acc_v = p->dv_accum != nullptr;
     if ((rc = make_tensor_map(&tdk, acc_k ? p->k : p->dk, Z, Nk, H, Dr,
-                              acc_k ? p->k_strides : p->dk_strides, kBf16)))
+                              acc_k ? p->k_strides : p->dk_strides, kBf16, 32)))
       return rc;
     if ((rc = make_tensor_map(&tdv, acc_v ? p->v : p->dv, Z, Nk, H, Dr,
-                              acc_v ? p->v_strides : p->dv_strides, kBf16)))
+                              acc_v ? p->v_strides : p->dv_strides, kBf16, 32)))
       return rc;
     fmha::BwdKernelParams kp;
-    kp.lse2 = w.lse2;
-    kp.delta = w.delta;
+    kp.neg_lse2 = w.lse2;
+    kp.neg_delta = w.delta;
     kp.dk_accum = p->dk_accum;
     kp.dv_accum = p->dv_accum;
     kp.accum_batch_stride =
@@ -387,6 +387,10 @@ int launch_bwd(const FmhaBwdParams* p, const BwdWorkspace& w, cudaStream_t strea
     kp.num_heads_total = Z * H;
     kp.head_group = bwd_head_group(kp.num_kv_blocks, p->causal != 0);
     kp.q_tile_begin = p->q_row_begin / 128;
+    kp.dk = static_cast<uint16_t*>(p->dk);
+    kp.dv = static_cast<uint16_t*>(p->dv);
+    kp.dk_strides = to3(p->dk_strides);
+    kp.dv_strides = to3(p->dv_strides);
     kp.scale = p->scale;
     kp.scale_log2 = p->scale * 1.4426950408889634f;
     kp.causal = p->causal ? 1 : 0;
@@ -400,13 +404,17 @@ int launch_bwd(const FmhaBwdParams* p, const BwdWorkspace& w, cudaStream_t strea
       if (cudaMemsetAsync(w.dq_order, 0, w.order_bytes, stream) != cudaSuccess) return FMHA_ERR_LAUNCH;
       kp.dq_order = w.dq_order;
     }
+    const unsigned grid = (unsigned)((long long)kp.num_kv_blocks * H * Z);
+    // One block per item, taken over by running blocks.  Not where every item has an SM of its own,
+    // nor in the deterministic mode: an item waits there for items with lower indices, and only the
+    // order in which blocks are dispatched says that these are under way.
+    kp.deal = (int)grid <= sm_count(current_device()) || kp.dq_order != nullptr;
     kp.timeline = g_timeline;
     kp.timeline_block = g_timeline_block;
     auto kernel = fmha::fmha_bwd_kernel<D, kBf16, DR>;
-    if (!allow_smem<fmha::fmha_bwd_kernel<D, kBf16, DR>>(current_device(), T::kSmemBytes))
-      return FMHA_ERR_LAUNCH;
-    const unsigned grid = (unsigned)((long long)kp.num_kv_blocks * H * Z);
-    kernel<<<grid, T::kThreads, T::kSmemBytes, stream>>>(tq, tk, tv, tdo, tdk, tdv, tacc, kp);
+    constexpr int smem = fmha::bwd_smem_bytes<D, kBf16>();
+    if (!allow_smem<fmha::fmha_bwd_kernel<D, kBf16, DR>>(current_device(), smem)) return FMHA_ERR_LAUNCH;
+    kernel<<<grid, T::kThreads, smem, stream>>>(tq, tk, tv, tdo, tdk, tdv, tacc, kp);
     if (cudaGetLastError() != cudaSuccess) return FMHA_ERR_LAUNCH;
   }
 
