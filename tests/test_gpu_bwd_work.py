@@ -1,0 +1,79 @@
+"""GPU parity tests of how the backward kernel's work is taken: more items (KV tiles) than SMs, so that
+a CTA runs several and hands its tiles and accumulators over from one to the next."""
+import pytest
+import torch
+
+from oracle import attention_oracle as oracle
+from tests import helpers
+from tests.test_gpu_padded import _oracle_padded
+
+pytestmark = pytest.mark.gpu
+
+
+def _tols(dtype):
+    if dtype == torch.float16:
+        return helpers.TOL_O_MAX_ABS, helpers.TOL_GRAD_REL_L2
+    return helpers.TOL_O_MAX_ABS_BF16, helpers.TOL_GRAD_REL_L2_BF16
+
+
+# H chosen so that Z * H * KV tiles is 2 to 4 times the 148 SMs
+@pytest.mark.parametrize("H,n_q,n_k,causal,shift", [
+    (100, 288, 288, False, 0),   # three KV tiles of three query tiles, ragged
+    (100, 320, 320, True, 0),    # items of 3, 2 and 1 query tiles
+    (25, 32, 2016, False, 0),    # one query tile per item, ragged last KV tile
+    (300, 640, 96, False, 0),    # one KV tile per head
+    (50, 256, 1152, True, 128),  # KV tiles that no query sees: runs of items without work
+])
+@pytest.mark.parametrize("D,dtype", [(64, torch.float16), (64, torch.bfloat16), (96, torch.float16),
+                                     (128, torch.float16), (128, torch.bfloat16)])
+def test_more_items_than_sms(H, n_q, n_k, causal, shift, D, dtype):
+    q, _, _, dout = oracle.make_inputs(1, n_q, H, D, seed=71)
+    _, k, v, _ = oracle.make_inputs(1, n_k, H, D, seed=72)
+    q, k, v, dout = (t.to(dtype) for t in (q, k, v, dout))
+    scale = oracle.default_scale(D)
+    got = helpers.gpu_fwd_bwd(q, k, v, dout, scale, causal, shift)
+    ref = oracle.attention_fwd_bwd(q, k, v, dout, scale, causal, shift)
+    helpers.check_against_oracle(got, ref, f"H{H} {n_q}x{n_k} D{D}", *_tols(dtype))
+    if causal:  # keys beyond the last one that is seen: exact zeros
+        assert not got[3][:, n_q + shift:].any() and not got[4][:, n_q + shift:].any()
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("overwrite", [False, True])
+def test_fp32_accumulation_over_many_items(D, overwrite):
+    """dK and dV added into (or in place of) fp32 buffers, with KV tiles that no query sees."""
+    from flash_attn_v100 import cabi
+
+    H, n_q, n_k, shift = 50, 256, 1152, 128
+    q, _, _, dout = oracle.make_inputs(1, n_q, H, D, seed=73)
+    _, k, v, _ = oracle.make_inputs(1, n_k, H, D, seed=74)
+    scale = oracle.default_scale(D)
+    ref = oracle.attention_fwd_bwd(q, k, v, dout, scale, True, shift)
+    q, k, v, dout = (t.cuda() for t in (q, k, v, dout))
+    out, lse = cabi.fwd(q, k, v, scale, True, shift)
+    acc = [torch.full((1, n_k, H, D), 3.0, device="cuda") for _ in range(2)]
+    cabi.bwd(q, k, v, out, dout, lse, scale, True, shift, dk_accum=acc[0], dv_accum=acc[1],
+             flags=cabi.FMHA_BWD_ACCUM_OVERWRITE if overwrite else 0)
+    for a, r in zip(acc, ref[3:]):
+        assert oracle.rel_l2(a.cpu() - (0.0 if overwrite else 3.0), r) <= helpers.TOL_GRAD_REL_L2
+        assert (a[:, n_q + shift:] == (0.0 if overwrite else 3.0)).all()
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("causal", [False, True])
+def test_runs_of_padding_between_items(D, causal):
+    """A padded batch whose short entries leave runs of far more empty items than are published ahead."""
+    from flash_attn_v100 import cabi
+
+    Z, H, N = 4, 24, 1024
+    lens = [1024, 33, 130, 700]
+    q, k, v, dout = oracle.make_inputs(Z, N, H, D, seed=75)
+    lens_d = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    scale = oracle.default_scale(D)
+    qd, kd, vd, dod = (t.cuda() for t in (q, k, v, dout))
+    out, lse = cabi.fwd(qd, kd, vd, scale, causal, status=status, seqused_q=lens_d, seqused_k=lens_d)
+    grads = cabi.bwd(qd, kd, vd, out, dod, lse, scale, causal, status=status, seqused_q=lens_d, seqused_k=lens_d)
+    assert int(status.item()) == 0
+    ref = _oracle_padded(q, k, v, dout, scale, causal, lens, lens)
+    helpers.check_against_oracle((out.cpu(), lse.cpu(), *(t.cpu() for t in grads)), ref, f"padding runs D{D}")
