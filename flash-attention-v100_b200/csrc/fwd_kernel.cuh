@@ -639,8 +639,12 @@ __global__ void __launch_bounds__(384, 1)
                 for (int i = 0; i < 32; ++i)
                   if (half * 64 + ch * 32 + i <= lim) m_new = fmaxf(m_new, __uint_as_float(x[i]));
               }
-              if (half == 1) mbar_wait(smem_u32(&bar_pv_half[t]), phase_s ^ 1u, &abort_word, 11);
-              if (half == 1 || j > 0) {
+              // In round 0 there is nothing to rescale: its reference is the maximum of all 128 keys, so
+              // that m_new is m_ref (what leads here is a sum that is not finite, or no score but
+              // -inf).  Nor may it wait for bar_pv_half: the first O_t += of an item follows
+              // bar_o_read, on which this warp arrives in the epilogue behind this round.
+              if (j > 0) {
+                if (half == 1) mbar_wait(smem_u32(&bar_pv_half[t]), phase_s ^ 1u, &abort_word, 11);
                 tc_fence_after();
                 const float alpha = isinf(m_new) ? 1.f : fast_exp2((m_ref - m_new) * c);
                 l *= alpha;
@@ -680,14 +684,14 @@ __global__ void __launch_bounds__(384, 1)
             if (lane == 0) mbar_arrive(smem_u32(&bar_p_full[t][half]));
           };
           if (j == 0) {
+            // over all 128 keys, so that half 1 never has to rescale in round 0 (see there)
             float mx[4];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              mx[k] = fmaxf(__uint_as_float(s[k >> 1][(k & 1) * 16]), __uint_as_float(s[k >> 1][(k & 1) * 16 + 1]));
+            for (int cc = 0; cc < 4; ++cc) {
+              mx[cc] = fmaxf(__uint_as_float(s[cc][0]), __uint_as_float(s[cc][1]));
 #pragma unroll
-              for (int i = 2; i < 16; i += 2)
-                mx[k] = max3(mx[k], __uint_as_float(s[k >> 1][(k & 1) * 16 + i]),
-                             __uint_as_float(s[k >> 1][(k & 1) * 16 + i + 1]));
+              for (int i = 2; i < 32; i += 2)
+                mx[cc] = max3(mx[cc], __uint_as_float(s[cc][i]), __uint_as_float(s[cc][i + 1]));
             }
             m_ref = fmaxf(max3(mx[0], mx[1], mx[2]), mx[3]);
             neg_mc = isinf(m_ref) ? 0.f : -m_ref * c;
