@@ -587,14 +587,16 @@ __global__ void __launch_bounds__(384, 1)
                 if (cc * 32 + i > lim) s[cc][i] = __float_as_uint(-CUDART_INF_F);
           }
           // P of 64 keys -> tensor memory.  The reference m_ref stays what it was unless an exponential
-          // comes out too large; what tells is their sum, which the row sum needs anyway, so that
-          // in the ordinary case no maximum is looked for at all.  (The first round has to look: it
+          // comes out too large; what tells is their sum, which the row sum needs anyway (and for those
+          // that are a polynomial, which wraps, their largest argument), so that in the ordinary case
+          // no maximum of the scores is looked for at all.  (The first round has to look: it
           // has no reference yet.)
           auto half_round = [&](auto half_tag) {
             constexpr int half = decltype(half_tag)::value;
             const uint64_t c2 = pack2f(c, c), nm2 = pack2f(neg_mc, neg_mc);
             uint64_t la = pack2f(0.f, 0.f), lb = pack2f(0.f, 0.f);
             uint32_t pk[32];
+            float top = 0.f;
 #pragma unroll
             for (int ch = 0; ch < 2; ++ch) {
               const int cc = half * 2 + ch;
@@ -604,7 +606,7 @@ __global__ void __launch_bounds__(384, 1)
                 uint64_t p2;
                 // kPolyPairs of every 8 pairs go through the FMA pipe instead of the MUFU unit
                 if (((i >> 1) & 7) < T::kPolyPairs) {
-                  p2 = poly_exp2_pair(x2);
+                  p2 = poly_exp2_pair(x2, top);
                 } else {
                   uint32_t x0, x1;
                   unpack2(x2, x0, x1);
@@ -620,7 +622,8 @@ __global__ void __launch_bounds__(384, 1)
             unpack2(add2(la, lb), a0, a1);
             float sum = __uint_as_float(a0) + __uint_as_float(a1);
             // (a row that has not seen anything yet has no reference to compare with)
-            const bool need = !(sum <= kRescaleSum) || (m_ref == -CUDART_INF_F && lim >= half * 64);
+            const bool need = !(sum <= kRescaleSum) || !(top <= kPolyExp2Top) ||
+                              (m_ref == -CUDART_INF_F && lim >= half * 64);
             if (!__any_sync(0xffffffffu, need)) {
               tmem_st32(tS + half * 32, pk);
             } else {

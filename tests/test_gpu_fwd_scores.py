@@ -15,11 +15,14 @@ FEW = (1, 2, 1024)    # 8 items: cut into chunks of the KV range where a workspa
 
 
 def _reference(q, k, v, scale, causal):
-    q, k, v = (t.float().transpose(1, 2) for t in (q, k, v))
-    s = q @ k.transpose(2, 3) * scale
-    if causal:
-        s = s.masked_fill(~torch.ones(s.shape[2:], dtype=torch.bool).tril(), float("-inf"))
-    return (s.softmax(-1) @ v).transpose(1, 2), s.logsumexp(-1)
+    out, lse = torch.empty(q.shape), torch.empty((q.shape[0], q.shape[2], q.shape[1]))
+    for z in range(q.shape[0]):
+        qz, kz, vz = (t[z].float().transpose(0, 1) for t in (q, k, v))
+        s = qz @ kz.transpose(1, 2) * scale
+        if causal:
+            s = s.masked_fill(~torch.ones(s.shape[1:], dtype=torch.bool).tril(), float("-inf"))
+        out[z], lse[z] = (s.softmax(-1) @ vz).transpose(0, 1), s.logsumexp(-1)
+    return out, lse
 
 
 def _run(q, k, v, scale, causal):
@@ -49,6 +52,12 @@ def _check(got, ref, tol_o):
     # fp32 on both sides: a few roundings of numbers as large as the LSE
     bound = helpers.TOL_LSE_MAX_ABS + 2.0 ** -21 * r_lse[good].abs().max().item()
     assert oracle.max_abs(lse[good], r_lse[good]) <= bound
+
+
+def _bound_few_keys(v, ref):
+    """Max-abs error of rows with all their weight on a key or two, where O is as large as V: every
+    weight is rounded to fp16 (relative 2^-11, the row sum is not), and so is O."""
+    return 2.0 ** -11 * (v.float().abs().max().item() + ref[0].abs().max().item())
 
 
 @pytest.mark.parametrize("shape", [MANY])
@@ -97,7 +106,57 @@ def test_leap_in_the_second_half_of_the_first_round(D, shape):
     k[:, 128:] *= 0.5
     scale = oracle.default_scale(D)
     ref = _reference(q, k, v, scale, False)
-    # rows with all their weight on a key or two: P is rounded to fp16 (2^-11, the row sum is not), so is O
-    bound = 2.0 ** -11 * (v.float().abs().max().item() + ref[0].abs().max().item())
     for got in _run(q, k, v, scale, False):
-        _check(got, ref, bound)
+        _check(got, ref, _bound_few_keys(v, ref))
+
+
+@pytest.mark.parametrize("D", [64, 96, 128])
+def test_one_key_far_above_the_rest(D):
+    """A single key above all others by 95 to 400, once in each of 16 neighbouring columns (some of whose
+    exponentials are a polynomial), in either half of the first, a middle and the last round.  Only
+    every second row sees it so; the others are ordinary rows of the same warps."""
+    Z, H, N = 5, 96, 512
+    q, k, v, _ = oracle.make_inputs(Z, N, H, D, seed=73)
+    scale = oracle.default_scale(D)
+    q[:, ::2, :, 0], q[:, 1::2, :, 0], k[..., 0] = 20.0, -20.0, 0.0
+    for z, leap in enumerate((95.0, 130.0, 180.0, 256.0, 400.0)):
+        for h in range(H):
+            column, half, rnd = h % 16, (h // 16) % 2, (0, 1, 3)[h // 32]
+            k[z, rnd * 128 + half * 64 + 16 * (h % 4) + column, h, 0] = leap / (20.0 * scale)
+    ref = _reference(q, k, v, scale, False)
+    for got in _run(q, k, v, scale, False):
+        _check(got, ref, _bound_few_keys(v, ref))
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_scores_of_large_standard_deviation(D):
+    """q and k ten times as large as usual: nearly all the weight of a row is on one key, and every row
+    meets its maximum somewhere in the middle.  Forward and gradients."""
+    from flash_attn_v100 import flash_attn_func
+
+    Z, H, N = 2, 4, 2048
+    q, k, v, dout = oracle.make_inputs(Z, N, H, D, seed=74)
+    q, k = q * 10, k * 10
+    scale = oracle.default_scale(D)
+    ref = _reference(q, k, v, scale, False)
+    for got in _run(q, k, v, scale, False):
+        _check(got, ref, _bound_few_keys(v, ref))
+    leaves = [t.cuda().requires_grad_() for t in (q, k, v)]
+    grads = torch.autograd.grad(flash_attn_func(*leaves), leaves, dout.cuda())
+    for z in range(Z):
+        qz, kz, vz, doz, oz = (t[z].float().transpose(0, 1) for t in (q, k, v, dout, ref[0]))
+        x = (qz @ kz.transpose(1, 2) * scale - ref[1][z][..., None])
+        p, dp = x.exp(), doz @ vz.transpose(1, 2)
+        delta = (doz * oz).sum(-1, keepdim=True)
+        ds = p * (dp - delta) * scale
+        # relative error of P: its fp16 argument (x / ln 2 in base 2), the fp16 exponential (2^-9.9) and
+        # its rounding; of dP, O (in delta), delta, P delta and dS: one fp16 rounding each
+        e_p = p * (x.abs() * 2.0 ** -11 + 2.0 ** -9.9 + 2.0 ** -11)
+        e_ds = scale * (e_p + p * 5 * 2.0 ** -11) * (dp.abs() + (doz * oz).abs().sum(-1, keepdim=True))
+        for got, want, bound in ((grads[0], ds @ kz, e_ds @ kz.abs()),
+                                 (grads[1], ds.transpose(1, 2) @ qz, e_ds.transpose(1, 2) @ qz.abs()),
+                                 (grads[2], p.transpose(1, 2) @ doz, e_p.transpose(1, 2) @ doz.abs())):
+            got = got[z].float().cpu().transpose(0, 1)
+            # ... and the result itself; 1e-4: weights below the fp16 range (6e-8 each, 2048 of them)
+            worst = ((got - want).abs() / (bound + want.abs() * 2.0 ** -11 + 1e-4 * 50)).max().item()
+            assert worst <= 1.0, worst
