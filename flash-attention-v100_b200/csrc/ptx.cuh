@@ -490,20 +490,31 @@ __device__ __forceinline__ float min3(float a, float b, float c) {
   asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
   return d;
 }
+// maxima that a NaN operand turns into NaN
+__device__ __forceinline__ float max_nan(float a, float b) {
+  float d;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b));
+  return d;
+}
+__device__ __forceinline__ float max3_nan(float a, float b, float c) {
+  float d;
+  asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
 // exp2 on the FMA / ALU pipes (no MUFU): x = n + f with n = floor(x) from a round-down add of
 // 1.5 * 2^23, 2^f on [0, 1) by the degree-4 polynomial with constant term 1 of least maximal
 // relative error (2.9e-6, found by iterated weighted least squares; an order of magnitude below
 // the fp16 rounding that P gets anyway), 2^n by adding n into the exponent field.  x is clamped to
 // >= -127, where the result is exactly 0 (a masked -inf score).  Above it is not: from 2^128 on the
 // exponent field wraps, and the result is anything.  `top` is raised to the largest floor(x) +
-// kPolyExp2Magic; where it exceeds kPolyExp2Top, the results are not to be used.  (One three-input
+// kPolyExp2Magic, or to NaN; where it is not <= kPolyExp2Top, the results are not to be used.  (One three-input
 // maximum per pair; a clamp from above would be two operations, on the pipe that is short of room.)
 // Works on a packed pair; the result is the packed pair of 2^x.
 constexpr float kPolyExp2Magic = 12582912.f, kPolyExp2Top = kPolyExp2Magic + 64.f;
 __device__ __forceinline__ uint64_t poly_exp2_pair(uint64_t x2, float& top) {
   uint32_t x0, x1;
   unpack2(x2, x0, x1);
-  x2 = pack2f(fmaxf(__uint_as_float(x0), -127.f), fmaxf(__uint_as_float(x1), -127.f));
+  x2 = pack2f(max_nan(__uint_as_float(x0), -127.f), max_nan(__uint_as_float(x1), -127.f));
   const uint64_t magic = pack2f(kPolyExp2Magic, kPolyExp2Magic);
   const uint64_t t2 = add2_rm(x2, magic);
   const uint64_t f2 = sub2(x2, sub2(t2, magic));
@@ -514,7 +525,7 @@ __device__ __forceinline__ uint64_t poly_exp2_pair(uint64_t x2, float& top) {
   uint32_t p0, p1, t0, t1;
   unpack2(p2, p0, p1);
   unpack2(t2, t0, t1);
-  top = max3(top, __uint_as_float(t0), __uint_as_float(t1));
+  top = max3_nan(top, __uint_as_float(t0), __uint_as_float(t1));
   // 2^n: n sits in the low mantissa bits of t; n * 2^23 added into the exponent field
   p0 += t0 << 23;
   p1 += t1 << 23;

@@ -78,6 +78,39 @@ def test_query_rows_that_are_not_finite(D, causal, shape):
         _check(got, ref, helpers.TOL_O_MAX_ABS)
 
 
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("D", [64, 96, 128])
+def test_a_key_row_that_is_nan(D, causal):
+    """NaN in one row of K, in another of 31 neighbouring columns from head to head: every row that sees
+    the key is NaN, whichever unit its exponential comes from, and no other (the last head has none)."""
+    Z, H, N = 8, 32, 512
+    q, k, v, _ = oracle.make_inputs(Z, N, H, D, seed=75)
+    scale = oracle.default_scale(D)
+    for z in range(Z):
+        for h in range(H - 1):
+            k[z, 64 * z + h, h, 7] = float("nan")
+    ref = _reference(q, k, v, scale, causal)
+    for got in _run(q, k, v, scale, causal):
+        _check(got, ref, helpers.TOL_O_MAX_ABS)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_a_value_row_that_is_not_finite(D):
+    """NaN and inf in V reach the column they are in, of every row."""
+    Z, H, N = 8, 32, 512
+    q, k, v, _ = oracle.make_inputs(Z, N, H, D, seed=76)
+    scale = oracle.default_scale(D)
+    for z in range(Z):
+        for h in range(H):
+            v[z, 64 * z + h, h, h] = float("nan") if h % 2 else float("inf")
+    r_out, r_lse = _reference(q, k, v, scale, False)
+    good = torch.isfinite(r_out)
+    for out, lse in _run(q, k, v, scale, False):
+        assert torch.equal(torch.isfinite(out), good)
+        assert oracle.max_abs(out[good].float(), r_out[good]) <= helpers.TOL_O_MAX_ABS
+        assert oracle.max_abs(lse, r_lse) <= helpers.TOL_LSE_MAX_ABS
+
+
 @pytest.mark.parametrize("shape", [MANY, FEW])
 @pytest.mark.parametrize("D", [64, 128])
 def test_rows_whose_first_keys_are_all_minus_inf(D, shape):
