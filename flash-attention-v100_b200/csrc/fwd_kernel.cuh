@@ -33,8 +33,7 @@
 //     warps is made warp-uniform for the compiler, slow paths are rolled loops;
 //   - no row maximum in the ordinary round (see the softmax groups), and the epilogue of an item waits
 //     for nothing;
-//   - 1/8 (D = 128) or 1/4 (D = 64) of the exponentials are a polynomial on the FMA pipe; more gives
-//     nothing (1/2: 6 % slower).
+//   - 1/8 of the exponentials are a polynomial on the FMA pipe (see kFwdPolyPairs).
 //
 // While the groups run an item's epilogue the producers and the MMA warp already work on the next
 // item, so that the load latency at the head of an item and the store at its tail are hidden.
@@ -89,8 +88,11 @@ struct FwdKernelParams {
   int row_elems;        // elements per row of the tensors (head_dim)
 };
 
-// pairs out of every 8 whose exponential is a polynomial on the FMA pipe (the rest use MUFU)
-constexpr int kFwdPolyPairsD128 = 1, kFwdPolyPairsD64 = 2;
+// Pairs out of every 8 whose exponential is a polynomial on the FMA pipe (the rest use MUFU).  None / 1 / 2
+// (3 at D = 64), us: D = 128, Z=8, H=32, N=2048 without a mask 551 / 537 / -, Z=1, H=16, N=16384 causal
+// 1136 / 1108 / -; D = 64, Z=2, H=16, N=8192 without a mask 799 / 783 / 784 (806), Z=64, H=16, N=512
+// 126.7 / 124.2 / 127.7 (131.8); no difference between none and 1 at D = 128, N = 2048 causal.
+constexpr int kFwdPolyPairs = 1;
 
 template <int D, bool kBf16 = false>
 struct FwdTraits {
@@ -106,7 +108,6 @@ struct FwdTraits {
   // Q tiles, K/V ring, one 64-column output box per softmax group
   static constexpr int kSmemBytes = 1024 + kTilesM * (kTileBytes + kBoxBytes) + kStages * kTileBytes;
   static constexpr int kTmemCols = 512;
-  static constexpr int kPolyPairs = (D == 128) ? kFwdPolyPairsD128 : kFwdPolyPairsD64;
   static constexpr uint32_t kIdescQK = umma_idesc_f16(128, kBlockN, 0, 0, kBf16);
   static constexpr uint32_t kIdescPV = umma_idesc_f16(128, D, 0, 1, kBf16);
 };
@@ -604,8 +605,8 @@ __global__ void __launch_bounds__(384, 1)
               for (int i = 0; i < 32; i += 2) {
                 const uint64_t x2 = fma2(pack2(s[cc][i], s[cc][i + 1]), c2, nm2);
                 uint64_t p2;
-                // kPolyPairs of every 8 pairs go through the FMA pipe instead of the MUFU unit
-                if (((i >> 1) & 7) < T::kPolyPairs) {
+                // kFwdPolyPairs of every 8 pairs go through the FMA pipe instead of the MUFU unit
+                if (((i >> 1) & 7) < kFwdPolyPairs) {
                   p2 = poly_exp2_pair(x2, top);
                 } else {
                   uint32_t x0, x1;

@@ -502,13 +502,15 @@ __device__ __forceinline__ float max3_nan(float a, float b, float c) {
   return d;
 }
 // exp2 on the FMA / ALU pipes (no MUFU): x = n + f with n = floor(x) from a round-down add of
-// 1.5 * 2^23, 2^f on [0, 1) by the degree-4 polynomial with constant term 1 of least maximal
-// relative error (2.9e-6, found by iterated weighted least squares; an order of magnitude below
-// the fp16 rounding that P gets anyway), 2^n by adding n into the exponent field.  x is clamped to
-// >= -127, where the result is exactly 0 (a masked -inf score).  Above it is not: from 2^128 on the
-// exponent field wraps, and the result is anything.  `top` is raised to the largest floor(x) +
-// kPolyExp2Magic, or to NaN; where it is not <= kPolyExp2Top, the results are not to be used.  (One three-input
-// maximum per pair; a clamp from above would be two operations, on the pipe that is short of room.)
+// 1.5 * 2^23, 2^f on [0, 1) by the degree-6 polynomial with constant term 1 of least maximal
+// relative error (2.0e-9, found by iterated weighted least squares), 2^n by adding n into the exponent
+// field.  Over all of fp32 it is off by 8.7e-8 at most, the hardware's ex2.approx by 1.46e-7.  (P is
+// rounded to 16 bits, but the row sum and the LSE are not.  Degree 4 is off by 2.9e-6, which showed in
+// the LSE; degree 5 by 1.65e-7, and the forward gets 0 to 1.5 % faster with it.)
+// x is clamped to >= -127, where the result is exactly 0 (a masked -inf score).  Above it is not: from
+// 2^128 on the exponent field wraps, and the result is anything.  `top` is raised to the largest
+// floor(x) + kPolyExp2Magic, or to NaN; where it is not <= kPolyExp2Top, the results are not to be
+// used.  (One three-input maximum per pair; a clamp from above would be two operations.)
 // Works on a packed pair; the result is the packed pair of 2^x.
 constexpr float kPolyExp2Magic = 12582912.f, kPolyExp2Top = kPolyExp2Magic + 64.f;
 __device__ __forceinline__ uint64_t poly_exp2_pair(uint64_t x2, float& top) {
@@ -518,9 +520,11 @@ __device__ __forceinline__ uint64_t poly_exp2_pair(uint64_t x2, float& top) {
   const uint64_t magic = pack2f(kPolyExp2Magic, kPolyExp2Magic);
   const uint64_t t2 = add2_rm(x2, magic);
   const uint64_t f2 = sub2(x2, sub2(t2, magic));
-  uint64_t p2 = fma2(f2, pack2f(0.0134266876f, 0.0134266876f), pack2f(0.0522424690f, 0.0522424690f));
-  p2 = fma2(p2, f2, pack2f(0.241280213f, 0.241280213f));
-  p2 = fma2(p2, f2, pack2f(0.693044841f, 0.693044841f));
+  uint64_t p2 = fma2(f2, pack2f(0.000216129163f, 0.000216129163f), pack2f(0.00124678458f, 0.00124678458f));
+  p2 = fma2(p2, f2, pack2f(0.00967545155f, 0.00967545155f));
+  p2 = fma2(p2, f2, pack2f(0.0554852821f, 0.0554852821f));
+  p2 = fma2(p2, f2, pack2f(0.240229309f, 0.240229309f));
+  p2 = fma2(p2, f2, pack2f(0.693147063f, 0.693147063f));
   p2 = fma2(p2, f2, pack2f(1.f, 1.f));
   uint32_t p0, p1, t0, t1;
   unpack2(p2, p0, p1);

@@ -193,3 +193,26 @@ def test_scores_of_large_standard_deviation(D):
             # ... and the result itself; 1e-4: weights below the fp16 range (6e-8 each, 2048 of them)
             worst = ((got - want).abs() / (bound + want.abs() * 2.0 ** -11 + 1e-4 * 50)).max().item()
             assert worst <= 1.0, worst
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_row_sum_where_the_polynomial_makes_up_most_of_it(D):
+    """LSE of rows with one key of score 0 and two of score -r / 1024 in columns whose exponential is a
+    polynomial, all else being far below; inputs and products are exact.  The exponential has to be
+    as good as the hardware's (2 ulp)."""
+    from flash_attn_v100 import cabi
+
+    n_q, n_k = 1024, 128
+    q, k = torch.zeros(1, n_q, 1, D), torch.zeros(1, n_k, 1, D)
+    q[0, :, 0, 0], q[0, :, 0, 1] = -torch.arange(n_q) / 1024, 1.0
+    k[0, :, 0, 1] = -1000.0
+    k[0, 8, 0] = 0.0
+    k[0, :2, 0, 0], k[0, :2, 0, 1] = 1.0, 0.0
+    v = torch.zeros(1, n_k, 1, D).half()
+    _, lse = cabi.fwd(q.half().cuda(), k.half().cuda(), v.cuda(), 1.0, False)
+    want = torch.log1p(2 * torch.exp(-torch.arange(n_q).double() / 1024))
+    # exponentials 2 ulp (2^-22) times their share of the sum (2/3); their arguments (up to 1.44 in base
+    # 2) two roundings; the sum two; the logarithm 1 ulp of up to 1.6, its product with ln 2 one
+    u = 2.0 ** -24
+    bound = 4 * u * 2 / 3 + 2 * u * 1.44 * 0.7 * 2 / 3 + 2 * u + 2 * u * 1.1 + u * 1.1
+    assert oracle.max_abs(lse[0, 0].cpu(), want) <= bound
