@@ -18,6 +18,8 @@
 
 #include <type_traits>
 
+#include "ptx.cuh"
+
 namespace fmha {
 
 struct Strides3 {
@@ -164,10 +166,10 @@ __global__ void __launch_bounds__(256)
     stat_idx = ((long long)z * heads + h) * acc_rows + row_offset + q;
     la = lse_acc[stat_idx];
     lb = lse_part[((long long)z * heads + h) * rows + q];
-    const float mx = fmaxf(la, lb);
+    const float mx = max_nan(la, lb);  // a part that is NaN makes the row NaN
     float wa = 0.f, wb = 0.f;
     ln = -CUDART_INF_F;
-    if (mx > -CUDART_INF_F) {
+    if (mx != -CUDART_INF_F) {
       const float ea = __expf(la - mx), eb = __expf(lb - mx);
       const float inv = 1.f / (ea + eb);
       wa = ea * inv;
@@ -178,7 +180,7 @@ __global__ void __launch_bounds__(256)
     // a row whose accumulated LSE is -inf holds nothing yet: its o_acc is not read (it may be
     // uninitialised memory), so the first merge of a row initialises it
     float4 a0 = make_float4(0.f, 0.f, 0.f, 0.f), a1 = a0;
-    if (la > -CUDART_INF_F) a0 = acc[0], a1 = acc[1];
+    if (la != -CUDART_INF_F) a0 = acc[0], a1 = acc[1];
     const uint4 up =
         *reinterpret_cast<const uint4*>(o_part + z * sp.batch + q * sp.row + h * sp.head + part * 8);
     float fp[8];

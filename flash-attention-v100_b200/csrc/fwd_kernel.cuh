@@ -711,10 +711,12 @@ __global__ void __launch_bounds__(384, 1)
         const int row = done.q0 + t * T::kBlockM + row_in_tile;
         const int nd = t == 0 ? done.n0 : done.n1;
         const bool split = done.chunk >= 0;
-        const float inv_l = (done_l > 0.f) ? 1.f / done_l : 0.f;
+        // (a row sum that is NaN leaves NaN in both: an LSE of -inf means that the row sees nothing, and
+        // whoever joins partial results leaves such a part out)
+        const float inv_l = (done_l == 0.f) ? 0.f : 1.f / done_l;
         if (row < p.seqlen_q) {
           const float lse =
-              (done_l > 0.f) ? (done_m * c + log2f(done_l)) * 0.6931471805599453f : -CUDART_INF_F;
+              (done_l == 0.f) ? -CUDART_INF_F : (done_m * c + log2f(done_l)) * 0.6931471805599453f;
           const size_t stat = (size_t)done.zh * p.seqlen_q + row;
           if (split) p.lse_part[(size_t)done.chunk * p.num_heads_total * p.seqlen_q + stat] = lse;
           else p.lse[stat] = lse;
@@ -821,26 +823,27 @@ __global__ void __launch_bounds__(256)
                                 p.chunk_tiles);
   if (chunks <= 1) return;
   const size_t stat = (size_t)zh * p.seqlen_q + row, plane = (size_t)p.num_heads_total * p.seqlen_q;
+  // a part that is NaN makes the row NaN
   float mx = -CUDART_INF_F;
-  for (int c = lane; c < chunks; c += 32) mx = fmaxf(mx, p.lse_part[c * plane + stat]);
+  for (int c = lane; c < chunks; c += 32) mx = max_nan(mx, p.lse_part[c * plane + stat]);
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-  const float base = mx > -CUDART_INF_F ? mx : 0.f;
+  for (int off = 16; off > 0; off >>= 1) mx = max_nan(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+  const float base = mx == -CUDART_INF_F ? 0.f : mx;
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
   float sum = 0.f;
   const int col = lane * 4;
   for (int c = 0; c < chunks; ++c) {
     const float lp = p.lse_part[c * plane + stat];
     if (lp == -CUDART_INF_F) continue;  // nothing visible in this chunk: its row was not written
-    const float w = expf(lp - base);
+    const float w = lp == base ? 1.f : expf(lp - base);  // (inf - inf would be NaN)
     sum += w;
     if (col < p.row_elems) {
       const float4 v = *reinterpret_cast<const float4*>(p.o_part + (c * plane + stat) * p.row_elems + col);
       acc.x += w * v.x, acc.y += w * v.y, acc.z += w * v.z, acc.w += w * v.w;
     }
   }
-  const float inv = sum > 0.f ? 1.f / sum : 0.f;
-  if (lane == 0) p.lse[stat] = sum > 0.f ? base + logf(sum) : -CUDART_INF_F;
+  const float inv = sum == 0.f ? 0.f : 1.f / sum;
+  if (lane == 0) p.lse[stat] = sum == 0.f ? -CUDART_INF_F : base + logf(sum);
   if (col < p.row_elems) {
     constexpr bool kBf16 = std::is_same<E, __nv_bfloat16>::value;
     uint2 v;

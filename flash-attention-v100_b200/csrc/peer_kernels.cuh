@@ -121,15 +121,15 @@ __global__ void __launch_bounds__(256)
   const long long zn = row_id / heads;
   const int n = (int)(zn % rows);
   const int z = (int)(zn / rows);
-  float mx = -CUDART_INF_F;
+  float mx = -CUDART_INF_F;  // NaN if any part is: then the row is
   for (int s = 0; s < parts.n; ++s) {
     const int r = n - parts.row0[s];
     if (r >= 0 && r < parts.rows[s])
-      mx = fmaxf(mx, parts.lse[s][((long long)z * heads + h) * parts.rows[s] + r]);
+      mx = max_nan(mx, parts.lse[s][((long long)z * heads + h) * parts.rows[s] + r]);
   }
   float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   float sum = 0.f;
-  if (mx > -CUDART_INF_F) {
+  if (mx != -CUDART_INF_F) {
     for (int s = 0; s < parts.n; ++s) {
       const int r = n - parts.row0[s];
       if (r < 0 || r >= parts.rows[s]) continue;
@@ -149,7 +149,7 @@ __global__ void __launch_bounds__(256)
   }
   *reinterpret_cast<uint4*>(out + row_id * DR + part * 8) = pack8<E>(f);
   if (part == 0)
-    lse_out[((long long)z * heads + h) * rows + n] = mx > -CUDART_INF_F ? mx + __logf(sum) : -CUDART_INF_F;
+    lse_out[((long long)z * heads + h) * rows + n] = mx != -CUDART_INF_F ? mx + __logf(sum) : -CUDART_INF_F;
 }
 
 }  // namespace fmha

@@ -11,7 +11,7 @@ from tests import helpers
 pytestmark = pytest.mark.gpu
 
 MANY = (30, 16, 256)  # 480 items of 256 query rows: more than three per SM
-FEW = (1, 2, 1024)    # 8 items: cut into chunks of the KV range where a workspace is given
+FEW = (1, 2, 1024)    # 8 items: cut into chunks of the KV range where the extension gives a workspace
 
 
 def _reference(q, k, v, scale, causal):
@@ -60,7 +60,7 @@ def _bound_few_keys(v, ref):
     return 2.0 ** -11 * (v.float().abs().max().item() + ref[0].abs().max().item())
 
 
-@pytest.mark.parametrize("shape", [MANY])
+@pytest.mark.parametrize("shape", [MANY, FEW])
 @pytest.mark.parametrize("causal", [False, True])
 @pytest.mark.parametrize("D", [64, 96, 128])
 def test_query_rows_that_are_not_finite(D, causal, shape):
@@ -92,6 +92,42 @@ def test_a_key_row_that_is_nan(D, causal):
     ref = _reference(q, k, v, scale, causal)
     for got in _run(q, k, v, scale, causal):
         _check(got, ref, helpers.TOL_O_MAX_ABS)
+
+
+@pytest.mark.parametrize("key", [0, 8, 700])
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("D", [64, 96, 128])
+def test_a_key_row_that_is_nan_in_one_of_several_chunks(D, causal, key):
+    """The chunk that holds the key is NaN for the rows that see it, the others are not: so is the result."""
+    Z, H, N = FEW
+    q, k, v, _ = oracle.make_inputs(Z, N, H, D, seed=77)
+    k[0, key, 0, 7] = float("nan")
+    scale = oracle.default_scale(D)
+    ref = _reference(q, k, v, scale, causal)
+    for got in _run(q, k, v, scale, causal):
+        _check(got, ref, helpers.TOL_O_MAX_ABS)
+
+
+@pytest.mark.parametrize("D", [64, 96, 128])
+def test_merged_partial_results_that_are_nan(D):
+    """Both merges of ring attention: a row that is NaN in any of its parts, or in all of them, is NaN."""
+    from flash_attn_v100 import cabi
+
+    Z, H, N = 1, 2, 128
+    q, k, v, _ = oracle.make_inputs(Z, N, H, D, seed=78, n_k=384)
+    k[0, 130, 0, 3] = float("nan")  # head 0: the second part of three
+    q[0, 5, 1, 3] = float("nan")    # head 1: row 5 of every part
+    r_out, r_lse = _reference(q, k, v, 0.1, False)
+    qd, kd, vd = q.cuda(), k.cuda(), v.cuda()
+    o_acc = torch.empty((Z, N, H, D), device="cuda")
+    l_acc = torch.full((Z, H, N), float("-inf"), device="cuda")
+    parts = [cabi.fwd(qd, kd[:, lo:lo + 128], vd[:, lo:lo + 128], 0.1, False) for lo in (0, 128, 256)]
+    for o, l in parts:
+        cabi.merge(o_acc, l_acc, o, l)
+    out, lse = torch.empty((Z, N, H, D), dtype=torch.float16, device="cuda"), torch.empty((Z, H, N), device="cuda")
+    cabi.merge_parts([o for o, _ in parts], [l for _, l in parts], [0, 0, 0], out, lse)
+    for got in ((o_acc.cpu(), l_acc.cpu()), (out.cpu(), lse.cpu())):
+        _check(got, (r_out, r_lse), helpers.TOL_O_MAX_ABS)
 
 
 @pytest.mark.parametrize("D", [64, 128])
