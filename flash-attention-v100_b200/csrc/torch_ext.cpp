@@ -18,6 +18,7 @@
 //     D = rowsum(dO o O) itself in fp32.
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/core/AutogradState.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/csrc/autograd/autograd_not_implemented_fallback.h>
 #include <torch/extension.h>
@@ -353,6 +354,11 @@ at::Tensor attention(const at::Tensor& q, const at::Tensor& k, const at::Tensor&
                      const OptTensor& seqused_k, bool deterministic) {
   TORCH_CHECK(q.dim() > 0 && k.dim() > 0 && v.dim() > 0, "q, k and v must have shape (batch, seqlen, heads, head_size)");
   const double scale = softmax_scale.has_value() ? *softmax_scale : std::pow((double)q.size(-1), -0.5);
+  // What autograd refuses has to be refused here, too: without gradients to record it is passed by.
+  if (c10::AutogradState::get_tls_state().get_fw_grad_mode())
+    for (const at::Tensor* t : {&q, &k, &v})
+      TORCH_CHECK_NOT_IMPLEMENTED(!t->_fw_grad(/*level=*/0).defined(),
+                                  "flash_attn_func has no forward-mode derivative (an input carries a tangent)");
   if (at::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad()))
     return AttentionFunction::apply(q, k, v, seqused_q, seqused_k, scale, causal, deterministic);
   at::AutoDispatchBelowADInplaceOrView guard;
