@@ -16,6 +16,7 @@
 //     still holds for a caller that uses the pair;
 //   - `bwd` ignores the fp16 `D` argument (flash_attn_interface.py:43-44) and computes
 //     D = rowsum(dO o O) itself in fp32.
+#include <ATen/FuncTorchTLS.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/core/AutogradState.h>
@@ -355,6 +356,7 @@ at::Tensor attention(const at::Tensor& q, const at::Tensor& k, const at::Tensor&
   TORCH_CHECK(q.dim() > 0 && k.dim() > 0 && v.dim() > 0, "q, k and v must have shape (batch, seqlen, heads, head_size)");
   const double scale = softmax_scale.has_value() ? *softmax_scale : std::pow((double)q.size(-1), -0.5);
   // What autograd refuses has to be refused here, too: without gradients to record it is passed by.
+  if (const auto& functorch = at::functorch::functorchTLSAccessor()) functorch->checkSupportsCppAutogradFunction();
   if (c10::AutogradState::get_tls_state().get_fw_grad_mode())
     for (const at::Tensor* t : {&q, &k, &v})
       TORCH_CHECK_NOT_IMPLEMENTED(!t->_fw_grad(/*level=*/0).defined(),

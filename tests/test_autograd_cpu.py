@@ -44,3 +44,19 @@ def test_a_forward_mode_tangent_is_refused(ops_on_cpu, which, no_grad, requires_
                 call(*inputs)
             with fw._set_fwd_grad_enabled(False):
                 call(*inputs)
+
+
+@pytest.mark.parametrize("no_grad", [False, True])
+def test_function_transforms_are_refused(ops_on_cpu, no_grad):
+    """vmap, grad and jvp, with and without gradients to record: the autograd function has no rules for them
+    (vmap would run the op in a loop over the batch)."""
+    for call in _calls():
+        q, k, v = _qkv()
+        with torch.set_grad_enabled(not no_grad):
+            with pytest.raises(RuntimeError, match="functorch"):
+                torch.vmap(lambda a: call(a, k, v))(torch.stack([q, q]))
+            with pytest.raises(RuntimeError, match="functorch"):
+                torch.func.grad(lambda a: call(a, k, v).sum())(q)
+            with pytest.raises(RuntimeError, match="functorch"):
+                torch.func.jvp(lambda a: call(a, k, v), (q,), (torch.ones_like(q),))
+            call(q, k, v)
