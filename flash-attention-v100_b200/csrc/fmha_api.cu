@@ -271,7 +271,7 @@ int fwd_head_group(const FmhaFwdParams* p) {
 // (96 runs at D = 128: the tensor maps describe 96 columns, the loads fill the rest of a
 // 128-wide tile with zeros and the stores clip it)
 template <int D, bool kBf16>
-int launch_fwd(const FmhaFwdParams* p, cudaStream_t stream) {
+int launch_fwd(const FmhaFwdParams* p, void* workspace, size_t workspace_bytes, cudaStream_t stream) {
   using T = fmha::FwdTraits<D, kBf16>;
   using E = typename std::conditional<kBf16, __nv_bfloat16, __half>::type;
   CUtensorMap tq, tk, tv, to;
@@ -288,8 +288,8 @@ int launch_fwd(const FmhaFwdParams* p, cudaStream_t stream) {
   const int dev = current_device();
   const int sms = std::max(1, sm_count(dev) - std::max(0, (int)p->sm_margin));
   FwdPlan plan;
-  if (p->workspace != nullptr) plan = plan_fwd(p, sms);
-  if (plan.workspace > p->workspace_bytes || plan.max_chunks <= 1) {
+  if (workspace != nullptr) plan = plan_fwd(p, sms);
+  if (plan.workspace > workspace_bytes || plan.max_chunks <= 1) {
     plan = FwdPlan();
     plan.items_per_head = (p->seqlen_q + 255) / 256;
   }
@@ -315,7 +315,7 @@ int launch_fwd(const FmhaFwdParams* p, cudaStream_t stream) {
   kp.o_part = nullptr;
   kp.lse_part = nullptr;
   if (plan.max_chunks > 1) {
-    kp.o_part = static_cast<float*>(p->workspace);
+    kp.o_part = static_cast<float*>(workspace);
     kp.lse_part = kp.o_part + (size_t)plan.max_chunks * kp.num_heads_total * p->seqlen_q * Dr;
   }
   auto kernel = fmha::fmha_fwd_kernel<D, kBf16>;
@@ -472,13 +472,15 @@ void* static_scratch_for_current_device(int* rc) {
 
 extern "C" {
 
-int fmha_fwd(const FmhaFwdParams* p, void* stream) {
+int fmha_fwd(const FmhaFwdParams* p, void* stream) { return fmha_fwd_with_workspace(p, nullptr, 0, stream); }
+
+int fmha_fwd_with_workspace(const FmhaFwdParams* p, void* workspace, size_t workspace_bytes, void* stream) {
   if (p == nullptr || p->q == nullptr || p->k == nullptr || p->v == nullptr || p->o == nullptr ||
       p->lse == nullptr)
     return FMHA_ERR_NULL_POINTER;
   int rc = check_common(p->batch, p->heads, p->seqlen_q, p->seqlen_k, p->head_dim, p->scale, p->dtype);
   if (rc) return rc;
-  if (!aligned16(p->q) || !aligned16(p->k) || !aligned16(p->v) || !aligned16(p->o) || !aligned16(p->workspace))
+  if (!aligned16(p->q) || !aligned16(p->k) || !aligned16(p->v) || !aligned16(p->o) || !aligned16(workspace))
     return FMHA_ERR_BAD_ALIGNMENT;
   if ((rc = check_strides(p->q_strides, p->seqlen_q, p->heads, p->batch))) return rc;
   if ((rc = check_strides(p->k_strides, p->seqlen_k, p->heads, p->batch))) return rc;
@@ -486,8 +488,10 @@ int fmha_fwd(const FmhaFwdParams* p, void* stream) {
   if ((rc = check_strides(p->o_strides, p->seqlen_q, p->heads, p->batch))) return rc;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (p->dtype == FMHA_DTYPE_BF16)
-    return p->head_dim > 64 ? launch_fwd<128, true>(p, s) : launch_fwd<64, true>(p, s);
-  return p->head_dim > 64 ? launch_fwd<128, false>(p, s) : launch_fwd<64, false>(p, s);
+    return p->head_dim > 64 ? launch_fwd<128, true>(p, workspace, workspace_bytes, s)
+                            : launch_fwd<64, true>(p, workspace, workspace_bytes, s);
+  return p->head_dim > 64 ? launch_fwd<128, false>(p, workspace, workspace_bytes, s)
+                          : launch_fwd<64, false>(p, workspace, workspace_bytes, s);
 }
 
 size_t fmha_fwd_workspace_bytes(const FmhaFwdParams* p) {
@@ -899,7 +903,7 @@ const char* fmha_status_string(int status) {
   }
 }
 
-const char* fmha_version(void) { return "0.2.0"; }
+const char* fmha_version(void) { return "0.3.0"; }
 
 #ifdef FMHA_TIMELINE
 // debug builds only: device buffer (>= 3 * 512 int64) and the CTA whose events are recorded

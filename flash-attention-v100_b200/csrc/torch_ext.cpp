@@ -130,12 +130,11 @@ std::vector<at::Tensor> fwd_impl(const at::Tensor& q, const at::Tensor& k, const
   p.seqused_q = seqused_ptr(seqused_q, q, "seqused_q");
   p.seqused_k = seqused_ptr(seqused_k, q, "seqused_k");
   at::Tensor ws;
-  if (const size_t ws_bytes = fmha_fwd_workspace_bytes(&p)) {
-    ws = empty_on(q, {static_cast<int64_t>(ws_bytes)}, at::kByte);
-    p.workspace = ws.data_ptr();
-    p.workspace_bytes = ws_bytes;
-  }
-  check_status(fmha_fwd(&p, at::cuda::getCurrentCUDAStream().stream()), "fmha_fwd");
+  const size_t ws_bytes = fmha_fwd_workspace_bytes(&p);
+  if (ws_bytes > 0) ws = empty_on(q, {static_cast<int64_t>(ws_bytes)}, at::kByte);
+  check_status(fmha_fwd_with_workspace(&p, ws_bytes > 0 ? ws.data_ptr() : nullptr, ws_bytes,
+                                       at::cuda::getCurrentCUDAStream().stream()),
+               "fmha_fwd");
   if (!want_sum) return {out, lse};
   return {out, lse, at::ones({B, H, Nq}, q.options().dtype(at::kFloat))};
 }

@@ -29,7 +29,8 @@ FMHA_DTYPE_FP16 = 0
 FMHA_DTYPE_BF16 = 1
 
 EXPORTED_SYMBOLS = (
-    "fmha_fwd", "fmha_fwd_workspace_bytes", "fmha_bwd_workspace_bytes", "fmha_bwd", "fmha_bwd_static_scratch", "fmha_bwd_convert_dq", "fmha_merge", "fmha_merge_rows", "fmha_b200_forward",
+    "fmha_fwd", "fmha_fwd_with_workspace", "fmha_fwd_workspace_bytes", "fmha_bwd_workspace_bytes", "fmha_bwd",
+    "fmha_bwd_static_scratch", "fmha_bwd_convert_dq", "fmha_merge", "fmha_merge_rows", "fmha_b200_forward",
     "fmha_b200_backward", "fmha_status_string", "fmha_version",
     "fmha_ipc_export", "fmha_ipc_open", "fmha_ipc_close", "fmha_peer_copy", "fmha_peer_copy_2d",
     "fmha_counter_bump", "fmha_peer_signal", "fmha_peer_wait", "fmha_sum_partials", "fmha_merge_parts",
@@ -51,7 +52,6 @@ class FmhaFwdParams(ctypes.Structure):
         ("scale", ctypes.c_float), ("causal", ctypes.c_int32), ("causal_shift", ctypes.c_int32),
         ("status", ctypes.c_void_p), ("sm_margin", ctypes.c_int32), ("dtype", ctypes.c_int32),
         ("seqused_q", ctypes.c_void_p), ("seqused_k", ctypes.c_void_p),
-        ("workspace", ctypes.c_void_p), ("workspace_bytes", ctypes.c_size_t),
     ]
 
 
@@ -89,6 +89,11 @@ def load_library() -> ctypes.CDLL:
     lib = ctypes.CDLL(_LIB_PATH)
     lib.fmha_fwd.restype = ctypes.c_int
     lib.fmha_fwd.argtypes = [ctypes.POINTER(FmhaFwdParams), ctypes.c_void_p]
+    lib.fmha_fwd_with_workspace.restype = ctypes.c_int
+    lib.fmha_fwd_with_workspace.argtypes = [ctypes.POINTER(FmhaFwdParams), ctypes.c_void_p, ctypes.c_size_t,
+                                            ctypes.c_void_p]
+    lib.fmha_fwd_workspace_bytes.restype = ctypes.c_size_t
+    lib.fmha_fwd_workspace_bytes.argtypes = [ctypes.POINTER(FmhaFwdParams)]
     lib.fmha_bwd_workspace_bytes.restype = ctypes.c_size_t
     lib.fmha_bwd_workspace_bytes.argtypes = [ctypes.POINTER(FmhaBwdParams)]
     lib.fmha_bwd.restype = ctypes.c_int

@@ -104,11 +104,6 @@ typedef struct {
    * the contract "the caller pads" (README.md:3) and computes the padding like real rows. */
   const int32_t* seqused_q;
   const int32_t* seqused_k;
-  /* Optional device scratch of fmha_fwd_workspace_bytes bytes, 16-byte aligned.  With it, a call whose
-   * query blocks alone would leave SMs idle (few queries over a long context) cuts their KV
-   * ranges into chunks and joins the partial results; without it such a call runs uncut. */
-  void* workspace;
-  size_t workspace_bytes;
 } FmhaFwdParams;
 
 typedef struct {
@@ -180,8 +175,16 @@ typedef struct {
 
 /* Forward: O = softmax(scale * Q K^T [+ causal mask]) V and LSE.
  * Replaces fused_mha_forward (include/fused_mha.h:1-2, kernel/fused_mha_kernel.cu:891-902). */
-size_t fmha_fwd_workspace_bytes(const FmhaFwdParams* p); /* 0 where a workspace would not be used */
 int fmha_fwd(const FmhaFwdParams* p, void* stream);
+
+/* The same with device scratch of fmha_fwd_workspace_bytes(p) bytes, 16-byte aligned.  With it, a call
+ * whose query blocks alone would leave SMs idle (few queries over a long context) cuts their KV
+ * ranges into chunks and joins the partial results; with less, or NULL, it runs uncut like fmha_fwd.
+ * fmha_fwd_workspace_bytes returns 0 where a workspace would not be used.  (An entry point of its own
+ * and not two more fields of FmhaFwdParams, which a host built against an earlier header of the
+ * library would not have.) */
+size_t fmha_fwd_workspace_bytes(const FmhaFwdParams* p);
+int fmha_fwd_with_workspace(const FmhaFwdParams* p, void* workspace, size_t workspace_bytes, void* stream);
 
 /* Bytes of device workspace the backward needs for these sizes: an fp32 dQ accumulator
  * (Z, seqlen_q, H, D) followed by fp32 lse * log2(e) and D = rowsum(dO * O), each (Z, H, seqlen_q

@@ -91,6 +91,26 @@ def test_forward_rejects_bad_strides(built_library):
     assert lib.fmha_fwd(None, None) == 1
 
 
+def test_forward_reads_nothing_behind_its_parameters(built_library):
+    """The struct ends with seqused_k, as in every header so far that hosts were built against: what lies
+    behind it in the host's memory is not the library's.  The workspace has an entry point of its own."""
+    from flash_attn_v100 import cabi
+
+    lib = cabi.load_library()
+
+    class WithTail(ctypes.Structure):
+        _fields_ = [("p", cabi.FmhaFwdParams), ("tail", ctypes.c_uint64 * 2)]
+
+    assert cabi.FmhaFwdParams.seqused_k.offset + 8 == ctypes.sizeof(cabi.FmhaFwdParams) == WithTail.tail.offset
+    host = WithTail(_fwd_params(cabi), (ctypes.c_uint64 * 2)(1, 1 << 30))
+    host.p.k_strides.row = 2 * 128 + 4  # refused after the alignments have been looked at
+    assert lib.fmha_fwd(ctypes.byref(host.p), None) == 4
+    assert lib.fmha_fwd_with_workspace(ctypes.byref(host.p), None, 0, None) == 4
+    assert lib.fmha_fwd_with_workspace(ctypes.byref(host.p), 0x1000, 1 << 20, None) == 4
+    assert lib.fmha_fwd_with_workspace(ctypes.byref(host.p), 0x1008, 1 << 20, None) == 5
+    assert lib.fmha_fwd_with_workspace(None, None, 0, None) == 1
+
+
 def test_backward_workspace_size_and_validation(built_library):
     from flash_attn_v100 import cabi
 
