@@ -130,8 +130,14 @@ std::vector<at::Tensor> fwd_impl(const at::Tensor& q, const at::Tensor& k, const
   p.seqused_q = seqused_ptr(seqused_q, q, "seqused_q");
   p.seqused_k = seqused_ptr(seqused_k, q, "seqused_k");
   at::Tensor ws;
-  const size_t ws_bytes = fmha_fwd_workspace_bytes(&p);
-  if (ws_bytes > 0) ws = empty_on(q, {static_cast<int64_t>(ws_bytes)}, at::kByte);
+  size_t ws_bytes = fmha_fwd_workspace_bytes(&p);
+  if (ws_bytes > 0) {
+    try {
+      ws = empty_on(q, {static_cast<int64_t>(ws_bytes)}, at::kByte);
+    } catch (const c10::OutOfMemoryError&) {
+      ws_bytes = 0;  // the call does not need it: uncut, it is only slower
+    }
+  }
   check_status(fmha_fwd_with_workspace(&p, ws_bytes > 0 ? ws.data_ptr() : nullptr, ws_bytes,
                                        at::cuda::getCurrentCUDAStream().stream()),
                "fmha_fwd");

@@ -57,6 +57,27 @@ def test_cut_query_blocks_of_a_padded_batch():
     _check((out, lse), (ref_o, ref_l))
 
 
+def test_no_memory_for_the_workspace():
+    """A call that would be cut runs uncut where the workspace cannot be had (here 97 MiB), as it did before
+    there was one."""
+    Z, H, N, D = 1, 1, 32768, 128
+    q, k, v, _ = oracle.make_inputs(Z, N, H, D, seed=66)
+    q, k, v = q.cuda(), k.cuda(), v.cuda()
+    scale = oracle.default_scale(D)
+    want = _fwd(q, k, v, scale, True)
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (60 << 20)) / total)
+    try:
+        with pytest.raises(torch.cuda.OutOfMemoryError):
+            torch.empty(90 << 20, dtype=torch.uint8, device="cuda")
+        got = _fwd(q, k, v, scale, True)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert oracle.max_abs(got[0].float(), want[0].float()) <= 2 * helpers.TOL_O_MAX_ABS
+    assert oracle.max_abs(got[1], want[1]) <= 2 * helpers.TOL_LSE_MAX_ABS
+
+
 @pytest.mark.parametrize("D", [64, 128])
 def test_runs_of_items_without_work(D):
     """Far more items than SMs, most of them of entries without a single row, in runs longer than the
@@ -76,7 +97,7 @@ def test_runs_of_items_without_work(D):
 
 
 @pytest.mark.parametrize("D", [64, 128])
-@pytest.mark.parametrize("first_large", [0, 64, 192, 448])
+@pytest.mark.parametrize("first_large", [0, 64, 128, 192, 448])
 def test_new_reference_in_mid_round(first_large, D):
     """Scores that leap by far more than 2^10 at a key in the first or second half of a 128-key round, in
     the first, a middle and the last round: the reference found before it must be replaced, the
