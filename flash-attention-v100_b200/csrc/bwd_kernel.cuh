@@ -37,7 +37,9 @@
 // the roles compete for shared memory (MMA operands, dQ staging, statistics) and for the
 // instruction cache.  The latter decides more than it seems: the same kernel with its MMA loops and
 // write-outs unrolled fetched 1.7 times the instructions from behind the first-level cache
-// and ran 10-18 % SLOWER than one CTA per item did, rolled up it is faster.  Hence the loops below.
+// and ran 5-18 % SLOWER than one CTA per item did, rolled up it is 5-10 % faster.  Hence the loops below.
+// They ease it and do not settle it: 1.04 stalled cycles per issue for want of instructions, 0.57
+// with one CTA per item (Z8 H32 N2048 D128 causal).
 // One CTA per item spent about 7 us of its life on its head and tail (a causal item at N = 2048 has
 // 8.5 tiles of 2.2 us).  Whole backward, one CTA per item -> this, steady state: Z8 H32 N2048 D128
 // causal 1025 -> 955 us, without a mask 1665 -> 1570, Z64 H16 N512 D64 422 -> 385, Z1 H16 N16384
@@ -652,7 +654,7 @@ __global__ void __launch_bounds__(512, 1)
 #pragma unroll 1
         for (int n = 0; n < it.cnt; ++n, ++g) {
           const int qbase = (it.i_begin + n) * T::kBlock;
-          const uint32_t sb = stat_smem + (g & 1) * T::kStatBytes;  // lse2 at [0, 512), delta at [512, 1024)
+          const uint32_t sb = stat_smem + (g & 1) * T::kStatBytes;  // -lse2 at 0, -delta at 512
 
           // first visible query column of this thread's half (>= 64: none)
           int first_visible = 0;

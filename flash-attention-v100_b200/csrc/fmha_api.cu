@@ -78,7 +78,8 @@ int make_accum_map(CUtensorMap* map, float* base, int Z, int N, int H, int D) {
   return r == CUDA_SUCCESS ? FMHA_OK : FMHA_ERR_TENSOR_MAP;
 }
 
-// debug builds (-DFMHA_TIMELINE) set these through fmha_debug_set_timeline; otherwise unused
+// debug builds (-DFMHA_TIMELINE) set these through fmha_debug_set_timeline for the backward kernel;
+// otherwise unused
 long long* g_timeline = nullptr;
 int g_timeline_block = 0;
 
@@ -196,6 +197,18 @@ BwdWorkspace carve_workspace(void* ws, int Z, int H, int Nq, int D) {
 // How the forward's work is cut.  A query block (256 rows) is one item unless that leaves SMs
 // idle: then its KV range is cut into chunks of chunk_tiles tiles, each an item of its own that
 // leaves an fp32 partial result, and a second kernel joins them.
+//
+// Measured, uncut / as cut by plan_fwd (chunks), us, fp16, D = 128:
+//   64 queries x 8192 keys     8 heads 115.0 / 25.8 (13), 32: 116.6 / 43.2 (4), 64: 117.0 / 69.8 (2)
+//   256 queries x 4096 keys    8 heads 59.5 / 26.8 (8), 64: 61.7 / 53.4 (2)
+//   causal, 1 head             N = 1024 24.2 / 22.7 (4), 4096 59.8 / 28.8 (8), 16384 214.5 / 113.7 (6)
+//   causal, 4 heads            N = 1024 24.3 / 22.7 (4), 4096 60.9 / 43.2 (3)
+// and what it leaves uncut, uncut / cut in two: 128 heads of 64 x 8192 120.7 / 139.5, 64 heads of 512 x
+// 2048 37.0 / 67.7, causal 16 heads N = 4096 63.6 / 97.9, 4 heads N = 16384 227.9 / 261.5.  Over 150 shapes
+// (D = 64 and 128, 1 to 296 heads) no cut of its was slower than none.  It is a rough estimate on
+// the cautious side: where the items are just fewer than the SMs a cut that it does not make
+// would be up to 1.4 times as fast (causal, 4 heads, N = 8192: 113.1 / 80.3), and under a mask fewer chunks
+// than it makes up to 1.3 times (1 head, N = 16384: 113.7 in 6, 86.6 in 4).
 // ---------------------------------------------------------------------------------------
 struct FwdPlan {
   int chunk_tiles = 1 << 30;
@@ -211,8 +224,8 @@ FwdPlan plan_fwd(const FmhaFwdParams* p, int sms) {
   const int nqb = (p->seqlen_q + 255) / 256, nk = (p->seqlen_k + 127) / 128;
   const double heads = (double)p->batch * p->heads;
   plan.items_per_head = nqb;
-  // In units of one round (256 query rows x 128 keys, about 1.2 us): an item costs its rounds and
-  // half a round of its own.
+  // In units of one round (256 query rows x 128 keys; about 1.2 us with the whole chip at work, 1.9 us
+  // with a few SMs): an item costs its rounds and half a round of its own.
   auto visible = [&](int qb) {
     return fmha::fwd_visible_tiles(causal, p->causal_shift, std::min(qb * 256 + 255, p->seqlen_q - 1), nk);
   };
@@ -261,7 +274,10 @@ FwdPlan plan_fwd(const FmhaFwdParams* p, int sms) {
 }
 
 // Heads whose items are interleaved in the forward's order, so that the last items are the short
-// ones of a causal mask: as many as have their K and V in 48 of the 126 MB of L2.
+// ones of a causal mask: as many as have their K and V in 48 of the 126 MB of L2.  One head at a time /
+// 24 / 48 / 96 / 1000 MB, us, fp16: Z8 H32 N2048 D128 causal 371 / 328 / 328 / 343 / 377, without a mask 607 /
+// 536 / 546 / 604 / 652, Z4 H32 N4096 causal 637 / 572 / 561 / 592 / 648, Z2 H32 N8192 without a mask 2038 /
+// 1973 / 1988 / 2070 / 2161.
 int fwd_head_group(const FmhaFwdParams* p) {
   const double kv_bytes = 4.0 * p->seqlen_k * p->head_dim;
   return (int)std::max(1.0, std::min((double)p->batch * p->heads, 48e6 / kv_bytes));

@@ -23,16 +23,17 @@
 // its operands with the TMA writes are 256 KB, which at 128 bytes/clk is 2048 clk as well; a round takes
 // 2850 clk with the exponentials left out and 3250 with them (1500-1700 clk per group).  At D = 64
 // it is the softmax groups.  What made it faster than S tiles of 64 keys, double buffered, with two
-// issuing warps (Z=8, H=32, N=2048 / Z=1, N=16384 sustained, TFLOP/s; D=128 without a mask 947 / 1055
-// -> 1024 / 1195, causal 847 / 1057 -> 902 / 1136; D=64 614 -> 698):
+// issuing warps (us, that form -> this one, sustained, in turn in one process; D = 128, Z=8, H=32, N=2048 without
+// a mask, bf16 636 -> 531, causal, bf16 345 -> 312, Z=1, H=16, N=16384 without a mask, fp16 2608 -> 1918, causal, bf16
+// 1175 -> 1055; D = 64, Z=2, H=16, N=8192 without a mask, fp16 1005 -> 759):
 //   - S tiles of 128 keys read Q from shared memory half as often;
 //   - the turns come in a fixed order, which keeps the two softmax groups half a round apart: while
 //     one group's exponentials run, the tensor pipe works for the other;
 //   - the code is small: the roles of a CTA share one instruction cache, and at 200 KB of code the MMA
 //     warp waited for instructions (2850 clk of a round became 4000).  Control flow of the issuing
 //     warps is made warp-uniform for the compiler, slow paths are rolled loops;
-//   - no row maximum in the ordinary round (see the softmax groups), and the epilogue of an item waits
-//     for nothing;
+//   - no row maximum in the ordinary round (see the softmax groups; what has to be watched instead, so
+//     that no score is too large for it, costs 1 %), and the epilogue of an item waits for nothing;
 //   - 1/8 of the exponentials are a polynomial on the FMA pipe (see kFwdPolyPairs).
 //
 // While the groups run an item's epilogue the producers and the MMA warp already work on the next

@@ -11,10 +11,11 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-// Timeline instrumentation, compiled in only with -DFMHA_TIMELINE: the chosen CTA's elected
-// threads store clock64() at pipeline events so that stalls can be located without a profiler.
+// Timeline instrumentation of the backward kernel, compiled in only with -DFMHA_TIMELINE: the chosen
+// CTA's elected threads store clock64() at pipeline events so that stalls can be located without a
+// profiler.
 #ifndef FMHA_ABLATE
-#define FMHA_ABLATE 0  // debug builds: bit 0 no exp2, bit 1 no row max, bit 2 no P store
+#define FMHA_ABLATE 0  // debug builds: bit 0 no exp2
 #endif
 #ifdef FMHA_TIMELINE
 #define FMHA_TL(role, j, k)                                                        \
@@ -373,18 +374,6 @@ __device__ __forceinline__ void umma_ts_elect(uint32_t d_tmem, uint32_t a_tmem, 
 __device__ __forceinline__ void umma_commit_elect(uint32_t bar) {
   if (elect_one()) umma_commit(bar);
 }
-// has the phase completed?  A single test by a whole converged warp, without waiting.
-__device__ __forceinline__ bool mbar_probe_warp(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return __all_sync(0xffffffffu, ok != 0);
-}
 // bounded wait by a whole converged warp, with a warp-uniform result
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity,
                                                volatile int* abort_word, int who) {
@@ -479,15 +468,10 @@ __device__ __forceinline__ uint64_t add2_rm(uint64_t a, uint64_t b) {
   asm("add.rm.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
 }
-// three-input maximum / minimum
+// three-input maximum
 __device__ __forceinline__ float max3(float a, float b, float c) {
   float d;
   asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-  return d;
-}
-__device__ __forceinline__ float min3(float a, float b, float c) {
-  float d;
-  asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
   return d;
 }
 // maxima that a NaN operand turns into NaN
