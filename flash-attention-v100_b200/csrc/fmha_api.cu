@@ -102,15 +102,22 @@ int sm_count(int dev) {
   return n;
 }
 
-// Raises a kernel's dynamic shared-memory limit, once per kernel and device.
-template <auto kKernel>
-bool allow_smem(int dev, int bytes) {
-  static std::atomic<bool> done[kMaxDevices];
-  if (dev >= 0 && done[dev].load(std::memory_order_acquire)) return true;
-  if (cudaFuncSetAttribute(kKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess)
-    return false;
-  if (dev >= 0) done[dev].store(true, std::memory_order_release);
-  return true;
+// Launches a kernel whose dynamic shared memory needs its limit raised, which is done once per kernel and
+// device, and again where a launch is refused: the limit goes with the context when the host resets
+// the device.
+template <auto kKernel, typename... Args>
+bool launch_with_smem(int dev, unsigned grid, unsigned threads, int bytes, cudaStream_t stream, const Args&... args) {
+  static std::atomic<bool> raised[kMaxDevices];
+  for (int attempt = 0; attempt < 2; ++attempt) {
+    if (attempt > 0 || dev < 0 || !raised[dev].load(std::memory_order_acquire)) {
+      if (cudaFuncSetAttribute(kKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess)
+        return false;
+      if (dev >= 0) raised[dev].store(true, std::memory_order_release);
+    }
+    kKernel<<<grid, threads, bytes, stream>>>(args...);
+    if (cudaGetLastError() == cudaSuccess) return true;
+  }
+  return false;
 }
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
@@ -334,14 +341,13 @@ int launch_fwd(const FmhaFwdParams* p, void* workspace, size_t workspace_bytes, 
     kp.o_part = static_cast<float*>(workspace);
     kp.lse_part = kp.o_part + (size_t)plan.max_chunks * kp.num_heads_total * p->seqlen_q * Dr;
   }
-  auto kernel = fmha::fmha_fwd_kernel<D, kBf16>;
-  if (!allow_smem<fmha::fmha_fwd_kernel<D, kBf16>>(dev, T::kSmemBytes)) return FMHA_ERR_LAUNCH;
   // One block per item, taken over by running blocks; dealt out instead where every item has an SM
   // of its own (nothing to take over) or the caller wants SMs left free.
   kp.deal = kp.num_items <= sms || p->sm_margin > 0;
   const unsigned grid = kp.deal ? (unsigned)std::min(kp.num_items, sms) : (unsigned)kp.num_items;
-  kernel<<<grid, T::kThreads, T::kSmemBytes, stream>>>(tq, tk, tv, to, kp);
-  if (cudaGetLastError() != cudaSuccess) return FMHA_ERR_LAUNCH;
+  if (!launch_with_smem<fmha::fmha_fwd_kernel<D, kBf16>>(dev, grid, T::kThreads, T::kSmemBytes, stream, tq, tk, tv, to,
+                                                         kp))
+    return FMHA_ERR_LAUNCH;
   if (plan.max_chunks > 1) {
     const long long rows = (long long)kp.num_heads_total * (p->seqlen_q - plan.first_cut_row);
     fmha::fmha_fwd_combine_kernel<E><<<(unsigned)((rows + 7) / 8), 256, 0, stream>>>(
@@ -424,14 +430,14 @@ int launch_bwd(const FmhaBwdParams* p, const BwdWorkspace& w, cudaStream_t strea
     // One block per item, taken over by running blocks.  Not where every item has an SM of its own,
     // nor in the deterministic mode: an item waits there for items with lower indices, and only the
     // order in which blocks are dispatched says that these are under way.
-    kp.deal = (int)grid <= sm_count(current_device()) || kp.dq_order != nullptr;
+    const int dev = current_device();
+    kp.deal = (int)grid <= sm_count(dev) || kp.dq_order != nullptr;
     kp.timeline = g_timeline;
     kp.timeline_block = g_timeline_block;
-    auto kernel = fmha::fmha_bwd_kernel<D, kBf16, DR>;
     constexpr int smem = fmha::bwd_smem_bytes<D, kBf16>();
-    if (!allow_smem<fmha::fmha_bwd_kernel<D, kBf16, DR>>(current_device(), smem)) return FMHA_ERR_LAUNCH;
-    kernel<<<grid, T::kThreads, smem, stream>>>(tq, tk, tv, tdo, tdk, tdv, tacc, kp);
-    if (cudaGetLastError() != cudaSuccess) return FMHA_ERR_LAUNCH;
+    if (!launch_with_smem<fmha::fmha_bwd_kernel<D, kBf16, DR>>(dev, grid, T::kThreads, smem, stream, tq, tk, tv, tdo, tdk,
+                                                               tdv, tacc, kp))
+      return FMHA_ERR_LAUNCH;
   }
 
   if (!(p->flags & FMHA_BWD_SKIP_DQ_CONVERT)) {
