@@ -212,10 +212,12 @@ def fwd_params(q, k, v, o, lse, scale, causal, causal_shift=0, status=None, sm_m
 def fwd(q, k, v, scale: float, causal: bool = False, causal_shift: int = 0,
         out: Optional[torch.Tensor] = None, lse: Optional[torch.Tensor] = None,
         status: Optional[torch.Tensor] = None, stream=None, sm_margin: int = 0,
-        seqused_q: Optional[torch.Tensor] = None, seqused_k: Optional[torch.Tensor] = None):
+        seqused_q: Optional[torch.Tensor] = None, seqused_k: Optional[torch.Tensor] = None,
+        workspace: Optional[torch.Tensor] = None):
     """O, LSE through ``fmha_fwd`` on the current (or given) stream; outputs allocated with torch
     unless passed in.  ``sm_margin``: SMs the persistent kernel leaves to other streams' kernels.
-    ``seqused_q`` / ``seqused_k``: per-batch real lengths of right-padded batches (int32)."""
+    ``seqused_q`` / ``seqused_k``: per-batch real lengths of right-padded batches (int32).
+    ``workspace``: a contiguous CUDA tensor as scratch for ``fmha_fwd_with_workspace``."""
     _require_cuda_half(q, k, v, out)
     Z, Nq, H, D = q.shape
     if out is None:
@@ -224,7 +226,9 @@ def fwd(q, k, v, scale: float, causal: bool = False, causal_shift: int = 0,
         lse = torch.empty((Z, H, Nq), dtype=torch.float32, device=q.device)
     p = fwd_params(q, k, v, out, lse, scale, causal, causal_shift, status, sm_margin, seqused_q, seqused_k)
     with torch.cuda.device(q.device):
-        _check(load_library().fmha_fwd(ctypes.byref(p), _stream(stream)), "fmha_fwd")
+        nbytes = 0 if workspace is None else workspace.numel() * workspace.element_size()
+        _check(load_library().fmha_fwd_with_workspace(ctypes.byref(p), _ptr(workspace), nbytes, _stream(stream)),
+               "fmha_fwd")
     return out, lse
 
 

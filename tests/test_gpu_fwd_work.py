@@ -1,6 +1,9 @@
 """GPU parity tests of how the forward kernel's work is cut and taken: query blocks whose KV range is
 cut into chunks (partial results joined by a second kernel), items taken over through cluster
 launch control, runs of items with nothing to do, and a new softmax reference in mid-round."""
+import ctypes
+import random
+
 import pytest
 import torch
 
@@ -55,6 +58,52 @@ def test_cut_query_blocks_of_a_padded_batch():
         r = oracle.attention_forward(q[z:z + 1, :sq[z]], k[z:z + 1, :sk[z]], v[z:z + 1, :sk[z]], scale, False)
         ref_o[z, :sq[z]], ref_l[z, :, :sq[z]] = r[0][0], r[1][0]
     _check((out, lse), (ref_o, ref_l))
+
+
+# seeds whose sizes make a call that is cut
+@pytest.mark.parametrize("seed", [1, 4, 8, 12, 15, 19, 21, 25, 29, 30, 44, 52, 64, 71, 72, 76])
+def test_cut_and_uncut_calls_agree(seed):
+    """The same call with and without a workspace, over what the C ABI takes: odd lengths, shifted masks,
+    per-batch lengths (zero among them), packed and transposed tensors, all head dims and types, SMs
+    left free; a workspace one byte short is as good as none."""
+    from flash_attn_v100 import cabi
+
+    rng = random.Random(seed)
+    Z, H, D = rng.choice([1, 2]), rng.choice([1, 3]), (64, 96, 128)[seed % 3]
+    n_q, n_k = rng.choice([1, 33, 200, 513]), rng.choice([1025, 1999, 4000])
+    if seed % 4 == 1:
+        n_q = n_k = rng.choice([1025, 1999])
+    dtype = rng.choice([torch.float16, torch.bfloat16])
+    causal = seed % 4 == 1 or rng.random() < 0.4
+    shift = 0 if not causal else rng.choice([0, n_k - n_q, 700, -150 if n_q > 150 else 0])
+    layout = rng.choice(["dense", "packed", "heads first"])
+    g = torch.Generator(device="cuda").manual_seed(seed)
+
+    def tensor(n):
+        x = torch.randn((Z, n, H, D), generator=g, device="cuda").to(dtype)
+        if layout == "packed":
+            return x.unsqueeze(2).expand(Z, n, 3, H, D).contiguous()[:, :, 1]
+        return x.transpose(1, 2).contiguous().transpose(1, 2) if layout == "heads first" else x
+
+    q, k, v, out = tensor(n_q), tensor(n_k), tensor(n_k), tensor(n_q)
+    lens = [None, None]
+    if rng.random() < 0.5:
+        lens = [torch.tensor([rng.choice([n, n // 2 + 1] + [0] * z) for z in range(Z)], dtype=torch.int32, device="cuda")
+                for n in (n_q, n_k)]
+    kw = dict(sm_margin=rng.choice([0, 0, 20]), seqused_q=lens[0], seqused_k=lens[1])
+    scale = rng.choice([1, -1]) * D ** -0.5
+    want = cabi.fwd(q, k, v, scale, causal, shift, **kw)
+    lse = torch.empty((Z, H, n_q), device="cuda")
+    p = cabi.fwd_params(q, k, v, out, lse, scale, causal, shift, **kw)
+    nbytes = cabi.load_library().fmha_fwd_workspace_bytes(ctypes.byref(p))
+    assert nbytes > 0, "not a call that is cut"
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    guard = torch.full((nbytes + 256,), 0xFF, dtype=torch.uint8, device="cuda")  # NaN
+    cabi.fwd(q, k, v, scale, causal, shift, out=out, lse=lse, status=status, workspace=guard[:nbytes], **kw)
+    assert int(status.item()) == 0 and bool((guard[nbytes:] == 0xFF).all())
+    _check((out.cpu(), lse.cpu()), (want[0].float().cpu(), want[1].cpu()), dtype)
+    short = cabi.fwd(q, k, v, scale, causal, shift, workspace=guard[:nbytes - 1], **kw)
+    assert torch.equal(short[0], want[0]) and torch.equal(short[1], want[1])
 
 
 def test_no_memory_for_the_workspace():
