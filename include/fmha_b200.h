@@ -36,7 +36,8 @@
  *    (README.md:3) is enforced one level up, by the torch extension's `fwd` / `bwd`.
  *  - Thread safety: entry points may be called from any thread with the target device
  *    current.  The only process-wide state is read-mostly: the resolved driver entry point
- *    for tensor-map encoding, and, for fmha_bwd_static_scratch, the per-device address of the
+ *    for tensor-map encoding, per device the number of SMs and whether the kernels' shared-memory
+ *    limits have been raised (done again where the device was reset), and, for fmha_bwd_static_scratch, the per-device address of the
  *    built-in scratch area (looked up once per device ordinal in the primary context; it
  *    goes stale if that context is destroyed with cudaDeviceReset) and the area itself,
  *    which every call of that entry point on a device shares (see there).
