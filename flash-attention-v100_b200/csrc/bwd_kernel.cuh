@@ -74,10 +74,9 @@ struct BwdKernelParams {
   int causal, causal_shift;
   int* status;
   // Deterministic dQ (not NULL): one word per (batch*head, query tile), zero at launch.  The
-  // CTAs that add into a query tile's dQ do so in the order of their KV tiles: CTA kb waits
-  // for the word to reach kb, adds, waits for its adds to complete and sets kb + 1.  The fp32
-  // additions then happen in one fixed order and dQ is the same bits on every run; the price
-  // is that the CTAs of a head run staggered by one query tile each.
+  // CTAs that add into a query tile's dQ take turns (bwd_turn): a CTA waits for the word to reach
+  // its turn, adds, and once its adds have completed sets turn + 1.  The fp32 additions then
+  // happen in one fixed order and dQ is the same bits on every run.
   int* dq_order;
   // optional per-batch lengths (right-padded batches), see FmhaBwdParams
   const int* seqused_q;
@@ -156,6 +155,7 @@ constexpr int bwd_smem_bytes() {
 // items in work at any time still belong to a handful of heads (their Q / dO tiles and dQ
 // accumulators stay in L2), and what comes last, at the end of a group and of the grid, are the
 // short ones.  head_group = 1: all items of a head in a row.
+template <bool kDet>
 __device__ __forceinline__ BwdItem bwd_item(const BwdKernelParams& p, int id) {
   BwdItem it;
   it.id = id;
@@ -164,6 +164,7 @@ __device__ __forceinline__ BwdItem bwd_item(const BwdKernelParams& p, int id) {
   const int heads_here = min(p.head_group, p.num_heads_total - group * p.head_group);
   it.zh = group * p.head_group + within % heads_here;
   it.kb = within / heads_here;
+  if (kDet && p.causal) it.kb = p.num_kv_blocks - 1 - it.kb;  // see bwd_turn
   it.z = it.zh / p.heads;
   it.h = it.zh % p.heads;
   // the lengths that count for this batch entry: query tiles and keys beyond them are padding
@@ -182,10 +183,26 @@ __device__ __forceinline__ BwdItem bwd_item(const BwdKernelParams& p, int id) {
   return it;
 }
 
+// Deterministic dQ: the turn of an item's KV tile among those that add into a query tile.  An item only
+// ever waits for items with lower indices, whose blocks are dispatched before its own.
+// Without a mask: KV tile after KV tile, and the items of a head run staggered by one query tile each.
+// Under a causal mask: from the diagonal downwards, and the items of a head are dispatched in that order.
+// The item on the diagonal comes first to its query tile, the one below it a tile later, and so on: no item
+// waits that has not been held up itself.  (In ascending order the item of KV tile kb had to wait for all kb
+// before it when it came to its first query tile.  Whole backward, us, ascending / so: Z2 H16 N2048 D128 256 / 206,
+// Z8 H32 N2048 D128 1777 / 1313, Z1 H8 N16384 D128 4272 / 2229, Z4 H16 N1024 D64 138 / 100.)
+__device__ __forceinline__ int bwd_turn(const BwdKernelParams& p, const BwdItem& it, int tile) {
+  if (!p.causal) return it.kb;
+  const long long diagonal = ((long long)(tile + 1) * 128 + p.causal_shift - 1) / 128;  // last KV tile it sees
+  return (int)min(diagonal, (long long)(it.sk - 1) / 128) - it.kb;
+}
+
 // DR <= D: elements per row of the tensors.  96 runs at D = 128: the tile loads fill columns
 // 96-127 with zeros, so those columns of dQ, dK and dV are zeros that are never written out, and
 // the fp32 buffers have DR elements per row.
-template <int D, bool kBf16 = false, int DR = D>
+// kDet: deterministic dQ, with the items dealt out.  An instantiation of its own: the turns cost the other mode
+// 1 to 3 % when they were a branch in the dQ group's loop.
+template <int D, bool kBf16 = false, int DR = D, bool kDet = false>
 __global__ void __launch_bounds__(512, 1)
     fmha_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                     const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
@@ -255,7 +272,7 @@ __global__ void __launch_bounds__(512, 1)
       fence_barrier_init();
     }
     __syncwarp();
-    const BwdItem it = bwd_item(p, blockIdx.x);
+    const BwdItem it = bwd_item<kDet>(p, blockIdx.x);
     if (it.cnt > 0) {
       const int row0 = it.i_begin * T::kBlock;
       send(3, &tm_q, it, row0, true);
@@ -317,7 +334,7 @@ __global__ void __launch_bounds__(512, 1)
       uint32_t published = 0, asked = 0;
       bool pending = false;  // a request is out
       auto ask = [&]() {
-        if (p.deal || pending) return;
+        if (kDet || p.deal || pending) return;
         if (elect_one()) {
           fence_proxy_async_smem();  // the last answer has been read
           mbar_arrive_expect_tx(smem_u32(&sh.bar_clc), 16);
@@ -356,7 +373,7 @@ __global__ void __launch_bounds__(512, 1)
         for (;; first = false) {
           if (first) {
             id = blockIdx.x;
-          } else if (p.deal) {
+          } else if (kDet || p.deal) {
             id = -1;
           } else {
             ask();
@@ -369,7 +386,7 @@ __global__ void __launch_bounds__(512, 1)
           it.id = -1;
           it.cnt = 0;
           if (id < 0) break;
-          it = bwd_item(p, id);
+          it = bwd_item<kDet>(p, id);
           it.cnt = __shfl_sync(0xffffffffu, it.cnt, 0);
           if (it.cnt > 0) break;
           ask();
@@ -817,8 +834,12 @@ __global__ void __launch_bounds__(512, 1)
           __syncwarp();
           if (lane == 0) mbar_arrive(smem_u32(&sh.bar_dq_empty));
           if (tl) FMHA_TL(1, g, 2);
-          int* const order_word =
-              p.dq_order == nullptr ? nullptr : p.dq_order + (size_t)it.zh * (p.seqlen_q_pad / T::kBlock) + tile;
+          int* order_word = nullptr;
+          int turn = 0;
+          if constexpr (kDet) {
+            order_word = p.dq_order + (size_t)it.zh * (p.seqlen_q_pad / T::kBlock) + tile;
+            turn = bwd_turn(p, it, tile);
+          }
 #pragma unroll
           for (int cc = 0; cc < kChunks; ++cc) {
             // One reduce-add per 32-column chunk for the whole 128-row tile (16 KB): few large
@@ -841,18 +862,18 @@ __global__ void __launch_bounds__(512, 1)
             fence_proxy_async_smem();
             named_bar_sync(2, 128);
             if (r == 0) {
-              if (order_word != nullptr && cc == 0) {
-                // the KV tiles before this one have added their share of this query tile
-                global_flag_wait(order_word, it.kb, &sh.abort_word, p.status, 17);
+              if (kDet && cc == 0) {
+                // those whose turn comes before have added their share of this query tile
+                global_flag_wait(order_word, turn, &sh.abort_word, p.status, 17);
                 fence_proxy_async_all();
               }
               tma_reduce_add_4d(&tm_dqacc, stg_buf, cc * 32, tile * T::kBlock, it.h, it.z);
               tma_commit_group();
-              if (order_word != nullptr && cc == kChunks - 1) {
+              if (kDet && cc == kChunks - 1) {
                 tma_wait_group<0>();  // the adds have been performed, not just read from shared memory
                 fence_proxy_async_all();
                 __threadfence();
-                global_flag_release(order_word, it.kb + 1);
+                global_flag_release(order_word, turn + 1);
               }
             }
           }

@@ -160,10 +160,10 @@ typedef struct {
  * before the first K/V block arrives, and for timing the three kernels of a backward pass one by
  * one.  Not combinable with FMHA_BWD_KEEP_WORKSPACE (FMHA_ERR_WORKSPACE). */
 #define FMHA_BWD_PREPROCESS_ONLY 4
-/* Deterministic dQ: the fp32 partial sums of dQ from different key/value tiles are added in the
- * order of the tiles instead of the order in which they happen to finish, so dQ is bit-for-bit
- * the same on every run (dK, dV, O and LSE always are).  The CTAs of a (batch, head) then run
- * staggered, one query tile apart, which costs up to a factor of two in the fused kernel.  The
+/* Deterministic dQ: the fp32 partial sums of dQ from different key/value tiles are added in a
+ * fixed order instead of the order in which they happen to finish, so dQ is bit-for-bit
+ * the same on every run (dK, dV, O and LSE always are).  The CTAs of a (batch, head) then wait
+ * for one another, which costs up to a factor of two in the fused kernel.  The
  * reference's dQ is a 64-way fp16 atomicAdd (kernel/fused_mha_kernel.cu:543,693) and has no
  * such mode.  The order words live in the workspace (fmha_bwd_workspace_bytes accounts for
  * them) and are cleared by every call that carries the flag. */

@@ -1,0 +1,58 @@
+"""GPU tests of the order in which deterministic dQ is added: under a causal mask from the diagonal
+downwards, where the diagonal depends on the shift and on the lengths of a padded batch."""
+import pytest
+import torch
+
+from oracle import attention_oracle as oracle
+from tests import helpers
+from tests.test_gpu_padded import _oracle_padded
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("H,n_q,n_k,causal,shift", [
+    (40, 640, 640, True, 0),      # more items than SMs, several head groups, the last one not full
+    (3, 640, 640, True, 37),      # the diagonal crosses tiles
+    (3, 640, 640, True, -200),    # query rows that see nothing
+    (3, 256, 1000, True, 300),    # KV tiles that no query sees
+    (3, 1000, 256, True, 0),      # more query tiles than KV tiles
+    (3, 300, 300, True, 100000),  # every key seen
+    (40, 640, 384, False, 0),
+])
+@pytest.mark.parametrize("D", [64, 96, 128])
+def test_order_of_dq(H, n_q, n_k, causal, shift, D):
+    from flash_attn_v100 import cabi
+
+    q, _, _, dout = oracle.make_inputs(1, n_q, H, D, seed=91)
+    _, k, v, _ = oracle.make_inputs(1, n_k, H, D, seed=92)
+    scale = oracle.default_scale(D)
+    qd, kd, vd, dod = (t.cuda() for t in (q, k, v, dout))
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    out, lse = cabi.fwd(qd, kd, vd, scale, causal, shift)
+    runs = [cabi.bwd(qd, kd, vd, out, dod, lse, scale, causal, shift, flags=cabi.FMHA_BWD_DETERMINISTIC, status=status)
+            for _ in range(2)]
+    assert int(status.item()) == 0
+    assert all(torch.equal(a, b) for a, b in zip(*runs))
+    ref = oracle.attention_fwd_bwd(q, k, v, dout, scale, causal, shift)
+    helpers.check_against_oracle((out.cpu(), lse.cpu(), *(t.cpu() for t in runs[0])), ref, f"order D{D}")
+
+
+@pytest.mark.parametrize("q_row_begin", [0, 256])
+def test_order_of_dq_in_a_padded_batch(q_row_begin):
+    from flash_attn_v100 import cabi
+
+    Z, N, H, D = 5, 640, 4, 128
+    sq, sk = [640, 130, 0, 513, 300], [640, 640, 128, 1, 0]
+    q, k, v, dout = oracle.make_inputs(Z, N, H, D, seed=93)
+    qd, kd, vd, dod = (t.cuda() for t in (q, k, v, dout))
+    sqd, skd = (torch.tensor(x, dtype=torch.int32, device="cuda") for x in (sq, sk))
+    scale = oracle.default_scale(D)
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    out, lse = cabi.fwd(qd, kd, vd, scale, True, seqused_q=sqd, seqused_k=skd)
+    runs = [cabi.bwd(qd, kd, vd, out, dod, lse, scale, True, flags=cabi.FMHA_BWD_DETERMINISTIC, status=status,
+                     seqused_q=sqd, seqused_k=skd, q_row_begin=q_row_begin) for _ in range(2)]
+    assert int(status.item()) == 0
+    assert all(torch.equal(a, b) for a, b in zip(*runs))
+    if q_row_begin == 0:
+        ref = _oracle_padded(q, k, v, dout, scale, True, sq, sk)
+        helpers.check_against_oracle((out.cpu(), lse.cpu(), *(t.cpu() for t in runs[0])), ref, "order, padded")
