@@ -373,6 +373,9 @@ int launch_bwd(const FmhaBwdParams* p, const BwdWorkspace& w, cudaStream_t strea
   const int Z = p->batch, H = p->heads, Nq = p->seqlen_q, Nk = p->seqlen_k;
   const int Nq_pad = round_up_128(Nq);
   constexpr int Dr = DR;
+  // The accumulator rows of padding queries are skipped where the call both zeroes and converts the
+  // accumulator.  Otherwise they are zeros for whoever converts it later, without the lengths.
+  const bool whole = !(p->flags & (FMHA_BWD_KEEP_WORKSPACE | FMHA_BWD_PREPROCESS_ONLY | FMHA_BWD_SKIP_DQ_CONVERT));
 
   if (!(p->flags & FMHA_BWD_KEEP_WORKSPACE)) {
     const long long rows = (long long)Z * H * Nq_pad;
@@ -380,7 +383,7 @@ int launch_bwd(const FmhaBwdParams* p, const BwdWorkspace& w, cudaStream_t strea
     const unsigned grid = (unsigned)((rows + rows_per_block - 1) / rows_per_block);
     fmha::fmha_bwd_preprocess_kernel<D, E, DR><<<grid, 256, 0, stream>>>(
         static_cast<const E*>(p->o), to3(p->o_strides), static_cast<const E*>(p->dout),
-        to3(p->dout_strides), p->lse, w.dq_accum, w.lse2, w.delta, H, Nq, Nq_pad, rows, p->seqused_q);
+        to3(p->dout_strides), p->lse, w.dq_accum, w.lse2, w.delta, H, Nq, Nq_pad, rows, p->seqused_q, whole ? 0 : 1);
     if (cudaGetLastError() != cudaSuccess) return FMHA_ERR_LAUNCH;
   }
   if (p->flags & FMHA_BWD_PREPROCESS_ONLY) return FMHA_OK;
@@ -460,7 +463,8 @@ int launch_bwd(const FmhaBwdParams* p, const BwdWorkspace& w, cudaStream_t strea
     constexpr int rows_per_block = 256 / (D / 8);
     const unsigned grid = (unsigned)((rows + rows_per_block - 1) / rows_per_block);
     fmha::fmha_bwd_convert_dq_kernel<D, E, DR><<<grid, 256, 0, stream>>>(
-        w.dq_accum, static_cast<E*>(p->dq), to3(p->dq_strides), H, Nq, p->scale, rows);
+        w.dq_accum, static_cast<E*>(p->dq), to3(p->dq_strides), H, Nq, p->scale, rows,
+        whole ? p->seqused_q : nullptr);
     if (cudaGetLastError() != cudaSuccess) return FMHA_ERR_LAUNCH;
   }
   return FMHA_OK;
@@ -633,12 +637,12 @@ int fmha_bwd_convert_dq(const void* workspace, void* dq, FmhaStrides dq_strides,
     auto* out = static_cast<__nv_bfloat16*>(dq);
     FMHA_DISPATCH_DIMS(head_dim,
                        fmha::fmha_bwd_convert_dq_kernel<D, __nv_bfloat16, DR><<<grid, 256, 0, s>>>(
-                           acc, out, sd, heads, seqlen_q, scale, rows);)
+                           acc, out, sd, heads, seqlen_q, scale, rows, nullptr);)
   } else {
     auto* out = static_cast<__half*>(dq);
     FMHA_DISPATCH_DIMS(head_dim,
                        fmha::fmha_bwd_convert_dq_kernel<D, __half, DR><<<grid, 256, 0, s>>>(
-                           acc, out, sd, heads, seqlen_q, scale, rows);)
+                           acc, out, sd, heads, seqlen_q, scale, rows, nullptr);)
   }
   return cudaGetLastError() == cudaSuccess ? FMHA_OK : FMHA_ERR_LAUNCH;
 }
