@@ -20,8 +20,8 @@
 //                      (aliases dP^T, which is dead once dS^T is in shared memory)
 //
 //   warps 0-3, 4-7  two compute groups: one thread per KV row, group g owns query columns
-//                   [64g, 64g+64) of the tile: P^T = exp2(S^T*c - lse2) (two exp2 per MUFU op,
-//                   fp16) and dS^T = P^T o (dP^T - D)
+//                   [64g, 64g+64) of the tile: P^T = exp2(S^T*c - lse2) and
+//                   dS^T = P^T o (dP^T - D)
 //   warps 8-11      dQ group: one thread per query row; tensor memory -> registers ->
 //                   shared-memory staging -> TMA reduce-add into the fp32 dQ accumulator
 //                   (bulk async adds: no per-thread atomics in the load/store pipeline)
@@ -43,7 +43,9 @@
 // One CTA per item spent about 7 us of its life on its head and tail (a causal item at N = 2048 has
 // 8.5 tiles of 2.2 us).  Whole backward, one CTA per item -> this, steady state: Z8 H32 N2048 D128
 // causal 1025 -> 955 us, without a mask 1665 -> 1570, Z64 H16 N512 D64 422 -> 385, Z1 H16 N16384
-// causal 2870 -> 2740.
+// causal 2870 -> 2740.  Where a period goes at D = 128 (bf16, clk): the compute warps take 1800 for P^T, 1250 for
+// dS^T and 900 for four waits and the loop; the MMA warp issues for 2600 and waits for them.  Shorter periods
+// (sixteen compute warps: -10 %) did not shorten the time, the clock fell instead: the power cap.
 #pragma once
 #include <cuda.h>
 #include <math_constants.h>
@@ -99,8 +101,12 @@ struct BwdTraits {
   static constexpr int kTileBytes = kBoxes * kBoxBytes;  // a 128 x D fp16 tile
   static constexpr int kDsBytes = 2 * kBoxBytes;         // dS^T: 128 x 128 fp16
   // Tile slots.  K, V and dO are in slots 0-2 and change places from item to item (see the kernel);
-  // slots 3 and 4 take the query tiles in turn.
-  static constexpr int kSlots = 5;
+  // the slots behind them take the query tiles in turn.  Where there is room for four (D = 64), a query tile's
+  // load need not wait for dK of the tile two before: behind the reduce-adds of dQ, which go through the
+  // same unit, it came too late for its S^T.  Whole backward, us, two slots / four: Z64 H16 N512 no mask, bf16
+  // 379 / 353, Z4 H16 N1024 causal 55.6 / 53.4, Z2 H16 N8192 no mask, bf16 1680 / 1601.
+  static constexpr int kQSlots = D == 64 ? 4 : 2;
+  static constexpr int kSlots = 3 + kQSlots;
   static constexpr int kStageBytes = 2 * 16384;          // dQ staging: 2 x (128 rows x 32 fp32)
   // statistics of one query tile: -lse2[128] (fp32), -delta[128] (fp32 with bf16 tensors, else fp16)
   static constexpr int kDeltaBytes = kBf16 ? 512 : 256;
@@ -146,7 +152,7 @@ struct __align__(16) BwdControl {
 template <int D, bool kBf16>
 constexpr int bwd_smem_bytes() {
   using T = BwdTraits<D, kBf16>;
-  return T::kSlots * T::kTileBytes + T::kDsBytes + T::kStageBytes + 2 * T::kStatBytes +
+  return T::kSlots * T::kTileBytes + T::kDsBytes + T::kStageBytes + T::kQSlots * T::kStatBytes +
          (int)sizeof(BwdControl<D, kBf16>);
 }
 
@@ -216,7 +222,7 @@ __global__ void __launch_bounds__(512, 1)
   const uint32_t stg_smem = ds_smem + T::kDsBytes;                  // dQ staging, 2 x 16 KB
   const uint32_t stat_smem = stg_smem + T::kStageBytes;             // statistics, one block per query slot
   auto& sh = *reinterpret_cast<BwdControl<D, kBf16>*>(smem_raw + T::kSlots * T::kTileBytes + T::kDsBytes +
-                                                      T::kStageBytes + 2 * T::kStatBytes);
+                                                      T::kStageBytes + T::kQSlots * T::kStatBytes);
   volatile int* const abort_word = &sh.abort_word;
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);  // warp-uniform for the compiler, too
@@ -430,7 +436,7 @@ __global__ void __launch_bounds__(512, 1)
           }
           __syncwarp();
           // in the order in which the slots fall free
-          load(3 + (g & 1), &tm_q, it, row0, true);
+          load(3 + g % T::kQSlots, &tm_q, it, row0, true);
           load(slot_k, &tm_k, it, kv0, false);
           load(slot_v, &tm_v, it, kv0, false);
           load(slot_do, &tm_do, it, row0, false);
@@ -441,7 +447,7 @@ __global__ void __launch_bounds__(512, 1)
         for (int n = 1; ok && n < it.cnt; ++n, ++g) {
           const int row = (it.i_begin + n) * T::kBlock;
           if (n == it.cnt - 1) ask();  // the answer takes a microsecond
-          load(3 + (g & 1), &tm_q, it, row, true);
+          load(3 + g % T::kQSlots, &tm_q, it, row, true);
           load(slot_do, &tm_do, it, row, false);
         }
       }
@@ -499,7 +505,7 @@ __global__ void __launch_bounds__(512, 1)
 #pragma unroll 1
       for (uint32_t g = 0; ok; ++g) {  // one pass per query tile, from one item into the next
         const bool last = n == cur.cnt - 1;
-        const uint32_t q_addr = slot_addr(3 + (g & 1));
+        const uint32_t q_addr = slot_addr(3 + g % T::kQSlots);
         // ---- dV += P^T dO_i; the first one overwrites the last item's dV
         FMHA_TL(2, g, 0);
         if (n == 0 && item_no > 0 && !mbar_wait_warp(smem_u32(&sh.bar_dv_read), (item_no - 1) & 1, abort_word, 19)) break;
@@ -520,9 +526,9 @@ __global__ void __launch_bounds__(512, 1)
         if (last) nxt = take_item();
         if (nxt.id >= 0) {
           if (last && !wait_full(slot_v, 3)) break;  // the next K is where V was
-          if (!wait_full(3 + ((g + 1) & 1), 7)) break;
+          if (!wait_full(3 + (g + 1) % T::kQSlots, 7)) break;
           tc_fence_after();
-          issue_kmajor(T::kColS, slot_addr(last ? slot_v : slot_k), slot_addr(3 + ((g + 1) & 1)));
+          issue_kmajor(T::kColS, slot_addr(last ? slot_v : slot_k), slot_addr(3 + (g + 1) % T::kQSlots));
           umma_commit_elect(smem_u32(&sh.bar_s_full));
         }
         // ---- dQ_i = dS K first (its read-out is on the critical path), then dK += dS^T Q_i
@@ -540,7 +546,7 @@ __global__ void __launch_bounds__(512, 1)
         }
         const uint32_t q_lo_mn = umma_desc_lo(q_addr, kLboMnMajor);
         issue_ss(2, T::kColDK, ds_lo_k, kBlockK, kStepK, q_lo_mn, kBlockMn, kStepMn, T::kIdescDV, n > 0 ? 1u : 0u);
-        umma_commit_elect(smem_u32(&sh.bar_empty[3 + (g & 1)]));  // Q_i, and dS^T, have been read
+        umma_commit_elect(smem_u32(&sh.bar_empty[3 + g % T::kQSlots]));  // Q_i, and dS^T, have been read
         if (last) umma_commit_elect(smem_u32(&sh.bar_acc_full));
         FMHA_TL(2, g, 4);
         if (nxt.id < 0) break;
@@ -671,7 +677,7 @@ __global__ void __launch_bounds__(512, 1)
 #pragma unroll 1
         for (int n = 0; n < it.cnt; ++n, ++g) {
           const int qbase = (it.i_begin + n) * T::kBlock;
-          const uint32_t sb = stat_smem + (g & 1) * T::kStatBytes;  // -lse2 at 0, -delta at 512
+          const uint32_t sb = stat_smem + g % T::kQSlots * T::kStatBytes;  // -lse2 at 0, -delta at 512
 
           // first visible query column of this thread's half (>= 64: none)
           int first_visible = 0;
@@ -684,12 +690,9 @@ __global__ void __launch_bounds__(512, 1)
           const int fvh = first_visible - cg * 64;
 
           uint32_t pp[32];  // P^T of this row and half, 16-bit pairs
-          // fp16 only: -(P^T o delta) as fp16 pairs, so that dS^T = P^T o dP^T - P^T o delta is one
-          // half2 FMA per pair; with bf16 (8 mantissa bits) dS^T is formed in fp32 instead
-          uint32_t npd[kBf16 ? 1 : 32];
           if (tl) FMHA_TL(0, g, 0);
           // on a time-out: keep going, every later wait returns at once
-          mbar_wait(smem_u32(&sh.bar_full[3 + (g & 1)]), (g >> 1) & 1, abort_word, 21);  // the statistics
+          mbar_wait(smem_u32(&sh.bar_full[3 + g % T::kQSlots]), g / T::kQSlots & 1, abort_word, 21);  // the statistics
           mbar_wait(smem_u32(&sh.bar_s_full), g & 1, abort_word, 11);
           tc_fence_after();
           if (tl) FMHA_TL(0, g, 1);
@@ -706,13 +709,12 @@ __global__ void __launch_bounds__(512, 1)
                 uint32_t x[4];
                 unpack2(fma2(pack2(s[cc][i + 0], s[cc][i + 1]), c2, pack2f(nl.x, nl.y)), x[0], x[1]);
                 unpack2(fma2(pack2(s[cc][i + 2], s[cc][i + 3]), c2, pack2f(nl.z, nl.w)), x[2], x[3]);
+                // (in fp32 for either type: a pair in fp16 takes the MUFU unit as long as two of these, and a
+                // 16-bit argument costs P two to three digits)
 #pragma unroll
-                for (int k = 0; k < 2; ++k) {
-                  const float xa = __uint_as_float(x[2 * k]), xb = __uint_as_float(x[2 * k + 1]);
-                  // a bf16 argument would cost P two to three digits: exponentials in fp32
-                  if constexpr (kBf16) pp[cc * 16 + (i >> 1) + k] = pack_bf16x2(fast_exp2(xa), fast_exp2(xb));
-                  else pp[cc * 16 + (i >> 1) + k] = exp2_half2(pack_half2(xa, xb));
-                }
+                for (int k = 0; k < 2; ++k)
+                  pp[cc * 16 + (i >> 1) + k] =
+                      pack16x2<kBf16>(fast_exp2(__uint_as_float(x[2 * k])), fast_exp2(__uint_as_float(x[2 * k + 1])));
               }
             if (fvh > 0) {
 #pragma unroll
@@ -732,23 +734,10 @@ __global__ void __launch_bounds__(512, 1)
             drain(done);
             pending = false;
           }
-          // off the critical path (dP^T is not there yet): -(P o delta)
-          if constexpr (!kBf16) {
-#pragma unroll
-            for (int j = 0; j < 32; j += 4) {
-              const float4 nd = lds128(sb + 512 + (cg * 32 + j) * 4);  // eight fp16 values
-              npd[j + 0] = mul_half2(pp[j + 0], __float_as_uint(nd.x));
-              npd[j + 1] = mul_half2(pp[j + 1], __float_as_uint(nd.y));
-              npd[j + 2] = mul_half2(pp[j + 2], __float_as_uint(nd.z));
-              npd[j + 3] = mul_half2(pp[j + 3], __float_as_uint(nd.w));
-            }
-          }
-
           mbar_wait(smem_u32(&sh.bar_dp_full), g & 1, abort_word, 12);
           if (tl) FMHA_TL(0, g, 3);
-          // dS^T of the previous tile must have been consumed by its dK / dQ MMAs (which also
-          // released its query tile), and dK / dV must have left the staging area
-          if (g > 0) mbar_wait(smem_u32(&sh.bar_empty[3 + ((g - 1) & 1)]), ((g - 1) >> 1) & 1, abort_word, 13);
+          // dS^T of the previous tile has been read: its dQ and dK MMAs were issued before this dP^T, and the
+          // commit that told of it covers them.  dK / dV must have left the staging area.
           if (n == 0) {
             if (lane == 0) tma_wait_group_read<0>();
             __syncwarp();
@@ -765,13 +754,13 @@ __global__ void __launch_bounds__(512, 1)
 #pragma unroll
               for (int k8 = 0; k8 < 4; ++k8) {  // 8 columns = one 16-byte chunk
                 uint32_t w[4];
-                uint64_t nd[4];  // bf16 only: -delta of this chunk's 8 query columns, in pairs
-                if constexpr (kBf16) {
-                  const float4 a = lds128(sb + 512 + (cg * 64 + cc * 32 + k8 * 8) * 4);
-                  const float4 b = lds128(sb + 512 + (cg * 64 + cc * 32 + k8 * 8 + 4) * 4);
-                  nd[0] = pack2f(a.x, a.y), nd[1] = pack2f(a.z, a.w);
-                  nd[2] = pack2f(b.x, b.y), nd[3] = pack2f(b.z, b.w);
-                }
+                // -delta of this chunk's 8 query columns: fp16 pairs, with bf16 (8 mantissa bits) pairs of fp32
+                const uint32_t at = sb + 512 + (cg * 64 + cc * 32 + k8 * 8) * (kBf16 ? 4 : 2);
+                const float4 a = lds128(at), b = kBf16 ? lds128(at + 16) : a;
+                [[maybe_unused]] const uint64_t nd[4] = {pack2f(a.x, a.y), pack2f(a.z, a.w), pack2f(b.x, b.y),
+                                                         pack2f(b.z, b.w)};
+                [[maybe_unused]] const uint32_t nd16[4] = {__float_as_uint(a.x), __float_as_uint(a.y),
+                                                           __float_as_uint(a.z), __float_as_uint(a.w)};
 #pragma unroll
                 for (int q2 = 0; q2 < 4; ++q2) {
                   const int i = k8 * 8 + q2 * 2;     // column within this 32-column block
@@ -782,9 +771,8 @@ __global__ void __launch_bounds__(512, 1)
                             lo, hi);
                     w[q2] = pack_bf16x2(__uint_as_float(lo), __uint_as_float(hi));
                   } else {
-                    w[q2] = fma_half2(pp[j],
-                                      pack_half2(__uint_as_float(dp[cc][i]), __uint_as_float(dp[cc][i + 1])),
-                                      npd[j]);
+                    w[q2] = mul_half2(
+                        pp[j], add_half2(pack_half2(__uint_as_float(dp[cc][i]), __uint_as_float(dp[cc][i + 1])), nd16[q2]));
                   }
                 }
                 const int ch = cc * 4 + k8;  // chunk of this thread's 128-byte row

@@ -519,20 +519,14 @@ __device__ __forceinline__ uint64_t poly_exp2_pair(uint64_t x2, float& top) {
   p1 += t1 << 23;
   return pack2(p0, p1);
 }
-// two exp2 per MUFU operation, fp16 in and out (inputs here are <= ~0, results in [0, 1])
-__device__ __forceinline__ uint32_t exp2_half2(uint32_t x) {
-  uint32_t y;
-  asm("ex2.approx.f16x2 %0, %1;" : "=r"(y) : "r"(x));
-  return y;
-}
 __device__ __forceinline__ uint32_t mul_half2(uint32_t a, uint32_t b) {
   uint32_t y;
   asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(y) : "r"(a), "r"(b));
   return y;
 }
-__device__ __forceinline__ uint32_t fma_half2(uint32_t a, uint32_t b, uint32_t c) {
+__device__ __forceinline__ uint32_t add_half2(uint32_t a, uint32_t b) {
   uint32_t y;
-  asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(y) : "r"(a), "r"(b), "r"(c));
+  asm("add.rn.f16x2 %0, %1, %2;" : "=r"(y) : "r"(a), "r"(b));
   return y;
 }
 __device__ __forceinline__ float4 lds128(uint32_t addr) {
