@@ -231,6 +231,7 @@ struct FwdPlan {
   int items_per_head = 0;
   int first_cut_row = 0;   // rows from here on belong to cut query blocks
   size_t workspace = 0;    // bytes of the partial results
+  bool pair = false;       // up to 128 query rows: an item is two chunks, both in work
 };
 
 FwdPlan plan_fwd(const FmhaFwdParams* p, int sms) {
@@ -245,7 +246,9 @@ FwdPlan plan_fwd(const FmhaFwdParams* p, int sms) {
     return fmha::fwd_visible_tiles(causal, p->causal_shift, std::min(qb * 256 + 255, p->seqlen_q - 1), nk);
   };
   const int n_max = visible(nqb - 1);
-  if (n_max < 4 || heads * nqb > 8.0 * sms) return plan;  // nothing to cut, or enough items to balance
+  if (n_max < 4) return plan;
+  const bool can_pair = p->seqlen_q <= (p->head_dim > 64 ? 64 : 128);
+  if (heads * nqb > 8.0 * sms && !can_pair) return plan;  // enough items to balance
   auto cost = [&](int chunk, int& items) {  // makespan with chunks of `chunk` tiles
     double total = 0;
     items = 0;
@@ -266,7 +269,7 @@ FwdPlan plan_fwd(const FmhaFwdParams* p, int sms) {
   int items = 0;
   double best = 0.85 * cost(n_max, items);  // a cut has to be worth it: the estimate is rough
   // without a mask the work per SM is what it is unless SMs idle; under one, unless one block dominates
-  for (int k = 2; k <= 64 && n_max / k >= 2; ++k) {
+  for (int k = 2; heads * nqb <= 8.0 * sms && k <= 64 && n_max / k >= 2; ++k) {
     const int chunk = (n_max + k - 1) / k;
     const double t0 = cost(chunk, items);
     // the joining kernel: its launch, and the partial rows written and read (at about 4 TB/s)
@@ -278,6 +281,28 @@ FwdPlan plan_fwd(const FmhaFwdParams* p, int sms) {
       plan.max_chunks = (n_max + chunk - 1) / chunk;
     }
     if (heads * items > 8.0 * sms) break;
+  }
+  if (can_pair) {
+    // Few queries: an item with one query tile is a chain of MMA, softmax and MMA, 1.9 us per KV tile, and half
+    // of the SM idles.  Items of two chunks, in us: a round 2.2 at D = 64 and 3.0 at D = 128, where there is room
+    // for one K and one V tile per chunk only.  Not for chunks of less than 8 tiles (8 heads of 64 x 8192, D = 128:
+    // 25.6 as cut above, 30.7 in pairs), nor at D = 128 for more than 64 rows, whose partial rows weigh more
+    // (128 heads of 128 x 4096: 61 / 73).  Taken: 64 heads of 64 x 8192 70 / 59, at D = 64 66 / 49.
+    const double now = 1.9 * (plan.max_chunks > 1 ? best : cost(n_max, items));
+    double best_us = 0.9 * now;
+    for (int k = 1; k <= 32; ++k) {
+      const int chunk = (n_max + 2 * k - 1) / (2 * k), n = (n_max + 2 * chunk - 1) / (2 * chunk);
+      if (chunk < 8) break;
+      const double parts = heads * n * 2 * p->seqlen_q * p->head_dim * 8.0;  // written, and read by the join
+      const double t = std::ceil(heads * n / sms) * (chunk + 1.0) * (p->head_dim > 64 ? 3.0 : 2.2) + 3.0 + parts / 4e6;
+      if (t < best_us) {
+        best_us = t;
+        plan.pair = true;
+        plan.chunk_tiles = chunk;
+        plan.items_per_head = n;
+        plan.max_chunks = 2 * n;
+      }
+    }
   }
   if (plan.max_chunks > 1) {
     int qb = 0;
@@ -353,9 +378,12 @@ int launch_fwd(const FmhaFwdParams* p, void* workspace, size_t workspace_bytes, 
   // of its own (nothing to take over) or the caller wants SMs left free.
   kp.deal = kp.num_items <= sms || p->sm_margin > 0;
   const unsigned grid = kp.deal ? (unsigned)std::min(kp.num_items, sms) : (unsigned)kp.num_items;
-  if (!launch_with_smem<fmha::fmha_fwd_kernel<D, kBf16>>(dev, grid, T::kThreads, T::kSmemBytes, stream, tq, tk, tv, to,
-                                                         kp))
-    return FMHA_ERR_LAUNCH;
+  const bool launched =
+      plan.pair ? launch_with_smem<fmha::fmha_fwd_kernel<D, kBf16, true>>(dev, grid, T::kThreads, T::kSmemBytes, stream,
+                                                                          tq, tk, tv, to, kp)
+                : launch_with_smem<fmha::fmha_fwd_kernel<D, kBf16>>(dev, grid, T::kThreads, T::kSmemBytes, stream, tq, tk,
+                                                                    tv, to, kp);
+  if (!launched) return FMHA_ERR_LAUNCH;
   if (plan.max_chunks > 1) {
     const long long rows = (long long)kp.num_heads_total * (p->seqlen_q - plan.first_cut_row);
     fmha::fmha_fwd_combine_kernel<E><<<(unsigned)((rows + 7) / 8), 256, 0, stream>>>(

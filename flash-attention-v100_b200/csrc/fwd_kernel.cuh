@@ -123,8 +123,9 @@ static_assert(kFwdRegsIssue <= 168 && kFwdRegsSoftmax >= 168 && kFwdRegsSoftmax 
 constexpr float kRescaleSum = 1024.0f;
 
 // A work item: 256 query rows from q0 of head zh = z * heads + h, KV tiles [kv_first, kv_first + n_t)
-// for its query tile t (n_t = 0: the tile sees nothing of this chunk).  The producer warp works it
-// out and publishes it in shared memory.
+// for its query tile t (n_t = 0: the tile sees nothing of this chunk).  A paired item (see the kernel) has
+// the same 128 rows twice, and its tile 1 the next chunk of the keys.  The producer warp works it out and
+// publishes it in shared memory.
 struct __align__(16) FwdItem {
   int id;      // -1: no more items
   int n0, n1;  // KV tiles of the two query tiles
@@ -132,7 +133,7 @@ struct __align__(16) FwdItem {
   int z, h, zh;
   int kv_first;
   int sq, sk;  // lengths of the batch entry
-  int chunk;   // index of the chunk among those of its query block, -1: the block is not cut
+  int chunk;   // index of the (first) chunk among those of its query block, -1: the block is not cut
   int pad;
 };
 
@@ -160,6 +161,7 @@ __host__ __device__ __forceinline__ int fwd_chunks(bool causal, int shift, int q
 
 // Items in groups of head_group heads (their K and V share the L2); in a group the last query
 // blocks first (under a causal mask the heaviest), heads innermost.
+template <bool kPair>
 __device__ __forceinline__ FwdItem fwd_item(const FwdKernelParams& p, int id) {
   FwdItem it;
   it.id = id;
@@ -175,7 +177,11 @@ __device__ __forceinline__ FwdItem fwd_item(const FwdKernelParams& p, int id) {
   it.chunk = -1;
   it.kv_first = 0;
   int most = 0x7fffffff;
-  if (p.o_part == nullptr) {
+  if (kPair) {
+    it.chunk = 2 * u;
+    it.kv_first = it.chunk * p.chunk_tiles;
+    most = p.chunk_tiles;
+  } else if (p.o_part == nullptr) {
     qb -= u;
   } else {
     for (;; --qb) {
@@ -195,17 +201,21 @@ __device__ __forceinline__ FwdItem fwd_item(const FwdKernelParams& p, int id) {
   it.q0 = qb * 256;
   fwd_lengths(p, it.z, it.sq, it.sk);
   const int nk_total = (it.sk + 127) / 128;
-  auto tiles = [&](int r0) {
+  auto tiles = [&](int r0, int first) {
     if (r0 >= it.sq) return 0;
     const int n = fwd_visible_tiles(p.causal != 0, p.causal_shift, min(r0 + 127, it.sq - 1), nk_total);
-    return max(0, min(most, n - it.kv_first));
+    return max(0, min(most, n - first));
   };
-  it.n0 = tiles(it.q0);
-  it.n1 = tiles(it.q0 + 128);
+  it.n0 = tiles(it.q0, it.kv_first);
+  it.n1 = kPair ? tiles(it.q0, it.kv_first + most) : tiles(it.q0 + 128, it.kv_first);
   return it;
 }
 
-template <int D, bool kBf16 = false>
+// kPair: no more than 128 query rows.  Both query tiles are these rows, each against a chunk of the keys of its
+// own, and both chunks leave partial results.  K and V of tile t come through a ring of their own, half of the
+// slots.  (With one query tile, cut or not, a CTA takes 1.9 us per KV tile: MMA, softmax and MMA one after the
+// other, and half of the SM idle.  64 queries x 8192 keys, 64 heads, us: D = 128, bf16 70 -> 59, D = 64 66 -> 49.)
+template <int D, bool kBf16 = false, bool kPair = false>
 __global__ void __launch_bounds__(384, 1)
     fmha_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                     const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o,
@@ -244,6 +254,7 @@ __global__ void __launch_bounds__(384, 1)
   const uint32_t q_smem = smem_base;                                    // 2 query tiles
   const uint32_t ring_smem = smem_base + T::kTilesM * T::kTileBytes;    // K/V ring
   const uint32_t ostage_smem = ring_smem + T::kStages * T::kTileBytes;  // 2 output boxes
+  constexpr uint32_t kRingSlots = T::kStages / 2;  // kPair: of each tile's ring
 
   // ---- set-up: barriers (thread 0), tensor memory (warp 9)
   if (threadIdx.x == 0) {
@@ -349,7 +360,7 @@ __global__ void __launch_bounds__(384, 1)
         FwdItem it;
         it.id = -1;
         it.n0 = it.n1 = 0;
-        if (id >= 0) it = fwd_item(p, id);
+        if (id >= 0) it = fwd_item<kPair>(p, id);
         it.n0 = __shfl_sync(0xffffffffu, it.n0, 0);
         it.n1 = __shfl_sync(0xffffffffu, it.n1, 0);
         const uint32_t s = published % T::kItemStages, round = published / T::kItemStages;
@@ -364,7 +375,13 @@ __global__ void __launch_bounds__(384, 1)
         return it;
       };
       uint32_t slot = 0, phase = 1;  // the next ring slot, parity of its last release (none yet: passes)
-      auto load = [&](const CUtensorMap* tm, const FwdItem& it, int tile) {
+      uint32_t loaded[2] = {0, 0};   // kPair: tiles that went through each ring
+      auto load = [&](const CUtensorMap* tm, const FwdItem& it, int tile, int ring) {
+        if constexpr (kPair) {
+          const uint32_t n = ring ? loaded[1]++ : loaded[0]++;
+          slot = ring * kRingSlots + n % kRingSlots;
+          phase = n / kRingSlots % 2 ^ 1;
+        }
         if (!(ok = mbar_wait_warp(smem_u32(&bar_kv_empty[slot]), phase, &abort_word, 2))) return;
         if (elect_one()) {
           const uint32_t fbar = smem_u32(&bar_kv_full[slot]);
@@ -375,12 +392,12 @@ __global__ void __launch_bounds__(384, 1)
                         (it.kv_first + tile) * T::kBlockN, it.h, it.z);
         }
         __syncwarp();
-        if (++slot == T::kStages) {
+        if (!kPair && ++slot == T::kStages) {
           slot = 0;
           phase ^= 1u;
         }
       };
-      // K(0) V(0) K(1) V(1) ... of one item after the other
+      // K(0) V(0) K(1) V(1) ... of one item after the other (kPair: of its tiles in turn; tile 0 has no fewer)
       while (ok) {
         const FwdItem it = next_item();
         if (it.id < 0) break;
@@ -388,7 +405,8 @@ __global__ void __launch_bounds__(384, 1)
 #pragma unroll 1
         for (int i = 0; ok && i < 2 * n; ++i) {
           if (i >= 2 * n - 5) ask();
-          load((i & 1) ? &tm_v : &tm_k, it, i >> 1);
+          load((i & 1) ? &tm_v : &tm_k, it, i >> 1, 0);
+          if (kPair && ok && (i >> 1) < it.n1) load((i & 1) ? &tm_v : &tm_k, it, p.chunk_tiles + (i >> 1), 1);
         }
       }
     } else if (warp == 10) {
@@ -404,7 +422,7 @@ __global__ void __launch_bounds__(384, 1)
 #pragma unroll 1
         for (int t = 0; t < T::kTilesM; ++t) {
           if ((t == 0 ? it.n0 : it.n1) == 0) continue;
-          const int row = it.q0 + t * T::kBlockM;
+          const int row = it.q0 + (kPair ? 0 : t * T::kBlockM);
           if ((used >> t) & 1) {
             // cold from HBM this takes microseconds: start towards L2 before waiting for the buffer
             if (elect_one())
@@ -451,6 +469,12 @@ __global__ void __launch_bounds__(384, 1)
           slot_phase ^= 1u;
         }
       };
+      uint32_t taken[2] = {0, 0};  // kPair: tiles that came through each ring
+      [[maybe_unused]] auto ring_next = [&](int t) {
+        const uint32_t n = t ? taken[1]++ : taken[0]++;
+        slot = t * kRingSlots + n % kRingSlots;
+        slot_phase = n / kRingSlots % 2;
+      };
       FwdItem cur = take_item();
       int j = -1;
       bool ok = true;
@@ -472,7 +496,7 @@ __global__ void __launch_bounds__(384, 1)
         const uint32_t k_slot = j < 0 ? slot : (slot + 1 == T::kStages ? 0 : slot + 1);
         const uint32_t k_addr = ring_smem + k_slot * T::kTileBytes;
         const uint32_t k_phase = k_slot < slot ? slot_phase ^ 1u : slot_phase;
-        if (j >= 0 && !(ok = slot_wait())) break;
+        if (!kPair && j >= 0 && !(ok = slot_wait())) break;
 #pragma unroll 1
         for (int t = 0; t < 2; ++t) {
           const int nt = t == 0 ? cur.n0 : cur.n1;
@@ -487,7 +511,11 @@ __global__ void __launch_bounds__(384, 1)
               }
               used_o |= 1u << t;
             }
-            const uint32_t v_lo = umma_desc_lo(v_addr, kLboMnMajor);
+            if (kPair) {
+              ring_next(t);
+              if (!(ok = slot_wait())) break;
+            }
+            const uint32_t v_lo = umma_desc_lo(kPair ? ring_smem + slot * T::kTileBytes : v_addr, kLboMnMajor);
             const uint32_t d = tmem_base + 256 + t * D, a = tmem_base + t * 128;
 #pragma unroll
             for (int half = 0; half < 2; ++half) {
@@ -501,13 +529,20 @@ __global__ void __launch_bounds__(384, 1)
             }
             phase_p ^= 1u << t;
             if (j == nt - 1) umma_commit_elect(smem_u32(&bar_o_full[t]));
+            if (kPair) umma_commit_elect(smem_u32(&bar_kv_empty[slot]));
             if (!ok) break;
           }
-          if (t == 1 && j >= 0) slot_next();
+          if (!kPair && t == 1 && j >= 0) slot_next();
           // ---- S_t = Q_t K^T of the round after, which may be the first of the next item
-          if (t == 0 && has_k && !(ok = mbar_wait_warp(smem_u32(&bar_kv_full[k_slot]), k_phase, &abort_word, 5))) break;
+          if (!kPair && t == 0 && has_k &&
+              !(ok = mbar_wait_warp(smem_u32(&bar_kv_full[k_slot]), k_phase, &abort_word, 5)))
+            break;
           const int nk = t == 0 ? nxt.n0 : nxt.n1;
           if (jk < nk) {
+            if (kPair) {
+              ring_next(t);
+              if (!(ok = slot_wait())) break;
+            }
             if (jk == 0) {
               ok = mbar_wait_warp(smem_u32(&bar_q_full[t]), (phase_q >> t) & 1, &abort_word, 3);
               phase_q ^= 1u << t;
@@ -515,18 +550,19 @@ __global__ void __launch_bounds__(384, 1)
             }
             tc_fence_after();
             const uint32_t a_lo = q_lo0 + ((t * T::kTileBytes) >> 4);
-            const uint32_t b_lo = umma_desc_lo(k_addr, kLboKMajor);
+            const uint32_t b_lo = umma_desc_lo(kPair ? ring_smem + slot * T::kTileBytes : k_addr, kLboKMajor);
 #pragma unroll
             for (int ks = 0; ks < D / 16; ++ks) {
               const uint32_t off = ((ks >> 2) * T::kBoxBytes + (ks & 3) * 32) >> 4;
               umma_ss_elect(tmem_base + t * 128, a_lo + off, b_lo + off, idesc_qk, ks > 0 ? 1u : 0u);
             }
             umma_commit_elect(smem_u32(&bar_s_full[t]));
+            if (kPair) umma_commit_elect(smem_u32(&bar_kv_empty[slot]));
             if (jk == nk - 1) umma_commit_elect(smem_u32(&bar_q_free[t]));
           }
         }
         if (!ok) break;
-        if (has_k) slot_next();
+        if (!kPair && has_k) slot_next();
         ++j;
         if (last) {
           cur = nxt;
@@ -563,11 +599,11 @@ __global__ void __launch_bounds__(384, 1)
       float l = 0.f;                // running sum of exp2((s - m_ref) * c)
       int lim;                      // last visible column of this row in the round
       {
-        const int row = it.q0 + t * T::kBlockM + row_in_tile;
+        const int row = it.q0 + (kPair ? 0 : t * T::kBlockM) + row_in_tile;
         long long last_key = p.causal ? (long long)row + p.causal_shift : (long long)it.sk - 1;
         last_key = min(last_key, (long long)it.sk - 1);
         if (row >= it.sq) last_key = -1;  // a padding row sees nothing: O = 0, LSE = -inf
-        lim = (int)max(last_key, -1ll) - it.kv_first * T::kBlockN;
+        lim = (int)max(last_key, -1ll) - (it.kv_first + (kPair ? t * p.chunk_tiles : 0)) * T::kBlockN;
       }
 
       for (int j = 0; j < n || j == 0; ++j, lim -= T::kBlockN) {
@@ -709,9 +745,10 @@ __global__ void __launch_bounds__(384, 1)
         // ---- epilogue of the item before: O_t / l -> registers (tensor memory released) -> 16 bit ->
         //      staging box -> TMA store; LSE.  A chunk of a query block leaves fp32 rows instead.
         pending = false;
-        const int row = done.q0 + t * T::kBlockM + row_in_tile;
+        const int row = done.q0 + (kPair ? 0 : t * T::kBlockM) + row_in_tile;
         const int nd = t == 0 ? done.n0 : done.n1;
-        const bool split = done.chunk >= 0;
+        const bool split = kPair || done.chunk >= 0;
+        const int chunk = done.chunk + (kPair ? t : 0);
         // (a row sum that is NaN leaves NaN in both: an LSE of -inf means that the row sees nothing, and
         // whoever joins partial results leaves such a part out)
         const float inv_l = (done_l == 0.f) ? 0.f : 1.f / done_l;
@@ -719,7 +756,7 @@ __global__ void __launch_bounds__(384, 1)
           const float lse =
               (done_l == 0.f) ? -CUDART_INF_F : (done_m * c + log2f(done_l)) * 0.6931471805599453f;
           const size_t stat = (size_t)done.zh * p.seqlen_q + row;
-          if (split) p.lse_part[(size_t)done.chunk * p.num_heads_total * p.seqlen_q + stat] = lse;
+          if (split) p.lse_part[(size_t)chunk * p.num_heads_total * p.seqlen_q + stat] = lse;
           else p.lse[stat] = lse;
         }
         if (nd > 0) {
@@ -729,7 +766,7 @@ __global__ void __launch_bounds__(384, 1)
         }
         if (split) {
           if (nd == 0) continue;  // LSE = -inf: the combine kernel reads no row
-          float* dst = p.o_part + (((size_t)done.chunk * p.num_heads_total + done.zh) * p.seqlen_q + row) * p.row_elems;
+          float* dst = p.o_part + (((size_t)chunk * p.num_heads_total + done.zh) * p.seqlen_q + row) * p.row_elems;
 #pragma unroll 1
           for (int cc = 0; cc < D / 16; ++cc) {
             uint32_t o[16];
@@ -787,7 +824,7 @@ __global__ void __launch_bounds__(384, 1)
         }
       }
       if (it.id < 0) break;
-      pending = it.q0 + t * T::kBlockM < p.seqlen_q;
+      pending = kPair || it.q0 + t * T::kBlockM < p.seqlen_q;
       done = it;
       done_m = m_ref;
       done_l = l;
