@@ -64,9 +64,10 @@ __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
 
 // Rows are indexed (zh, q) over the PADDED query length so that lse2 / delta are complete.  Both kernels are
 // bound by HBM, so the padding rows of a right-padded batch are left alone: their O and dO are not
-// read, and where the conversion knows the lengths, too (zero_padding = 0), their accumulator rows are
-// neither zeroed nor read.  Z8 H16 N2048 D128 causal, lengths spread evenly over [N/8, N], whole backward: 256 us ->
-// 234; Z64 H16 N512 D64 255 -> 231.
+// read, and their accumulator rows are not read where the conversion knows the lengths, nor zeroed where the
+// workspace is not used again either (zero_padding = 0).
+// Whole backward, us, lengths spread evenly over [N/8, N], all rows read and zeroed / zeroed only / neither:
+// Z8 H16 N2048 D128 bf16 causal 240 / 223 / 219; zeroed only / neither: Z64 H16 N512 D64 bf16 231 / 225.
 template <int D, typename E, int DR = D>
 __global__ void __launch_bounds__(256)
     fmha_bwd_preprocess_kernel(const E* __restrict__ o, Strides3 so,

@@ -401,9 +401,10 @@ int launch_bwd(const FmhaBwdParams* p, const BwdWorkspace& w, cudaStream_t strea
   const int Z = p->batch, H = p->heads, Nq = p->seqlen_q, Nk = p->seqlen_k;
   const int Nq_pad = round_up_128(Nq);
   constexpr int Dr = DR;
-  // The accumulator rows of padding queries are skipped where the call both zeroes and converts the
-  // accumulator.  Otherwise they are zeros for whoever converts it later, without the lengths.
+  // Where the call both zeroes and converts the accumulator, the conversion need not read the rows of padding
+  // queries.  They are zeroed all the same, for later calls on this workspace, unless the caller has none in mind.
   const bool whole = !(p->flags & (FMHA_BWD_KEEP_WORKSPACE | FMHA_BWD_PREPROCESS_ONLY | FMHA_BWD_SKIP_DQ_CONVERT));
+  const int zero_padding = whole && (p->flags & FMHA_BWD_DROP_WORKSPACE) ? 0 : 1;
 
   if (!(p->flags & FMHA_BWD_KEEP_WORKSPACE)) {
     const long long rows = (long long)Z * H * Nq_pad;
@@ -411,7 +412,7 @@ int launch_bwd(const FmhaBwdParams* p, const BwdWorkspace& w, cudaStream_t strea
     const unsigned grid = (unsigned)((rows + rows_per_block - 1) / rows_per_block);
     fmha::fmha_bwd_preprocess_kernel<D, E, DR><<<grid, 256, 0, stream>>>(
         static_cast<const E*>(p->o), to3(p->o_strides), static_cast<const E*>(p->dout),
-        to3(p->dout_strides), p->lse, w.dq_accum, w.lse2, w.delta, H, Nq, Nq_pad, rows, p->seqused_q, whole ? 0 : 1);
+        to3(p->dout_strides), p->lse, w.dq_accum, w.lse2, w.delta, H, Nq, Nq_pad, rows, p->seqused_q, zero_padding);
     if (cudaGetLastError() != cudaSuccess) return FMHA_ERR_LAUNCH;
   }
   if (p->flags & FMHA_BWD_PREPROCESS_ONLY) return FMHA_OK;
@@ -642,7 +643,9 @@ int fmha_bwd_static_scratch(const FmhaBwdParams* p, void* stream) {
   void* scratch = static_scratch_for_current_device(&rc);
   if (scratch == nullptr) return rc;
   // same validation, kernels and launch order as the caller-workspace entry point
-  return fmha_bwd(p, scratch, (size_t)FMHA_STATIC_SCRATCH_BYTES, stream);
+  FmhaBwdParams own = *p;
+  own.flags |= FMHA_BWD_DROP_WORKSPACE;  // the caller never sees it
+  return fmha_bwd(&own, scratch, (size_t)FMHA_STATIC_SCRATCH_BYTES, stream);
 }
 
 int fmha_bwd_convert_dq(const void* workspace, void* dq, FmhaStrides dq_strides, int32_t batch,

@@ -231,7 +231,7 @@ std::vector<at::Tensor> bwd_impl(const at::Tensor& dout, const at::Tensor& q, co
   p.dtype = q.scalar_type() == at::kBFloat16 ? FMHA_DTYPE_BF16 : FMHA_DTYPE_FP16;
   p.seqused_q = seqused_ptr(seqused_q, q, "seqused_q");
   p.seqused_k = seqused_ptr(seqused_k, q, "seqused_k");
-  p.flags = deterministic ? FMHA_BWD_DETERMINISTIC : 0;
+  p.flags = FMHA_BWD_DROP_WORKSPACE | (deterministic ? FMHA_BWD_DETERMINISTIC : 0);
   const size_t ws_bytes = fmha_bwd_workspace_bytes(&p);
   at::Tensor ws = empty_on(q, {static_cast<int64_t>(ws_bytes)}, at::kByte);
   check_status(fmha_bwd(&p, ws.data_ptr(), ws_bytes, at::cuda::getCurrentCUDAStream().stream()),

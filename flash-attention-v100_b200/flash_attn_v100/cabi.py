@@ -25,6 +25,7 @@ FMHA_BWD_SKIP_DQ_CONVERT = 2
 FMHA_BWD_PREPROCESS_ONLY = 4
 FMHA_BWD_DETERMINISTIC = 8
 FMHA_BWD_ACCUM_OVERWRITE = 16
+FMHA_BWD_DROP_WORKSPACE = 32
 FMHA_DTYPE_FP16 = 0
 FMHA_DTYPE_BF16 = 1
 
@@ -296,6 +297,7 @@ def bwd(q, k, v, o, dout, lse, scale: float, causal: bool = False, causal_shift:
         dv = torch.empty_like(v)
     if workspace is None:
         workspace = torch.empty(bwd_workspace_bytes(Z, Nq, H, D), dtype=torch.uint8, device=q.device)
+        flags |= FMHA_BWD_DROP_WORKSPACE
     p = bwd_params(q, k, v, o, dout, lse, dq, dk, dv, scale, causal, causal_shift, dk_accum,
                    dv_accum, flags, status, seqused_q, seqused_k, q_row_begin)
     with torch.cuda.device(q.device):

@@ -136,7 +136,8 @@ typedef struct {
    * bit 0 set = do not zero the dQ accumulator nor recompute D (workspace carries both over
    * from an earlier call); bit 1 set = do not convert dQ (a later call will); bit 2 set = run
    * the preprocess step only; bit 3 set = deterministic dQ (see FMHA_BWD_DETERMINISTIC); bit 4 set =
-   * dk_accum / dv_accum are overwritten, not added into (FMHA_BWD_ACCUM_OVERWRITE). */
+   * dk_accum / dv_accum are overwritten, not added into (FMHA_BWD_ACCUM_OVERWRITE); bit 5 set = the
+   * workspace is not used again (FMHA_BWD_DROP_WORKSPACE). */
   int32_t flags;
   int32_t* status;
   int32_t dtype; /* FMHA_DTYPE_FP16 (0) or FMHA_DTYPE_BF16 */
@@ -173,6 +174,11 @@ typedef struct {
  * sees a key), so the caller need not clear them first (ring attention: the partial result of
  * one step, sent to the block's owner). */
 #define FMHA_BWD_ACCUM_OVERWRITE 16
+/* The workspace is not used again after this call, and what it holds then is undefined: the
+ * accumulator rows of padding queries need not be zeroed.  Without it they are zeros, whichever call
+ * continues on the workspace or converts it.  Of no effect together with FMHA_BWD_KEEP_WORKSPACE,
+ * FMHA_BWD_PREPROCESS_ONLY or FMHA_BWD_SKIP_DQ_CONVERT. */
+#define FMHA_BWD_DROP_WORKSPACE 32
 
 /* Forward: O = softmax(scale * Q K^T [+ causal mask]) V and LSE.
  * Replaces fused_mha_forward (include/fused_mha.h:1-2, kernel/fused_mha_kernel.cu:891-902). */
