@@ -213,14 +213,14 @@ BwdWorkspace carve_workspace(void* ws, int Z, int H, int Nq, int D) {
 // idle: then its KV range is cut into chunks of chunk_tiles tiles, each an item of its own that
 // leaves an fp32 partial result, and a second kernel joins them.
 //
-// Measured, uncut / as cut by plan_fwd (chunks), us, fp16, D = 128:
-//   64 queries x 8192 keys     8 heads 115.0 / 25.8 (13), 32: 116.6 / 43.2 (4), 64: 117.0 / 69.8 (2)
+// Measured, uncut / as cut by plan_fwd (chunks), us, fp16, D = 128, the ordinary cut (pairs of chunks: below):
+//   64 queries x 8192 keys     8 heads 115.0 / 25.8 (13)
 //   256 queries x 4096 keys    8 heads 59.5 / 26.8 (8), 64: 61.7 / 53.4 (2)
 //   causal, 1 head             N = 1024 24.2 / 22.7 (4), 4096 59.8 / 28.8 (8), 16384 214.5 / 113.7 (6)
 //   causal, 4 heads            N = 1024 24.3 / 22.7 (4), 4096 60.9 / 43.2 (3)
-// and what it leaves uncut, uncut / cut in two: 128 heads of 64 x 8192 120.7 / 139.5, 64 heads of 512 x
+// and what it leaves uncut, uncut / cut in two: 64 heads of 512 x
 // 2048 37.0 / 67.7, causal 16 heads N = 4096 63.6 / 97.9, 4 heads N = 16384 227.9 / 261.5.  Over 150 shapes
-// (D = 64 and 128, 1 to 296 heads) no cut of its was slower than none.  It is a rough estimate on
+// (D = 64 and 128, 1 to 296 heads) no ordinary cut of its was slower than none.  It is a rough estimate on
 // the cautious side: where the items are just fewer than the SMs a cut that it does not make
 // would be up to 1.4 times as fast (causal, 4 heads, N = 8192: 113.1 / 80.3), and under a mask fewer chunks
 // than it makes up to 1.3 times (1 head, N = 16384: 113.7 in 6, 86.6 in 4).
@@ -247,7 +247,9 @@ FwdPlan plan_fwd(const FmhaFwdParams* p, int sms) {
   };
   const int n_max = visible(nqb - 1);
   if (n_max < 4) return plan;
-  const bool can_pair = p->seqlen_q <= (p->head_dim > 64 ? 64 : 128);
+  // partial rows of pairs of chunks, written, and read by the join
+  auto part_bytes = [&](int n) { return heads * n * 2 * p->seqlen_q * p->head_dim * 8.0; };
+  const bool can_pair = p->seqlen_q <= (p->head_dim > 64 ? 127 : 128);  // full tiles at D = 128: 0.86 to 1.1 times as fast
   if (heads * nqb > 8.0 * sms && !can_pair) return plan;  // enough items to balance
   auto cost = [&](int chunk, int& items) {  // makespan with chunks of `chunk` tiles
     double total = 0;
@@ -286,15 +288,14 @@ FwdPlan plan_fwd(const FmhaFwdParams* p, int sms) {
     // Few queries: an item with one query tile is a chain of MMA, softmax and MMA, 1.9 us per KV tile, and half
     // of the SM idles.  Items of two chunks, in us: a round 2.2 at D = 64 and 3.0 at D = 128, where there is room
     // for one K and one V tile per chunk only.  Not for chunks of less than 8 tiles (8 heads of 64 x 8192, D = 128:
-    // 25.6 as cut above, 30.7 in pairs), nor at D = 128 for more than 64 rows, whose partial rows weigh more
-    // (128 heads of 128 x 4096: 61 / 73).  Taken: 64 heads of 64 x 8192 70 / 59, at D = 64 66 / 49.
-    const double now = 1.9 * (plan.max_chunks > 1 ? best : cost(n_max, items));
-    double best_us = 0.9 * now;
+    // 25.6 as cut above, 30.7 in pairs).
+    const FwdPlan before = plan;
+    double best_us = 0.9 * 1.9 * (plan.max_chunks > 1 ? best : cost(n_max, items));
     for (int k = 1; k <= 32; ++k) {
       const int chunk = (n_max + 2 * k - 1) / (2 * k), n = (n_max + 2 * chunk - 1) / (2 * chunk);
       if (chunk < 8) break;
-      const double parts = heads * n * 2 * p->seqlen_q * p->head_dim * 8.0;  // written, and read by the join
-      const double t = std::ceil(heads * n / sms) * (chunk + 1.0) * (p->head_dim > 64 ? 3.0 : 2.2) + 3.0 + parts / 4e6;
+      const double t = std::ceil(heads * n / sms) * (chunk + 1.0) * (p->head_dim > 64 ? 3.0 : 2.2) + 3.0 +
+                       part_bytes(n) / 4e6;
       if (t < best_us) {
         best_us = t;
         plan.pair = true;
@@ -302,6 +303,22 @@ FwdPlan plan_fwd(const FmhaFwdParams* p, int sms) {
         plan.items_per_head = n;
         plan.max_chunks = 2 * n;
       }
+    }
+    // That is good enough to choose among the numbers of chunks, but not to choose between pairs and the plan before: it
+    // has the partial rows at half of what they cost, and full tiles, which take less time than others, like others.
+    // Pairs / before, us, D = 64, 2048 keys: 128 rows 148 heads 39 / 31, 1200 heads 246 / 192, 64 rows 1200 heads 198 / 228.
+    // So straight lines through 480 shapes (1 to 128 rows, 1024 to 16384 keys, 8 to 1200 heads, bf16) decide.  Of 3168
+    // shapes 6 are then slower in pairs than before, by 1 to 6 %; without them 89 were, by 2 to 28 %.  Taken, before /
+    // pairs, 64 x 8192: D = 64 64 heads 64 / 46, 128 heads 105 / 76, D = 96 75 / 62 and 118 / 99, D = 128 74 / 64 and 122 /
+    // 103; 96 x 8192: D = 128 75 / 66 and 120 / 107.
+    if (plan.pair) {
+      const bool wide = p->head_dim > 64, full = p->seqlen_q == 128;
+      const double round_us = wide ? 1.75 : full ? 1.35 : 1.5;
+      const double now = before.max_chunks > 1 ? 1.85 * best : round_us * cost(n_max, items) + (wide ? 12.0 : 8.0);
+      const double waves = std::ceil(heads * plan.items_per_head / sms);
+      const double t = (wide ? waves * (2.7 * plan.chunk_tiles + 0.5) + 14.0 : waves * (1.87 * plan.chunk_tiles + 1.8) + 10.5) +
+                       0.55 * part_bytes(plan.items_per_head) / 1e6;
+      if (t >= now) plan = before;
     }
   }
   if (plan.max_chunks > 1) {

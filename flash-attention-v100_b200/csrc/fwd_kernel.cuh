@@ -214,7 +214,7 @@ __device__ __forceinline__ FwdItem fwd_item(const FwdKernelParams& p, int id) {
 // kPair: no more than 128 query rows.  Both query tiles are these rows, each against a chunk of the keys of its
 // own, and both chunks leave partial results.  K and V of tile t come through a ring of their own, half of the
 // slots.  (With one query tile, cut or not, a CTA takes 1.9 us per KV tile: MMA, softmax and MMA one after the
-// other, and half of the SM idle.  64 queries x 8192 keys, 64 heads, us: D = 128, bf16 70 -> 59, D = 64 66 -> 49.)
+// other, and half of the SM idle.  64 queries x 8192 keys, 64 heads, bf16, us: D = 128 74 -> 64, D = 64 64 -> 46.)
 template <int D, bool kBf16 = false, bool kPair = false>
 __global__ void __launch_bounds__(384, 1)
     fmha_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,

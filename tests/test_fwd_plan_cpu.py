@@ -1,0 +1,48 @@
+"""CPU tests of how the forward's work is cut for few queries: the workspace that a call asks for (one plane of fp32 rows and
+LSE per chunk) tells the number of chunks.  Without a device the plan is that for 148 SMs."""
+import ctypes
+
+import pytest
+
+from flash_attn_v100 import cabi
+
+
+def _chunks(heads, n_q, n_k, D, causal=0, shift=0):
+    p = cabi.FmhaFwdParams()
+    p.batch, p.heads, p.seqlen_q, p.seqlen_k, p.head_dim = 1, heads, n_q, n_k, D
+    p.scale, p.causal, p.causal_shift = D ** -0.5, causal, shift
+    plane = heads * n_q * (D + 1) * 4
+    nbytes = cabi.load_library().fmha_fwd_workspace_bytes(ctypes.byref(p))
+    assert nbytes % plane == 0
+    return nbytes // plane
+
+
+# pairs of chunks against whole items, us, bf16, where the partial rows weigh more than the idle half of the SM costs
+@pytest.mark.parametrize("heads,n_q,n_k,D", [
+    (1200, 128, 2048, 64),  # 246 / 192
+    (296, 128, 2048, 64),   # 66 / 53
+    (128, 128, 2048, 64),   # 35 / 30
+    (148, 112, 2048, 64),   # 39 / 34
+    (1200, 128, 2500, 64),  # 275 / 239
+    (148, 127, 2500, 64),   # 45 / 41
+])
+def test_not_cut_where_that_is_slower(built_library, heads, n_q, n_k, D):
+    assert _chunks(heads, n_q, n_k, D) == 0
+
+
+# more than eight items per SM are cut in pairs of chunks only
+@pytest.mark.parametrize("D", [64, 96, 128])
+@pytest.mark.parametrize("n_q", [1, 16, 64, 80])
+def test_pairs_however_many_items(built_library, n_q, D):
+    assert _chunks(1200, n_q, 8192, D) % 2 == 0
+    assert _chunks(1200, n_q, 8192, D) >= 2
+    assert _chunks(1200, n_q, 512, D) == 0  # chunks of less than 8 tiles
+
+
+@pytest.mark.parametrize("D", [64, 96, 128])
+def test_more_query_rows_are_not_cut_sooner(built_library, D):
+    """Partial rows cost and nothing else depends on their number, up to full tiles."""
+    for n_k in (2048, 2500, 3000, 4096, 8192):
+        for heads in (64, 148, 296, 600, 1200):
+            cut = [_chunks(heads, n_q, n_k, D) > 0 for n_q in (1, 32, 64, 96, 112, 127)]
+            assert cut == sorted(cut, reverse=True), (heads, n_k, cut)
