@@ -5,6 +5,7 @@ import torch
 
 from oracle import attention_oracle as oracle
 from tests import helpers
+from tests.test_gpu_fwd_scores import _check
 from tests.test_gpu_padded import _oracle_padded
 
 pytestmark = pytest.mark.gpu
@@ -71,3 +72,107 @@ def test_pairs_of_chunks_in_a_padded_batch():
     assert torch.equal(torch.isfinite(lse), torch.isfinite(ref[1]))
     finite = torch.isfinite(lse)
     assert oracle.max_abs(lse[finite], ref[1][finite]) <= helpers.TOL_LSE_MAX_ABS
+
+
+# ------------------------------------------------------------------------------------------
+# More than eight items per SM, where nothing but pairs asks for a workspace: items follow one another on
+# their SM, through rings of two slots at D = 96 and 128.
+# ------------------------------------------------------------------------------------------
+Z, H = 5, 266  # nine waves of 148, the last one full
+
+
+def _many(n_q, n_k, D, dtype, seed):
+    assert Z * H > 8 * torch.cuda.get_device_properties(0).multi_processor_count
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return tuple(torch.randn((Z, n, H, D), generator=g, device="cuda", dtype=dtype) for n in (n_q, n_k, n_k))
+
+
+def _reference(q, k, v, scale, causal=False, shift=0, sq=None, sk=None):
+    """fp32 softmax on the GPU; rows that see nothing: O = 0, LSE = -inf."""
+    out, lse = torch.empty(q.shape, device="cuda"), torch.empty((Z, H, q.shape[1]), device="cuda")
+    row, key = (torch.arange(t.shape[1], device="cuda") for t in (q, k))
+    for z in range(Z):
+        qz, kz, vz = (t[z].float().transpose(0, 1) for t in (q, k, v))
+        s = qz @ kz.transpose(1, 2) * scale
+        hidden = (key >= (len(key) if sk is None else sk[z]))[None, :] | (row >= (len(row) if sq is None else sq[z]))[:, None]
+        if causal:
+            hidden = hidden | (key[None, :] > row[:, None] + shift)
+        s = s.masked_fill(hidden, float("-inf"))
+        p = s.softmax(-1).masked_fill(hidden.all(-1)[:, None], 0.0)
+        out[z], lse[z] = (p @ vz).transpose(0, 1), s.logsumexp(-1)
+    return out, lse
+
+
+def _tol(dtype):
+    return helpers.TOL_O_MAX_ABS if dtype == torch.float16 else helpers.TOL_O_MAX_ABS_BF16
+
+
+def _run_pairs(q, k, v, scale, causal=False, shift=0, **kw):
+    out, lse = _run(q, k, v, scale, causal, shift, **kw)
+    return out.cuda(), lse.cuda()
+
+
+@pytest.mark.parametrize("n_q,n_k,causal,shift", [
+    (16, 3200, False, 0), (16, 3150, False, 0),  # 25 tiles: the second chunk is a tile shorter
+    (1, 3072, False, 0), (64, 6100, False, 0),
+    (16, 3300, True, 3000),  # the diagonal and keys that no row sees in the second chunk
+    (16, 3300, True, 3064),  # ... the diagonal crosses tiles
+])
+@pytest.mark.parametrize("D", [64, 96, 128])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_pairs_one_after_the_other(n_q, n_k, causal, shift, D, dtype):
+    q, k, v = _many(n_q, n_k, D, dtype, seed=67)
+    scale = oracle.default_scale(D)
+    out, lse = _run_pairs(q, k, v, scale, causal, shift)
+    r_out, r_lse = _reference(q, k, v, scale, causal, shift)
+    assert oracle.max_abs(out.float(), r_out) <= _tol(dtype)
+    assert oracle.max_abs(lse, r_lse) <= helpers.TOL_LSE_MAX_ABS
+
+
+@pytest.mark.parametrize("D", [64, 96, 128])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_pairs_one_after_the_other_in_a_padded_batch(D, dtype):
+    # 25 tiles in chunks of 13 and 12; entries with one tile in the second chunk, with none, with none at all
+    n_q, n_k, sq, sk = 16, 3200, [16, 1, 16, 0, 9], [3200, 1665, 1664, 77, 0]
+    q, k, v = _many(n_q, n_k, D, dtype, seed=68)
+    scale = oracle.default_scale(D)
+    lens = {"seqused_q": sq, "seqused_k": sk}
+    out, lse = _run_pairs(q, k, v, scale, **{n: torch.tensor(x, dtype=torch.int32, device="cuda") for n, x in lens.items()})
+    r_out, r_lse = _reference(q, k, v, scale, sq=sq, sk=sk)
+    assert oracle.max_abs(out.float(), r_out) <= _tol(dtype)
+    seen = torch.isfinite(r_lse)
+    assert torch.equal(torch.isfinite(lse), seen)
+    assert oracle.max_abs(lse[seen], r_lse[seen]) <= helpers.TOL_LSE_MAX_ABS
+    assert not out[~seen.transpose(1, 2)].any()
+
+
+@pytest.mark.parametrize("what", ["query rows", "keys of the first chunk", "keys of the second chunk"])
+@pytest.mark.parametrize("D", [64, 96, 128])
+def test_pairs_with_rows_that_are_not_finite(D, what):
+    """Every row that sees one is not finite, the rows of other heads are right."""
+    q, k, v = _many(16, 3200, D, torch.float16, seed=69)
+    scale = oracle.default_scale(D)
+    for h in range(0, H, 3):
+        for z in range(Z):
+            if what == "query rows":
+                q[z, h % 16, h, 3] = float("nan") if h % 2 else float("inf")
+            else:  # in either half of a round and in every column that may take a path of its own
+                k[z, (0 if "first" in what else 1664) + 128 * z + h % 128, h, 7] = float("nan")
+    _check(_run_pairs(q, k, v, scale), _reference(q, k, v, scale), helpers.TOL_O_MAX_ABS)
+
+
+@pytest.mark.parametrize("D", [64, 96, 128])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_pairs_with_leaping_scores(D, dtype):
+    """One key far above all others, in either half of the first, a middle and the last round of either chunk."""
+    q, k, v = _many(16, 3200, D, dtype, seed=70)
+    scale = oracle.default_scale(D)
+    q[:, ::2, :, 0], q[:, 1::2, :, 0], k[..., 0] = 20.0, -20.0, 0.0
+    for z, leap in enumerate((95.0, 130.0, 180.0, 256.0, 400.0)):
+        for h in range(H):
+            tile = (0, 6, 12, 13, 19, 24)[h % 6]
+            k[z, tile * 128 + (h // 6 * 16 + h // 48) % 128, h, 0] = leap / (20.0 * scale)
+    ref = _reference(q, k, v, scale)
+    # weights on a key or two, each rounded to the 16-bit type, and so is O
+    bound = (2.0 ** -11 if dtype == torch.float16 else 2.0 ** -8) * (v.abs().max().item() + ref[0].abs().max().item())
+    _check(_run_pairs(q, k, v, scale), ref, bound)
