@@ -89,9 +89,9 @@ def _many(n_q, n_k, D, dtype, seed):
 
 def _reference(q, k, v, scale, causal=False, shift=0, sq=None, sk=None):
     """fp32 softmax on the GPU; rows that see nothing: O = 0, LSE = -inf."""
-    out, lse = torch.empty(q.shape, device="cuda"), torch.empty((Z, H, q.shape[1]), device="cuda")
+    out, lse = torch.empty(q.shape, device="cuda"), torch.empty((q.shape[0], q.shape[2], q.shape[1]), device="cuda")
     row, key = (torch.arange(t.shape[1], device="cuda") for t in (q, k))
-    for z in range(Z):
+    for z in range(q.shape[0]):
         qz, kz, vz = (t[z].float().transpose(0, 1) for t in (q, k, v))
         s = qz @ kz.transpose(1, 2) * scale
         hidden = (key >= (len(key) if sk is None else sk[z]))[None, :] | (row >= (len(row) if sq is None else sq[z]))[:, None]
@@ -176,3 +176,15 @@ def test_pairs_with_leaping_scores(D, dtype):
     # weights on a key or two, each rounded to the 16-bit type, and so is O
     bound = (2.0 ** -11 if dtype == torch.float16 else 2.0 ** -8) * (v.abs().max().item() + ref[0].abs().max().item())
     _check(_run_pairs(q, k, v, scale), ref, bound)
+
+
+@pytest.mark.parametrize("D", [64, 96, 128])
+def test_pairs_with_sms_left_free(D):
+    """Items dealt out over eight SMs, nine to each."""
+    q, k, v = (t[:1, :, :72].contiguous() for t in _many(16, 3200, D, torch.bfloat16, seed=71))
+    scale = oracle.default_scale(D)
+    margin = torch.cuda.get_device_properties(0).multi_processor_count - 8
+    out, lse = _run_pairs(q, k, v, scale, sm_margin=margin)
+    r_out, r_lse = _reference(q, k, v, scale)
+    assert oracle.max_abs(out.float(), r_out) <= _tol(torch.bfloat16)
+    assert oracle.max_abs(lse, r_lse) <= helpers.TOL_LSE_MAX_ABS
