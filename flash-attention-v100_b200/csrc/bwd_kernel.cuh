@@ -25,7 +25,7 @@
 //   warps 8-11      dQ group: one thread per query row; tensor memory -> registers ->
 //                   shared-memory staging -> TMA reduce-add into the fp32 dQ accumulator
 //                   (bulk async adds: no per-thread atomics in the load/store pipeline)
-//   warp 12         TMA producer (K, V once; Q_i through a 2-stage ring, dO_i single stage) and
+//   warp 12         TMA producer (K, V once; Q_i through a ring of two slots, four at D = 64, dO_i through one) and
 //                   source of the items
 //   warp 13         MMA issuer: the whole warp runs the loop, one elected lane issues
 //
@@ -38,8 +38,8 @@
 // instruction cache.  The latter decides more than it seems: the same kernel with its MMA loops and
 // write-outs unrolled fetched 1.7 times the instructions from behind the first-level cache
 // and ran 5-18 % SLOWER than one CTA per item did, rolled up it is 5-10 % faster.  Hence the loops below.
-// They ease it and do not settle it: 1.04 stalled cycles per issue for want of instructions, 0.57
-// with one CTA per item (Z8 H32 N2048 D128 causal).
+// They settle it: 0.56 stalled cycles per issue for want of instructions, as with one CTA per item (0.57; 1.04 as long
+// as the deterministic turns and P o D in registers were in the loops; Z8 H32 N2048 D128 causal).
 // One CTA per item spent about 7 us of its life on its head and tail (a causal item at N = 2048 has
 // 8.5 tiles of 2.2 us).  Whole backward, one CTA per item -> this, steady state: Z8 H32 N2048 D128
 // causal 1025 -> 955 us, without a mask 1665 -> 1570, Z64 H16 N512 D64 422 -> 385, Z1 H16 N16384
@@ -195,8 +195,8 @@ __device__ __forceinline__ BwdItem bwd_item(const BwdKernelParams& p, int id) {
 // Under a causal mask: from the diagonal downwards, and the items of a head are dispatched in that order.
 // The item on the diagonal comes first to its query tile, the one below it a tile later, and so on: no item
 // waits that has not been held up itself.  (In ascending order the item of KV tile kb had to wait for all kb
-// before it when it came to its first query tile.  Whole backward, us, ascending / so: Z2 H16 N2048 D128 256 / 206,
-// Z8 H32 N2048 D128 1777 / 1313, Z1 H8 N16384 D128 4272 / 2229, Z4 H16 N1024 D64 138 / 100.)
+// before it when it came to its first query tile.  Whole backward, us, ascending / so: Z2 H16 N2048 D128 257 / 202,
+// Z8 H32 N2048 D128 1757 / 1284, Z1 H8 N16384 D128 4289 / 2182, Z4 H16 N1024 D64 137 / 97.)
 __device__ __forceinline__ int bwd_turn(const BwdKernelParams& p, const BwdItem& it, int tile) {
   if (!p.causal) return it.kb;
   const long long diagonal = ((long long)(tile + 1) * 128 + p.causal_shift - 1) / 128;  // last KV tile it sees

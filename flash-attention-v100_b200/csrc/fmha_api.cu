@@ -168,8 +168,12 @@ int round_up_128(int x) { return (x + 127) / 128 * 128; }
 // time: their grids are long, and many heads' query tiles would not share the L2.
 // FMHA_BWD_HEAD_GROUP overrides (tuning experiments).
 // Deterministic, without a mask: the items of a head run staggered by a query tile, and the more heads have their
-// first KV tiles in work, the less of that is waiting: as many as fit the L2, up to 32, in even groups.  Z2 H16
-// N2048 D128, us: groups of 8 342, 16 329, 32 315; of 30 (and one of 2) 369.
+// first KV tiles in work, the less of that is waiting: as many as fit the L2, up to 32, in even groups.  Whole backward,
+// us, one head / 8 / 16 / 32 / this rule: D128 Z2 H16 N2048 433 / 346 / 326 / 311 / 311, Z3 H11 N2048 444 / 398 / 382 /
+// 368 / 331 (two groups of 17 and 16), Z1 H8 N8192 1456 / 1117 / 1117 / 1117 / 1117, Z2 H9 N8192 2912 / 2402 / 2357 /
+// 2184 / 2246, Z1 H5 N16384 2953 / 2715 / 2715 / 2715 / 2815; D64 Z16 H16 N512 187 / 178 / 168 / 157 / 157, Z2 H16 N4096 1027
+// / 753 / 715 / 699 / 698.  Over 60 shapes (D = 64, 96, 128, N = 512 to 16384, 5 to 256 heads) 0.89 to 1.04 of the
+// best of the four.  (The waiting is worth more here than the L2, so the limit is higher than the forward's 48 MB.)
 int bwd_head_group(int num_kv_blocks, bool causal, bool deterministic, int num_heads, double bytes_per_head) {
   static const int forced = []() {
     const char* e = std::getenv("FMHA_BWD_HEAD_GROUP");
