@@ -318,7 +318,9 @@ FwdPlan plan_fwd(const FmhaFwdParams* p, int sms) {
     if (plan.pair) {
       const bool wide = p->head_dim > 64, full = p->seqlen_q == 128;
       const double round_us = wide ? 1.75 : full ? 1.35 : 1.5;
-      const double now = before.max_chunks > 1 ? 1.85 * best : round_us * cost(n_max, items) + (wide ? 12.0 : 8.0);
+      // (the items of a head with one query block are equal under a mask, too: whole waves, other than in cost())
+      const double whole = round_us * std::ceil(heads / sms) * (n_max + 0.5) + (wide ? 12.0 : 8.0);
+      const double now = before.max_chunks > 1 ? 1.85 * best : whole;
       const double waves = std::ceil(heads * plan.items_per_head / sms);
       const double t = (wide ? waves * (2.7 * plan.chunk_tiles + 0.5) + 14.0 : waves * (1.87 * plan.chunk_tiles + 1.8) + 10.5) +
                        0.55 * part_bytes(plan.items_per_head) / 1e6;

@@ -46,3 +46,9 @@ def test_more_query_rows_are_not_cut_sooner(built_library, D):
         for heads in (64, 148, 296, 600, 1200):
             cut = [_chunks(heads, n_q, n_k, D) > 0 for n_q in (1, 32, 64, 96, 112, 127)]
             assert cut == sorted(cut, reverse=True), (heads, n_k, cut)
+
+
+@pytest.mark.parametrize("heads,n_q,n_k,D", [(160, 64, 8192, 64), (600, 64, 3000, 64), (160, 96, 8192, 64), (64, 32, 8192, 128)])
+def test_a_mask_that_hides_nothing_changes_no_plan(built_library, heads, n_q, n_k, D):
+    """(two waves of 160 whole items under a causal mask 199 us, in pairs 108)"""
+    assert _chunks(heads, n_q, n_k, D, 1, n_k) == _chunks(heads, n_q, n_k, D) >= 2
