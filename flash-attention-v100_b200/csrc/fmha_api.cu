@@ -322,8 +322,12 @@ FwdPlan plan_fwd(const FmhaFwdParams* p, int sms) {
       const double whole = round_us * std::ceil(heads / sms) * (n_max + 0.5) + (wide ? 12.0 : 8.0);
       const double now = before.max_chunks > 1 ? 1.85 * best : whole;
       const double waves = std::ceil(heads * plan.items_per_head / sms);
+      // The lengths of a padded batch are not known here; taken as half on average, which is the same as counting the
+      // partial rows twice.  8 entries of n/8 to n keys, 412 shapes: 8 are slower in pairs then, by 9 % at most (D = 64, 96 x 4096,
+      // 600 heads 142 / 154), without it 26, by up to 32 % (96 x 2048, 600 heads 77 / 101).
+      const bool unequal = p->seqused_k != nullptr && before.max_chunks <= 1;
       const double t = (wide ? waves * (2.7 * plan.chunk_tiles + 0.5) + 14.0 : waves * (1.87 * plan.chunk_tiles + 1.8) + 10.5) +
-                       0.55 * part_bytes(plan.items_per_head) / 1e6;
+                       (unequal ? 1.1 : 0.55) * part_bytes(plan.items_per_head) / 1e6;
       if (t >= now) plan = before;
     }
   }

@@ -7,8 +7,9 @@ import pytest
 from flash_attn_v100 import cabi
 
 
-def _chunks(heads, n_q, n_k, D, causal=0, shift=0):
+def _chunks(heads, n_q, n_k, D, causal=0, shift=0, padded=False):
     p = cabi.FmhaFwdParams()
+    p.seqused_k = 16 if padded else None  # an address that a plan does not follow
     p.batch, p.heads, p.seqlen_q, p.seqlen_k, p.head_dim = 1, heads, n_q, n_k, D
     p.scale, p.causal, p.causal_shift = D ** -0.5, causal, shift
     plane = heads * n_q * (D + 1) * 4
@@ -52,3 +53,20 @@ def test_more_query_rows_are_not_cut_sooner(built_library, D):
 def test_a_mask_that_hides_nothing_changes_no_plan(built_library, heads, n_q, n_k, D):
     """(two waves of 160 whole items under a causal mask 199 us, in pairs 108)"""
     assert _chunks(heads, n_q, n_k, D, 1, n_k) == _chunks(heads, n_q, n_k, D) >= 2
+
+
+# 8 entries of n_k / 8 to n_k keys, pairs against whole items, us
+@pytest.mark.parametrize("heads,n_q,n_k,D", [
+    (600, 96, 2048, 64),   # 101 / 77
+    (600, 128, 4096, 64),  # 152 / 119
+    (296, 64, 2048, 64),   # 52 / 45
+    (600, 64, 4096, 128),  # 179 / 159
+])
+def test_a_padded_batch_is_not_cut_where_that_is_slower(built_library, heads, n_q, n_k, D):
+    assert _chunks(heads, n_q, n_k, D, padded=True) == 0
+
+
+# ... 43 / 35 where the alternative is cut, too, and 105 / 76 for many keys
+@pytest.mark.parametrize("heads,n_q,n_k,D", [(64, 64, 4096, 128), (128, 64, 8192, 64), (1200, 16, 8192, 128)])
+def test_a_padded_batch_is_cut_in_pairs(built_library, heads, n_q, n_k, D):
+    assert _chunks(heads, n_q, n_k, D, padded=True) >= 2
