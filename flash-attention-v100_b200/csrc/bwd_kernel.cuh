@@ -93,7 +93,7 @@ constexpr int kBwdRegsDq = 128 + (128 - kBwdRegsIssue) + 2 * (128 - kBwdRegsComp
 static_assert(kBwdRegsIssue <= 128 && kBwdRegsCompute <= 128 && kBwdRegsDq >= 128,
               "setmaxnreg.dec must not raise and .inc must not lower the 128 registers of the launch");
 
-template <int D, bool kBf16 = false>
+template <int D, bool kBf16 = false, int DR = D>
 struct BwdTraits {
   static constexpr int kBlock = 128;
   static constexpr int kBoxes = D / 64;
@@ -118,8 +118,8 @@ struct BwdTraits {
   // warps that read dK (and as many dV) out of tensor memory at the end of an item
   static constexpr int kDrainWarps = (D == 128) ? 8 : 4;
   static constexpr uint32_t kIdescST = umma_idesc_f16(128, 128, 0, 0, kBf16);  // S^T, dP^T
-  static constexpr uint32_t kIdescDV = umma_idesc_f16(128, D, 0, 1, kBf16);    // dV, dK
-  static constexpr uint32_t kIdescDQ = umma_idesc_f16(128, D, 1, 1, kBf16);    // dQ
+  static constexpr uint32_t kIdescDV = umma_idesc_f16(128, DR, 0, 1, kBf16);   // dV, dK
+  static constexpr uint32_t kIdescDQ = umma_idesc_f16(128, DR, 1, 1, kBf16);   // dQ
 };
 
 // A work item: one KV tile of one (batch, head) and the query tiles that see it.  The producer warp
@@ -203,9 +203,11 @@ __device__ __forceinline__ int bwd_turn(const BwdKernelParams& p, const BwdItem&
   return (int)min(diagonal, (long long)(it.sk - 1) / 128) - it.kb;
 }
 
-// DR <= D: elements per row of the tensors.  96 runs at D = 128: the tile loads fill columns
-// 96-127 with zeros, so those columns of dQ, dK and dV are zeros that are never written out, and
-// the fp32 buffers have DR elements per row.
+// DR <= D: elements per row of the tensors.  96 runs on the tiles of D = 128: the tile loads fill columns
+// 96-127 with zeros, the MMAs leave them out (six steps instead of eight, N = 96 instead of 128), columns 96-127 of
+// dQ, dK and dV do not exist (what the write-out reads there is clipped by the store), and the fp32 buffers have DR
+// elements per row.  Z8 H32 N2048 D96 causal, fp16, forward and backward, the zeros multiplied too / left out: 1206 /
+// 1165 us (the tensor cores spend little power on zeros, and it is the power cap that bounds both).
 // kDet: deterministic dQ, with the items dealt out.  An instantiation of its own: the turns cost the other mode
 // 1 to 3 % when they were a branch in the dQ group's loop.
 template <int D, bool kBf16 = false, int DR = D, bool kDet = false>
@@ -214,7 +216,7 @@ __global__ void __launch_bounds__(512, 1)
                     const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
                     const __grid_constant__ CUtensorMap tm_dk, const __grid_constant__ CUtensorMap tm_dv,
                     const __grid_constant__ CUtensorMap tm_dqacc, const BwdKernelParams p) {
-  using T = BwdTraits<D, kBf16>;
+  using T = BwdTraits<D, kBf16, DR>;
   // (no static shared memory: the tiles need every byte, and 1024-byte alignment)
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t smem_base = smem_u32(smem_raw);
@@ -470,10 +472,22 @@ __global__ void __launch_bounds__(512, 1)
       // steps of 16 along the contraction and blocks of 64, in descriptor units
       constexpr uint32_t kStepK = 32 >> 4, kBlockK = T::kBoxBytes >> 4;  // K-major operand
       constexpr uint32_t kStepMn = 2048 >> 4, kBlockMn = 4 * kStepMn;    // MN-major operand
-      // C[128 x 128] = A[128 x D] B[128 x D]^T, both K-major
+      // C[128 x 128] = A[128 x DR] B[128 x DR]^T, both K-major
       auto issue_kmajor = [&](uint32_t d_col, uint32_t a_addr, uint32_t b_addr) {
-        issue_ss(T::kBoxes, d_col, umma_desc_lo(a_addr, kLboKMajor), kBlockK, kStepK, umma_desc_lo(b_addr, kLboKMajor),
-                 kBlockK, kStepK, T::kIdescST, 0u);
+        uint32_t a_lo = umma_desc_lo(a_addr, kLboKMajor), b_lo = umma_desc_lo(b_addr, kLboKMajor);
+        if constexpr (DR % 64 == 0) {
+          issue_ss(T::kBoxes, d_col, a_lo, kBlockK, kStepK, b_lo, kBlockK, kStepK, T::kIdescST, 0u);
+        } else {  // 96: six steps, two at a time, the last two in the second box
+#pragma unroll 1
+          for (int b = 0; b < DR / 32; ++b) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+              umma_ss_elect(tmem_base + d_col, a_lo + i * kStepK, b_lo + i * kStepK, T::kIdescST, b + i > 0 ? 1u : 0u);
+            const uint32_t step = b == 0 ? 2 * kStepK : kBlockK - 2 * kStepK;
+            a_lo += step;
+            b_lo += step;
+          }
+        }
       };
       auto slot_addr = [&](int slot) { return smem_base + slot * T::kTileBytes; };
       uint32_t filled = 0;  // bit s: fills of slot s waited for so far, modulo 2
@@ -798,7 +812,7 @@ __global__ void __launch_bounds__(512, 1)
       reg_alloc<kBwdRegsDq>();
       const uint32_t tDQ = tmem_base + lane_addr + T::kColDQ;
       const bool tl = (r == 0);
-      constexpr int kChunks = (DR + 31) / 32;  // 32-column chunks of a dQ row
+      constexpr int kChunks = DR / 32;  // 32-column chunks of a dQ row
       // an odd number of chunks per tile breaks the alternation of the two staging buffers by
       // chunk index: count the chunks staged so far instead
       [[maybe_unused]] uint32_t chunk_no = 0;
@@ -817,9 +831,9 @@ __global__ void __launch_bounds__(512, 1)
           if (tl) FMHA_TL(1, g, 1);
           // The whole dQ row goes to registers first so that the dQ columns are released to the
           // next dP^T as early as possible; then 32-column chunks go out through shared memory.
-          uint32_t acc[D / 32][32];
+          uint32_t acc[kChunks][32];
 #pragma unroll
-          for (int cc = 0; cc < D / 32; ++cc) tmem_ld32(tDQ + cc * 32, acc[cc]);
+          for (int cc = 0; cc < kChunks; ++cc) tmem_ld32(tDQ + cc * 32, acc[cc]);
           tmem_wait_ld();
           tc_fence_before();
           __syncwarp();

@@ -350,16 +350,16 @@ int fwd_head_group(const FmhaFwdParams* p) {
   return (int)std::max(1.0, std::min((double)p->batch * p->heads, 48e6 / kv_bytes));
 }
 
-// D is the head dimension the kernel runs at; the tensors have p->head_dim <= D elements per row
-// (96 runs at D = 128: the tensor maps describe 96 columns, the loads fill the rest of a
-// 128-wide tile with zeros and the stores clip it)
-template <int D, bool kBf16>
+// D is the head dimension the tiles have; the tensors have DR <= D elements per row (96 runs on the tiles of
+// 128: the tensor maps describe 96 columns, the loads fill the rest of a 128-wide tile with zeros, the MMAs leave it
+// out and the stores clip it)
+template <int D, bool kBf16, int DR = D>
 int launch_fwd(const FmhaFwdParams* p, void* workspace, size_t workspace_bytes, cudaStream_t stream) {
-  using T = fmha::FwdTraits<D, kBf16>;
+  using T = fmha::FwdTraits<D, kBf16, DR>;
   using E = typename std::conditional<kBf16, __nv_bfloat16, __half>::type;
   CUtensorMap tq, tk, tv, to;
   int rc;
-  const int Dr = p->head_dim;
+  constexpr int Dr = DR;
   if ((rc = make_tensor_map(&tq, p->q, p->batch, p->seqlen_q, p->heads, Dr, p->q_strides, kBf16)))
     return rc;
   if ((rc = make_tensor_map(&tk, p->k, p->batch, p->seqlen_k, p->heads, Dr, p->k_strides, kBf16)))
@@ -406,10 +406,10 @@ int launch_fwd(const FmhaFwdParams* p, void* workspace, size_t workspace_bytes, 
   kp.deal = kp.num_items <= sms || p->sm_margin > 0;
   const unsigned grid = kp.deal ? (unsigned)std::min(kp.num_items, sms) : (unsigned)kp.num_items;
   const bool launched =
-      plan.pair ? launch_with_smem<fmha::fmha_fwd_kernel<D, kBf16, true>>(dev, grid, T::kThreads, T::kSmemBytes, stream,
-                                                                          tq, tk, tv, to, kp)
-                : launch_with_smem<fmha::fmha_fwd_kernel<D, kBf16>>(dev, grid, T::kThreads, T::kSmemBytes, stream, tq, tk,
-                                                                    tv, to, kp);
+      plan.pair ? launch_with_smem<fmha::fmha_fwd_kernel<D, kBf16, true, DR>>(dev, grid, T::kThreads, T::kSmemBytes,
+                                                                              stream, tq, tk, tv, to, kp)
+                : launch_with_smem<fmha::fmha_fwd_kernel<D, kBf16, false, DR>>(dev, grid, T::kThreads, T::kSmemBytes,
+                                                                               stream, tq, tk, tv, to, kp);
   if (!launched) return FMHA_ERR_LAUNCH;
   if (plan.max_chunks > 1) {
     const long long rows = (long long)kp.num_heads_total * (p->seqlen_q - plan.first_cut_row);
@@ -584,11 +584,11 @@ int fmha_fwd_with_workspace(const FmhaFwdParams* p, void* workspace, size_t work
   if ((rc = check_strides(p->v_strides, p->seqlen_k, p->heads, p->batch))) return rc;
   if ((rc = check_strides(p->o_strides, p->seqlen_q, p->heads, p->batch))) return rc;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (p->dtype == FMHA_DTYPE_BF16)
-    return p->head_dim > 64 ? launch_fwd<128, true>(p, workspace, workspace_bytes, s)
-                            : launch_fwd<64, true>(p, workspace, workspace_bytes, s);
-  return p->head_dim > 64 ? launch_fwd<128, false>(p, workspace, workspace_bytes, s)
-                          : launch_fwd<64, false>(p, workspace, workspace_bytes, s);
+  if (p->dtype == FMHA_DTYPE_BF16) {
+    FMHA_DISPATCH_DIMS(p->head_dim, return launch_fwd<D, true, DR>(p, workspace, workspace_bytes, s);)
+  } else {
+    FMHA_DISPATCH_DIMS(p->head_dim, return launch_fwd<D, false, DR>(p, workspace, workspace_bytes, s);)
+  }
 }
 
 size_t fmha_fwd_workspace_bytes(const FmhaFwdParams* p) {

@@ -95,7 +95,9 @@ struct FwdKernelParams {
 // 126.7 / 124.2 / 127.7 (131.8); no difference between none and 1 at D = 128, N = 2048 causal.
 constexpr int kFwdPolyPairs = 1;
 
-template <int D, bool kBf16 = false>
+// DR <= D: elements per row of the tensors.  96 runs on the tiles of 128: the second box of a tile load holds 32
+// columns and zeros, which the MMAs leave out.
+template <int D, bool kBf16 = false, int DR = D>
 struct FwdTraits {
   static constexpr int kBlockM = 128;  // rows per query tile
   static constexpr int kTilesM = 2;    // query tiles per work item
@@ -110,7 +112,7 @@ struct FwdTraits {
   static constexpr int kSmemBytes = 1024 + kTilesM * (kTileBytes + kBoxBytes) + kStages * kTileBytes;
   static constexpr int kTmemCols = 512;
   static constexpr uint32_t kIdescQK = umma_idesc_f16(128, kBlockN, 0, 0, kBf16);
-  static constexpr uint32_t kIdescPV = umma_idesc_f16(128, D, 0, 1, kBf16);
+  static constexpr uint32_t kIdescPV = umma_idesc_f16(128, DR, 0, 1, kBf16);
 };
 
 constexpr int kFwdRegsIssue = 88;                                 // warps 8-11
@@ -215,12 +217,12 @@ __device__ __forceinline__ FwdItem fwd_item(const FwdKernelParams& p, int id) {
 // own, and both chunks leave partial results.  K and V of tile t come through a ring of their own, half of the
 // slots.  (With one query tile, cut or not, a CTA takes 1.9 us per KV tile: MMA, softmax and MMA one after the
 // other, and half of the SM idle.  64 queries x 8192 keys, 64 heads, bf16, us: D = 128 74 -> 64, D = 64 64 -> 46.)
-template <int D, bool kBf16 = false, bool kPair = false>
+template <int D, bool kBf16 = false, bool kPair = false, int DR = D>
 __global__ void __launch_bounds__(384, 1)
     fmha_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                     const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o,
                     const FwdKernelParams p) {
-  using T = FwdTraits<D, kBf16>;
+  using T = FwdTraits<D, kBf16, DR>;
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(16) uint8_t clc_word[16];
   __shared__ uint64_t bar_clc;                        // the answer to the last request is in clc_word
@@ -552,7 +554,7 @@ __global__ void __launch_bounds__(384, 1)
             const uint32_t a_lo = q_lo0 + ((t * T::kTileBytes) >> 4);
             const uint32_t b_lo = umma_desc_lo(kPair ? ring_smem + slot * T::kTileBytes : k_addr, kLboKMajor);
 #pragma unroll
-            for (int ks = 0; ks < D / 16; ++ks) {
+            for (int ks = 0; ks < DR / 16; ++ks) {
               const uint32_t off = ((ks >> 2) * T::kBoxBytes + (ks & 3) * 32) >> 4;
               umma_ss_elect(tmem_base + t * 128, a_lo + off, b_lo + off, idesc_qk, ks > 0 ? 1u : 0u);
             }
@@ -690,7 +692,7 @@ __global__ void __launch_bounds__(384, 1)
                 const float alpha = isinf(m_new) ? 1.f : fast_exp2((m_ref - m_new) * c);
                 l *= alpha;
 #pragma unroll 1
-                for (int cc = 0; cc < D / 16; ++cc) {
+                for (int cc = 0; cc < DR / 16; ++cc) {
                   uint32_t o[16];
                   tmem_ld16(tO + cc * 16, o);
                   tmem_wait_ld();
@@ -766,13 +768,13 @@ __global__ void __launch_bounds__(384, 1)
         }
         if (split) {
           if (nd == 0) continue;  // LSE = -inf: the combine kernel reads no row
-          float* dst = p.o_part + (((size_t)chunk * p.num_heads_total + done.zh) * p.seqlen_q + row) * p.row_elems;
+          float* dst = p.o_part + (((size_t)chunk * p.num_heads_total + done.zh) * p.seqlen_q + row) * DR;
 #pragma unroll 1
-          for (int cc = 0; cc < D / 16; ++cc) {
+          for (int cc = 0; cc < DR / 16; ++cc) {
             uint32_t o[16];
             tmem_ld16(tO + cc * 16, o);
             tmem_wait_ld();
-            if (row < p.seqlen_q && cc * 16 < p.row_elems) {
+            if (row < p.seqlen_q) {
 #pragma unroll
               for (int i = 0; i < 16; i += 4)
                 *reinterpret_cast<float4*>(dst + cc * 16 + i) =
@@ -785,17 +787,17 @@ __global__ void __launch_bounds__(384, 1)
           if (lane == 0) mbar_arrive(smem_u32(&bar_o_read[t]));
           continue;
         }
-        uint32_t o[D / 32][32];
+        uint32_t o[DR / 32][32];
         if (nd > 0) {
 #pragma unroll
-          for (int cc = 0; cc < D / 32; ++cc) tmem_ld32(tO + cc * 32, o[cc]);
+          for (int cc = 0; cc < DR / 32; ++cc) tmem_ld32(tO + cc * 32, o[cc]);
           tmem_wait_ld();
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(smem_u32(&bar_o_read[t]));
         } else {
 #pragma unroll
-          for (int cc = 0; cc < D / 32; ++cc)
+          for (int cc = 0; cc < DR / 32; ++cc)
 #pragma unroll
             for (int i = 0; i < 32; ++i) o[cc][i] = 0u;
         }
@@ -806,7 +808,7 @@ __global__ void __launch_bounds__(384, 1)
           if (row_in_tile == 0 && stored) tma_wait_group_read<0>();  // the box's last store has been read
           named_bar_sync(1 + t, 128);
 #pragma unroll
-          for (int ch = 0; ch < 8; ++ch) {  // 16-byte chunk (8 fp16) of this row
+          for (int ch = 0; ch < (DR - b * 64 < 64 ? 4 : 8); ++ch) {  // 16-byte chunk (8 fp16) of this row
             const uint32_t* w = &o[b * 2 + (ch >> 2)][(ch & 3) * 8];
             uint32_t h4[4];
 #pragma unroll
