@@ -26,7 +26,7 @@ EXT_PATH = os.path.join(HERE, EXT_NAME + (sysconfig.get_config_var("EXT_SUFFIX")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
-    "-shared", "-Xcompiler", "-fPIC", "--split-compile=0",  # kernels are optimised in parallel
+    "-shared", "-Xcompiler", "-fPIC",
 ]
 
 
