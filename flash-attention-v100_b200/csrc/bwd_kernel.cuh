@@ -6,46 +6,47 @@
 // 503-506), with dQ accumulated in fp32 instead of the reference's fp16 atomics (:543,693).
 //
 // A work item is one 128-row KV tile of one (batch, head) and the query tiles (128 rows) that can
-// see it.  A CTA stays on its SM and takes item after item (cluster launch control); the first S^T
-// and P^T of an item run beside the last dS^T, dQ and dK of the one before.  Everything is computed
-// TRANSPOSED so that the KV rows sit on the 128
+// see it.  A CTA stays on its SM and takes item after item (cluster launch control); dK and dV of an item are
+// written out beside the first P^T of the next.  Everything is computed TRANSPOSED so that the KV rows sit on the 128
 // tensor-memory lanes, which lets P^T feed the dV MMA straight from tensor memory:
 //
 //   S^T  = K  Q_i^T    (A = K  smem K-major,  B = Q_i  smem K-major)      -> TMEM [0,128)
 //   dP^T = V  dO_i^T   (A = V  smem K-major,  B = dO_i smem K-major)      -> TMEM [128,256)
 //   dV  += P^T dO_i    (A = P^T TMEM fp16 over S^T, B = dO_i smem MN-major)-> TMEM [256+D, ..)
-//                      (P^T columns [0,32) and [64,96): one 32-column block per compute group)
+//                      (P^T: each compute group's packed columns at the start of its own part of S^T)
 //   dK  += dS^T Q_i    (A = dS^T smem K-major, B = Q_i smem MN-major)      -> TMEM [256, 256+D)
 //   dQ_i = dS  K       (A = dS^T smem read MN-major, B = K smem MN-major)  -> TMEM [128,128+D)
 //                      (aliases dP^T, which is dead once dS^T is in shared memory)
 //
-//   warps 0-3, 4-7  two compute groups: one thread per KV row, group g owns query columns
-//                   [64g, 64g+64) of the tile: P^T = exp2(S^T*c - lse2) and
-//                   dS^T = P^T o (dP^T - D)
-//   warps 8-11      dQ group: one thread per query row; tensor memory -> registers ->
+//   compute groups  two of four warps, four at D = 64: one thread per KV row, group g owns 128 / groups query
+//                   columns of the tile: P^T = exp2(S^T*c - lse2) and dS^T = P^T o (dP^T - D)
+//   dQ group        four warps, one thread per query row; tensor memory -> registers ->
 //                   shared-memory staging -> TMA reduce-add into the fp32 dQ accumulator
-//                   (bulk async adds: no per-thread atomics in the load/store pipeline)
-//   warp 12         TMA producer (K, V once; Q_i through a ring of two slots, four at D = 64, dO_i through one) and
+//                   (bulk async adds: no per-thread atomics in the load/store pipeline); at the end of an
+//                   item dV and dK the same way, as 16-bit stores
+//   producer warp   TMA (K, V once; Q_i through a ring of two slots, four at D = 64, dO_i through one) and
 //                   source of the items
-//   warp 13         MMA issuer: the whole warp runs the loop, one elected lane issues
+//   MMA warp        the whole warp runs the loop, one elected lane issues
 //
 // The per-row statistics come from the workspace the preprocess kernel fills, negated (they are
 // added): lse2 = lse * log2(e) (+inf on padding rows) and delta = rowsum(dO o O) (0 on padding rows),
 // both padded to a multiple of 128 rows per (batch, head); a tile's 2 x 128 values come in with Q_i.
 //
-// What bounds it: per query tile 2560 clk of MMA at D = 128, in a period of about 4000, beside which
-// the roles compete for shared memory (MMA operands, dQ staging, statistics) and for the
-// instruction cache.  The latter decides more than it seems: the same kernel with its MMA loops and
-// write-outs unrolled fetched 1.7 times the instructions from behind the first-level cache
-// and ran 5-18 % SLOWER than one CTA per item did, rolled up it is 5-10 % faster.  Hence the loops below.
-// They settle it: 0.56 stalled cycles per issue for want of instructions, as with one CTA per item (0.57; 1.04 as long
-// as the deterministic turns and P o D in registers were in the loops; Z8 H32 N2048 D128 causal).
-// One CTA per item spent about 7 us of its life on its head and tail (a causal item at N = 2048 has
-// 8.5 tiles of 2.2 us).  Whole backward, one CTA per item -> this, steady state: Z8 H32 N2048 D128
-// causal 1025 -> 955 us, without a mask 1665 -> 1570, Z64 H16 N512 D64 422 -> 385, Z1 H16 N16384
-// causal 2870 -> 2740.  Where a period goes at D = 128 (bf16, clk): the compute warps take 1800 for P^T, 1250 for
-// dS^T and 900 for four waits and the loop; the MMA warp issues for 2600 and waits for them.  Shorter periods
-// (sixteen compute warps: -10 %) did not shorten the time, the clock fell instead: the power cap.
+// What bounds it at D = 128: the SM's port towards L2, and the power cap.  Per query tile there are 2560 clk of MMA
+// and 64 KB of fp32 reduce-adds, which take 3000 clk through the port (about 20 bytes/clk; l1tex__m_l1tex2xbar_req is
+// active 77 % of the time at Z4 H32 N2048 without a mask, the tensor pipe 60 %), in a period of 3700 to 3900.  At D = 64
+// (port 43 %, tensor pipe 31 %) it is a chain: P^T, wait, dS^T, wait.  The end of an item costs extra, 4000 clk of loads that come
+// in late and 64 KB of dK and dV through the same port.  What was measured about that end (whole backward, us,
+// first S^T of the next item ahead of the last dQ and dK, dK and dV written by the compute groups behind its P^T -> as
+// it is now: S^T behind them, written by the dQ group; no prefetch towards L2, which shares the TMA unit): Z64 H16 N512
+// D64 bf16 356 -> 331, Z4 H16 N1024 D64 causal 53.6 -> 49.3, Z2 H16 N8192 D64 causal 914 -> 860; Z8 H32 N2048 D128 causal
+// 978 -> 940, without a mask, bf16 1545 -> 1500, D96 causal 838 -> 805; a padded batch of it 251 -> 242.  Sixteen compute warps
+// of 32 columns at D = 64 instead of eight of 64: Z2 H16 N8192 causal 909 -> 888, Z64 H16 N512 345 -> 342.
+// The instruction cache decides more than it seems: with MMA loops and
+// write-outs unrolled the same kernel fetched 1.7 times the instructions from behind the first-level cache
+// and ran 5-18 % SLOWER than one CTA per item, rolled up 5-10 % faster (0.56 stalled cycles per issue for want of
+// instructions).  Hence the loops below.  At D = 128 shorter periods alone
+// (sixteen compute warps there, too: -10 %) do not shorten the time, the clock falls instead: the power cap.
 #pragma once
 #include <cuda.h>
 #include <math_constants.h>
@@ -87,12 +88,6 @@ struct BwdKernelParams {
   int timeline_block;
 };
 
-constexpr int kBwdRegsIssue = 80;     // warps 12-15
-constexpr int kBwdRegsCompute = 128;  // warps 0-7
-constexpr int kBwdRegsDq = 128 + (128 - kBwdRegsIssue) + 2 * (128 - kBwdRegsCompute);  // warps 8-11
-static_assert(kBwdRegsIssue <= 128 && kBwdRegsCompute <= 128 && kBwdRegsDq >= 128,
-              "setmaxnreg.dec must not raise and .inc must not lower the 128 registers of the launch");
-
 template <int D, bool kBf16 = false, int DR = D>
 struct BwdTraits {
   static constexpr int kBlock = 128;
@@ -104,7 +99,8 @@ struct BwdTraits {
   // the slots behind them take the query tiles in turn.  Where there is room for four (D = 64), a query tile's
   // load need not wait for dK of the tile two before: behind the reduce-adds of dQ, which go through the
   // same unit, it came too late for its S^T.  Whole backward, us, two slots / four: Z64 H16 N512 no mask, bf16
-  // 379 / 353, Z4 H16 N1024 causal 55.6 / 53.4, Z2 H16 N8192 no mask, bf16 1680 / 1601.
+  // 379 / 353, Z4 H16 N1024 causal 55.6 / 53.4, Z2 H16 N8192 no mask, bf16 1680 / 1601.  (Room is left at D = 64 for a
+  // second K and a second dO: Z64 H16 N512 no mask, bf16 334 -> 327, but Z2 H16 N8192 causal 875 -> 922.)
   static constexpr int kQSlots = D == 64 ? 4 : 2;
   static constexpr int kSlots = 3 + kQSlots;
   static constexpr int kStageBytes = 2 * 16384;          // dQ staging: 2 x (128 rows x 32 fp32)
@@ -112,11 +108,22 @@ struct BwdTraits {
   static constexpr int kDeltaBytes = kBf16 ? 512 : 256;
   static constexpr int kStatBytes = 512 + kDeltaBytes;
   static constexpr int kItemStages = 4;                  // item ids published ahead
-  static constexpr int kThreads = 512;  // 4 warpgroups; warps 14, 15 only take part in barriers
+
+  // Warps: compute groups of four, the dQ group, {producer, MMA issuer, two that only take part in barriers}.
+  static constexpr int kGroups = D == 64 ? 4 : 2;   // compute groups
+  static constexpr int kCols = 128 / kGroups;       // query columns each owns
+  static constexpr int kComputeWarps = 4 * kGroups;
+  static constexpr int kProducerWarp = kComputeWarps + 4, kMmaWarp = kProducerWarp + 1;
+  static constexpr int kThreads = 32 * (kComputeWarps + 8);
+  // Registers per thread: of the launch, and after setmaxnreg
+  static constexpr int kRegs = D == 64 ? 80 : 128;
+  static constexpr int kRegsIssue = 80, kRegsCompute = D == 64 ? 72 : 128;
+  static constexpr int kRegsDq = kRegs + (kRegs - kRegsIssue) + kGroups * (kRegs - kRegsCompute);
+  static_assert(kThreads * kRegs <= 65536 && kRegsIssue <= kRegs && kRegsCompute <= kRegs && kRegsDq >= kRegs &&
+                    kRegsIssue % 8 == 0 && kRegsCompute % 8 == 0 && kRegsDq % 8 == 0,
+                "setmaxnreg.dec must not raise and .inc must not lower the registers of the launch");
   static constexpr int kTmemCols = 512;
   static constexpr int kColS = 0, kColDP = 128, kColDQ = 128, kColDK = 256, kColDV = 256 + D;
-  // warps that read dK (and as many dV) out of tensor memory at the end of an item
-  static constexpr int kDrainWarps = (D == 128) ? 8 : 4;
   static constexpr uint32_t kIdescST = umma_idesc_f16(128, 128, 0, 0, kBf16);  // S^T, dP^T
   static constexpr uint32_t kIdescDV = umma_idesc_f16(128, DR, 0, 1, kBf16);   // dV, dK
   static constexpr uint32_t kIdescDQ = umma_idesc_f16(128, DR, 1, 1, kBf16);   // dQ
@@ -211,7 +218,7 @@ __device__ __forceinline__ int bwd_turn(const BwdKernelParams& p, const BwdItem&
 // kDet: deterministic dQ, with the items dealt out.  An instantiation of its own: the turns cost the other mode
 // 1 to 3 % when they were a branch in the dQ group's loop.
 template <int D, bool kBf16 = false, int DR = D, bool kDet = false>
-__global__ void __launch_bounds__(512, 1)
+__global__ void __launch_bounds__(BwdTraits<D, kBf16, DR>::kThreads, 1)
     fmha_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                     const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
                     const __grid_constant__ CUtensorMap tm_dk, const __grid_constant__ CUtensorMap tm_dv,
@@ -257,12 +264,12 @@ __global__ void __launch_bounds__(512, 1)
 
   // The producer warp sets the barriers up itself and sends the first tiles of its first item off at
   // once, before the CTA-wide barrier below that waits for the tensor-memory allocation.
-  if (warp == 12) {
+  if (warp == T::kProducerWarp) {
     if (lane == 0) {
       mbar_init(smem_u32(&sh.bar_clc), 1);
       for (int s = 0; s < T::kItemStages; ++s) {
         mbar_init(smem_u32(&sh.bar_item_full[s]), 1);
-        mbar_init(smem_u32(&sh.bar_item_empty[s]), 13);  // MMA warp, four dQ warps, eight compute warps
+        mbar_init(smem_u32(&sh.bar_item_empty[s]), 5 + T::kComputeWarps);  // MMA warp, four dQ warps
       }
       for (int s = 0; s < T::kSlots; ++s) {
         mbar_init(smem_u32(&sh.bar_full[s]), 1);
@@ -270,13 +277,13 @@ __global__ void __launch_bounds__(512, 1)
       }
       mbar_init(smem_u32(&sh.bar_s_full), 1);
       mbar_init(smem_u32(&sh.bar_dp_full), 1);
-      mbar_init(smem_u32(&sh.bar_p_ready), 8);  // one arrival per warp
-      mbar_init(smem_u32(&sh.bar_ds_ready), 8);
+      mbar_init(smem_u32(&sh.bar_p_ready), T::kComputeWarps);  // one arrival per warp
+      mbar_init(smem_u32(&sh.bar_ds_ready), T::kComputeWarps);
       mbar_init(smem_u32(&sh.bar_dq_full), 1);
       mbar_init(smem_u32(&sh.bar_dq_empty), 4);
       mbar_init(smem_u32(&sh.bar_acc_full), 1);
-      mbar_init(smem_u32(&sh.bar_dv_read), T::kDrainWarps);
-      mbar_init(smem_u32(&sh.bar_dk_read), T::kDrainWarps);
+      mbar_init(smem_u32(&sh.bar_dv_read), 4);
+      mbar_init(smem_u32(&sh.bar_dk_read), 4);
       fence_barrier_init();
     }
     __syncwarp();
@@ -289,7 +296,7 @@ __global__ void __launch_bounds__(512, 1)
       send(2, &tm_do, it, row0, false);
     }
   }
-  if (warp == 13) {
+  if (warp == T::kMmaWarp) {
     tmem_alloc(smem_u32(&sh.tmem_base), T::kTmemCols);
     tmem_relinquish();
   }
@@ -318,17 +325,16 @@ __global__ void __launch_bounds__(512, 1)
     return it;
   };
 
-  // Register budget: 512 threads leave 128 per thread.  The producer / MMA warpgroup and the
+  // Register budget: the producer / MMA warpgroup and, at D = 64, the
   // compute warpgroups hand part of their share to the dQ warpgroup, which must hold a whole
-  // 128-column dQ row per thread to drain tensor memory in one go (the next dP^T waits for
+  // dQ row per thread to drain tensor memory in one go (the next dP^T waits for
   // those columns).  Each setmaxnreg sits at the top of its warpgroup's own branch: the
   // compiler budgets registers per region only when the instruction dominates the region.
-  if (warp >= 12) {
-    reg_dealloc<kBwdRegsIssue>();
+  if (warp >= T::kProducerWarp) {
+    reg_dealloc<T::kRegsIssue>();
     // Slots of the running item's K, V and dO.  At the end of an item they fall free in the order
     // V (after the last dP^T), dO (after the last dV), K (after the last dQ), and the next item
-    // needs K first, V and dO a while later: it takes them over in that order, so that its first
-    // S^T is issued like any other query tile's.
+    // needs K first, V and dO a while later: it takes them over in that order.
     int slot_k = 0, slot_v = 1, slot_do = 2;
     auto next_slots = [&]() {
       const int k = slot_k;
@@ -336,7 +342,7 @@ __global__ void __launch_bounds__(512, 1)
       slot_v = slot_do;
       slot_do = k;
     };
-    if (warp == 12) {
+    if (warp == T::kProducerWarp) {
       // =========================== TMA producer, item source ===========================
       bool ok = true;
       uint32_t published = 0, asked = 0;
@@ -418,6 +424,10 @@ __global__ void __launch_bounds__(512, 1)
         used ^= 1u << slot;
       };
       uint32_t g = 0;  // query tiles so far, over all items
+      // The answer to a request takes a microsecond, so it is asked for ahead of the item's last loads: two tiles ahead at
+      // D = 128; where there are four slots for the query tiles the loads run ahead as it is, and asking later balances
+      // better (Z4 H16 N1024 D64 causal 51.2 two ahead, 49.9 us one).
+      constexpr int kAskAhead = T::kQSlots > 2 ? 1 : 2;
       while (ok) {
         const BwdItem it = next_item();
         if (it.id < 0) break;
@@ -427,16 +437,6 @@ __global__ void __launch_bounds__(512, 1)
           first = false;
         } else {
           if (published > 1) next_slots();
-          // cold from HBM these take microseconds: start towards L2 before waiting for the slots
-          if (elect_one()) {
-#pragma unroll
-            for (int b = 0; b < T::kBoxes; ++b) {
-              tma_prefetch_l2_4d(&tm_k, b * 64, kv0, it.h, it.z);
-              tma_prefetch_l2_4d(&tm_v, b * 64, kv0, it.h, it.z);
-              tma_prefetch_l2_4d(&tm_do, b * 64, row0, it.h, it.z);
-            }
-          }
-          __syncwarp();
           // in the order in which the slots fall free
           load(3 + g % T::kQSlots, &tm_q, it, row0, true);
           load(slot_k, &tm_k, it, kv0, false);
@@ -444,16 +444,16 @@ __global__ void __launch_bounds__(512, 1)
           load(slot_do, &tm_do, it, row0, false);
         }
         ++g;
-        if (it.cnt == 1) ask();
+        if (it.cnt <= kAskAhead) ask();
 #pragma unroll 1
         for (int n = 1; ok && n < it.cnt; ++n, ++g) {
           const int row = (it.i_begin + n) * T::kBlock;
-          if (n == it.cnt - 1) ask();  // the answer takes a microsecond
+          if (n >= it.cnt - kAskAhead) ask();
           load(3 + g % T::kQSlots, &tm_q, it, row, true);
           load(slot_do, &tm_do, it, row, false);
         }
       }
-    } else if (warp == 13) {
+    } else if (warp == T::kMmaWarp) {
       // =========================== MMA issuer (converged warp) ===========================
       // D (+)= A B with A and B in shared memory, the contraction in blocks of 64.  Loops, not straight
       // code: what the roles of the CTA execute has to fit the instruction cache together.
@@ -499,89 +499,75 @@ __global__ void __launch_bounds__(512, 1)
       const uint32_t ds_lo_k = umma_desc_lo(ds_smem, kLboKMajor);    // dS^T as K-major A (dK)
       const uint32_t ds_lo_mn = umma_desc_lo(ds_smem, kLboMnMajor);  // dS^T read as MN-major A (dQ)
 
-      BwdItem cur = take_item();
-      bool ok = cur.id >= 0;
-      ok = ok && wait_full(slot_k, 3) && wait_full(3, 4);
-      if (ok) {
+      uint32_t g = 0;  // query tiles so far, over all items
+      bool ok = true;
+#pragma unroll 1
+      for (uint32_t item_no = 0; ok; ++item_no) {
+        // S^T of the item's first query tile.  It comes behind dQ and dK of the item before: K and Q come late more often
+        // than not, and what is left of the item before would wait for them.
+        const BwdItem cur = take_item();
+        if (cur.id < 0) break;
+        if (item_no > 0) next_slots();
+        if (!wait_full(slot_k, 3) || !wait_full(3 + g % T::kQSlots, 4)) break;
         tc_fence_after();
-        issue_kmajor(T::kColS, slot_addr(slot_k), slot_addr(3));
+        issue_kmajor(T::kColS, slot_addr(slot_k), slot_addr(3 + g % T::kQSlots));
         umma_commit_elect(smem_u32(&sh.bar_s_full));
-      }
-      ok = ok && wait_full(slot_v, 5) && wait_full(slot_do, 5);
-      if (ok) {
-        tc_fence_after();
-        issue_kmajor(T::kColDP, slot_addr(slot_v), slot_addr(slot_do));
-        umma_commit_elect(smem_u32(&sh.bar_dp_full));
-        if (cur.cnt == 1) umma_commit_elect(smem_u32(&sh.bar_empty[slot_v]));
-      }
-      uint32_t item_no = 0;
-      int n = 0;  // query tile of the item
 #pragma unroll 1
-      for (uint32_t g = 0; ok; ++g) {  // one pass per query tile, from one item into the next
-        const bool last = n == cur.cnt - 1;
-        const uint32_t q_addr = slot_addr(3 + g % T::kQSlots);
-        // ---- dV += P^T dO_i; the first one overwrites the last item's dV
-        FMHA_TL(2, g, 0);
-        if (n == 0 && item_no > 0 && !mbar_wait_warp(smem_u32(&sh.bar_dv_read), (item_no - 1) & 1, abort_word, 19)) break;
-        if (!mbar_wait_warp(smem_u32(&sh.bar_p_ready), g & 1, abort_word, 6)) break;
-        tc_fence_after();
-        FMHA_TL(2, g, 1);
-        const uint32_t do_lo_mn = umma_desc_lo(slot_addr(slot_do), kLboMnMajor);  // dO as MN-major B
+        for (int n = 0; ok && n < cur.cnt; ++n, ++g) {
+          const bool last = n == cur.cnt - 1;
+          // ---- dP^T of this query tile (its columns hold dQ of the one before until the dQ group read it)
+          FMHA_TL(2, g, 0);
+          ok = (n > 0 || wait_full(slot_v, 5)) && wait_full(slot_do, 9) &&
+               (g == 0 || mbar_wait_warp(smem_u32(&sh.bar_dq_empty), (g - 1) & 1, abort_word, 10));
+          if (!ok) break;
+          tc_fence_after();
+          FMHA_TL(2, g, 1);
+          issue_kmajor(T::kColDP, slot_addr(slot_v), slot_addr(slot_do));
+          umma_commit_elect(smem_u32(&sh.bar_dp_full));
+          if (last) umma_commit_elect(smem_u32(&sh.bar_empty[slot_v]));
+          // ---- dV += P^T dO_i; the first one overwrites the last item's dV
+          FMHA_TL(2, g, 2);
+          ok = (n > 0 || item_no == 0 ||
+                mbar_wait_warp(smem_u32(&sh.bar_dv_read), (item_no - 1) & 1, abort_word, 19)) &&
+               mbar_wait_warp(smem_u32(&sh.bar_p_ready), g & 1, abort_word, 6);
+          if (!ok) break;
+          tc_fence_after();
+          FMHA_TL(2, g, 3);
+          const uint32_t do_lo_mn = umma_desc_lo(slot_addr(slot_do), kLboMnMajor);  // dO as MN-major B
 #pragma unroll 1
-        for (int b = 0; b < 2; ++b)
+          for (int b = 0; b < 2; ++b)
 #pragma unroll
-          for (int i = 0; i < 4; ++i)
-            umma_ts_elect(tmem_base + T::kColDV, tmem_base + T::kColS + b * 64 + i * 8,
-                          do_lo_mn + b * kBlockMn + i * kStepMn, T::kIdescDV, (n > 0 || b > 0 || i > 0) ? 1u : 0u);
-        umma_commit_elect(smem_u32(&sh.bar_empty[slot_do]));
-        // ---- S^T of the next query tile (the S region is free once dV has read P^T), which may be
-        // the first one of the next item
-        BwdItem nxt = cur;
-        if (last) nxt = take_item();
-        if (nxt.id >= 0) {
-          if (last && !wait_full(slot_v, 3)) break;  // the next K is where V was
-          if (!wait_full(3 + (g + 1) % T::kQSlots, 7)) break;
+            for (int i = 0; i < 4; ++i)
+              umma_ts_elect(tmem_base + T::kColDV,
+                            tmem_base + T::kColS + b * 64 + (T::kGroups == 2 ? i * 8 : (i >> 1) * 32 + (i & 1) * 8),
+                            do_lo_mn + b * kBlockMn + i * kStepMn, T::kIdescDV, (n > 0 || b > 0 || i > 0) ? 1u : 0u);
+          umma_commit_elect(smem_u32(&sh.bar_empty[slot_do]));
+          // ---- S^T of the item's next query tile (the S region is free once dV has read P^T)
+          if (!last) {
+            if (!(ok = wait_full(3 + (g + 1) % T::kQSlots, 7))) break;
+            tc_fence_after();
+            issue_kmajor(T::kColS, slot_addr(slot_k), slot_addr(3 + (g + 1) % T::kQSlots));
+            umma_commit_elect(smem_u32(&sh.bar_s_full));
+          }
+          // ---- dQ_i = dS K first (its read-out is on the critical path), then dK += dS^T Q_i
+          FMHA_TL(2, g, 4);
+          if (!(ok = mbar_wait_warp(smem_u32(&sh.bar_ds_ready), g & 1, abort_word, 8))) break;
           tc_fence_after();
-          issue_kmajor(T::kColS, slot_addr(last ? slot_v : slot_k), slot_addr(3 + (g + 1) % T::kQSlots));
-          umma_commit_elect(smem_u32(&sh.bar_s_full));
+          FMHA_TL(2, g, 5);
+          const uint32_t k_lo_mn = umma_desc_lo(slot_addr(slot_k), kLboMnMajor);  // K as MN-major B
+          issue_ss(2, T::kColDQ, ds_lo_mn, kBlockMn, kStepMn, k_lo_mn, kBlockMn, kStepMn, T::kIdescDQ, 0u);
+          umma_commit_elect(smem_u32(&sh.bar_dq_full));
+          if (last) umma_commit_elect(smem_u32(&sh.bar_empty[slot_k]));
+          if (n == 0 && item_no > 0) {
+            if (!(ok = mbar_wait_warp(smem_u32(&sh.bar_dk_read), (item_no - 1) & 1, abort_word, 20))) break;
+            tc_fence_after();
+          }
+          const uint32_t q_lo_mn = umma_desc_lo(slot_addr(3 + g % T::kQSlots), kLboMnMajor);
+          issue_ss(2, T::kColDK, ds_lo_k, kBlockK, kStepK, q_lo_mn, kBlockMn, kStepMn, T::kIdescDV, n > 0 ? 1u : 0u);
+          umma_commit_elect(smem_u32(&sh.bar_empty[3 + g % T::kQSlots]));  // Q_i, and dS^T, have been read
+          if (last) umma_commit_elect(smem_u32(&sh.bar_acc_full));
+          FMHA_TL(2, g, 6);
         }
-        // ---- dQ_i = dS K first (its read-out is on the critical path), then dK += dS^T Q_i
-        FMHA_TL(2, g, 2);
-        if (!mbar_wait_warp(smem_u32(&sh.bar_ds_ready), g & 1, abort_word, 8)) break;
-        tc_fence_after();
-        FMHA_TL(2, g, 3);
-        const uint32_t k_lo_mn = umma_desc_lo(slot_addr(slot_k), kLboMnMajor);  // K as MN-major B
-        issue_ss(2, T::kColDQ, ds_lo_mn, kBlockMn, kStepMn, k_lo_mn, kBlockMn, kStepMn, T::kIdescDQ, 0u);
-        umma_commit_elect(smem_u32(&sh.bar_dq_full));
-        if (last) umma_commit_elect(smem_u32(&sh.bar_empty[slot_k]));
-        if (n == 0 && item_no > 0) {
-          if (!mbar_wait_warp(smem_u32(&sh.bar_dk_read), (item_no - 1) & 1, abort_word, 20)) break;
-          tc_fence_after();
-        }
-        const uint32_t q_lo_mn = umma_desc_lo(q_addr, kLboMnMajor);
-        issue_ss(2, T::kColDK, ds_lo_k, kBlockK, kStepK, q_lo_mn, kBlockMn, kStepMn, T::kIdescDV, n > 0 ? 1u : 0u);
-        umma_commit_elect(smem_u32(&sh.bar_empty[3 + g % T::kQSlots]));  // Q_i, and dS^T, have been read
-        if (last) umma_commit_elect(smem_u32(&sh.bar_acc_full));
-        FMHA_TL(2, g, 4);
-        if (nxt.id < 0) break;
-        // ---- dP^T of the next query tile (its columns hold dQ_i until the dQ group read it)
-        if (last) {
-          next_slots();
-          cur = nxt;
-          ++item_no;
-          n = 0;
-          if (!wait_full(slot_v, 5)) break;
-        } else {
-          ++n;
-        }
-        if (!wait_full(slot_do, 9)) break;
-        if (!mbar_wait_warp(smem_u32(&sh.bar_dq_empty), g & 1, abort_word, 10)) break;
-        tc_fence_after();
-        FMHA_TL(2, g, 5);
-        issue_kmajor(T::kColDP, slot_addr(slot_v), slot_addr(slot_do));
-        umma_commit_elect(smem_u32(&sh.bar_dp_full));
-        if (n == cur.cnt - 1) umma_commit_elect(smem_u32(&sh.bar_empty[slot_v]));
-        FMHA_TL(2, g, 6);
       }
     }
   } else {
@@ -589,101 +575,22 @@ __global__ void __launch_bounds__(512, 1)
     const int r = quad * 32 + lane;  // TMEM lane of this thread
     const uint32_t lane_addr = uint32_t(quad * 32) << 16;
 
-    if (warp < 8) {
+    if (warp < T::kComputeWarps) {
       // =========================== compute groups: P^T, dS^T; dK, dV out ===================
-      reg_dealloc<kBwdRegsCompute>();
-      const int cg = warp >> 2;           // query-column half of this group
+      reg_dealloc<T::kRegsCompute>();
+      const int cg = warp >> 2;           // query columns [cg * kCols, (cg + 1) * kCols) are this group's
       const uint64_t c2 = pack2f(p.scale_log2, p.scale_log2);
-      const uint32_t tS = tmem_base + lane_addr + T::kColS + cg * 64;
-      // P^T (32 packed columns) goes over the start of this group's own S^T half, which only
-      // this group reads: no ordering between the two groups is needed
+      const uint32_t tS = tmem_base + lane_addr + T::kColS + cg * T::kCols;
+      // P^T (packed columns) goes over the start of this group's own part of S^T, which only
+      // this group reads: no ordering between the groups is needed
       const uint32_t tP = tS;
-      const uint32_t tDP = tmem_base + lane_addr + T::kColDP + cg * 64;
-      // this thread's 128-byte row of dS^T; a warp's 32 rows (4 KB) are also its own staging area for
-      // dK and dV
-      const uint32_t row_addr = ds_smem + cg * T::kBoxBytes + r * 128;
+      const uint32_t tDP = tmem_base + lane_addr + T::kColDP + cg * T::kCols;
+      // this thread's 128-byte row of dS^T; where the compute groups write dK and dV out, a warp's 32 rows (4 KB) are
+      // also its own staging area for them
+      const uint32_t row_addr = ds_smem + (cg * T::kCols / 64) * T::kBoxBytes + r * 128;
+      const int chunk0 = (cg * T::kCols % 64) / 8;  // this group's first 16-byte chunk of it
       const bool tl = (threadIdx.x == 0);
-      uint32_t g = 0, drained = 0;
-
-      // dK (is_dk) or dV columns [col0, col0 + 64) of an item: tensor memory -> 16-bit, staging, TMA
-      // store; or (ring attention) into an fp32 buffer, added to what is there or, with
-      // accum_overwrite, in its place
-      auto drain_half = [&](bool is_dk, const BwdItem& it, int col0, bool restage) {
-        const uint32_t tAcc = tmem_base + lane_addr + (is_dk ? T::kColDK : T::kColDV) + col0;
-        const float mul = is_dk ? p.scale : 1.f;
-        float* accum = is_dk ? p.dk_accum : p.dv_accum;
-        const uint32_t read_bar = smem_u32(is_dk ? &sh.bar_dk_read : &sh.bar_dv_read);
-        if (accum != nullptr) {
-          const int kvi = it.kb * T::kBlock + r;
-          const bool have = kvi < it.sk;  // this thread's row has a result
-          const bool touch = kvi < p.seqlen_k && (have || p.accum_overwrite != 0);
-          float* dst = accum + (size_t)it.z * p.accum_batch_stride + ((size_t)kvi * p.heads + it.h) * DR + col0;
-#pragma unroll 1
-          for (int cc = 0; cc < 4; ++cc) {
-            uint32_t a[16];
-            tmem_ld16(tAcc + cc * 16, a);
-            tmem_wait_ld();
-            if (touch && col0 + cc * 16 < DR) {
-#pragma unroll
-              for (int i = 0; i < 16; i += 4) {
-                float4 cur = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (p.accum_overwrite == 0) cur = *reinterpret_cast<float4*>(dst + cc * 16 + i);
-                if (have) {
-                  cur.x += __uint_as_float(a[i + 0]) * mul;
-                  cur.y += __uint_as_float(a[i + 1]) * mul;
-                  cur.z += __uint_as_float(a[i + 2]) * mul;
-                  cur.w += __uint_as_float(a[i + 3]) * mul;
-                }
-                *reinterpret_cast<float4*>(dst + cc * 16 + i) = cur;
-              }
-            }
-          }
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(read_bar);
-          return;
-        }
-        uint32_t w[32];
-#pragma unroll
-        for (int cc = 0; cc < 2; ++cc) {
-          uint32_t a[32];
-          tmem_ld32(tAcc + cc * 32, a);
-          tmem_wait_ld();
-#pragma unroll
-          for (int i = 0; i < 16; ++i)
-            w[cc * 16 + i] =
-                pack16x2<kBf16>(__uint_as_float(a[2 * i]) * mul, __uint_as_float(a[2 * i + 1]) * mul);
-        }
-        tc_fence_before();
-        if (restage && lane == 0) tma_wait_group_read<0>();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(read_bar);
-#pragma unroll
-        for (int ch = 0; ch < 8; ++ch)
-          sts128(row_addr + ((ch ^ (r & 7)) << 4), w[4 * ch], w[4 * ch + 1], w[4 * ch + 2], w[4 * ch + 3]);
-        fence_proxy_async_smem();
-        __syncwarp();
-        const int row = it.kb * T::kBlock + quad * 32;
-        if (lane == 0 && row < p.seqlen_k) {
-          tma_store_4d(is_dk ? &tm_dk : &tm_dv, row_addr, col0, row, it.h, it.z);
-          tma_commit_group();
-        }
-      };
-      // dK and dV of an item whose MMAs have all been issued
-      auto drain = [&](const BwdItem& it) {
-        mbar_wait(smem_u32(&sh.bar_acc_full), drained & 1, abort_word, 15);
-        ++drained;
-        tc_fence_after();
-        // dV, then dK (D = 64: one group each)
-#pragma unroll 1
-        for (int i = 0; i < T::kBoxes; ++i)
-          drain_half(D == 128 ? i == 1 : cg == 1, it, D == 128 ? cg * 64 : 0, i > 0);
-      };
-      // An item's dK and dV are written out behind the first P^T of the next item: they are complete
-      // by then, and the group would wait for the next item's first dP^T (whose V and dO tiles come
-      // in last) anyway.
-      bool pending = false;
-      BwdItem done;
+      uint32_t g = 0;
       for (;;) {
         const BwdItem it = take_item();
         if (it.id < 0) break;
@@ -701,9 +608,9 @@ __global__ void __launch_bounds__(512, 1)
             const long long fv = (long long)kvi - p.causal_shift - qbase;
             first_visible = fv <= 0 ? 0 : (int)min(fv, (long long)T::kBlock);
           }
-          const int fvh = first_visible - cg * 64;
+          const int fvh = first_visible - cg * T::kCols;
 
-          uint32_t pp[32];  // P^T of this row and half, 16-bit pairs
+          uint32_t pp[T::kCols / 2];  // P^T of this row and group, 16-bit pairs
           if (tl) FMHA_TL(0, g, 0);
           // on a time-out: keep going, every later wait returns at once
           mbar_wait(smem_u32(&sh.bar_full[3 + g % T::kQSlots]), g / T::kQSlots & 1, abort_word, 21);  // the statistics
@@ -711,15 +618,15 @@ __global__ void __launch_bounds__(512, 1)
           tc_fence_after();
           if (tl) FMHA_TL(0, g, 1);
           {
-            uint32_t s[2][32];
-            tmem_ld32(tS, s[0]);
-            tmem_ld32(tS + 32, s[1]);
+            uint32_t s[T::kCols / 32][32];
+#pragma unroll
+            for (int cc = 0; cc < T::kCols / 32; ++cc) tmem_ld32(tS + cc * 32, s[cc]);
             tmem_wait_ld();
 #pragma unroll
-            for (int cc = 0; cc < 2; ++cc)
+            for (int cc = 0; cc < T::kCols / 32; ++cc)
 #pragma unroll
               for (int i = 0; i < 32; i += 4) {
-                const float4 nl = lds128(sb + (cg * 64 + cc * 32 + i) * 4);
+                const float4 nl = lds128(sb + (cg * T::kCols + cc * 32 + i) * 4);
                 uint32_t x[4];
                 unpack2(fma2(pack2(s[cc][i + 0], s[cc][i + 1]), c2, pack2f(nl.x, nl.y)), x[0], x[1]);
                 unpack2(fma2(pack2(s[cc][i + 2], s[cc][i + 3]), c2, pack2f(nl.z, nl.w)), x[2], x[3]);
@@ -732,44 +639,37 @@ __global__ void __launch_bounds__(512, 1)
               }
             if (fvh > 0) {
 #pragma unroll
-              for (int j = 0; j < 32; ++j) {  // pair j = columns 2j, 2j+1 of this half
+              for (int j = 0; j < T::kCols / 2; ++j) {  // pair j = columns 2j, 2j+1 of this group's
                 if (2 * j + 1 < fvh) pp[j] = 0u;
                 else if (2 * j < fvh) pp[j] &= 0xffff0000u;
               }
             }
           }
-          tmem_st32(tP, pp);
+          if constexpr (T::kCols == 64) tmem_st32(tP, pp);
+          else tmem_st16(tP, pp);
           tmem_wait_st();
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(smem_u32(&sh.bar_p_ready));
           if (tl) FMHA_TL(0, g, 2);
-          if (pending) {
-            drain(done);
-            pending = false;
-          }
           mbar_wait(smem_u32(&sh.bar_dp_full), g & 1, abort_word, 12);
           if (tl) FMHA_TL(0, g, 3);
           // dS^T of the previous tile has been read: its dQ and dK MMAs were issued before this dP^T, and the
-          // commit that told of it covers them.  dK / dV must have left the staging area.
-          if (n == 0) {
-            if (lane == 0) tma_wait_group_read<0>();
-            __syncwarp();
-          }
+          // commit that told of it covers them.
           tc_fence_after();
           if (tl) FMHA_TL(0, g, 4);
           {
-            uint32_t dp[2][32];
-            tmem_ld32(tDP, dp[0]);
-            tmem_ld32(tDP + 32, dp[1]);
+            uint32_t dp[T::kCols / 32][32];
+#pragma unroll
+            for (int cc = 0; cc < T::kCols / 32; ++cc) tmem_ld32(tDP + cc * 32, dp[cc]);
             tmem_wait_ld();
 #pragma unroll
-            for (int cc = 0; cc < 2; ++cc)
+            for (int cc = 0; cc < T::kCols / 32; ++cc)
 #pragma unroll
               for (int k8 = 0; k8 < 4; ++k8) {  // 8 columns = one 16-byte chunk
                 uint32_t w[4];
                 // -delta of this chunk's 8 query columns: fp16 pairs, with bf16 (8 mantissa bits) pairs of fp32
-                const uint32_t at = sb + 512 + (cg * 64 + cc * 32 + k8 * 8) * (kBf16 ? 4 : 2);
+                const uint32_t at = sb + 512 + (cg * T::kCols + cc * 32 + k8 * 8) * (kBf16 ? 4 : 2);
                 const float4 a = lds128(at), b = kBf16 ? lds128(at + 16) : a;
                 [[maybe_unused]] const uint64_t nd[4] = {pack2f(a.x, a.y), pack2f(a.z, a.w), pack2f(b.x, b.y),
                                                          pack2f(b.z, b.w)};
@@ -792,7 +692,7 @@ __global__ void __launch_bounds__(512, 1)
                                       mul_half2(pp[j], nd16[q2]));
                   }
                 }
-                const int ch = cc * 4 + k8;  // chunk of this thread's 128-byte row
+                const int ch = chunk0 + cc * 4 + k8;  // chunk of this thread's 128-byte row
                 sts128(row_addr + ((ch ^ (r & 7)) << 4), w[0], w[1], w[2], w[3]);
               }
           }
@@ -802,21 +702,17 @@ __global__ void __launch_bounds__(512, 1)
           if (lane == 0) mbar_arrive(smem_u32(&sh.bar_ds_ready));
           if (tl) FMHA_TL(0, g, 5);
         }
-        pending = true;
-        done = it;
       }
-      if (pending) drain(done);
-      if (lane == 0) tma_wait_group<0>();
     } else {
       // =========================== dQ group ===========================
-      reg_alloc<kBwdRegsDq>();
+      reg_alloc<T::kRegsDq>();
       const uint32_t tDQ = tmem_base + lane_addr + T::kColDQ;
       const bool tl = (r == 0);
       constexpr int kChunks = DR / 32;  // 32-column chunks of a dQ row
       // an odd number of chunks per tile breaks the alternation of the two staging buffers by
       // chunk index: count the chunks staged so far instead
       [[maybe_unused]] uint32_t chunk_no = 0;
-      uint32_t g = 0;
+      uint32_t g = 0, drained = 0;
       for (;;) {
         const BwdItem it = take_item();
         if (it.id < 0) break;
@@ -884,6 +780,76 @@ __global__ void __launch_bounds__(512, 1)
           }
           if (tl) FMHA_TL(1, g, 3);
         }
+        // dV and dK of the item: tensor memory -> 16 bit -> TMA stores through the staging buffers; or (ring attention)
+        // into an fp32 buffer, added to what is there or, with accum_overwrite, in its place.  (This group does it
+        // because it has time to until the next item's first dQ.  Written by the compute groups they hold up the next
+        // item's P^T and dS^T: the SM's port towards L2, at 20 bytes/clk, has the last dQ to send, too.)
+        mbar_wait(smem_u32(&sh.bar_acc_full), drained & 1, abort_word, 15);
+        ++drained;
+        tc_fence_after();
+#pragma unroll 1
+        for (int i = 0; i < 2; ++i) {
+          const bool is_dk = i == 1;
+          const uint32_t tAcc = tmem_base + lane_addr + (is_dk ? T::kColDK : T::kColDV);
+          const float mul = is_dk ? p.scale : 1.f;
+          float* accum = is_dk ? p.dk_accum : p.dv_accum;
+          uint32_t acc[kChunks][32];
+#pragma unroll
+          for (int cc = 0; cc < kChunks; ++cc) tmem_ld32(tAcc + cc * 32, acc[cc]);
+          tmem_wait_ld();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(smem_u32(is_dk ? &sh.bar_dk_read : &sh.bar_dv_read));
+          if (accum != nullptr) {
+            const int kvi = it.kb * T::kBlock + r;
+            const bool have = kvi < it.sk;  // this thread's row has a result
+            if (kvi < p.seqlen_k && (have || p.accum_overwrite != 0)) {
+              float* dst = accum + (size_t)it.z * p.accum_batch_stride + ((size_t)kvi * p.heads + it.h) * DR;
+#pragma unroll
+              for (int cc = 0; cc < kChunks; ++cc)
+#pragma unroll
+                for (int k = 0; k < 32; k += 4) {
+                  float4 cur = make_float4(0.f, 0.f, 0.f, 0.f);
+                  if (p.accum_overwrite == 0) cur = *reinterpret_cast<float4*>(dst + cc * 32 + k);
+                  if (have) {
+                    cur.x += __uint_as_float(acc[cc][k + 0]) * mul;
+                    cur.y += __uint_as_float(acc[cc][k + 1]) * mul;
+                    cur.z += __uint_as_float(acc[cc][k + 2]) * mul;
+                    cur.w += __uint_as_float(acc[cc][k + 3]) * mul;
+                  }
+                  *reinterpret_cast<float4*>(dst + cc * 32 + k) = cur;
+                }
+            }
+            continue;
+          }
+#pragma unroll
+          for (int b = 0; b < T::kBoxes; ++b) {  // 64 columns (128 bytes) of each row
+            uint32_t stg_buf;
+            if constexpr (kChunks % 2 == 0) {
+              stg_buf = stg_smem + ((T::kBoxes == 1 ? i : b) & 1) * 16384;
+            } else {
+              stg_buf = stg_smem + (chunk_no & 1u) * 16384;
+              ++chunk_no;
+            }
+            if (r == 0) tma_wait_group_read<1>();
+            named_bar_sync(2, 128);
+#pragma unroll
+            for (int ch = 0; ch < (DR - b * 64 < 64 ? 4 : 8); ++ch) {
+              const uint32_t* a = &acc[b * 2 + ch / 4][ch % 4 * 8];
+              uint32_t w[4];
+#pragma unroll
+              for (int k = 0; k < 4; ++k)
+                w[k] = pack16x2<kBf16>(__uint_as_float(a[2 * k]) * mul, __uint_as_float(a[2 * k + 1]) * mul);
+              sts128(stg_buf + r * 128 + ((ch ^ (r & 7)) << 4), w[0], w[1], w[2], w[3]);
+            }
+            fence_proxy_async_smem();
+            named_bar_sync(2, 128);
+            if (r == 0) {
+              tma_store_4d(is_dk ? &tm_dk : &tm_dv, stg_buf, b * 64, it.kb * T::kBlock, it.h, it.z);
+              tma_commit_group();
+            }
+          }
+        }
       }
       if (r == 0) tma_wait_group<0>();
     }
@@ -897,7 +863,7 @@ __global__ void __launch_bounds__(512, 1)
     // let copies that may still be in flight land before the shared memory is released
     for (int i = 0; i < 64; ++i) __nanosleep(1000);
   }
-  if (warp == 13) {
+  if (warp == T::kMmaWarp) {
     tc_fence_after();
     tmem_dealloc(tmem_base, T::kTmemCols);
   }

@@ -41,10 +41,10 @@ EncodeTiledFn get_encode_fn() {
   return fn;
 }
 
-// 16-bit (Z, N, H, D) tensor with element strides -> 4-D map (D, N, H, Z), box 64 x box_rows x 1
+// 16-bit (Z, N, H, D) tensor with element strides -> 4-D map (D, N, H, Z), box 64 x 128 x 1
 // x 1, 128-byte swizzle, zero fill outside the tensor
 int make_tensor_map(CUtensorMap* map, const void* base, int Z, int N, int H, int D,
-                    const FmhaStrides& s, bool bf16, unsigned box_rows = 128) {
+                    const FmhaStrides& s, bool bf16) {
   EncodeTiledFn encode = get_encode_fn();
   if (encode == nullptr) return FMHA_ERR_NO_DEVICE;
   // a stride of a size-1 dimension is never used for addressing; make it well-formed
@@ -53,7 +53,7 @@ int make_tensor_map(CUtensorMap* map, const void* base, int Z, int N, int H, int
   const int64_t batch = (Z > 1) ? s.batch : row * N;
   const cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)N, (cuuint64_t)H, (cuuint64_t)Z};
   const cuuint64_t strides[3] = {(cuuint64_t)row * 2, (cuuint64_t)head * 2, (cuuint64_t)batch * 2};
-  const cuuint32_t box[4] = {64, box_rows, 1, 1};
+  const cuuint32_t box[4] = {64, 128, 1, 1};
   const cuuint32_t estr[4] = {1, 1, 1, 1};
   const CUresult r = encode(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
                             4, const_cast<void*>(base), dims,
@@ -452,13 +452,11 @@ int launch_bwd(const FmhaBwdParams* p, const BwdWorkspace& w, cudaStream_t strea
     if ((rc = make_tensor_map(&tk, p->k, Z, Nk, H, Dr, p->k_strides, kBf16))) return rc;
     if ((rc = make_tensor_map(&tv, p->v, Z, Nk, H, Dr, p->v_strides, kBf16))) return rc;
     if ((rc = make_tensor_map(&tdo, p->dout, Z, Nq, H, Dr, p->dout_strides, kBf16))) return rc;
-    // with fp32 accumulation the fp16 outputs are not touched: any valid map will do
+    // with fp32 accumulation the 16-bit outputs are not touched: any valid map will do
     const bool acc_k = p->dk_accum != nullptr, acc_v = p->dv_accum != nullptr;
-    if ((rc = make_tensor_map(&tdk, acc_k ? p->k : p->dk, Z, Nk, H, Dr,
-                              acc_k ? p->k_strides : p->dk_strides, kBf16, 32)))
+    if ((rc = make_tensor_map(&tdk, acc_k ? p->k : p->dk, Z, Nk, H, Dr, acc_k ? p->k_strides : p->dk_strides, kBf16)))
       return rc;
-    if ((rc = make_tensor_map(&tdv, acc_v ? p->v : p->dv, Z, Nk, H, Dr,
-                              acc_v ? p->v_strides : p->dv_strides, kBf16, 32)))
+    if ((rc = make_tensor_map(&tdv, acc_v ? p->v : p->dv, Z, Nk, H, Dr, acc_v ? p->v_strides : p->dv_strides, kBf16)))
       return rc;
     fmha::BwdKernelParams kp;
     kp.neg_lse2 = w.lse2;

@@ -77,3 +77,27 @@ def test_runs_of_padding_between_items(D, causal):
     assert int(status.item()) == 0
     ref = _oracle_padded(q, k, v, dout, scale, causal, lens, lens)
     helpers.check_against_oracle((out.cpu(), lse.cpu(), *(t.cpu() for t in grads)), ref, f"padding runs D{D}")
+
+
+@pytest.mark.parametrize("D,dtype", [(64, torch.float16), (96, torch.float16), (96, torch.bfloat16), (128, torch.bfloat16)])
+@pytest.mark.parametrize("wide", ["dk", "dv"])
+def test_one_of_dk_and_dv_in_fp32(D, dtype, wide):
+    """One of them goes through the staging buffers that dQ uses in turn (an odd number of chunks per tile at 96), the
+    other does not; more items than SMs, of one, two and three query tiles, the last rows of a tile missing."""
+    from flash_attn_v100 import cabi
+
+    H, N = 100, 352
+    q, k, v, dout = (t.to(dtype) for t in oracle.make_inputs(1, N, H, D, seed=76))
+    scale = oracle.default_scale(D)
+    ref = oracle.attention_fwd_bwd(q, k, v, dout, scale, True, 0)
+    q, k, v, dout = (t.cuda() for t in (q, k, v, dout))
+    out, lse = cabi.fwd(q, k, v, scale, True)
+    acc = torch.full((1, N, H, D), 3.0, device="cuda")
+    guard = torch.full((1, N + 32, H, D), 7.0, dtype=dtype, device="cuda")
+    kw = {"dk_accum": acc, "dv": guard[:, :N]} if wide == "dk" else {"dv_accum": acc, "dk": guard[:, :N]}
+    dq, _, _ = cabi.bwd(q, k, v, out, dout, lse, scale, True, flags=cabi.FMHA_BWD_ACCUM_OVERWRITE, **kw)
+    tol = _tols(dtype)[1]
+    assert oracle.rel_l2(dq.float().cpu(), ref[2]) <= tol
+    assert oracle.rel_l2(acc.cpu(), ref[3] if wide == "dk" else ref[4]) <= tol
+    assert oracle.rel_l2(guard[:, :N].float().cpu(), ref[4] if wide == "dk" else ref[3]) <= tol
+    assert (guard[:, N:] == 7.0).all()
