@@ -806,19 +806,24 @@ __global__ void __launch_bounds__(BwdTraits<D, kBf16, DR>::kThreads, 1)
             if (kvi < p.seqlen_k && (have || p.accum_overwrite != 0)) {
               float* dst = accum + (size_t)it.z * p.accum_batch_stride + ((size_t)kvi * p.heads + it.h) * DR;
 #pragma unroll
-              for (int cc = 0; cc < kChunks; ++cc)
+              for (int cc = 0; cc < kChunks; ++cc) {
+                float4 cur[8];  // read ahead of the stores
 #pragma unroll
-                for (int k = 0; k < 32; k += 4) {
-                  float4 cur = make_float4(0.f, 0.f, 0.f, 0.f);
-                  if (p.accum_overwrite == 0) cur = *reinterpret_cast<float4*>(dst + cc * 32 + k);
-                  if (have) {
-                    cur.x += __uint_as_float(acc[cc][k + 0]) * mul;
-                    cur.y += __uint_as_float(acc[cc][k + 1]) * mul;
-                    cur.z += __uint_as_float(acc[cc][k + 2]) * mul;
-                    cur.w += __uint_as_float(acc[cc][k + 3]) * mul;
-                  }
-                  *reinterpret_cast<float4*>(dst + cc * 32 + k) = cur;
+                for (int k = 0; k < 8; ++k) {
+                  cur[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+                  if (p.accum_overwrite == 0) cur[k] = *reinterpret_cast<float4*>(dst + cc * 32 + k * 4);
                 }
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                  if (have) {
+                    cur[k].x += __uint_as_float(acc[cc][4 * k + 0]) * mul;
+                    cur[k].y += __uint_as_float(acc[cc][4 * k + 1]) * mul;
+                    cur[k].z += __uint_as_float(acc[cc][4 * k + 2]) * mul;
+                    cur[k].w += __uint_as_float(acc[cc][4 * k + 3]) * mul;
+                  }
+                  *reinterpret_cast<float4*>(dst + cc * 32 + k * 4) = cur[k];
+                }
+              }
             }
             continue;
           }
