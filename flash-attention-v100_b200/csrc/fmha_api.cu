@@ -251,9 +251,7 @@ FwdPlan plan_fwd(const FmhaFwdParams* p, int sms) {
   };
   const int n_max = visible(nqb - 1);
   if (n_max < 4) return plan;
-  // partial rows of pairs of chunks, written, and read by the join
-  auto part_bytes = [&](int n) { return heads * n * 2 * p->seqlen_q * p->head_dim * 8.0; };
-  const bool can_pair = p->seqlen_q <= (p->head_dim > 64 ? 127 : 128);  // full tiles at D = 128: 0.86 to 1.1 times as fast
+  const bool can_pair = p->seqlen_q <= 128 && n_max >= 16;  // (shorter: nothing to gain beyond the noise)
   if (heads * nqb > 8.0 * sms && !can_pair) return plan;  // enough items to balance
   auto cost = [&](int chunk, int& items) {  // makespan with chunks of `chunk` tiles
     double total = 0;
@@ -289,46 +287,53 @@ FwdPlan plan_fwd(const FmhaFwdParams* p, int sms) {
     if (heads * items > 8.0 * sms) break;
   }
   if (can_pair) {
-    // Few queries: an item with one query tile is a chain of MMA, softmax and MMA, 1.9 us per KV tile, and half
-    // of the SM idles.  Items of two chunks, in us: a round 2.2 at D = 64 and 3.0 at D = 128, where there is room
-    // for one K and one V tile per chunk only.  Not for chunks of less than 8 tiles (8 heads of 64 x 8192, D = 128:
-    // 25.6 as cut above, 30.7 in pairs).
-    const FwdPlan before = plan;
-    double best_us = 0.9 * 1.9 * (plan.max_chunks > 1 ? best : cost(n_max, items));
+    // Few queries: an item with one query tile is a chain of MMA, softmax and MMA, 1.5 to 1.9 us per KV tile, and half
+    // of the SM idles.  Items of two chunks, or the plan so far?  Times in us,
+    //   fixed + max(waves * (round * tiles + item), MB of K and V / rate) + per_mb * MB of partial rows,
+    // 0.35 more per MB of partial rows beyond 40 MB, which the L2 does not keep, and in pairs 0.25 per chunk for the
+    // join.  Rates: 6.4 TB/s, with an item per head 6.2, 3.6 and 4.4 at D = 64, 96 and 128.  Fitted to 5000 times of 784
+    // shapes (D = 64, 96, 128, 1 to 128 rows, 1024 to 16384 keys, 8 to 600 heads, bf16), to 4 % on average at D = 64, 6 %
+    // else; then corrected where the choice came out wrong.  Over 3320 shapes (also padded, causal, half
+    // visible, fp16), against straight lines that had been fitted to a ring of four slots: 1.06 times as fast
+    // on average, 64 queries x 8192 keys, 64 heads, D = 128 64.3 -> 60.4, 64 x 3000 50 -> 32, 128 x 16384 126 -> 90, D = 96 64 x 2048
+    // 35 -> 26; slower by more than 3 % in about one shape of a hundred (padded ones with uneven lengths, 128 rows), by 13 % at most.
+    struct Times {
+      double fixed, round, item, per_mb;
+    };
+    static const Times kPairs[2][2] = {{{10.3, 1.88, 1.8, 0.33}, {10.0, 1.60, 0.6, 0.40}},    // D = 64: others, 128 rows
+                                       {{10.8, 2.08, 2.5, 0.37}, {10.0, 1.90, 5.0, 0.46}}};  // D = 96, 128
+    static const Times kWhole[2][2] = {{{8.8, 1.54, 0.4, 0}, {9.9, 1.30, 0.0, 0}},
+                                       {{12.0, 1.74, 0.0, 0}, {10.8, 1.45, 0.7, 0}}};
+    static const Times kCut[2][2] = {{{13.0, 1.53, 2.7, 0.06}, {11.0, 1.30, 4.1, 0.20}},
+                                     {{0.0, 1.70, 18.0, 0.05}, {0.0, 1.50, 19.0, 0.12}}};
+    const int wide = p->head_dim > 64, full = p->seqlen_q == 128;
+    const double kv_mb = heads * n_max * 128 * p->head_dim * 4 / 1e6;
+    // The lengths of a padded batch are not known here: taken as half on average, and as items that fill the gaps; the
+    // second chunk of a pair is the emptier one, so that a pair takes more than half of its rounds.
+    const bool padded = p->seqused_k != nullptr;
+    auto time = [&](const Times& t, int chunk, double items, double rate, double parts, double filled) {
+      const double per_sm = heads * items / sms, longest = t.round * chunk + t.item;
+      const double work = padded ? std::max(longest, per_sm * (filled * t.round * chunk + t.item) + 0.4 * longest)
+                                 : std::ceil(per_sm) * longest;
+      const double part_mb = heads * parts * p->seqlen_q * p->head_dim * 8.0 / 1e6;
+      return t.fixed + std::max(work, (padded ? 0.55 : 1.0) * kv_mb / rate) + t.per_mb * part_mb +
+             0.35 * std::max(0.0, part_mb - 40.0);
+    };
+    const bool cut = plan.max_chunks > 1;
+    double most = (padded ? 1.0 : wide ? 0.95 : 0.92) *  // a pair has to be worth it
+                  (cut ? time(kCut[wide][full], plan.chunk_tiles, plan.max_chunks, 6.4, plan.max_chunks, 0.55)
+                       : time(kWhole[wide][full], n_max, 1, p->head_dim == 64 ? 6.2 : p->head_dim == 96 ? 3.6 : 4.4, 0, 0.55));
     for (int k = 1; k <= 32; ++k) {
       const int chunk = (n_max + 2 * k - 1) / (2 * k), n = (n_max + 2 * chunk - 1) / (2 * chunk);
-      if (chunk < 8) break;
-      const double t = std::ceil(heads * n / sms) * (chunk + 1.0) * (p->head_dim > 64 ? 3.0 : 2.2) + 3.0 +
-                       part_bytes(n) / 4e6;
-      if (t < best_us) {
-        best_us = t;
+      if (chunk < 4) break;
+      const double t = time(kPairs[wide][full], chunk, n, 6.4, 2 * n, 0.55 + 0.15 / n) + (padded ? 0.5 : 0.25) * 2 * n;
+      if (t < most) {
+        most = t;
         plan.pair = true;
         plan.chunk_tiles = chunk;
         plan.items_per_head = n;
         plan.max_chunks = 2 * n;
       }
-    }
-    // That is good enough to choose among the numbers of chunks, but not to choose between pairs and the plan before: it
-    // has the partial rows at half of what they cost, and full tiles, which take less time than others, like others.
-    // Pairs / before, us, D = 64, 2048 keys: 128 rows 148 heads 39 / 31, 1200 heads 246 / 192, 64 rows 1200 heads 198 / 228.
-    // So straight lines through 480 shapes (1 to 128 rows, 1024 to 16384 keys, 8 to 1200 heads, bf16) decide.  Of 3168
-    // shapes 6 are then slower in pairs than before, by 1 to 6 %; without them 89 were, by 2 to 28 %.  Taken, before /
-    // pairs, 64 x 8192: D = 64 64 heads 64 / 46, 128 heads 105 / 76, D = 96 75 / 62 and 118 / 99, D = 128 74 / 64 and 122 /
-    // 103; 96 x 8192: D = 128 75 / 66 and 120 / 107.
-    if (plan.pair) {
-      const bool wide = p->head_dim > 64, full = p->seqlen_q == 128;
-      const double round_us = wide ? 1.75 : full ? 1.35 : 1.5;
-      // (the items of a head with one query block are equal under a mask, too: whole waves, other than in cost())
-      const double whole = round_us * std::ceil(heads / sms) * (n_max + 0.5) + (wide ? 12.0 : 8.0);
-      const double now = before.max_chunks > 1 ? 1.85 * best : whole;
-      const double waves = std::ceil(heads * plan.items_per_head / sms);
-      // The lengths of a padded batch are not known here; taken as half on average, which is the same as counting the
-      // partial rows twice.  8 entries of n/8 to n keys, 412 shapes: 8 are slower in pairs then, by 9 % at most (D = 64, 96 x 4096,
-      // 600 heads 142 / 154), without it 26, by up to 32 % (96 x 2048, 600 heads 77 / 101).
-      const bool unequal = p->seqused_k != nullptr && before.max_chunks <= 1;
-      const double t = (wide ? waves * (2.7 * plan.chunk_tiles + 0.5) + 14.0 : waves * (1.87 * plan.chunk_tiles + 1.8) + 10.5) +
-                       (unequal ? 1.1 : 0.55) * part_bytes(plan.items_per_head) / 1e6;
-      if (t >= now) plan = before;
     }
   }
   if (plan.max_chunks > 1) {
@@ -356,6 +361,7 @@ int fwd_head_group(const FmhaFwdParams* p) {
 template <int D, bool kBf16, int DR = D>
 int launch_fwd(const FmhaFwdParams* p, void* workspace, size_t workspace_bytes, cudaStream_t stream) {
   using T = fmha::FwdTraits<D, kBf16, DR>;
+  using TPair = fmha::FwdTraits<D, kBf16, DR, true>;
   using E = typename std::conditional<kBf16, __nv_bfloat16, __half>::type;
   CUtensorMap tq, tk, tv, to;
   int rc;
@@ -406,7 +412,7 @@ int launch_fwd(const FmhaFwdParams* p, void* workspace, size_t workspace_bytes, 
   kp.deal = kp.num_items <= sms || p->sm_margin > 0;
   const unsigned grid = kp.deal ? (unsigned)std::min(kp.num_items, sms) : (unsigned)kp.num_items;
   const bool launched =
-      plan.pair ? launch_with_smem<fmha::fmha_fwd_kernel<D, kBf16, true, DR>>(dev, grid, T::kThreads, T::kSmemBytes,
+      plan.pair ? launch_with_smem<fmha::fmha_fwd_kernel<D, kBf16, true, DR>>(dev, grid, TPair::kThreads, TPair::kSmemBytes,
                                                                               stream, tq, tk, tv, to, kp)
                 : launch_with_smem<fmha::fmha_fwd_kernel<D, kBf16, false, DR>>(dev, grid, T::kThreads, T::kSmemBytes,
                                                                                stream, tq, tk, tv, to, kp);

@@ -97,7 +97,7 @@ constexpr int kFwdPolyPairs = 1;
 
 // DR <= D: elements per row of the tensors.  96 runs on the tiles of 128: the second box of a tile load holds 32
 // columns and zeros, which the MMAs leave out.
-template <int D, bool kBf16 = false, int DR = D>
+template <int D, bool kBf16 = false, int DR = D, bool kPair = false>
 struct FwdTraits {
   static constexpr int kBlockM = 128;  // rows per query tile
   static constexpr int kTilesM = 2;    // query tiles per work item
@@ -105,11 +105,16 @@ struct FwdTraits {
   static constexpr int kBoxes = D / 64;
   static constexpr int kBoxBytes = 128 * 128;  // 128 rows x 128 bytes
   static constexpr int kTileBytes = kBoxes * kBoxBytes;
-  static constexpr int kStages = (D == 128) ? 4 : 8;  // ring slots of one K or V tile
+  // A paired item (see the kernel) has one query tile in shared memory and no output to stage: room for six K
+  // or V tiles at D = 128, three per chunk.  64 queries x 8192 keys, 64 heads, bf16, two per chunk / three: 65.1 / 61.1 us
+  // (K and V alone take 41 at the rate of a copy).
+  static constexpr int kQTiles = kPair ? 1 : kTilesM;
+  static constexpr int kStages = (D == 128 ? 4 : 8) + (kPair ? (D == 128 ? 2 : 4) : 0);  // ring slots of one K or V tile
   static constexpr int kItemStages = 4;  // item ids published ahead
   static constexpr int kThreads = 384;   // softmax 0, softmax 1, {K/V, MMA, Q, idle} warps
   // Q tiles, K/V ring, one 64-column output box per softmax group
-  static constexpr int kSmemBytes = 1024 + kTilesM * (kTileBytes + kBoxBytes) + kStages * kTileBytes;
+  static constexpr int kSmemBytes =
+      1024 + (kQTiles + kStages) * kTileBytes + (kPair ? 0 : kTilesM * kBoxBytes);
   static constexpr int kTmemCols = 512;
   static constexpr uint32_t kIdescQK = umma_idesc_f16(128, kBlockN, 0, 0, kBf16);
   static constexpr uint32_t kIdescPV = umma_idesc_f16(128, DR, 0, 1, kBf16);
@@ -222,7 +227,7 @@ __global__ void __launch_bounds__(384, 1)
     fmha_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                     const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o,
                     const FwdKernelParams p) {
-  using T = FwdTraits<D, kBf16, DR>;
+  using T = FwdTraits<D, kBf16, DR, kPair>;
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(16) uint8_t clc_word[16];
   __shared__ uint64_t bar_clc;                        // the answer to the last request is in clc_word
@@ -253,9 +258,9 @@ __global__ void __launch_bounds__(384, 1)
   if (skip_cta) return;
 
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  const uint32_t q_smem = smem_base;                                    // 2 query tiles
-  const uint32_t ring_smem = smem_base + T::kTilesM * T::kTileBytes;    // K/V ring
-  const uint32_t ostage_smem = ring_smem + T::kStages * T::kTileBytes;  // 2 output boxes
+  const uint32_t q_smem = smem_base;                                    // 2 query tiles (kPair: one)
+  const uint32_t ring_smem = smem_base + T::kQTiles * T::kTileBytes;    // K/V ring
+  const uint32_t ostage_smem = ring_smem + T::kStages * T::kTileBytes;  // 2 output boxes (kPair: none)
   constexpr uint32_t kRingSlots = T::kStages / 2;  // kPair: of each tile's ring
 
   // ---- set-up: barriers (thread 0), tensor memory (warp 9)
@@ -418,34 +423,53 @@ __global__ void __launch_bounds__(384, 1)
       uint32_t phase = 0;  // bit t: Q_t tiles loaded so far, modulo 2 (phase of the Q barriers)
       uint32_t used = 0;   // bit t: Q_t has been loaded before
       bool ok = true;
+      auto load = [&](int t, int row, const FwdItem& it) {
+        if (elect_one()) {
+          const uint32_t qbar = smem_u32(&bar_q_full[t]);
+          mbar_arrive_expect_tx(qbar, T::kTileBytes);
+#pragma unroll
+          for (int b = 0; b < T::kBoxes; ++b)
+            tma_load_4d(q_smem + t * T::kTileBytes + b * T::kBoxBytes, &tm_q, qbar, b * 64, row, it.h, it.z);
+        }
+        __syncwarp();
+      };
+      // cold from HBM a tile takes microseconds: start towards L2 before waiting for the buffer
+      auto prefetch = [&](int row, const FwdItem& it) {
+        if (elect_one())
+#pragma unroll
+          for (int b = 0; b < T::kBoxes; ++b) tma_prefetch_l2_4d(&tm_q, b * 64, row, it.h, it.z);
+        __syncwarp();
+      };
       while (ok) {
         const FwdItem it = take_item();
         if (it.id < 0) break;
+        if constexpr (kPair) {
+          // one tile for both: free once the last S of either of the item before is done
+          if (it.n0 == 0) continue;
+          if (used) prefetch(it.q0, it);
+          for (int t = 0; ok && t < 2; ++t)
+            if ((used >> t) & 1) ok = mbar_wait_warp(smem_u32(&bar_q_free[t]), ((phase >> t) & 1) ^ 1, &abort_word, 1);
+          if (!ok) break;
+          load(0, it.q0, it);
+          const uint32_t both = it.n1 > 0 ? 3u : 1u;
+          phase ^= both;
+          used |= both;
+        } else {
 #pragma unroll 1
-        for (int t = 0; t < T::kTilesM; ++t) {
-          if ((t == 0 ? it.n0 : it.n1) == 0) continue;
-          const int row = it.q0 + (kPair ? 0 : t * T::kBlockM);
-          if ((used >> t) & 1) {
-            // cold from HBM this takes microseconds: start towards L2 before waiting for the buffer
-            if (elect_one())
-#pragma unroll
-              for (int b = 0; b < T::kBoxes; ++b) tma_prefetch_l2_4d(&tm_q, b * 64, row, it.h, it.z);
-            __syncwarp();
-            if (!mbar_wait_warp(smem_u32(&bar_q_free[t]), ((phase >> t) & 1) ^ 1, &abort_word, 1)) {
-              ok = false;
-              break;
+          for (int t = 0; t < T::kTilesM; ++t) {
+            if ((t == 0 ? it.n0 : it.n1) == 0) continue;
+            const int row = it.q0 + t * T::kBlockM;
+            if ((used >> t) & 1) {
+              prefetch(row, it);
+              if (!mbar_wait_warp(smem_u32(&bar_q_free[t]), ((phase >> t) & 1) ^ 1, &abort_word, 1)) {
+                ok = false;
+                break;
+              }
             }
+            load(t, row, it);
+            phase ^= 1u << t;
+            used |= 1u << t;
           }
-          if (elect_one()) {
-            const uint32_t qbar = smem_u32(&bar_q_full[t]);
-            mbar_arrive_expect_tx(qbar, T::kTileBytes);
-#pragma unroll
-            for (int b = 0; b < T::kBoxes; ++b)
-              tma_load_4d(q_smem + t * T::kTileBytes + b * T::kBoxBytes, &tm_q, qbar, b * 64, row, it.h, it.z);
-          }
-          __syncwarp();
-          phase ^= 1u << t;
-          used |= 1u << t;
         }
       }
     } else if (warp == 9) {
@@ -545,13 +569,13 @@ __global__ void __launch_bounds__(384, 1)
               ring_next(t);
               if (!(ok = slot_wait())) break;
             }
-            if (jk == 0) {
+            if (jk == 0 && (!kPair || t == 0)) {
               ok = mbar_wait_warp(smem_u32(&bar_q_full[t]), (phase_q >> t) & 1, &abort_word, 3);
               phase_q ^= 1u << t;
               if (!ok) break;
             }
             tc_fence_after();
-            const uint32_t a_lo = q_lo0 + ((t * T::kTileBytes) >> 4);
+            const uint32_t a_lo = q_lo0 + (kPair ? 0 : (t * T::kTileBytes) >> 4);
             const uint32_t b_lo = umma_desc_lo(kPair ? ring_smem + slot * T::kTileBytes : k_addr, kLboKMajor);
 #pragma unroll
             for (int ks = 0; ks < DR / 16; ++ks) {

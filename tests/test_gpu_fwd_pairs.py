@@ -188,3 +188,17 @@ def test_pairs_with_sms_left_free(D):
     r_out, r_lse = _reference(q, k, v, scale)
     assert oracle.max_abs(out.float(), r_out) <= _tol(torch.bfloat16)
     assert oracle.max_abs(lse, r_lse) <= helpers.TOL_LSE_MAX_ABS
+
+
+# chunks of 4 to 17 tiles through a ring of three (six at D = 64) slots each, full tiles of 128 rows
+@pytest.mark.parametrize("n_k", [2500, 4100, 8200])
+@pytest.mark.parametrize("n_q", [1, 128])
+@pytest.mark.parametrize("D,dtype", [(64, torch.bfloat16), (96, torch.float16), (128, torch.float16), (128, torch.bfloat16)])
+def test_pairs_of_short_chunks(n_q, n_k, D, dtype):
+    g = torch.Generator(device="cuda").manual_seed(72)
+    q, k, v = (torch.randn((1, n, 32, D), generator=g, device="cuda", dtype=dtype) for n in (n_q, n_k, n_k))
+    scale = oracle.default_scale(D)
+    out, lse = _run_pairs(q, k, v, scale)
+    r_out, r_lse = _reference(q, k, v, scale)
+    assert oracle.max_abs(out.float(), r_out) <= _tol(dtype)
+    assert oracle.max_abs(lse, r_lse) <= helpers.TOL_LSE_MAX_ABS
