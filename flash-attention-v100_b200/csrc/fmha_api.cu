@@ -501,11 +501,9 @@ int launch_bwd(const FmhaBwdParams* p, const BwdWorkspace& w, cudaStream_t strea
       kp.dq_order = w.dq_order;
     }
     const unsigned grid = (unsigned)((long long)kp.num_kv_blocks * H * Z);
-    // One block per item, taken over by running blocks.  Not where every item has an SM of its own,
-    // nor in the deterministic mode: an item waits there for items with lower indices, and only the
-    // order in which blocks are dispatched says that these are under way.
+    // One block per item, taken over by running blocks, unless every item has an SM of its own.
     const int dev = current_device();
-    kp.deal = (int)grid <= sm_count(dev) || kp.dq_order != nullptr;
+    kp.deal = (int)grid <= sm_count(dev);
     kp.timeline = g_timeline;
     kp.timeline_block = g_timeline_block;
     constexpr int smem = fmha::bwd_smem_bytes<D, kBf16>();

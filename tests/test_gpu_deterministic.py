@@ -59,3 +59,25 @@ def test_order_of_dq_in_a_padded_batch(q_row_begin, H):
     ref = _oracle_padded(q, k, v, dout, scale, True, sq, sk)
     assert not runs[0][0][:, :q_row_begin].any()
     helpers.check_against_oracle((out.cpu(), lse.cpu(), *(t.cpu() for t in runs[0])), ref, "order, padded")
+
+
+@pytest.mark.parametrize("D,dtype", [(64, torch.bfloat16), (96, torch.float16), (128, torch.float16)])
+@pytest.mark.parametrize("causal", [False, True])
+def test_order_of_dq_over_many_items(D, dtype, causal):
+    """Six times as many items as SMs, of one to three query tiles: a CTA has the next one while the one in work waits
+    for its turns."""
+    from flash_attn_v100 import cabi
+
+    H, N = 300, 352
+    g = torch.Generator(device="cuda").manual_seed(94)
+    q, k, v, dout = (torch.randn((1, N, H, D), generator=g, device="cuda", dtype=dtype) for _ in range(4))
+    scale = oracle.default_scale(D)
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    out, lse = cabi.fwd(q, k, v, scale, causal)
+    a, b, c = (cabi.bwd(q, k, v, out, dout, lse, scale, causal, flags=f, status=status)
+               for f in (cabi.FMHA_BWD_DETERMINISTIC, cabi.FMHA_BWD_DETERMINISTIC, 0))
+    assert int(status.item()) == 0
+    for x, y, z in zip(a, b, c):
+        assert torch.equal(x, y)
+        # the other mode adds the same terms in another order and rounds once (2^-9 for bf16)
+        assert oracle.rel_l2(x.float().cpu(), z.float().cpu()) < 2e-3
