@@ -423,34 +423,23 @@ __global__ void __launch_bounds__(384, 1)
       uint32_t phase = 0;  // bit t: Q_t tiles loaded so far, modulo 2 (phase of the Q barriers)
       uint32_t used = 0;   // bit t: Q_t has been loaded before
       bool ok = true;
-      auto load = [&](int t, int row, const FwdItem& it) {
-        if (elect_one()) {
-          const uint32_t qbar = smem_u32(&bar_q_full[t]);
-          mbar_arrive_expect_tx(qbar, T::kTileBytes);
-#pragma unroll
-          for (int b = 0; b < T::kBoxes; ++b)
-            tma_load_4d(q_smem + t * T::kTileBytes + b * T::kBoxBytes, &tm_q, qbar, b * 64, row, it.h, it.z);
-        }
-        __syncwarp();
-      };
-      // cold from HBM a tile takes microseconds: start towards L2 before waiting for the buffer
-      auto prefetch = [&](int row, const FwdItem& it) {
-        if (elect_one())
-#pragma unroll
-          for (int b = 0; b < T::kBoxes; ++b) tma_prefetch_l2_4d(&tm_q, b * 64, row, it.h, it.z);
-        __syncwarp();
-      };
       while (ok) {
         const FwdItem it = take_item();
         if (it.id < 0) break;
         if constexpr (kPair) {
           // one tile for both: free once the last S of either of the item before is done
           if (it.n0 == 0) continue;
-          if (used) prefetch(it.q0, it);
           for (int t = 0; ok && t < 2; ++t)
             if ((used >> t) & 1) ok = mbar_wait_warp(smem_u32(&bar_q_free[t]), ((phase >> t) & 1) ^ 1, &abort_word, 1);
           if (!ok) break;
-          load(0, it.q0, it);
+          if (elect_one()) {
+            const uint32_t qbar = smem_u32(&bar_q_full[0]);
+            mbar_arrive_expect_tx(qbar, T::kTileBytes);
+#pragma unroll
+            for (int b = 0; b < T::kBoxes; ++b)
+              tma_load_4d(q_smem + b * T::kBoxBytes, &tm_q, qbar, b * 64, it.q0, it.h, it.z);
+          }
+          __syncwarp();
           const uint32_t both = it.n1 > 0 ? 3u : 1u;
           phase ^= both;
           used |= both;
@@ -460,13 +449,24 @@ __global__ void __launch_bounds__(384, 1)
             if ((t == 0 ? it.n0 : it.n1) == 0) continue;
             const int row = it.q0 + t * T::kBlockM;
             if ((used >> t) & 1) {
-              prefetch(row, it);
+              // cold from HBM this takes microseconds: start towards L2 before waiting for the buffer
+              if (elect_one())
+#pragma unroll
+                for (int b = 0; b < T::kBoxes; ++b) tma_prefetch_l2_4d(&tm_q, b * 64, row, it.h, it.z);
+              __syncwarp();
               if (!mbar_wait_warp(smem_u32(&bar_q_free[t]), ((phase >> t) & 1) ^ 1, &abort_word, 1)) {
                 ok = false;
                 break;
               }
             }
-            load(t, row, it);
+            if (elect_one()) {
+              const uint32_t qbar = smem_u32(&bar_q_full[t]);
+              mbar_arrive_expect_tx(qbar, T::kTileBytes);
+#pragma unroll
+              for (int b = 0; b < T::kBoxes; ++b)
+                tma_load_4d(q_smem + t * T::kTileBytes + b * T::kBoxBytes, &tm_q, qbar, b * 64, row, it.h, it.z);
+            }
+            __syncwarp();
             phase ^= 1u << t;
             used |= 1u << t;
           }
