@@ -419,9 +419,22 @@ int launch_fwd(const FmhaFwdParams* p, void* workspace, size_t workspace_bytes, 
   if (!launched) return FMHA_ERR_LAUNCH;
   if (plan.max_chunks > 1) {
     const long long rows = (long long)kp.num_heads_total * (p->seqlen_q - plan.first_cut_row);
-    fmha::fmha_fwd_combine_kernel<E><<<(unsigned)((rows + 7) / 8), 256, 0, stream>>>(
-        kp, static_cast<E*>(p->o), p->o_strides.batch, p->o_strides.row, p->o_strides.head, plan.first_cut_row, rows);
-    if (cudaGetLastError() != cudaSuccess) return FMHA_ERR_LAUNCH;
+    // set up while the chunks are still in work; it waits for them itself
+    cudaLaunchAttribute early;
+    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3((unsigned)((rows + 7) / 8));
+    config.blockDim = dim3(256);
+    config.stream = stream;
+    config.attrs = &early;
+    config.numAttrs = 1;
+    if (cudaLaunchKernelEx(&config, fmha::fmha_fwd_combine_kernel<E>, kp, static_cast<E*>(p->o),
+                           (long long)p->o_strides.batch, (long long)p->o_strides.row, (long long)p->o_strides.head,
+                           plan.first_cut_row, rows) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return FMHA_ERR_LAUNCH;
+    }
   }
   return FMHA_OK;
 }

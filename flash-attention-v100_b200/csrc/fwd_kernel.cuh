@@ -878,6 +878,7 @@ template <typename E>
 __global__ void __launch_bounds__(256)
     fmha_fwd_combine_kernel(const FwdKernelParams p, E* __restrict__ o, long long so_batch, long long so_row,
                             long long so_head, int row_begin, long long total_rows) {
+  grid_dependency_wait();
   const long long idx = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (idx >= total_rows) return;
   const int lane = threadIdx.x & 31;

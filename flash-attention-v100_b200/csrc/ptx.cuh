@@ -409,6 +409,9 @@ __device__ __forceinline__ int clc_answer(uint32_t answer_smem) {
   return got ? (int)x : -1;
 }
 
+// In a kernel that the launch allows to start early: the kernels before it are done, their writes visible
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // warpgroup-wide register re-budgeting: every warp of an aligned group of 4 warps executes it
 template <int N>
 __device__ __forceinline__ void reg_alloc() {
