@@ -419,7 +419,9 @@ int launch_fwd(const FmhaFwdParams* p, void* workspace, size_t workspace_bytes, 
   if (!launched) return FMHA_ERR_LAUNCH;
   if (plan.max_chunks > 1) {
     const long long rows = (long long)kp.num_heads_total * (p->seqlen_q - plan.first_cut_row);
-    // set up while the chunks are still in work; it waits for them itself
+    // Set up while the chunks are still in work; it waits for them itself (59.6 -> 56.7 us at 64 queries x 8192 keys, 64
+    // heads, D = 128).  Not so the kernels of a backward: Z4 H16 N1024 D64 causal 49.3 -> 47.1 us on the GPU, but this
+    // launch takes the host half a microsecond longer, and small training steps wait for the host (76.3 -> 77.7).
     cudaLaunchAttribute early;
     early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     early.val.programmaticStreamSerializationAllowed = 1;
