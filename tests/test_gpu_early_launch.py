@@ -10,7 +10,7 @@ pytestmark = pytest.mark.gpu
 
 SHAPES = [  # Z, H, n_q, n_k, D, deterministic
     (1, 32, 64, 8192, 128, False),  # pairs of chunks
-    (1, 300, 16, 4096, 64, False),  # ... more items than SMs
+    (1, 300, 32, 4096, 64, False),  # ... more items than SMs
     (1, 2, 512, 4096, 128, True),   # an ordinary cut
     (2, 40, 384, 384, 96, False),   # none
 ]
