@@ -840,7 +840,13 @@ __global__ void __launch_bounds__(BwdTraits<D, kBf16, DR>::kThreads, 1)
               stg_buf = stg_smem + (chunk_no & 1u) * 16384;
               ++chunk_no;
             }
-            if (r == 0) tma_wait_group_read<1>();
+            // At D = 64 an item leaves one box each of dV and dK.  If one of them is in fp32, the other breaks the
+            // alternation of the buffers: then nothing may be reading before it, nor behind it.
+            const bool alone = T::kBoxes == 1 && (p.dk_accum == nullptr) != (p.dv_accum == nullptr);
+            if (r == 0) {
+              if (alone) tma_wait_group_read<0>();
+              else tma_wait_group_read<1>();
+            }
             named_bar_sync(2, 128);
 #pragma unroll
             for (int ch = 0; ch < (DR - b * 64 < 64 ? 4 : 8); ++ch) {
@@ -856,6 +862,7 @@ __global__ void __launch_bounds__(BwdTraits<D, kBf16, DR>::kThreads, 1)
             if (r == 0) {
               tma_store_4d(is_dk ? &tm_dk : &tm_dv, stg_buf, b * 64, it.kb * T::kBlock, it.h, it.z);
               tma_commit_group();
+              if (alone) tma_wait_group_read<0>();
             }
           }
         }
