@@ -70,7 +70,7 @@ struct BwdKernelParams {
   int num_heads_total;  // batch * heads
   int head_group;       // heads whose CTAs are interleaved in the grid (>= 1)
   int q_tile_begin;     // query tiles before this one take no part (FmhaBwdParams.q_row_begin / 128)
-  int deal;             // 1: every block has the one item of its index; 0: cluster launch control
+  int deal;             // 1: every block has the one item of its index; 0: cluster launch control (dq_order: neither)
   uint16_t *dk, *dv;    // 16-bit outputs (element strides), for KV tiles that no query sees
   Strides3 dk_strides, dv_strides;
   float scale, scale_log2;
@@ -80,7 +80,10 @@ struct BwdKernelParams {
   // CTAs that add into a query tile's dQ take turns (bwd_turn): a CTA waits for the word to reach
   // its turn, adds, and once its adds have completed sets turn + 1.  The fp32 additions then
   // happen in one fixed order and dQ is the same bits on every run.
-  int* dq_order;
+  // The first two of them are the halves of word 0, for word 1 counts the items that have been handed out (the workspace
+  // has no other room, and its size is part of the ABI).
+  unsigned* dq_order;
+  int num_items;
   // optional per-batch lengths (right-padded batches), see FmhaBwdParams
   const int* seqused_q;
   const int* seqused_k;
@@ -197,11 +200,15 @@ __device__ __forceinline__ BwdItem bwd_item(const BwdKernelParams& p, int id) {
 }
 
 // Deterministic dQ: the turn of an item's KV tile among those that add into a query tile.  An item only
-// ever waits for items with lower indices.  Blocks are dispatched, and taken over, in the order of their indices, and a
-// CTA works through its items in that order: of the items that are not done, the one with the lowest index is
-// in work, and waits for nobody.  (Taken over by running CTAs instead of a CTA per item, whole backward, us: Z2 H16 N2048 D128
-// bf16 causal 199 -> 189, without a mask 308 -> 296, Z8 H32 N2048 causal 1290 -> 1215, D96 Z8 H32 N1024 causal 410 -> 368, D64 Z64 H16
-// N512 568 -> 508, Z4 H16 N1024 causal 99.6 -> 87.4.)
+// ever waits for items with lower indices.  A CTA draws every item, the first one too, from one counter (draw), and
+// works through its items in the order in which it drew them.  So of the items that are not done the one with the lowest
+// index waits for nobody, and is in work or drawn next, whatever the order in which blocks start.  (Half a word
+// holds a turn modulo 2^16, which is enough: of the items drawn only a handful per CTA are not done.)
+// Cluster launch control, by which the other mode takes items over, promises no order; an item per CTA, in the order
+// of the block indices, relied on their being started in that order.  Whole backward, us, an item per CTA / by cluster
+// launch control / drawn, bf16: Z2 H16 N2048 D128 causal 199 / 185 / 190 (the first draw, and which SMs get the first
+// items), without a mask 313 / 297 / 292, Z8 H32 N2016 causal 1350 / 1224 / 1243, Z64 H16 N512 causal 618 / 608 / 545,
+// D64 without a mask 558 / 500 / 468, Z1 H40 N640 without a mask 71 / 82 / 69; 126 shapes 1 / 1.055 / 1.073 times as fast.
 // Without a mask: KV tile after KV tile, and the items of a head run staggered by one query tile each.
 // Under a causal mask: from the diagonal downwards, and the items of a head are dispatched in that order.
 // The item on the diagonal comes first to its query tile, the one below it a tile later, and so on: no item
@@ -240,6 +247,11 @@ __global__ void __launch_bounds__(BwdTraits<D, kBf16, DR>::kThreads, 1)
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);  // warp-uniform for the compiler, too
   const int lane = threadIdx.x & 31;
+
+  auto draw = [&]() -> unsigned { return atomicAdd(p.dq_order + 1, 1u); };
+  // the first item (drawn ahead of the set-up: the answer takes a while)
+  unsigned first_id = blockIdx.x;
+  if (kDet && threadIdx.x == T::kProducerWarp * 32) first_id = draw();
 
   if (threadIdx.x == 0) {
     sh.skip_cta = (p.status != nullptr && *reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
@@ -291,7 +303,10 @@ __global__ void __launch_bounds__(BwdTraits<D, kBf16, DR>::kThreads, 1)
       fence_barrier_init();
     }
     __syncwarp();
-    const BwdItem it = bwd_item<kDet>(p, blockIdx.x);
+    first_id = __shfl_sync(0xffffffffu, first_id, 0);
+    BwdItem it;
+    it.cnt = 0;
+    if (first_id < (unsigned)p.num_items) it = bwd_item<kDet>(p, first_id);
     if (it.cnt > 0) {
       const int row0 = it.i_begin * T::kBlock;
       send(3, &tm_q, it, row0, true);
@@ -351,7 +366,13 @@ __global__ void __launch_bounds__(BwdTraits<D, kBf16, DR>::kThreads, 1)
       bool ok = true;
       uint32_t published = 0, asked = 0;
       bool pending = false;  // a request is out
+      [[maybe_unused]] unsigned drawn = 0;
       auto ask = [&]() {
+        if constexpr (kDet) {
+          if (!pending && lane == 0) drawn = draw();
+          pending = true;
+          return;
+        }
         if (p.deal || pending) return;
         if (elect_one()) {
           fence_proxy_async_smem();  // the last answer has been read
@@ -385,12 +406,16 @@ __global__ void __launch_bounds__(BwdTraits<D, kBf16, DR>::kThreads, 1)
 
       // finds the next item with query tiles to walk and publishes it
       int id = -1;
-      bool first = true;  // the item of the block's own index comes first
+      bool first = true;  // the block's own item comes first
       auto next_item = [&]() -> BwdItem {
         BwdItem it;
         for (;; first = false) {
           if (first) {
-            id = blockIdx.x;
+            id = first_id < (unsigned)p.num_items ? (int)first_id : -1;
+          } else if (kDet) {
+            ask();
+            pending = false;
+            id = drawn < (unsigned)p.num_items ? (int)drawn : -1;
           } else if (p.deal) {
             id = -1;
           } else {
@@ -430,8 +455,10 @@ __global__ void __launch_bounds__(BwdTraits<D, kBf16, DR>::kThreads, 1)
       uint32_t g = 0;  // query tiles so far, over all items
       // The answer to a request takes a microsecond, so it is asked for ahead of the item's last loads: two tiles ahead at
       // D = 128; where there are four slots for the query tiles the loads run ahead as it is, and asking later balances
-      // better (Z4 H16 N1024 D64 causal 51.2 two ahead, 49.9 us one).
-      constexpr int kAskAhead = T::kQSlots > 2 ? 1 : 2;
+      // better (Z4 H16 N1024 D64 causal 51.2 two ahead, 49.9 us one).  Deterministic, the items of a head end one after
+      // the other, and the first to end has to be the first to ask: not ahead (two ahead / one / none, us: Z64 H16 N512 D128
+      // bf16 causal 592 / 529 / 517, Z1 H40 N640 without a mask 75.5 / 68.0 / 67.8; 126 shapes 0.982 / 0.997 / 1).
+      constexpr int kAskAhead = kDet ? 0 : T::kQSlots > 2 ? 1 : 2;
       while (ok) {
         const BwdItem it = next_item();
         if (it.id < 0) break;
@@ -739,10 +766,14 @@ __global__ void __launch_bounds__(BwdTraits<D, kBf16, DR>::kThreads, 1)
           __syncwarp();
           if (lane == 0) mbar_arrive(smem_u32(&sh.bar_dq_empty));
           if (tl) FMHA_TL(1, g, 2);
-          int* order_word = nullptr;
-          int turn = 0;
+          unsigned* order_word = nullptr;
+          uint32_t order_shift = 0, order_mask = 0xffffffffu;
+          unsigned turn = 0;
           if constexpr (kDet) {
-            order_word = p.dq_order + (size_t)it.zh * (p.seqlen_q_pad / T::kBlock) + tile;
+            const size_t at = (size_t)it.zh * (p.seqlen_q_pad / T::kBlock) + tile;
+            order_word = p.dq_order + (at == 1 ? 0 : at);
+            order_shift = at == 1 ? 16 : 0;
+            order_mask = at < 2 ? 0xffffu : 0xffffffffu;
             turn = bwd_turn(p, it, tile);
           }
 #pragma unroll
@@ -769,7 +800,7 @@ __global__ void __launch_bounds__(BwdTraits<D, kBf16, DR>::kThreads, 1)
             if (r == 0) {
               if (kDet && cc == 0) {
                 // those whose turn comes before have added their share of this query tile
-                global_flag_wait(order_word, turn, &sh.abort_word, p.status, 17);
+                global_flag_wait(order_word, order_shift, order_mask, turn, &sh.abort_word, p.status, 17);
                 fence_proxy_async_all();
               }
               tma_reduce_add_4d(&tm_dqacc, stg_buf, cc * 32, tile * T::kBlock, it.h, it.z);
@@ -778,7 +809,9 @@ __global__ void __launch_bounds__(BwdTraits<D, kBf16, DR>::kThreads, 1)
                 tma_wait_group<0>();  // the adds have been performed, not just read from shared memory
                 fence_proxy_async_all();
                 __threadfence();
-                global_flag_release(order_word, turn + 1);
+                // (a half's carry is not the other half's)
+                const bool wraps = order_mask == 0xffffu && order_shift == 0 && (turn & 0xffffu) == 0xffffu;
+                global_flag_release(order_word, wraps ? 1u - 65536u : 1u << order_shift);
               }
             }
           }

@@ -193,7 +193,7 @@ struct BwdWorkspace {
   float* dq_accum;
   float* lse2;
   float* delta;
-  int* dq_order;       // one word per (batch*head, query tile): FMHA_BWD_DETERMINISTIC
+  unsigned* dq_order;  // one word per (batch*head, query tile), two at least: FMHA_BWD_DETERMINISTIC
   size_t order_bytes;
   size_t bytes;
 };
@@ -206,8 +206,8 @@ BwdWorkspace carve_workspace(void* ws, int Z, int H, int Nq, int D) {
   w.dq_accum = reinterpret_cast<float*>(base);
   w.lse2 = reinterpret_cast<float*>(base + dq_bytes);
   w.delta = reinterpret_cast<float*>(base + dq_bytes + stat_bytes);
-  w.dq_order = reinterpret_cast<int*>(base + dq_bytes + 2 * stat_bytes);
-  w.order_bytes = (size_t)Z * H * (round_up_128(Nq) / 128) * sizeof(int);
+  w.dq_order = reinterpret_cast<unsigned*>(base + dq_bytes + 2 * stat_bytes);
+  w.order_bytes = std::max((size_t)2, (size_t)Z * H * (round_up_128(Nq) / 128)) * sizeof(int);
   w.bytes = dq_bytes + 2 * stat_bytes + (w.order_bytes + 255) / 256 * 256;
   return w;
 }
@@ -515,10 +515,12 @@ int launch_bwd(const FmhaBwdParams* p, const BwdWorkspace& w, cudaStream_t strea
       if (cudaMemsetAsync(w.dq_order, 0, w.order_bytes, stream) != cudaSuccess) return FMHA_ERR_LAUNCH;
       kp.dq_order = w.dq_order;
     }
-    const unsigned grid = (unsigned)((long long)kp.num_kv_blocks * H * Z);
-    // One block per item, taken over by running blocks, unless every item has an SM of its own.
+    kp.num_items = kp.num_kv_blocks * H * Z;
+    // One block per item, taken over by running blocks, unless every item has an SM of its own.  Deterministic: a block
+    // per SM, which draw the items from a counter.
     const int dev = current_device();
-    kp.deal = (int)grid <= sm_count(dev);
+    kp.deal = kp.num_items <= sm_count(dev);
+    const unsigned grid = kp.dq_order != nullptr ? std::min(kp.num_items, sm_count(dev)) : kp.num_items;
     kp.timeline = g_timeline;
     kp.timeline_block = g_timeline_block;
     constexpr int smem = fmha::bwd_smem_bytes<D, kBf16>();

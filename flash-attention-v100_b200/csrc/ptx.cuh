@@ -101,16 +101,15 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   return true;
 }
 
-// Bounded wait for a word in global memory to reach `want`; another CTA of the same grid with a
-// LOWER block index sets it (blocks are dispatched in index order, so that CTA is running or
-// done).  Gives up at once when this CTA, or the grid (status word), is already aborting.
+// Bounded wait for a field of a word in global memory, (word >> shift) & mask, to reach `want` (modulo the field); another CTA of the same
+// grid adds to it (global_flag_release), for an item that was handed out before this one's.  Gives up at once when this CTA, or the grid (status word), is already aborting.
 constexpr uint32_t kFlagPollLimit = 1u << 21;
-__device__ __forceinline__ bool global_flag_wait(const int* flag, int want, volatile int* abort_word,
+__device__ __forceinline__ bool global_flag_wait(const unsigned* flag, uint32_t shift, uint32_t mask, uint32_t want, volatile int* abort_word,
                                                  const int* status, int who) {
   for (uint32_t i = 0; i < kFlagPollLimit; ++i) {
-    int v;
-    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(flag) : "memory");
-    if (v >= want) return true;
+    uint32_t v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(flag) : "memory");
+    if ((((v >> shift) - want) & mask) <= mask >> 1) return true;
     if (*abort_word != 0) return false;
     if (status != nullptr && (i & 31u) == 31u && *reinterpret_cast<const volatile int*>(status) != 0)
       break;
@@ -119,8 +118,8 @@ __device__ __forceinline__ bool global_flag_wait(const int* flag, int want, vola
   atomicCAS(const_cast<int*>(abort_word), 0, kErrWaitTimeout | (who & 0xff));
   return false;
 }
-__device__ __forceinline__ void global_flag_release(int* flag, int value) {
-  asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(flag), "r"(value) : "memory");
+__device__ __forceinline__ void global_flag_release(unsigned* flag, uint32_t add) {
+  asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(flag), "r"(add) : "memory");
 }
 
 // ---------------------------------------------------------------------------------
