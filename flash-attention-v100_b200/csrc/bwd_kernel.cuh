@@ -61,7 +61,7 @@ namespace fmha {
 struct BwdKernelParams {
   const float* neg_lse2;  // fp32 (Z*H, seqlen_q_pad)
   const void* neg_delta;  // (Z*H, seqlen_q_pad): fp32 with bf16 tensors, else fp16
-  float* dk_accum;      // optional fp32 (Z, seqlen_k, H, D) contiguous
+  float* dk_accum;      // optional fp32 (Z, seqlen_k, H, D) contiguous: tm_dk then describes it
   float* dv_accum;      // optional
   long long accum_batch_stride;  // elements between batch entries of dk_accum / dv_accum
   int accum_overwrite;  // 1: dK / dV REPLACE what dk_accum / dv_accum hold (FMHA_BWD_ACCUM_OVERWRITE)
@@ -818,7 +818,11 @@ __global__ void __launch_bounds__(BwdTraits<D, kBf16, DR>::kThreads, 1)
           if (tl) FMHA_TL(1, g, 3);
         }
         // dV and dK of the item: tensor memory -> 16 bit -> TMA stores through the staging buffers; or (ring attention)
-        // into an fp32 buffer, added to what is there or, with accum_overwrite, in its place.  (This group does it
+        // 32 columns of fp32 at a time, reduce-added to what is there or, with accum_overwrite, in its place.  (With
+        // loads and stores of a row per thread, eight warps behind the next P^T / these four / so, whole backward, us,
+        // bf16, adding: Z8 H16 N512 D128 120 / 130 / 81, D64 69 / 74 / 47, Z1 H32 N4096 D128 causal 479 / 500 / 383;
+        // in its place: 98 / 92 / 78, 57 / 52 / 46, 439 / 424 / 390.  Through the staging buffers, but by loads and
+        // stores of whole lines, which keep one fused multiply-add: 127, 67, 484.)  (This group does it
         // because it has time to until the next item's first dQ.  Written by the compute groups they hold up the next
         // item's P^T and dS^T: the SM's port towards L2, at 20 bytes/clk, has the last dQ to send, too.)
         mbar_wait(smem_u32(&sh.bar_acc_full), drained & 1, abort_word, 15);
@@ -838,28 +842,35 @@ __global__ void __launch_bounds__(BwdTraits<D, kBf16, DR>::kThreads, 1)
           __syncwarp();
           if (lane == 0) mbar_arrive(smem_u32(is_dk ? &sh.bar_dk_read : &sh.bar_dv_read));
           if (accum != nullptr) {
-            const int kvi = it.kb * T::kBlock + r;
-            const bool have = kvi < it.sk;  // this thread's row has a result
-            if (kvi < p.seqlen_k && (have || p.accum_overwrite != 0)) {
-              float* dst = accum + (size_t)it.z * p.accum_batch_stride + ((size_t)kvi * p.heads + it.h) * DR;
+            // a padding key has no result: nothing is added to its row, and what replaces it is zero
+            const bool have = it.kb * T::kBlock + r < it.sk;
+            const float none = p.accum_overwrite != 0 ? 0.f : -0.f;
 #pragma unroll
-              for (int cc = 0; cc < kChunks; ++cc) {
-                float4 cur[8];  // read ahead of the stores
+            for (int cc = 0; cc < kChunks; ++cc) {
+              uint32_t stg_buf;
+              if constexpr (kChunks % 2 == 0) {
+                stg_buf = stg_smem + (cc & 1) * 16384;
+              } else {
+                stg_buf = stg_smem + (chunk_no & 1u) * 16384;
+                ++chunk_no;
+              }
+              if (r == 0) tma_wait_group_read<1>();
+              named_bar_sync(2, 128);
 #pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                  cur[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-                  if (p.accum_overwrite == 0) cur[k] = *reinterpret_cast<float4*>(dst + cc * 32 + k * 4);
-                }
+              for (int k4 = 0; k4 < 8; ++k4) {
+                uint32_t w[4];
 #pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                  if (have) {
-                    cur[k].x += __uint_as_float(acc[cc][4 * k + 0]) * mul;
-                    cur[k].y += __uint_as_float(acc[cc][4 * k + 1]) * mul;
-                    cur[k].z += __uint_as_float(acc[cc][4 * k + 2]) * mul;
-                    cur[k].w += __uint_as_float(acc[cc][4 * k + 3]) * mul;
-                  }
-                  *reinterpret_cast<float4*>(dst + cc * 32 + k * 4) = cur[k];
-                }
+                for (int k = 0; k < 4; ++k)
+                  w[k] = __float_as_uint(have ? __uint_as_float(acc[cc][k4 * 4 + k]) * mul : none);
+                sts128(stg_buf + r * 128 + ((k4 ^ (r & 7)) << 4), w[0], w[1], w[2], w[3]);
+              }
+              fence_proxy_async_smem();
+              named_bar_sync(2, 128);
+              if (r == 0) {
+                const CUtensorMap* tm = is_dk ? &tm_dk : &tm_dv;
+                if (p.accum_overwrite != 0) tma_store_4d(tm, stg_buf, cc * 32, it.kb * T::kBlock, it.h, it.z);
+                else tma_reduce_add_4d(tm, stg_buf, cc * 32, it.kb * T::kBlock, it.h, it.z);
+                tma_commit_group();
               }
             }
             continue;
@@ -873,8 +884,8 @@ __global__ void __launch_bounds__(BwdTraits<D, kBf16, DR>::kThreads, 1)
               stg_buf = stg_smem + (chunk_no & 1u) * 16384;
               ++chunk_no;
             }
-            // At D = 64 an item leaves one box each of dV and dK.  If one of them is in fp32, the other breaks the
-            // alternation of the buffers: then nothing may be reading before it, nor behind it.
+            // At D = 64 an item leaves one box each of dV and dK.  If one of them is in fp32 (two boxes), the other
+            // breaks the alternation of the buffers: then nothing may be reading before it, nor behind it.
             const bool alone = T::kBoxes == 1 && (p.dk_accum == nullptr) != (p.dv_accum == nullptr);
             if (r == 0) {
               if (alone) tma_wait_group_read<0>();

@@ -65,11 +65,12 @@ int make_tensor_map(CUtensorMap* map, const void* base, int Z, int N, int H, int
 
 // fp32 dQ accumulator (Z, N, H, D) contiguous -> 4-D map, box 32 x 128 x 1 x 1 (a tile's 128 query
 // rows x 32 columns = 128-byte rows), 128-byte swizzle; used by TMA reduce-add
-int make_accum_map(CUtensorMap* map, float* base, int Z, int N, int H, int D) {
+int make_accum_map(CUtensorMap* map, float* base, int Z, int N, int H, int D, int64_t batch) {
   EncodeTiledFn encode = get_encode_fn();
   if (encode == nullptr) return FMHA_ERR_NO_DEVICE;
   const cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)N, (cuuint64_t)H, (cuuint64_t)Z};
-  const cuuint64_t strides[3] = {(cuuint64_t)H * D * 4, (cuuint64_t)D * 4, (cuuint64_t)N * H * D * 4};
+  if (Z == 1 || batch == 0) batch = (int64_t)N * H * D;
+  const cuuint64_t strides[3] = {(cuuint64_t)H * D * 4, (cuuint64_t)D * 4, (cuuint64_t)batch * 4};
   const cuuint32_t box[4] = {32, 128, 1, 1};
   const cuuint32_t estr[4] = {1, 1, 1, 1};
   const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, dims, strides, box, estr,
@@ -468,17 +469,18 @@ int launch_bwd(const FmhaBwdParams* p, const BwdWorkspace& w, cudaStream_t strea
   {
     CUtensorMap tq, tk, tv, tdo, tdk, tdv, tacc;
     int rc;
-    if ((rc = make_accum_map(&tacc, w.dq_accum, Z, Nq, H, Dr))) return rc;
+    if ((rc = make_accum_map(&tacc, w.dq_accum, Z, Nq, H, Dr, 0))) return rc;
     if ((rc = make_tensor_map(&tq, p->q, Z, Nq, H, Dr, p->q_strides, kBf16))) return rc;
     if ((rc = make_tensor_map(&tk, p->k, Z, Nk, H, Dr, p->k_strides, kBf16))) return rc;
     if ((rc = make_tensor_map(&tv, p->v, Z, Nk, H, Dr, p->v_strides, kBf16))) return rc;
     if ((rc = make_tensor_map(&tdo, p->dout, Z, Nq, H, Dr, p->dout_strides, kBf16))) return rc;
-    // with fp32 accumulation the 16-bit outputs are not touched: any valid map will do
-    const bool acc_k = p->dk_accum != nullptr, acc_v = p->dv_accum != nullptr;
-    if ((rc = make_tensor_map(&tdk, acc_k ? p->k : p->dk, Z, Nk, H, Dr, acc_k ? p->k_strides : p->dk_strides, kBf16)))
-      return rc;
-    if ((rc = make_tensor_map(&tdv, acc_v ? p->v : p->dv, Z, Nk, H, Dr, acc_v ? p->v_strides : p->dv_strides, kBf16)))
-      return rc;
+    // with fp32 accumulation the 16-bit outputs are not touched
+    auto kv_out_map = [&](CUtensorMap* map, float* accum, void* out, const FmhaStrides& strides) {
+      return accum != nullptr ? make_accum_map(map, accum, Z, Nk, H, Dr, p->accum_batch_stride)
+                              : make_tensor_map(map, out, Z, Nk, H, Dr, strides, kBf16);
+    };
+    if ((rc = kv_out_map(&tdk, p->dk_accum, p->dk, p->dk_strides))) return rc;
+    if ((rc = kv_out_map(&tdv, p->dv_accum, p->dv, p->dv_strides))) return rc;
     fmha::BwdKernelParams kp;
     kp.neg_lse2 = w.lse2;
     kp.neg_delta = w.delta;

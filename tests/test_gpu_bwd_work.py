@@ -101,3 +101,43 @@ def test_one_of_dk_and_dv_in_fp32(D, dtype, wide):
     assert oracle.rel_l2(acc.cpu(), ref[3] if wide == "dk" else ref[4]) <= tol
     assert oracle.rel_l2(guard[:, :N].float().cpu(), ref[4] if wide == "dk" else ref[3]) <= tol
     assert (guard[:, N:] == 7.0).all()
+
+
+@pytest.mark.parametrize("D", [64, 96, 128])
+@pytest.mark.parametrize("wide", ["both", "dk", "dv"])
+def test_fp32_dk_dv_are_added_and_replaced_alike(D, wide):
+    """What is added is what would replace: bit for bit, and nothing to rows of padding keys, behind the last key or
+    between batch entries.  More items than SMs, the last KV tile not full, KV tiles that no query sees."""
+    from flash_attn_v100 import cabi
+
+    Z, H, n_q, n_k, gap = 3, 40, 200, 500, 24
+    g = torch.Generator(device="cuda").manual_seed(97)
+    q, dout = (torch.randn((Z, n_q, H, D), generator=g, device="cuda", dtype=torch.float16) for _ in range(2))
+    k, v = (torch.randn((Z, n_k, H, D), generator=g, device="cuda", dtype=torch.float16) for _ in range(2))
+    used = torch.tensor([500, 130, 0], dtype=torch.int32, device="cuda")
+    start = [torch.randn((Z, n_k + gap, H, D), generator=g, device="cuda") for _ in range(2)]
+    out, lse = cabi.fwd(q, k, v, 0.1, True, 100, seqused_k=used)
+    names = {"both": ["dk", "dv"], "dk": ["dk"], "dv": ["dv"]}[wide]
+
+    def run(flags):
+        acc = dict(zip(("dk", "dv"), (t.clone() for t in start)))
+        kw = {name + "_accum": acc[name][:, :n_k] for name in names}
+        kw |= {name: torch.full_like(k, float("nan")) for name in ("dk", "dv") if name not in names}
+        _, dk, dv = cabi.bwd(q, k, v, out, dout, lse, 0.1, True, 100, flags=flags, seqused_k=used, **kw)
+        return acc, {"dk": dk, "dv": dv}
+
+    added, narrow = run(0)
+    replaced, again = run(cabi.FMHA_BWD_ACCUM_OVERWRITE)
+    plain = dict(zip(("dq", "dk", "dv"), cabi.bwd(q, k, v, out, dout, lse, 0.1, True, 100, seqused_k=used)))
+    for name, before in zip(("dk", "dv"), start):
+        if name not in names:
+            assert torch.equal(narrow[name], plain[name]) and torch.equal(again[name], plain[name])
+            assert torch.equal(added[name], before)
+            continue
+        new = replaced[name][:, :n_k]
+        assert torch.equal(new.half(), plain[name])
+        assert torch.equal(replaced[name][:, n_k:], before[:, n_k:])
+        assert torch.equal(added[name][:, :n_k], before[:, :n_k] + new)
+        assert torch.equal(added[name][:, n_k:], before[:, n_k:])
+        for z, n in enumerate(used.tolist()):
+            assert torch.equal(added[name][z, n:], before[z, n:]) and not new[z, n:].any()
