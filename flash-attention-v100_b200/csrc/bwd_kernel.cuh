@@ -800,7 +800,7 @@ __global__ void __launch_bounds__(BwdTraits<D, kBf16, DR>::kThreads, 1)
             if (r == 0) {
               if (kDet && cc == 0) {
                 // those whose turn comes before have added their share of this query tile
-                global_flag_wait(order_word, order_shift, order_mask, turn, &sh.abort_word, p.status, 17);
+                global_flag_wait(order_word, order_shift, order_mask, turn, &sh.abort_word, p.status, 22);
                 fence_proxy_async_all();
               }
               tma_reduce_add_4d(&tm_dqacc, stg_buf, cc * 32, tile * T::kBlock, it.h, it.z);
