@@ -288,46 +288,41 @@ FwdPlan plan_fwd(const FmhaFwdParams* p, int sms) {
     if (heads * items > 8.0 * sms) break;
   }
   if (can_pair) {
-    // Few queries: an item with one query tile is a chain of MMA, softmax and MMA, 1.5 to 1.9 us per KV tile, and half
-    // of the SM idles.  Items of two chunks, or the plan so far?  Times in us,
-    //   fixed + max(waves * (round * tiles + item), MB of K and V / rate) + per_mb * MB of partial rows,
-    // 0.35 more per MB of partial rows beyond 40 MB, which the L2 does not keep, and in pairs 0.25 per chunk for the
-    // join.  Rates: 6.4 TB/s, with an item per head 6.2, 3.6 and 4.4 at D = 64, 96 and 128.  Fitted to 5000 times of 784
-    // shapes (D = 64, 96, 128, 1 to 128 rows, 1024 to 16384 keys, 8 to 600 heads, bf16), to 4 % on average at D = 64, 6 %
-    // else; then corrected where the choice came out wrong.  Over 3320 shapes (also padded, causal, half
-    // visible, fp16), against straight lines that had been fitted to a ring of four slots: 1.06 times as fast
-    // on average, 64 queries x 8192 keys, 64 heads, D = 128 64.3 -> 60.4, 64 x 3000 50 -> 32, 128 x 16384 126 -> 90, D = 96 64 x 2048
-    // 35 -> 26; slower by more than 3 % in about one shape of a hundred (padded ones with uneven lengths, 128 rows), by 13 % at most.
-    struct Times {
-      double fixed, round, item, per_mb;
+    // Few queries: an item with one query tile is a chain of MMA, softmax and MMA, and half of the SM idles.  Items of
+    // two chunks, which idle less but leave partial rows, or the plan so far?  Estimates of each, in us: a fixed part and
+    // one per chunk (the join); the rounds of the longest item, wave after wave, and K and V from HBM, of which the longer
+    // one counts and the shorter one a little; the partial rows, more beyond 40 MB, which the L2 does not keep.  A
+    // round of one tile takes 1.5 to 1.7 us, of two chunks 1.8 to 2.1; rows that a tile does not have cost 0.1 to 0.2,
+    // for they are masked.  Pairs have to be estimated 8 % faster than whole items, 4 % faster than the ordinary cut.
+    // Constants from 2918 shapes (D = 64, 96, 128, 1 to 128 rows, 1921 to 32768 keys, 8 to 1200 heads, bf16), every way
+    // timed, searched on one half of them and as good on the other: 0.5 % slower than the best way on average, by more
+    // than 3 % in 110 of them, 17 % at most (without pairs 22 % slower on average).  148 heads of 128 rows over 4096 keys,
+    // D = 128: whole 59 us, one pair 73; 64 rows over 8192, 64 heads: whole 113, two pairs 54.
+    // Padded batches: the lengths are not known here.  Taken as 0.56 of the whole on average, and waves and margins as
+    // they were best for 1639 shapes with 8 entries of n/8 to n keys: 1.2 % slower than the best way on average, 22 % at
+    // most (without pairs 27 % on average).
+    const double wide = p->head_dim / 64.0;
+    const bool full = p->seqlen_q == 128, padded = p->seqused_k != nullptr;
+    const double one_tile = 1.37 + 0.19 * wide - (full ? 0.2 : 0.0), two_chunks = 1.52 + 0.32 * wide - (full ? 0.1 : 0.0);
+    auto waves = [&](int items, double filled) {  // items per head; of a padded batch, the part of their rounds that exists
+      const double per_sm = heads * items / sms;
+      if (!padded || per_sm <= 1) return std::ceil(per_sm);
+      return std::max(1.0, per_sm * filled + 0.25 * std::ceil(per_sm * filled));
     };
-    static const Times kPairs[2][2] = {{{10.3, 1.88, 1.8, 0.33}, {10.0, 1.60, 0.6, 0.40}},    // D = 64: others, 128 rows
-                                       {{10.8, 2.08, 2.5, 0.37}, {10.0, 1.90, 5.0, 0.46}}};  // D = 96, 128
-    static const Times kWhole[2][2] = {{{8.8, 1.54, 0.4, 0}, {9.9, 1.30, 0.0, 0}},
-                                       {{12.0, 1.74, 0.0, 0}, {10.8, 1.45, 0.7, 0}}};
-    static const Times kCut[2][2] = {{{13.0, 1.53, 2.7, 0.06}, {11.0, 1.30, 4.1, 0.20}},
-                                     {{0.0, 1.70, 18.0, 0.05}, {0.0, 1.50, 19.0, 0.12}}};
-    const int wide = p->head_dim > 64, full = p->seqlen_q == 128;
-    const double kv_mb = heads * n_max * 128 * p->head_dim * 4 / 1e6;
-    // The lengths of a padded batch are not known here: taken as half on average, and as items that fill the gaps; the
-    // second chunk of a pair is the emptier one, so that a pair takes more than half of its rounds.
-    const bool padded = p->seqused_k != nullptr;
-    auto time = [&](const Times& t, int chunk, double items, double rate, double parts, double filled) {
-      const double per_sm = heads * items / sms, longest = t.round * chunk + t.item;
-      const double work = padded ? std::max(longest, per_sm * (filled * t.round * chunk + t.item) + 0.4 * longest)
-                                 : std::ceil(per_sm) * longest;
-      const double part_mb = heads * parts * p->seqlen_q * p->head_dim * 8.0 / 1e6;
-      return t.fixed + std::max(work, (padded ? 0.55 : 1.0) * kv_mb / rate) + t.per_mb * part_mb +
-             0.35 * std::max(0.0, part_mb - 40.0);
+    auto time = [&](double rounds_us, int chunks) {
+      const double part = padded ? 0.56 : 1.0;
+      const double kv_us = part * heads * n_max * 128 * p->head_dim * 4 / 7.1e6;
+      const double parts_mb = part * heads * chunks * p->seqlen_q * p->head_dim * 8 / 1e6;
+      const double x = rounds_us * rounds_us, y = kv_us * kv_us;
+      return 6.0 + 0.27 * chunks + std::sqrt(std::sqrt(x * x + y * y)) + 0.34 * parts_mb + 0.1 * std::max(0.0, parts_mb - 40);
     };
-    const bool cut = plan.max_chunks > 1;
-    double most = (padded ? 1.0 : wide ? 0.95 : 0.92) *  // a pair has to be worth it
-                  (cut ? time(kCut[wide][full], plan.chunk_tiles, plan.max_chunks, 6.4, plan.max_chunks, 0.55)
-                       : time(kWhole[wide][full], n_max, 1, p->head_dim == 64 ? 6.2 : p->head_dim == 96 ? 3.6 : 4.4, 0, 0.55));
+    const int chunks = plan.max_chunks;
+    double most = chunks > 1 ? (padded ? 0.93 : 0.96) * time(waves(chunks, 0.58) * (one_tile * plan.chunk_tiles + 2.5), chunks)
+                             : (padded ? 0.88 : 0.92) * (time(waves(1, 0.67) * (one_tile * n_max - 0.5), 0) - 0.5);
     for (int k = 1; k <= 32; ++k) {
       const int chunk = (n_max + 2 * k - 1) / (2 * k), n = (n_max + 2 * chunk - 1) / (2 * chunk);
       if (chunk < 4) break;
-      const double t = time(kPairs[wide][full], chunk, n, 6.4, 2 * n, 0.55 + 0.15 / n) + (padded ? 0.5 : 0.25) * 2 * n;
+      const double t = time(waves(n, 0.58 + 0.27 / n) * (two_chunks * chunk + 1.3), 2 * n);
       if (t < most) {
         most = t;
         plan.pair = true;

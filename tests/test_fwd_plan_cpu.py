@@ -70,3 +70,23 @@ def test_a_padded_batch_is_not_cut_where_that_is_slower(built_library, heads, n_
 @pytest.mark.parametrize("heads,n_q,n_k,D", [(64, 64, 4096, 128), (128, 64, 8192, 64), (1200, 16, 8192, 128)])
 def test_a_padded_batch_is_cut_in_pairs(built_library, heads, n_q, n_k, D):
     assert _chunks(heads, n_q, n_k, D, padded=True) >= 2
+
+
+# one or two whole waves of items, us, whole items / pairs: full waves leave little idle, and many rows many partial results
+@pytest.mark.parametrize("heads,n_q,n_k,D", [
+    (148, 128, 4096, 128),  # 59 / 73
+    (148, 128, 2500, 96),   # 38 / 47
+    (296, 128, 3000, 96),   # 82 / 99
+    (148, 127, 2048, 96),   # 35 / 43
+    (296, 112, 4096, 128),  # 122 / 137
+    (200, 128, 3000, 128),  # 80 / 91
+])
+def test_full_waves_are_not_cut_in_pairs(built_library, heads, n_q, n_k, D):
+    assert _chunks(heads, n_q, n_k, D) == 0
+
+
+# 8 entries of n_k / 8 to n_k keys, us: two items per head / one, where one is a little more than an SM
+@pytest.mark.parametrize("heads,n_q,n_k,D", [(200, 128, 8192, 64), (200, 127, 6144, 64), (200, 96, 8192, 128)])
+def test_a_padded_batch_is_cut_twice_where_once_is_slower(built_library, heads, n_q, n_k, D):
+    """(83 / 110, 77 / 101, 107 / 140)"""
+    assert _chunks(heads, n_q, n_k, D, padded=True) == 4

@@ -146,6 +146,22 @@ def test_pairs_one_after_the_other_in_a_padded_batch(D, dtype):
     assert not out[~seen.transpose(1, 2)].any()
 
 
+@pytest.mark.parametrize("D", [64, 96, 128])
+def test_pairs_twice_per_head_in_a_padded_batch(D):
+    # 25 tiles in chunks of 7, 7, 7 and 4; entries that end with one tile in the fourth, third, second and first, and with none
+    n_q, n_k, sq, sk = 16, 3200, [16, 1, 16, 7, 9], [2689, 1793, 897, 1, 0]
+    q, k, v = _many(n_q, n_k, D, torch.bfloat16, seed=70)
+    scale = oracle.default_scale(D)
+    lens = {"seqused_q": sq, "seqused_k": sk}
+    out, lse = _run_pairs(q, k, v, scale, **{n: torch.tensor(x, dtype=torch.int32, device="cuda") for n, x in lens.items()})
+    r_out, r_lse = _reference(q, k, v, scale, sq=sq, sk=sk)
+    assert oracle.max_abs(out.float(), r_out) <= _tol(torch.bfloat16)
+    seen = torch.isfinite(r_lse)
+    assert torch.equal(torch.isfinite(lse), seen)
+    assert oracle.max_abs(lse[seen], r_lse[seen]) <= helpers.TOL_LSE_MAX_ABS
+    assert not out[~seen.transpose(1, 2)].any()
+
+
 @pytest.mark.parametrize("what", ["query rows", "keys of the first chunk", "keys of the second chunk"])
 @pytest.mark.parametrize("D", [64, 96, 128])
 def test_pairs_with_rows_that_are_not_finite(D, what):
