@@ -187,8 +187,9 @@ int fmha_fwd(const FmhaFwdParams* p, void* stream);
 /* The same with device scratch of fmha_fwd_workspace_bytes(p) bytes, 16-byte aligned.  With it, a call
  * whose query blocks alone would leave SMs idle (few queries over a long context) cuts their KV
  * ranges into chunks and joins the partial results; with less, or NULL, it runs uncut like fmha_fwd.
- * Up to 128 query rows over many keys are cut in pairs of chunks of at least 512 keys however many
- * items there are, which takes up to a quarter of the bytes of K and V.
+ * Up to 128 query rows over 1921 keys and more are cut, however many items there are, in pairs of
+ * chunks of 512 keys and more (the last ones less), which takes up to 0.34 of the bytes of K and V.  With
+ * fewer than 28 heads (batch * heads), or fewer keys, it can be chunks of 256, and up to 0.62.
  * fmha_fwd_workspace_bytes returns 0 where a workspace would not be used.  (An entry point of its own
  * and not two more fields of FmhaFwdParams, which a host built against an earlier header of the
  * library would not have.) */
