@@ -75,3 +75,41 @@ def test_call_after_call_on_two_streams(shape):
     for results, w in zip(got, want):
         for x in results:
             _close(x, w)
+
+
+@pytest.mark.parametrize("shape", SHAPES[:3])
+@pytest.mark.parametrize("poison", [False, True])
+def test_join_sees_the_chunks_of_its_own_call(shape, poison):
+    """A workspace holds the partial results of the call before, on other inputs, or NaN: a join that did not wait would
+    read them.  Against the uncut forward."""
+    import ctypes
+
+    from flash_attn_v100 import cabi
+
+    Z, H, n_q, n_k, D, _ = shape
+    scale = oracle.default_scale(D)
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    jobs = []
+    for i, s in enumerate(streams):
+        data = [_calls(shape, 10 + 2 * i + k, torch.float16)[1][:3] for k in range(2)]
+        out, lse = (torch.empty((8, Z, n_q, H, D), dtype=torch.float16, device="cuda"),
+                    torch.empty((8, Z, H, n_q), device="cuda"))
+        p = cabi.fwd_params(*data[0], out[0], lse[0], scale, False)
+        nbytes = cabi.load_library().fmha_fwd_workspace_bytes(ctypes.byref(p))
+        assert nbytes > 0
+        jobs.append((s, data, out, lse, torch.full((nbytes,), 255, dtype=torch.uint8, device="cuda")))
+    torch.cuda.synchronize()
+    for n in range(8):
+        for s, data, out, lse, workspace in jobs:
+            with torch.cuda.stream(s):
+                if poison:
+                    workspace.fill_(255)
+                cabi.fwd(*data[n % 2], scale, out=out[n], lse=lse[n], workspace=workspace)
+    torch.cuda.synchronize()
+    for _, data, out, lse, _ in jobs:
+        for k in range(2):
+            want, want_lse = cabi.fwd(*data[k], scale)
+            for n in range(k, 8, 2):
+                # (the probabilities, at most 1, are rounded to fp16, 2^-11, relative to other references)
+                assert oracle.max_abs(out[n].float(), want.float()) <= 2e-3
+                assert oracle.max_abs(lse[n], want_lse) <= 1e-4
