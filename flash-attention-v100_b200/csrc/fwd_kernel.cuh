@@ -792,13 +792,16 @@ __global__ void __launch_bounds__(384, 1)
         }
         if (split) {
           if (nd == 0) continue;  // LSE = -inf: the combine kernel reads no row
-          float* dst = p.o_part + (((size_t)chunk * p.num_heads_total + done.zh) * p.seqlen_q + row) * DR;
+          // (p.row_elems is DR.  Where it is left out here for good, the other code of the kernel comes out slower: without a
+          // mask, Z1 H8 N8192 D64 210.9 -> 213.2 us, D96 230.1 -> 233.2, D128 0.2 %; not so for pairs.)
+          const int row_elems = DR == D && !kPair ? p.row_elems : DR;
+          float* dst = p.o_part + (((size_t)chunk * p.num_heads_total + done.zh) * p.seqlen_q + row) * row_elems;
 #pragma unroll 1
           for (int cc = 0; cc < DR / 16; ++cc) {
             uint32_t o[16];
             tmem_ld16(tO + cc * 16, o);
             tmem_wait_ld();
-            if (row < p.seqlen_q) {
+            if (row < p.seqlen_q && ((kPair && DR == D) || cc * 16 < p.row_elems)) {
 #pragma unroll
               for (int i = 0; i < 16; i += 4)
                 *reinterpret_cast<float4*>(dst + cc * 16 + i) =
