@@ -6,9 +6,9 @@
 // 503-506), with dQ accumulated in fp32 instead of the reference's fp16 atomics (:543,693).
 //
 // A work item is one 128-row KV tile of one (batch, head) and the query tiles (128 rows) that can
-// see it.  A CTA stays on its SM and takes item after item (cluster launch control); dK and dV of an item are
-// written out beside the first P^T of the next.  Everything is computed TRANSPOSED so that the KV rows sit on the 128
-// tensor-memory lanes, which lets P^T feed the dV MMA straight from tensor memory:
+// see it.  A CTA stays on its SM and takes item after item (cluster launch control; deterministic, a counter).
+// Everything is computed TRANSPOSED so that the KV rows sit on the 128 tensor-memory lanes, which lets P^T feed the
+// dV MMA straight from tensor memory:
 //
 //   S^T  = K  Q_i^T    (A = K  smem K-major,  B = Q_i  smem K-major)      -> TMEM [0,128)
 //   dP^T = V  dO_i^T   (A = V  smem K-major,  B = dO_i smem K-major)      -> TMEM [128,256)
@@ -33,20 +33,21 @@
 // both padded to a multiple of 128 rows per (batch, head); a tile's 2 x 128 values come in with Q_i.
 //
 // What bounds it at D = 128: the SM's port towards L2, and the power cap.  Per query tile there are 2560 clk of MMA
-// and 64 KB of fp32 reduce-adds, which take 3000 clk through the port (about 20 bytes/clk; l1tex__m_l1tex2xbar_req is
-// active 77 % of the time at Z4 H32 N2048 without a mask, the tensor pipe 60 %), in a period of 3700 to 3900.  At D = 64
-// (port 43 %, tensor pipe 31 %) it is a chain: P^T, wait, dS^T, wait.  The end of an item costs extra, 4000 clk of loads that come
-// in late and 64 KB of dK and dV through the same port.  What was measured about that end (whole backward, us,
-// first S^T of the next item ahead of the last dQ and dK, dK and dV written by the compute groups behind its P^T -> as
-// it is now: S^T behind them, written by the dQ group; no prefetch towards L2, which shares the TMA unit): Z64 H16 N512
-// D64 bf16 356 -> 331, Z4 H16 N1024 D64 causal 53.6 -> 49.3, Z2 H16 N8192 D64 causal 914 -> 860; Z8 H32 N2048 D128 causal
-// 978 -> 940, without a mask, bf16 1545 -> 1500, D96 causal 838 -> 805; a padded batch of it 251 -> 242.  Sixteen compute warps
-// of 32 columns at D = 64 instead of eight of 64: Z2 H16 N8192 causal 909 -> 888, Z64 H16 N512 345 -> 342.
-// The instruction cache decides more than it seems: with MMA loops and
-// write-outs unrolled the same kernel fetched 1.7 times the instructions from behind the first-level cache
-// and ran 5-18 % SLOWER than one CTA per item, rolled up 5-10 % faster (0.56 stalled cycles per issue for want of
-// instructions).  Hence the loops below.  At D = 128 shorter periods alone
-// (sixteen compute warps there, too: -10 %) do not shorten the time, the clock falls instead: the power cap.
+// and 64 KB of fp32 reduce-adds, which take 3000 clk through the port (about 20 bytes/clk; it is active 81 % of the
+// time at Z8 H32 N2048 causal, the tensor pipe 62 %), in a period of 3700 to 3900.  At D = 64 (port 43 %, tensor
+// pipe 31 %) it is a chain: P^T, wait, dS^T, wait.
+// The end of an item costs extra: 4000 clk of loads that come in late, and 64 KB of dK and dV through the same port.
+// Hence the first S^T of the next item is issued behind the last dQ and dK, for its K comes late, and dK and dV are
+// written by the dQ group, which is idle there.  Against S^T ahead of them, dK and dV written by the compute groups
+// behind P^T, a prefetch of K, V and dO towards L2, and at D = 64 eight compute warps of 64 columns instead of
+// sixteen of 32, all together, whole backward, us: Z64 H16 N512 D64 bf16 363 -> 323, Z4 H16 N1024 D64 causal 51 -> 46,
+// Z2 H16 N8192 D64 causal 914 -> 860, Z8 H32 N2016 D128 bf16 without a mask 1481 -> 1432, causal 954 -> 904, D96
+// 838 -> 760.  The warps alone: Z2 H16 N8192 D64 causal 909 -> 888, Z64 H16 N512 345 -> 342.  With the prefetch again:
+// D = 64 no difference, D = 96 and 128 0 to 4 % slower (it shares the unit with the loads it is meant to help).
+// The instruction cache decides more than it seems: with MMA loops and write-outs unrolled the same kernel fetched
+// 1.7 times the instructions from behind the first-level cache and ran 5-18 % SLOWER than one CTA per item, rolled up
+// 5-10 % faster.  Hence the loops below.  At D = 128 shorter periods alone (sixteen compute warps there, too: -10 %) do
+// not shorten the time, the clock falls instead: the power cap.
 #pragma once
 #include <cuda.h>
 #include <math_constants.h>
@@ -80,8 +81,8 @@ struct BwdKernelParams {
   // CTAs that add into a query tile's dQ take turns (bwd_turn): a CTA waits for the word to reach
   // its turn, adds, and once its adds have completed sets turn + 1.  The fp32 additions then
   // happen in one fixed order and dQ is the same bits on every run.
-  // The first two of them are the halves of word 0, for word 1 counts the items that have been handed out (the workspace
-  // has no other room, and its size is part of the ABI).
+  // The first two of them are the halves of word 0, for word 1 counts the items that have been handed out (the
+  // workspace has no other room, and its size is part of the ABI).
   unsigned* dq_order;
   int num_items;
   // optional per-batch lengths (right-padded batches), see FmhaBwdParams
@@ -201,14 +202,15 @@ __device__ __forceinline__ BwdItem bwd_item(const BwdKernelParams& p, int id) {
 
 // Deterministic dQ: the turn of an item's KV tile among those that add into a query tile.  An item only
 // ever waits for items with lower indices.  A CTA draws every item, the first one too, from one counter (draw), and
-// works through its items in the order in which it drew them.  So of the items that are not done the one with the lowest
-// index waits for nobody, and is in work or drawn next, whatever the order in which blocks start.  (Half a word
-// holds a turn modulo 2^16, which is enough: of the items drawn only a handful per CTA are not done.)
+// works through its items in the order in which it drew them.  So of the items that are not done the one with the
+// lowest index waits for nobody, and is in work or drawn next, whatever the order in which blocks start.  (Half a
+// word holds a turn modulo 2^16, which is enough: of the items drawn only a handful per CTA are not done.)
 // Cluster launch control, by which the other mode takes items over, promises no order; an item per CTA, in the order
 // of the block indices, relied on their being started in that order.  Whole backward, us, an item per CTA / by cluster
 // launch control / drawn, bf16: Z2 H16 N2048 D128 causal 199 / 185 / 190 (the first draw, and which SMs get the first
 // items), without a mask 313 / 297 / 292, Z8 H32 N2016 causal 1350 / 1224 / 1243, Z64 H16 N512 causal 618 / 608 / 545,
-// D64 without a mask 558 / 500 / 468, Z1 H40 N640 without a mask 71 / 82 / 69; 126 shapes 1 / 1.055 / 1.073 times as fast.
+// D64 without a mask 558 / 500 / 468, Z1 H40 N640 without a mask 71 / 82 / 69; 126 shapes 1 / 1.055 / 1.073 times as
+// fast.
 // Without a mask: KV tile after KV tile, and the items of a head run staggered by one query tile each.
 // Under a causal mask: from the diagonal downwards, and the items of a head are dispatched in that order.
 // The item on the diagonal comes first to its query tile, the one below it a tile later, and so on: no item
@@ -238,8 +240,8 @@ __global__ void __launch_bounds__(BwdTraits<D, kBf16, DR>::kThreads, 1)
   // (no static shared memory: the tiles need every byte, and 1024-byte alignment)
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t smem_base = smem_u32(smem_raw);
-  const uint32_t ds_smem = smem_base + T::kSlots * T::kTileBytes;   // dS^T, later dK / dV on their way out
-  const uint32_t stg_smem = ds_smem + T::kDsBytes;                  // dQ staging, 2 x 16 KB
+  const uint32_t ds_smem = smem_base + T::kSlots * T::kTileBytes;   // dS^T
+  const uint32_t stg_smem = ds_smem + T::kDsBytes;                  // staging of dQ, dK and dV, 2 x 16 KB
   const uint32_t stat_smem = stg_smem + T::kStageBytes;             // statistics, one block per query slot
   auto& sh = *reinterpret_cast<BwdControl<D, kBf16>*>(smem_raw + T::kSlots * T::kTileBytes + T::kDsBytes +
                                                       T::kStageBytes + T::kQSlots * T::kStatBytes);
@@ -453,11 +455,11 @@ __global__ void __launch_bounds__(BwdTraits<D, kBf16, DR>::kThreads, 1)
         used ^= 1u << slot;
       };
       uint32_t g = 0;  // query tiles so far, over all items
-      // The answer to a request takes a microsecond, so it is asked for ahead of the item's last loads: two tiles ahead at
-      // D = 128; where there are four slots for the query tiles the loads run ahead as it is, and asking later balances
-      // better (Z4 H16 N1024 D64 causal 51.2 two ahead, 49.9 us one).  Deterministic, the items of a head end one after
-      // the other, and the first to end has to be the first to ask: not ahead (two ahead / one / none, us: Z64 H16 N512 D128
-      // bf16 causal 592 / 529 / 517, Z1 H40 N640 without a mask 75.5 / 68.0 / 67.8; 126 shapes 0.982 / 0.997 / 1).
+      // The answer to a request takes a microsecond, so it is asked for ahead of the item's last loads.  How far makes
+      // little difference: two tiles ahead take 0.99 to 1.01 times as long as one, over 52 shapes at each D, and 1.02 at
+      // Z4 H16 N1024 causal, where asking later balances better.  Deterministic, the items of a head end one after the
+      // other, and the first to end has to be the first to ask: not ahead (two ahead / one / none, us: Z64 H16 N512 D128
+      // bf16 causal 592 / 529 / 517, Z1 H40 N640 without a mask 75.5 / 68.0 / 67.8; 126 shapes 1.018 / 1.003 / 1).
       constexpr int kAskAhead = kDet ? 0 : T::kQSlots > 2 ? 1 : 2;
       while (ok) {
         const BwdItem it = next_item();
@@ -534,8 +536,8 @@ __global__ void __launch_bounds__(BwdTraits<D, kBf16, DR>::kThreads, 1)
       bool ok = true;
 #pragma unroll 1
       for (uint32_t item_no = 0; ok; ++item_no) {
-        // S^T of the item's first query tile.  It comes behind dQ and dK of the item before: K and Q come late more often
-        // than not, and what is left of the item before would wait for them.
+        // S^T of the item's first query tile.  It comes behind dQ and dK of the item before: K and Q come late more
+        // often than not, and what is left of the item before would wait for them.
         const BwdItem cur = take_item();
         if (cur.id < 0) break;
         if (item_no > 0) next_slots();
@@ -607,7 +609,7 @@ __global__ void __launch_bounds__(BwdTraits<D, kBf16, DR>::kThreads, 1)
     const uint32_t lane_addr = uint32_t(quad * 32) << 16;
 
     if (warp < T::kComputeWarps) {
-      // =========================== compute groups: P^T, dS^T; dK, dV out ===================
+      // =========================== compute groups: P^T, dS^T ===========================
       reg_dealloc<T::kRegsCompute>();
       const int cg = warp >> 2;           // query columns [cg * kCols, (cg + 1) * kCols) are this group's
       const uint64_t c2 = pack2f(p.scale_log2, p.scale_log2);
@@ -616,8 +618,7 @@ __global__ void __launch_bounds__(BwdTraits<D, kBf16, DR>::kThreads, 1)
       // this group reads: no ordering between the groups is needed
       const uint32_t tP = tS;
       const uint32_t tDP = tmem_base + lane_addr + T::kColDP + cg * T::kCols;
-      // this thread's 128-byte row of dS^T; where the compute groups write dK and dV out, a warp's 32 rows (4 KB) are
-      // also its own staging area for them
+      // this thread's 128-byte row of dS^T
       const uint32_t row_addr = ds_smem + (cg * T::kCols / 64) * T::kBoxBytes + r * 128;
       const int chunk0 = (cg * T::kCols % 64) / 8;  // this group's first 16-byte chunk of it
       const bool tl = (threadIdx.x == 0);
@@ -631,7 +632,7 @@ __global__ void __launch_bounds__(BwdTraits<D, kBf16, DR>::kThreads, 1)
           const int qbase = (it.i_begin + n) * T::kBlock;
           const uint32_t sb = stat_smem + g % T::kQSlots * T::kStatBytes;  // -lse2 at 0, -delta at 512
 
-          // first visible query column of this thread's half (>= 64: none)
+          // first visible query column of this thread's kCols (>= kCols: none)
           int first_visible = 0;
           if (kvi >= it.sk) {
             first_visible = T::kBlock;
@@ -735,7 +736,7 @@ __global__ void __launch_bounds__(BwdTraits<D, kBf16, DR>::kThreads, 1)
         }
       }
     } else {
-      // =========================== dQ group ===========================
+      // =========================== dQ group: dQ; dV, dK ===========================
       reg_alloc<T::kRegsDq>();
       const uint32_t tDQ = tmem_base + lane_addr + T::kColDQ;
       const bool tl = (r == 0);

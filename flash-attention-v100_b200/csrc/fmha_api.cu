@@ -169,11 +169,11 @@ int round_up_128(int x) { return (x + 127) / 128 * 128; }
 // time: their grids are long, and many heads' query tiles would not share the L2.
 // FMHA_BWD_HEAD_GROUP overrides (tuning experiments).
 // Deterministic, without a mask: the items of a head run staggered by a query tile, and the more heads have their
-// first KV tiles in work, the less of that is waiting: as many as fit the L2, up to 32, in even groups.  Whole backward,
-// us, one head / 8 / 16 / 32 / this rule: D128 Z2 H16 N2048 433 / 346 / 326 / 311 / 311, Z3 H11 N2048 444 / 398 / 382 /
+// first KV tiles in work, the less of that is waiting: as many as fit the L2, up to 32, in even groups.  Whole
+// backward, us, one head / 8 / 16 / 32 / this rule: D128 Z2 H16 N2048 433 / 346 / 326 / 311 / 311, Z3 H11 N2048 444 / 398 / 382 /
 // 368 / 331 (two groups of 17 and 16), Z1 H8 N8192 1456 / 1117 / 1117 / 1117 / 1117, Z2 H9 N8192 2912 / 2402 / 2357 /
-// 2184 / 2246, Z1 H5 N16384 2953 / 2715 / 2715 / 2715 / 2815; D64 Z16 H16 N512 187 / 178 / 168 / 157 / 157, Z2 H16 N4096 1027
-// / 753 / 715 / 699 / 698.  Over 60 shapes (D = 64, 96, 128, N = 512 to 16384, 5 to 256 heads) 0.89 to 1.04 of the
+// 2184 / 2246, Z1 H5 N16384 2953 / 2715 / 2715 / 2715 / 2815; D64 Z16 H16 N512 187 / 178 / 168 / 157 / 157, Z2 H16
+// N4096 1027 / 753 / 715 / 699 / 698.  Over 60 shapes (D = 64, 96, 128, N = 512 to 16384, 5 to 256 heads) 0.89 to 1.04 of the
 // best of the four.  (The waiting is worth more here than the L2, so the limit is higher than the forward's 48 MB.)
 int bwd_head_group(int num_kv_blocks, bool causal, bool deterministic, int num_heads, double bytes_per_head) {
   static const int forced = []() {
@@ -289,22 +289,24 @@ FwdPlan plan_fwd(const FmhaFwdParams* p, int sms) {
   }
   if (can_pair) {
     // Few queries: an item with one query tile is a chain of MMA, softmax and MMA, and half of the SM idles.  Items of
-    // two chunks, which idle less but leave partial rows, or the plan so far?  Estimates of each, in us: a fixed part and
-    // one per chunk (the join); the rounds of the longest item, wave after wave, and K and V from HBM, of which the longer
-    // one counts and the shorter one a little; the partial rows, more beyond 40 MB, which the L2 does not keep.  A
-    // round of one tile takes 1.5 to 1.7 us, of two chunks 1.8 to 2.1; rows that a tile does not have cost 0.1 to 0.2,
-    // for they are masked.  Pairs have to be estimated 8 % faster than whole items, 4 % faster than the ordinary cut.
-    // Constants from 2918 shapes (D = 64, 96, 128, 1 to 128 rows, 1921 to 32768 keys, 8 to 1200 heads, bf16), every way
-    // timed, searched on one half of them and as good on the other: 0.5 % slower than the best way on average, by more
-    // than 3 % in 110 of them, 17 % at most (without pairs 22 % slower on average).  148 heads of 128 rows over 4096 keys,
-    // D = 128: whole 59 us, one pair 73; 64 rows over 8192, 64 heads: whole 113, two pairs 54.
+    // two chunks, which idle less but leave partial rows, or the plan so far?  Estimates of each, in us: a fixed part
+    // and one per chunk (the join); the rounds of the longest item, wave after wave, and K and V from HBM, of which the
+    // longer one counts and the shorter one a little; the partial rows, more beyond 40 MB, which the L2 does not keep.
+    // A round of one tile takes 1.5 to 1.7 us, of two chunks 1.8 to 2.1; rows that a tile does not have cost 0.1 to
+    // 0.2, for they are masked.  Pairs have to be estimated 8 % faster than whole items, 4 % faster than the ordinary
+    // cut.  Constants from 2918 shapes (D = 64, 96, 128, 1 to 128 rows, 1921 to 32768 keys, 8 to 1200 heads, bf16),
+    // every way timed, searched on one half of them and as good on the other: 0.5 % slower than the best way on average,
+    // by more than 3 % in 110 of them, 17 % at most (without pairs 22 % slower on average).  148 heads of 128 rows over
+    // 4096 keys, D = 128: whole 59 us, one pair 73; 64 rows over 8192, 64 heads: whole 113, two pairs 54.
     // Padded batches: the lengths are not known here.  Taken as 0.56 of the whole on average, and waves and margins as
-    // they were best for 1639 shapes with 8 entries of n/8 to n keys: 1.2 % slower than the best way on average, 22 % at
-    // most (without pairs 27 % on average).
+    // they were best for 1639 shapes with 8 entries of n/8 to n keys: 1.2 % slower than the best way on average, 22 %
+    // at most (without pairs 27 % on average).
     const double wide = p->head_dim / 64.0;
     const bool full = p->seqlen_q == 128, padded = p->seqused_k != nullptr;
-    const double one_tile = 1.37 + 0.19 * wide - (full ? 0.2 : 0.0), two_chunks = 1.52 + 0.32 * wide - (full ? 0.1 : 0.0);
-    auto waves = [&](int items, double filled) {  // items per head; of a padded batch, the part of their rounds that exists
+    const double one_tile = 1.37 + 0.19 * wide - (full ? 0.2 : 0.0);
+    const double two_chunks = 1.52 + 0.32 * wide - (full ? 0.1 : 0.0);
+    // items per head; of a padded batch, the part of their rounds that exists
+    auto waves = [&](int items, double filled) {
       const double per_sm = heads * items / sms;
       if (!padded || per_sm <= 1) return std::ceil(per_sm);
       return std::max(1.0, per_sm * filled + 0.25 * std::ceil(per_sm * filled));
@@ -314,10 +316,12 @@ FwdPlan plan_fwd(const FmhaFwdParams* p, int sms) {
       const double kv_us = part * heads * n_max * 128 * p->head_dim * 4 / 7.1e6;
       const double parts_mb = part * heads * chunks * p->seqlen_q * p->head_dim * 8 / 1e6;
       const double x = rounds_us * rounds_us, y = kv_us * kv_us;
-      return 6.0 + 0.27 * chunks + std::sqrt(std::sqrt(x * x + y * y)) + 0.34 * parts_mb + 0.1 * std::max(0.0, parts_mb - 40);
+      return 6.0 + 0.27 * chunks + std::sqrt(std::sqrt(x * x + y * y)) + 0.34 * parts_mb +
+             0.1 * std::max(0.0, parts_mb - 40);
     };
     const int chunks = plan.max_chunks;
-    double most = chunks > 1 ? (padded ? 0.93 : 0.96) * time(waves(chunks, 0.58) * (one_tile * plan.chunk_tiles + 2.5), chunks)
+    double most = chunks > 1 ? (padded ? 0.93 : 0.96) *
+                                   time(waves(chunks, 0.58) * (one_tile * plan.chunk_tiles + 2.5), chunks)
                              : (padded ? 0.88 : 0.92) * (time(waves(1, 0.67) * (one_tile * n_max - 0.5), 0) - 0.5);
     for (int k = 1; k <= 32; ++k) {
       const int chunk = (n_max + 2 * k - 1) / (2 * k), n = (n_max + 2 * chunk - 1) / (2 * chunk);
@@ -415,9 +419,11 @@ int launch_fwd(const FmhaFwdParams* p, void* workspace, size_t workspace_bytes, 
   if (!launched) return FMHA_ERR_LAUNCH;
   if (plan.max_chunks > 1) {
     const long long rows = (long long)kp.num_heads_total * (p->seqlen_q - plan.first_cut_row);
-    // Set up while the chunks are still in work; it waits for them itself (59.6 -> 56.7 us at 64 queries x 8192 keys, 64
-    // heads, D = 128).  Not so the kernels of a backward: Z4 H16 N1024 D64 causal 49.3 -> 47.1 us on the GPU, but this
-    // launch takes the host half a microsecond longer, and small training steps wait for the host (76.3 -> 77.7).
+    // Launched as soon as no block of the chunks is left to start or run, and not only when their writes are visible:
+    // it waits for those itself.  64 queries x 8192 keys, 64 heads, D = 128, bf16, call after call 57.7 -> 55.6 us; 216
+    // shapes 1.06 times as fast, in a captured graph no difference.  Not so the kernels of a backward: Z4 H16 N1024 D64
+    // causal 49.3 -> 47.1 us on the GPU, but this launch takes the host half a microsecond longer, and small training
+    // steps wait for the host (76.3 -> 77.7).
     cudaLaunchAttribute early;
     early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     early.val.programmaticStreamSerializationAllowed = 1;

@@ -106,10 +106,11 @@ struct FwdTraits {
   static constexpr int kBoxBytes = 128 * 128;  // 128 rows x 128 bytes
   static constexpr int kTileBytes = kBoxes * kBoxBytes;
   // A paired item (see the kernel) has one query tile in shared memory and no output to stage: room for six K
-  // or V tiles at D = 128, three per chunk.  64 queries x 8192 keys, 64 heads, bf16, two per chunk / three: 65.1 / 61.1 us
-  // (K and V alone take 41 at the rate of a copy).
+  // or V tiles at D = 128, three per chunk.  64 queries x 8192 keys, 64 heads, bf16, two per chunk / three: 65.1 / 61.1
+  // us (K and V alone take 41 at the rate of a copy).
   static constexpr int kQTiles = kPair ? 1 : kTilesM;
-  static constexpr int kStages = (D == 128 ? 4 : 8) + (kPair ? (D == 128 ? 2 : 4) : 0);  // ring slots of one K or V tile
+  // ring slots of one K or V tile
+  static constexpr int kStages = (D == 128 ? 4 : 8) + (kPair ? (D == 128 ? 2 : 4) : 0);
   static constexpr int kItemStages = 4;  // item ids published ahead
   static constexpr int kThreads = 384;   // softmax 0, softmax 1, {K/V, MMA, Q, idle} warps
   // Q tiles, K/V ring, one 64-column output box per softmax group
@@ -792,8 +793,8 @@ __global__ void __launch_bounds__(384, 1)
         }
         if (split) {
           if (nd == 0) continue;  // LSE = -inf: the combine kernel reads no row
-          // (p.row_elems is DR.  Where it is left out here for good, the other code of the kernel comes out slower: without a
-          // mask, Z1 H8 N8192 D64 210.9 -> 213.2 us, D96 230.1 -> 233.2, D128 0.2 %; not so for pairs.)
+          // (p.row_elems is DR.  Where it is left out here for good, the other code of the kernel comes out slower:
+          // without a mask, Z1 H8 N8192 D64 210.9 -> 213.2 us, D96 230.1 -> 233.2, D128 0.2 %; not so for pairs.)
           const int row_elems = DR == D && !kPair ? p.row_elems : DR;
           float* dst = p.o_part + (((size_t)chunk * p.num_heads_total + done.zh) * p.seqlen_q + row) * row_elems;
 #pragma unroll 1

@@ -101,11 +101,12 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   return true;
 }
 
-// Bounded wait for a field of a word in global memory, (word >> shift) & mask, to reach `want` (modulo the field); another CTA of the same
-// grid adds to it (global_flag_release), for an item that was handed out before this one's.  Gives up at once when this CTA, or the grid (status word), is already aborting.
+// Bounded wait for a field of a word in global memory, (word >> shift) & mask, to reach `want` (modulo the field);
+// another CTA of the same grid adds to it (global_flag_release), for an item that was handed out before this one's.
+// Gives up at once when this CTA, or the grid (status word), is already aborting.
 constexpr uint32_t kFlagPollLimit = 1u << 21;
-__device__ __forceinline__ bool global_flag_wait(const unsigned* flag, uint32_t shift, uint32_t mask, uint32_t want, volatile int* abort_word,
-                                                 const int* status, int who) {
+__device__ __forceinline__ bool global_flag_wait(const unsigned* flag, uint32_t shift, uint32_t mask, uint32_t want,
+                                                 volatile int* abort_word, const int* status, int who) {
   for (uint32_t i = 0; i < kFlagPollLimit; ++i) {
     uint32_t v;
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(flag) : "memory");

@@ -1,6 +1,6 @@
-"""GPU tests of a kernel that is set up while the one before it is still in work (the join of a cut forward): in a
-captured graph, and call after call on two streams, it sees what the kernel before it wrote, and the backward what it
-wrote."""
+"""GPU tests of a kernel that is launched before the writes of the one before it are visible, and waits for them itself
+(the join of a cut forward): in a captured graph, and call after call on two streams, it sees what the kernel before it
+wrote, and the backward what it wrote."""
 import pytest
 import torch
 
