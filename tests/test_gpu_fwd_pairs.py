@@ -132,7 +132,7 @@ def test_pairs_one_after_the_other(n_q, n_k, causal, shift, D, dtype):
 @pytest.mark.parametrize("D", [64, 96, 128])
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 def test_pairs_one_after_the_other_in_a_padded_batch(D, dtype):
-    # 25 tiles in chunks of 13 and 12; entries with one tile in the second chunk, with none, with none at all
+    # 25 tiles; in chunks of 13 and 12, which the next test has, too, entries with one tile in the second chunk and with none
     n_q, n_k, sq, sk = 16, 3200, [16, 1, 16, 0, 9], [3200, 1665, 1664, 77, 0]
     q, k, v = _many(n_q, n_k, D, dtype, seed=68)
     scale = oracle.default_scale(D)
@@ -146,14 +146,23 @@ def test_pairs_one_after_the_other_in_a_padded_batch(D, dtype):
     assert not out[~seen.transpose(1, 2)].any()
 
 
+@pytest.mark.parametrize("heads,chunks,sk", [
+    (266, 4, [2689, 1793, 897, 1, 0]),  # 25 tiles in chunks of 7, 7, 7, 4: one tile in the fourth, third, second, first
+    (66, 2, [3200, 1665, 1664, 77, 0]),  # in chunks of 13 and 12: a full second chunk, one tile in it, none
+])
 @pytest.mark.parametrize("D", [64, 96, 128])
-def test_pairs_twice_per_head_in_a_padded_batch(D):
-    # 25 tiles in chunks of 7, 7, 7 and 4; entries that end with one tile in the fourth, third, second and first, and with none
-    n_q, n_k, sq, sk = 16, 3200, [16, 1, 16, 7, 9], [2689, 1793, 897, 1, 0]
-    q, k, v = _many(n_q, n_k, D, torch.bfloat16, seed=70)
+def test_pairs_once_and_twice_per_head_in_a_padded_batch(D, heads, chunks, sk):
+    import ctypes
+
+    from flash_attn_v100 import cabi
+
+    n_q, n_k, sq = 16, 3200, [16, 1, 16, 7, 9]
+    q, k, v = (t[:, :, :heads].contiguous() for t in _many(n_q, n_k, D, torch.bfloat16, seed=70))
+    lens = {n: torch.tensor(x, dtype=torch.int32, device="cuda") for n, x in (("seqused_q", sq), ("seqused_k", sk))}
+    p = cabi.fwd_params(q, k, v, q, torch.empty(1, device="cuda"), 1.0, False, **lens)
+    assert cabi.load_library().fmha_fwd_workspace_bytes(ctypes.byref(p)) == chunks * Z * heads * n_q * (D + 1) * 4
     scale = oracle.default_scale(D)
-    lens = {"seqused_q": sq, "seqused_k": sk}
-    out, lse = _run_pairs(q, k, v, scale, **{n: torch.tensor(x, dtype=torch.int32, device="cuda") for n, x in lens.items()})
+    out, lse = _run_pairs(q, k, v, scale, **lens)
     r_out, r_lse = _reference(q, k, v, scale, sq=sq, sk=sk)
     assert oracle.max_abs(out.float(), r_out) <= _tol(torch.bfloat16)
     seen = torch.isfinite(r_lse)
